@@ -7,6 +7,8 @@
 #include <vector>
 
 #include "../../include/hpt.h"
+#include "bvh.cuh"
+#include "bvh_build.h"
 #include "engine.h"
 #include "scene_pack.h"
 #include "shading.cuh"
@@ -68,17 +70,20 @@ __global__ void k_stage_intersect(const DevScene* s, int n, const float* o, cons
                                   int32_t* tri, float* t, float* u, float* v, DevErr* err) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  TravState st;
-  TravCold tc;
-  trav_init(*s, Ray{mk(o[3 * i], o[3 * i + 1], o[3 * i + 2]), mk(d[3 * i], d[3 * i + 1], d[3 * i + 2])},
-            st, tc);
+  const Ray r{mk(o[3 * i], o[3 * i + 1], o[3 * i + 2]), mk(d[3 * i], d[3 * i + 1], d[3 * i + 2])};
   TravCount cnt{};
-  while (!trav_leaf<true>(*s, st, tc, nullptr, 0, err, cnt)) {
+  int32_t hit;
+  float ht, hu = 0.f, hv = 0.f;
+  bvh_query(*s, r, hit, ht, err, cnt);
+  if (hit >= 0) {  // the winning test's u, v
+    const float4* rec = reinterpret_cast<const float4*>(s->tris + hit);
+    float t2;
+    mt_test(r, ldg(rec), ldg(rec + 1), ldg(rec + 2), t2, hu, hv);
   }
-  tri[i] = st.best.tri;
-  t[i] = st.best.rec >= 0 ? st.best.t : 0.f;
-  u[i] = st.best.rec >= 0 ? st.best.u : 0.f;
-  v[i] = st.best.rec >= 0 ? st.best.v : 0.f;
+  tri[i] = hit;
+  t[i] = ht;
+  u[i] = hu;
+  v[i] = hv;
 }
 
 __global__ void k_stage_shade(const DevScene* s, int n, const float* o, const float* d,
@@ -391,6 +396,21 @@ hpt_status upload_scene(const hpt_scene_desc& d, SceneDev& out) {
   if (pk.refs.empty()) pk.refs.push_back(0);
   if ((s = dev_upload(out, pk.refs.data(), pk.refs.size(), &refs)) != HPT_OK) return s;
   if ((s = dev_upload(out, pk.tris.data(), pk.tris.size(), &recs)) != HPT_OK) return s;
+  PackedBvh bvh;
+  float scale = 0.f;
+  for (int a = 0; a < 3; ++a) {
+    ds.root_lo[a] = pk.root_lo[a];
+    ds.root_hi[a] = pk.root_hi[a];
+    scale = std::max({scale, std::fabs(pk.root_lo[a]), std::fabs(pk.root_hi[a]),
+                      pk.root_hi[a] - pk.root_lo[a]});
+  }
+  ds.scene_eps = 2e-5f * scale;
+  build_bvh(pk, ds.scene_eps, 0, bvh);
+  if ((s = dev_upload(out, bvh.nodes.data(), bvh.nodes.size(), &ds.bvh)) != HPT_OK) return s;
+  if (bvh.tris.empty()) bvh.tris.emplace_back();
+  if ((s = dev_upload(out, bvh.tris.data(), bvh.tris.size(), &ds.btris)) != HPT_OK) return s;
+  ds.num_bvh = (int32_t)bvh.nodes.size();
+  ds.num_btris = (int32_t)bvh.tris.size();
   ds.nodes = nodes;
   ds.leaves = leaves;
   ds.leaf_refs = refs;
@@ -435,14 +455,6 @@ hpt_status upload_scene(const hpt_scene_desc& d, SceneDev& out) {
   ds.num_materials = d.num_materials;
   ds.num_lights = d.num_lights;
   ds.num_textures = d.num_textures;
-  float scale = 0.f;
-  for (int a = 0; a < 3; ++a) {
-    ds.root_lo[a] = pk.root_lo[a];
-    ds.root_hi[a] = pk.root_hi[a];
-    scale = std::max({scale, std::fabs(pk.root_lo[a]), std::fabs(pk.root_hi[a]),
-                      pk.root_hi[a] - pk.root_lo[a]});
-  }
-  ds.scene_eps = 2e-5f * scale;
   const int64_t cap = 8 * ((int64_t)pk.nodes.size() + (int64_t)pk.refs.size()) + 100000;
   ds.max_steps = (int32_t)std::min<int64_t>(cap, 1 << 30);
   void* p = nullptr;
@@ -475,8 +487,8 @@ void release_scene(SceneDev& s) {
 
 namespace {
 
-// Ranges the engine supports (capacity: queue entries; smem_nodes: shared
-// node prefix; trav_steps: 0 = leaf per round, 1..256 step units per round;
+// Ranges the engine supports (capacity: queue entries; smem_nodes: accepted,
+// without effect; trav_steps: 0 = the default, 1..256 rounds between refills;
 // isect_block / isect_min_blocks: a compiled traversal variant,
 // 0 min blocks = the block size's default).
 hpt_status check_tuning(const hpt_tuning& t) {

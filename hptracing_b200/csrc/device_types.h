@@ -56,6 +56,43 @@ struct DevTri {
 };
 static_assert(sizeof(DevTri) == 48, "48-byte triangle record");
 
+// --- Bounding volume hierarchy ---------------------------------------------
+// 8-wide node with child boxes quantised to 8 bits per plane (the published
+// compressed wide layout of Ylitie, Karras and Laine, "Efficient Incoherent
+// Ray Traversal on GPUs Through Compressed Wide BVHs", 2017), 80 bytes
+// (5 x 16 B). A child's plane q on axis a lies at p[a] + q * 2^e[a].
+//  slot i is an inner child when bit i of imask is set: its node is
+//  child_base + popcount(imask & ((1 << i) - 1)). Otherwise meta[i] is 0 (no
+//  child) or a leaf: bits 0-4 = first triangle relative to tri_base, bits
+//  5-7 = one bit per triangle (1 to 3 triangles).
+struct BvhNode {
+  float p[3];
+  uint8_t e[3];             // biased exponents (float bits e << 23)
+  uint8_t imask;
+  uint32_t child_base;
+  uint32_t tri_base;
+  uint8_t meta[8];
+  uint8_t qlo[3][8];        // x, y, z lower planes of the 8 slots
+  uint8_t qhi[3][8];        // upper planes
+};
+static_assert(sizeof(BvhNode) == 80, "80-byte wide node");
+
+// Triangle record in node order: the DevTri values and the lowest tree node
+// that holds every leaf listing the triangle (bvh_certain in bvh.cuh).
+struct BvhTri {
+  float a[3];
+  int32_t tri_id;
+  float e1[3];
+  int32_t start_node;
+  float e2[3];
+  int32_t pad;
+};
+static_assert(sizeof(BvhTri) == 48, "48-byte triangle record");
+
+// Entries of a ray's node stack; the builder bounds the depth below it (one
+// entry at most per level).
+constexpr int kBvhStack = 32;
+
 // Per-texture descriptor: texel offset into the RGBA8 pool, width, height.
 struct DevTexInfo {
   int64_t offset;
@@ -82,23 +119,10 @@ struct DevScene {
   float root_lo[3], root_hi[3];
   float scene_eps;          // termination slack in world units
   int32_t max_steps;        // traversal step cap per ray
+  const BvhNode* bvh;       // wide nodes, root first
+  const BvhTri* btris;      // triangle records in node order
+  int32_t num_bvh, num_btris;
 };
-
-// The fields of a DevScene the traversal reads (80 bytes): a launch whose
-// jobs render several scenes keeps one per job slot in shared memory, so a
-// traversal step reads its scene's pointers and sizes from there instead
-// of from the job table in global memory.
-struct TravScene {
-  const DevNode* nodes;
-  const DevLeaf* leaves;
-  const int32_t* leaf_refs;
-  const DevTri* tris;
-  int32_t num_nodes, num_leaves, num_leaf_tris, num_triangles;
-  float root_lo[3], root_hi[3];
-  float scene_eps;
-  int32_t max_steps;
-};
-static_assert(sizeof(TravScene) == 80, "80-byte traversal scene");
 
 // --- Wavefront job table ------------------------------------------------
 // One render job (a frame of one scene) in a slot of the engine's table.

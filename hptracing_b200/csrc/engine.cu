@@ -36,6 +36,7 @@
 #include <numeric>
 #include <type_traits>
 
+#include "bvh.cuh"
 #include "engine.h"
 #include "shading.cuh"
 #include "traverse.cuh"
@@ -68,26 +69,19 @@ struct EngineParams {
   float4* A_s[2];
   float4* A_r[2];
   int32_t* A_tri[2];
-  int32_t* A_leaf[2];   // leaf node of the hit (start hint for the next ray)
   float4* R_o;
   float4* R_d;
   float4* R_s;
   float4* R_r;
   int capacity;
-  int smem_nodes;       // > 0 only when every job uses shared_nodes' scene
-  int refill;
-  int trav_steps;       // > 0: step-at-a-time traversal, units per round
-  const DevNode* shared_nodes;
+  int refill;           // idle lanes that make a warp refill
+  int rounds;           // warp rounds between refills
   // When every job of the launch renders the same scene (a frame, or a
   // batch over one scene): a copy of its DevScene in the kernel's parameter
-  // space. The step loop then reads the scene's pointers and sizes as
-  // constant operands instead of loading them from the job table on every
-  // traversal unit (one dependent load less per unit).
+  // space, whose pointers the walk then reads as constant operands. With
+  // several scenes each lane keeps its own in registers.
   int uniform_scene;
   DevScene uscene;
-  // Several scenes, and their per-slot TravScene table fits the dynamic
-  // shared memory: the traversal reads its scene from there.
-  int scene_table;
 };
 
 __device__ __forceinline__ unsigned lanemask_lt() {
@@ -147,55 +141,16 @@ __device__ __forceinline__ void count_queries(DevSlot* slots, bool alive, int sl
     atomicAdd(&slots[slot].queries, (unsigned long long)__popc(same & m));
 }
 
-// A lane's work counters in shared memory (five words: an odd stride, so
-// the lanes of a warp hit distinct banks); they are touched once per
-// traversal unit and would otherwise hold four registers.
-struct CountSlot {
-  TravCount c;
-  uint32_t queries;  // the lane's queries in this launch
-};
-
-// Warp-level reduction of the per-lane query and work counters.
-__device__ __forceinline__ void flush_counts(DevCtrl* c, unsigned long long q, TravCount lane) {
-  unsigned long long nodes = lane.nodes, leaves = lane.leaves, tris = lane.tris,
-                     repeats = lane.repeats;
-  for (int o = 16; o > 0; o >>= 1) {
-    q += __shfl_down_sync(kFull, q, o);
-    nodes += __shfl_down_sync(kFull, nodes, o);
-    leaves += __shfl_down_sync(kFull, leaves, o);
-    tris += __shfl_down_sync(kFull, tris, o);
-    repeats += __shfl_down_sync(kFull, repeats, o);
-  }
-  if ((threadIdx.x & 31) == 0 && q) {
+// Adds a warp's query and work counts to the control block (lane 0 calls).
+__device__ __forceinline__ void add_counts(DevCtrl* c, uint32_t queries, uint32_t nodes,
+                                           uint32_t leaves, uint32_t tests) {
 #ifdef HPT_DEVICE_CHECKS
-    atomicAdd(&c->chk_isect_done, (int)q);
+  if (queries) atomicAdd(&c->chk_isect_done, (int)queries);
 #endif
-    atomicAdd(&c->isect_queries, q);
-    atomicAdd(&c->nodes_visited, nodes);
-    atomicAdd(&c->leaves_visited, leaves);
-    atomicAdd(&c->tri_tests, tris);
-    atomicAdd(&c->tri_repeats, repeats);
-  }
-}
-
-__device__ __forceinline__ int stage_nodes(const EngineParams& P, uint2* snodes) {
-  if (P.smem_nodes <= 0) return 0;
-  const uint2* src = reinterpret_cast<const uint2*>(P.shared_nodes);
-  for (int i = threadIdx.x; i < P.smem_nodes; i += blockDim.x) snodes[i] = __ldg(src + i);
-  __syncthreads();
-  return P.smem_nodes;
-}
-
-// A launch over several scenes copies each job slot's TravScene into the
-// dynamic shared memory (the node prefix is only used by one-scene
-// launches, so the table starts at offset 0): the traversal steps then read
-// their scene's pointers and sizes from shared memory.
-__device__ __forceinline__ const TravScene* stage_scenes(const EngineParams& P, uint2* smem) {
-  if (!P.scene_table) return nullptr;
-  TravScene* tab = reinterpret_cast<TravScene*>(smem);
-  for (int i = threadIdx.x; i < P.num_slots; i += blockDim.x) tab[i] = trav_scene(P.jobs[i].scene);
-  __syncthreads();
-  return tab;
+  if (queries) atomicAdd(&c->isect_queries, (unsigned long long)queries);
+  if (nodes) atomicAdd(&c->nodes_visited, (unsigned long long)nodes);
+  if (leaves) atomicAdd(&c->leaves_visited, (unsigned long long)leaves);
+  if (tests) atomicAdd(&c->tri_tests, (unsigned long long)tests);
 }
 
 // Grants the free wavefront capacity to active slots in priority order
@@ -247,237 +202,10 @@ __device__ void schedule(const EngineParams& P) {
 }
 
 // ---------------------------------------------------------------------------
-// Primary pass: raygen + closest hit, lanes refilled from a global counter.
-// Traversal modes of k_primary / k_isect.
-constexpr int kTravLeaf = 0;      // trav_leaf, one leaf per lane per round
-constexpr int kTravStep = 1;      // trav_step, nodes from global memory
-constexpr int kTravStepSmem = 2;  // trav_step with the shared-memory node prefix
+// Closest hits: queue rays and camera rays, persistent warps with lane refill.
+// ---------------------------------------------------------------------------
 
-// Phase vote (default; -DHPT_PHASE_VOTE=0 builds the per-lane loop for
-// comparison): in each warp round of the step-at-a-time walk only the lanes
-// of the more common phase (descent / leaf set-up, or triangle test) run a
-// unit, so that a round executes one phase's code instead of both. Measured
-// on the spheres frame 107.9 -> 105.7 ms and on the terrain frame 85.1 ->
-// 79.0 ms per frame (4 spp), images unchanged (each lane still runs its own
-// units in order).
-#ifndef HPT_PHASE_VOTE
-#define HPT_PHASE_VOTE 1
-#endif
-// The tests' phase runs when it holds at least this many sixths of the
-// warp's live lanes: with one test per testing lane a round (3, the
-// majority), and with cooperative tests (1; a cooperative round tests up to
-// 32 references whatever the number of testing lanes).
-#ifndef HPT_VOTE_TEST_SIXTHS
-#define HPT_VOTE_TEST_SIXTHS 3
-#endif
-#ifndef HPT_COOP_TEST_SIXTHS
-#define HPT_COOP_TEST_SIXTHS 1
-#endif
-
-// k_primary tests one reference per testing lane a round unless built with
-// -DHPT_COOP_PRIMARY=1: camera rays are coherent, neighbouring lanes test
-// the same triangles and share their loads, and the terrain frame's
-// primary pass measured 9.6 ms with per-lane tests against 11.3 ms with
-// cooperative ones (the spheres frame's 1.16 against 0.87 ms).
-#ifndef HPT_COOP_PRIMARY
-#define HPT_COOP_PRIMARY 0
-#endif
-constexpr bool kCoopPrimary = HPT_COOP_PRIMARY != 0;
-
-// Scene accessors of the traversal loops: scene_of(slot) is the scene of a
-// job slot's rays - the launch's one scene (kernel parameters), the
-// per-block table of a several-scene launch, or the job table.
-struct OneScene {
-  const DevScene& s;
-  __device__ __forceinline__ const DevScene& operator()(int) const { return s; }
-};
-struct TableScene {
-  const TravScene* tab;
-  __device__ __forceinline__ const TravScene& operator()(int slot) const { return tab[slot]; }
-};
-struct JobScene {
-  const DevJob* jobs;
-  __device__ __forceinline__ const DevScene& operator()(int slot) const {
-    return jobs[slot].scene;
-  }
-};
-
-// Warp-cooperative triangle tests (default with the phase vote;
-// -DHPT_COOP_TESTS=0 builds the one-test-per-lane rounds): in a test round
-// the untested references of every testing lane's current leaf are dealt
-// out over the warp's 32 lanes, one test per lane, and a segmented minimum
-// over (t, rank) hands each ray the best of its candidates. The reference's
-// rule - the smallest t wins, the lower rank on an exact tie - is a
-// lexicographic minimum, so the order in which the tests run does not
-// change any result.
-#ifndef HPT_COOP_TESTS
-#define HPT_COOP_TESTS 1
-#endif
-
-#if HPT_PHASE_VOTE
-#if HPT_COOP_TESTS
-// One cooperative test round; every lane of the warp calls it. `testing`:
-// this lane's ray is in the test phase; `slot`: its job slot, whose scene
-// scene_of(slot) gives (a lane may test for a ray of another job, so it
-// reads that ray's scene). Returns true when this lane's ray finished (its
-// leaf's last reference was tested and the exit ended it).
-template <class SceneOf, class Cnt>
-__device__ __forceinline__ bool coop_tests(const SceneOf& scene_of, int slot, bool testing,
-                                           TravState& st, TravCold& tc, DevErr* err, Cnt& cnt) {
-  const int lane = threadIdx.x & 31;
-  const int rem = testing ? st.end - st.k : 0;
-  // This lane's references take slots [excl, incl) of the round.
-  int incl = rem;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(kFull, incl, o);
-    if (lane >= o) incl += v;
-  }
-  const int excl = incl - rem;
-  const int total = __shfl_sync(kFull, incl, 31);
-  // Slot `lane` belongs to the first lane whose inclusive end exceeds it.
-  int owner = 0;
-#pragma unroll
-  for (int step = 16; step > 0; step >>= 1) {
-    const int v = __shfl_sync(kFull, incl, owner + step - 1);
-    if (v <= lane) owner += step;
-  }
-  const bool valid = lane < total;
-  const int o_k = __shfl_sync(kFull, st.k, owner);
-  const int o_excl = __shfl_sync(kFull, excl, owner);
-  const int o_mb = __shfl_sync(kFull, st.mb_id[0], owner);
-  const int o_slot = __shfl_sync(kFull, slot, owner);
-  Ray r;
-  r.o.x = __shfl_sync(kFull, st.ray.o.x, owner);
-  r.o.y = __shfl_sync(kFull, st.ray.o.y, owner);
-  r.o.z = __shfl_sync(kFull, st.ray.o.z, owner);
-  r.d.x = __shfl_sync(kFull, st.ray.d.x, owner);
-  r.d.y = __shfl_sync(kFull, st.ray.d.y, owner);
-  r.d.z = __shfl_sync(kFull, st.ray.d.z, owner);
-  int id = -1;
-  uint32_t key = ~0u;  // t's bits for a hit (t > 0: ordered like t), else the maximum
-  if (valid) {
-    const auto& so = scene_of(o_slot);
-    const int j = o_k + (lane - o_excl);
-    bool ok = true;
-    HPT_DCHECK(err, j >= 0 && j < so.num_leaf_tris, 107, j, ok = false);
-    if (ok) {
-      id = ldg(so.leaf_refs + j);
-      HPT_DCHECK(err, id >= 0 && id < so.num_triangles, 104, id, ok = false);
-    }
-    if (ok) {
-      const float4* rec = reinterpret_cast<const float4*>(so.tris) + 3 * (size_t)id;
-      float t, u, v;
-      if (mt_test(r, ldg(rec), ldg(rec + 1), ldg(rec + 2), t, u, v)) key = __float_as_uint(t);
-    }
-  }
-  // Work counters as the one-test-per-lane walk counts them: a reference
-  // equal to the one before it in its ray's sequence is a mailbox repeat.
-  const int up = __shfl_up_sync(kFull, id, 1);
-  if (valid) {
-    if (id == (lane == o_excl ? o_mb : up)) count_repeat(cnt);
-    else count_test(cnt);
-  }
-  // Segmented minimum of t: the first slot of each ray's range ends with
-  // its range's minimum. Bit s of `starts`: slot s begins a range.
-  const unsigned starts = __ballot_sync(kFull, valid && lane == o_excl);
-  const uint32_t mine = key;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t other = __shfl_down_sync(kFull, key, o);
-    const bool same =
-        lane + o < 32 &&
-        ((unsigned)((unsigned long long)starts >> (lane + 1)) & ((1u << o) - 1)) == 0;
-    if (same && other < key) key = other;
-  }
-  // Of the slots that hold their range's minimum the lowest one - the
-  // lowest rank - wins, as the reference's strict comparison in list order
-  // keeps the first of equal t.
-  const uint32_t seg_min = __shfl_sync(kFull, key, o_excl);
-  const unsigned wins = __ballot_sync(kFull, valid && mine != ~0u && mine == seg_min);
-  const int first = excl < 32 ? excl : 31;
-  const int last = incl < 32 ? incl - 1 : 31;
-  const unsigned my_wins = (unsigned)(((unsigned long long)wins >> first) << first);
-  const int w = my_wins ? __ffs(my_wins) - 1 : 0;
-  const int last_id = __shfl_sync(kFull, id, last < 0 ? 0 : last);
-  const int win_id = __shfl_sync(kFull, id, w);
-  const uint32_t best = __shfl_sync(kFull, key, first);
-  if (!testing) return false;
-  if (rem > 0 && excl < 32) {
-    const int k0 = st.k;
-    st.k += last + 1 - excl;
-    st.mb_id[0] = last_id;
-    // When the range holds a hit, w is its lowest slot at the range's
-    // minimum (the slots past the range belong to other rays).
-    if (best != ~0u && w <= last) {
-      const float t = __uint_as_float(best);
-      const int jb = k0 + (w - excl);
-      if (st.best.rec < 0 || t < st.best.t || (t == st.best.t && jb < st.best.rec)) {
-        const auto& s = scene_of(slot);
-        if (tc.pierced < 0) {
-          const float4* L = reinterpret_cast<const float4*>(s.leaves + tc.leaf);
-          tc.pierced = ref_box_test(st.ray, ldg(L), ldg(L + 1)) ? 1 : 0;
-        }
-        if (tc.pierced) {
-          st.best.rec = jb;
-          st.best.tri = win_id;
-          st.best.t = t;
-          tc.best_node = tc.leaf_node;
-        }
-      }
-    }
-  }
-  if (st.k < st.end) return false;
-  return trav_exit(scene_of(slot), st, tc, err);
-}
-#endif
-
-// Up to `units` warp rounds. Every lane of the warp calls it; `live` is
-// false for a lane without a ray; scene_of(slot) is the scene of this
-// lane's job. kCoop: test rounds are cooperative (coop_tests). Returns true
-// when this lane's ray finished.
-template <int kMode, bool kCoop, class SceneOf>
-__device__ __forceinline__ bool vote_units(const SceneOf& scene_of, int slot, bool live,
-                                           TravState& st, TravCold& tc, const uint2* snodes,
-                                           int n_smem, DevErr* err, TravCount& cnt, int units) {
-  bool finished = false;
-  // The cooperative loop's work counts stay in one register and are added
-  // to the shared-memory counters at most 128 rounds apart and on return
-  // (a shared-memory update per unit measured 1-2 % slower).
-  PackedCount ucnt{0};
-  for (int u = 0; u < units; ++u) {
-    const bool go = live && !finished;
-    const unsigned lm = __ballot_sync(kFull, go);
-    if (lm == 0) break;
-    const bool testing = go && st.phase == kStepTest;
-    const unsigned tm = __ballot_sync(kFull, testing);
-#if HPT_COOP_TESTS
-    if constexpr (kCoop) {
-      using SceneT = std::decay_t<decltype(scene_of(slot))>;
-      // Every round moves a lane on: a test round needs a testing lane
-      // (whatever the threshold), else the descending lanes run.
-      if (tm != 0 && 6 * __popc(tm) >= HPT_COOP_TEST_SIXTHS * __popc(lm)) {
-        if (coop_tests(scene_of, slot, testing, st, tc, err, ucnt)) finished = true;
-      } else if (go && !testing) {
-        finished = trav_step<false, kMode == kTravStepSmem, SceneT, false>(
-            scene_of(slot), st, tc, snodes, n_smem, err, ucnt);
-      }
-      if ((u & 127) == 127) count_flush(ucnt, cnt);
-      continue;
-    }
-#endif
-    const bool pick_test = 6 * __popc(tm) >= HPT_VOTE_TEST_SIXTHS * __popc(lm);
-    if (go && testing == pick_test)
-      finished = trav_step<false, kMode == kTravStepSmem>(scene_of(slot), st, tc, snodes, n_smem,
-                                                          err, cnt);
-  }
-  count_flush(ucnt, cnt);
-  return finished;
-}
-#endif
-
-// --- Camera rays of a launch's primary-pass entries (P.prim_*), shared by
-// k_primary and the k_isect launches that carry them.
+// --- Camera rays of a launch's primary-pass entries (P.prim_*).
 // Entry g: its slot and ray index within the job.
 __device__ __forceinline__ bool prim_locate(const EngineParams& P, int64_t g, int& slot,
                                             int64_t& ray) {
@@ -491,136 +219,342 @@ __device__ __forceinline__ bool prim_locate(const EngineParams& P, int64_t g, in
   return ok;
 }
 
-// Starts the walk of the job's camera ray (set_viewdirs / set_viewdirs_vr,
-// kernel.cl:559-613).
-__device__ __forceinline__ void prim_init(const DevJob& J, int64_t ray, TravState& st,
-                                          TravCold& tc) {
+// The job's camera ray (set_viewdirs / set_viewdirs_vr, kernel.cl:559-613).
+__device__ __forceinline__ Ray prim_ray(const DevJob& J, int64_t ray) {
   const int x = (int)(ray % J.nx), y = (int)(ray / J.nx);
   const f3 d = J.pano ? pano_dir(x, y, J.vr_x_shift, J.ny)
                       : pinhole_dir(J.top, J.right, J.width, J.height, x, y, J.nx, J.ny);
-  trav_init(J.scene, Ray{mk(J.view_p[0], J.view_p[1], J.view_p[2]), d}, st, tc);
+  return Ray{mk(J.view_p[0], J.view_p[1], J.view_p[2]), d};
 }
 
-// A finished camera ray: its hit goes to the job's primary-hit cache; a
-// miss adds the background (kernel.cl:193-206: the first pass assigns
-// background * strength * sample_n with strength (1,1,1)).
-__device__ __forceinline__ void prim_finish(const EngineParams& P, int slot, int64_t ray,
-                                            const TravState& st, const TravCold& tc) {
-  const DevJob& J = P.jobs[slot];
-  if (st.best.rec >= 0) {
-    int k = atomicAdd(J.prim_count, 1);
-    HPT_DCHECK(&P.ctrl->err, k < job_rays(J), 203, k, k = -1);
-    if (k >= 0) {
-      float4* dst = reinterpret_cast<float4*>(J.prim) + 2 * (size_t)k;
-      dst[0] = make_float4(st.ray.d.x, st.ray.d.y, st.ray.d.z, __int_as_float((int)ray));
-      dst[1] = make_float4(__int_as_float(st.best.tri), st.best.t, __int_as_float(tc.best_node),
-                           0.f);
+// Rays a warp has finished walking, waiting to be certified and written out
+// 32 at a time with every lane busy (a lane that finishes takes its next ray
+// at once). item: index in the intersect queue, or -1 - ray for a camera ray.
+struct HitList {
+  int32_t item[64], slot[64];
+  uint32_t best[64];
+  float t[64];
+};
+// Rays of a warp that need the tree walk.
+struct WalkList {
+  int32_t item[64], slot[64];
+};
+
+__device__ __forceinline__ Ray list_ray(const EngineParams& P, int item, int slot) {
+  if (item < 0) return prim_ray(P.jobs[slot], -1 - (int64_t)item);
+  const float4 o = P.R_o[item], d = P.R_d[item];
+  return Ray{mk(o.x, o.y, o.z), mk(d.x, d.y, d.z)};
+}
+
+// Writes out one finished ray per lane (`have`): a hit goes to the next shade
+// queue (or, for a camera ray, to its job's primary-hit cache), a miss adds
+// the background. Every lane of the warp calls it.
+__device__ __forceinline__ void write_hits(const EngineParams& P, bool have, int item, int slot,
+                                           const f3& dir, int tri, float t) {
+  DevCtrl* c = P.ctrl;
+  const int lane = threadIdx.x & 31;
+  const int out_par = c->parity ^ 1;
+  const bool queued = have && item >= 0, camera = have && item < 0;
+  const bool hit = queued && tri >= 0;
+  const unsigned hm = __ballot_sync(kFull, hit);
+  if (hm) {
+    const int leader = __ffs(hm) - 1;
+    int base = 0;
+    if (lane == leader) base = atomicAdd(&c->nA_next, __popc(hm));
+    base = __shfl_sync(kFull, base, leader);
+    if (hit) {
+      const int pos = base + __popc(hm & lanemask_lt());
+      bool ok = true;
+      HPT_DCHECK(&c->err, pos < P.capacity, 223, pos, ok = false);
+      if (ok) {
+        const float4 r4 = P.R_r[item];
+        P.A_o[out_par][pos] = P.R_o[item];
+        P.A_d[out_par][pos] = P.R_d[item];
+        P.A_s[out_par][pos] = P.R_s[item];
+        P.A_r[out_par][pos] = make_float4(r4.x, r4.y, r4.z, t);
+        P.A_tri[out_par][pos] = tri;
+      }
     }
-  } else {
+  }
+  const bool missed = queued && !hit;
+  if (missed) {
+    // kernel.cl:195-200: miss adds background * strength (sample_n = 1).
+    const DevJob& J = P.jobs[slot];
+    const float4 s4 = P.R_s[item], r4 = P.R_r[item];
+    const int64_t ray = __float_as_int(P.R_o[item].w);
+    bool ok = true;
+    HPT_DCHECK(&c->err, ray >= 0 && ray < job_rays(J), 224, ray, ok = false);
+    if (ok) {
+      f3 rad = mk(r4.x, r4.y, r4.z);
+      rad = add(rad, mul(mk(J.bg[0], J.bg[1], J.bg[2]), mk(s4.x, s4.y, s4.z)));
+      flush_radiance(J, ray, rad);
+    }
+  }
+  count_done(P.slots, missed, slot);
+  // Camera rays: a hit goes to the job's primary-hit cache; a miss adds the
+  // background (kernel.cl:193-206: the first pass assigns background *
+  // strength * sample_n with strength (1,1,1)).
+  const unsigned cm = __ballot_sync(kFull, camera && tri >= 0);
+  if (cm) {
+    const unsigned same = __match_any_sync(kFull, camera && tri >= 0 ? slot : -1) & cm;
+    int base = 0;
+    const int leader = __ffs(same) - 1;
+    if (camera && tri >= 0 && lane == leader)
+      base = atomicAdd(P.jobs[slot].prim_count, __popc(same));
+    base = __shfl_sync(kFull, base, leader < 0 ? 0 : leader);
+    if (camera && tri >= 0) {
+      const DevJob& J = P.jobs[slot];
+      int k = base + __popc(same & lanemask_lt());
+      HPT_DCHECK(&c->err, k < job_rays(J), 203, k, k = -1);
+      if (k >= 0) {
+        float4* dst = reinterpret_cast<float4*>(J.prim) + 2 * (size_t)k;
+        dst[0] = make_float4(dir.x, dir.y, dir.z, __int_as_float(-1 - item));
+        dst[1] = make_float4(__int_as_float(tri), t, 0.f, 0.f);
+      }
+    }
+  }
+  if (camera && tri < 0) {
+    const DevJob& J = P.jobs[slot];
     const f3 val = scale((float)J.spp, mul(mk(J.bg[0], J.bg[1], J.bg[2]), mk(1.f, 1.f, 1.f)));
-    flush_radiance(J, ray, val);
+    flush_radiance(J, -1 - (int64_t)item, val);
   }
 }
 
-// ---------------------------------------------------------------------------
-// kMode: traversal as in k_isect.
-template <int BS, int MINB, int kMode>
-__global__ void __launch_bounds__(BS, MINB) k_primary(EngineParams P) {
-  constexpr bool kStep = kMode != kTravLeaf;
-  extern __shared__ uint2 snodes[];
-  const int n_smem = kMode == kTravStep ? 0 : stage_nodes(P, snodes);
-  const TravScene* scene_tab = stage_scenes(P, snodes);
+// Tree walk of the rays [first, first + n) of the list, n <= 32. Not inlined:
+// few rays need it, and its registers must not weigh on the main loop.
+__device__ __noinline__ void walk_rays(const EngineParams& P, const WalkList& W, int first,
+                                       int n) {
   DevCtrl* c = P.ctrl;
   const int lane = threadIdx.x & 31;
-  const int64_t total = P.prim_prefix[P.prim_n];
-  bool active = false;
+  const bool have = lane < n;
+  int item = 0, slot = 0;
+  TravCount cnt{};
   TravState st;
-  __shared__ TravCold cold_sh[BS];
-  __shared__ CountSlot count_sh[BS];
-  TravCold& tc = cold_sh[threadIdx.x];
-  TravCount& cnt = count_sh[threadIdx.x].c;
-  cnt = TravCount{};
-  uint32_t& queries = count_sh[threadIdx.x].queries;
-  queries = 0;
-  int slot = 0;
-  // The lane's camera ray (read when it finishes; shared memory keeps the
-  // registers for the traversal).
-  __shared__ int64_t ray_sh[BS];
-  int64_t& ray = ray_sh[threadIdx.x];
-  ray = 0;
-  // Once a refill finds the rays exhausted the warp stops asking (the value
-  // is warp-uniform), so the cursor overshoots by at most one grab per warp.
+  st.best.tri = -1;
+  st.best.t = 0.f;
+  Ray r{};
+  if (have) {
+    item = W.item[first + lane];
+    slot = W.slot[first + lane];
+    const DevScene& s = P.jobs[slot].scene;
+    r = list_ray(P, item, slot);
+    TravCold tc;
+    trav_init(s, r, st, tc);
+    while (!trav_leaf(s, st, tc, nullptr, 0, &c->err, cnt)) {
+    }
+  }
+  __syncwarp();
+  write_hits(P, have, item, slot, r.d, have && st.best.rec >= 0 ? st.best.tri : -1, st.best.t);
+  const uint32_t nodes = __reduce_add_sync(kFull, cnt.nodes);
+  const uint32_t leaves = __reduce_add_sync(kFull, cnt.leaves);
+  const uint32_t tests = __reduce_add_sync(kFull, cnt.tris);
+  const uint32_t repeats = __reduce_add_sync(kFull, cnt.repeats);
+  if (lane == 0) {
+    add_counts(c, 0, nodes, leaves, tests);
+    if (repeats) atomicAdd(&c->tri_repeats, (unsigned long long)repeats);
+  }
+}
+
+// Certifies the finished rays [first, first + n) of the list, n <= 32, and
+// writes them out; those that need the tree walk go to W at n_walk. Returns
+// the new length of W.
+__device__ __noinline__ int finish_rays(const EngineParams& P, const HitList& L, int first, int n,
+                                        WalkList& W, int n_walk) {
+  DevCtrl* c = P.ctrl;
+  const int lane = threadIdx.x & 31;
+  const bool have = lane < n;
+  int item = 0, slot = 0, tri = -1;
+  float t = 0.f;
+  bool certain = false;
+  Ray r{};
+  if (have) {
+    item = L.item[first + lane];
+    slot = L.slot[first + lane];
+    const uint32_t best = L.best[first + lane];
+    t = L.t[first + lane];
+    const DevScene& s = P.jobs[slot].scene;
+    r = list_ray(P, item, slot);
+    certain = bvh_certain(s, r, best, t, &c->err);
+    if (certain && best != kBvhNone)
+      tri = __float_as_int(__ldg(reinterpret_cast<const float4*>(s.btris + best)).w);
+  }
+  __syncwarp();
+  const unsigned wm = __ballot_sync(kFull, have && !certain);
+  if (have && !certain) {
+    const int k = n_walk + __popc(wm & lanemask_lt());
+    W.item[k] = item;
+    W.slot[k] = slot;
+  }
+  __syncwarp();
+  write_hits(P, have && certain, item, slot, r.d, tri, t);
+  return n_walk + __popc(wm);
+}
+
+// Test rounds run when at least this share (in eighths) of the warp's live
+// lanes hold pending triangles.
+#ifndef HPT_TEST_EIGHTHS
+#define HPT_TEST_EIGHTHS 4
+#endif
+
+// kUniform: every job of the launch renders P.uscene. kQueue: traces the
+// intersect queue; kPrim: traces the camera rays of the launch's primary-pass
+// entries (P.prim_*), after the queue's; k_admit (or, with kQueue, k_ctrl)
+// then starts the paths of the jobs whose primary pass completed. A serving
+// loop admits requests with both, with no launch of its own.
+//
+// A round of the warp runs one code path: a node visit for the lanes without
+// pending triangles, or one triangle test for those with some.
+template <int BS, int MINB, bool kUniform, bool kQueue, bool kPrim>
+__global__ void __launch_bounds__(BS, MINB) k_trace(const __grid_constant__ EngineParams P) {
+  __shared__ HitList hit_lists[BS / 32];
+  __shared__ WalkList walk_lists[BS / 32];
+  HitList& L = hit_lists[threadIdx.x >> 5];
+  WalkList& W = walk_lists[threadIdx.x >> 5];
+  DevCtrl* c = P.ctrl;
+  const int n = kQueue ? c->nR : 0;
+  const int64_t total = kPrim ? (int64_t)n + P.prim_prefix[P.prim_n] : (int64_t)n;
+  unsigned long long* head = kQueue ? &c->isect_head : &c->prim_head;
+  const int lane = threadIdx.x & 31;
+  bool active = false;
+  BvhRay b;
+  b.tri_bits = 0;
+  uint2 stack[kBvhStack];
+  int item = 0, slot = 0, steps = 0;
+  const BvhNode* bvh = P.uscene.bvh;
+  const BvhTri* btris = P.uscene.btris;
+  uint32_t num_bvh = (uint32_t)P.uscene.num_bvh;
+  int max_steps = P.uscene.max_steps;
+  // The warp's counts and list lengths (the same value in every lane).
+  uint32_t queries = 0, nodes = 0, leaves = 0, tests = 0;
+  int n_hits = 0, n_walk = 0;
+  // Once a refill finds the rays exhausted the warp stops asking, so the
+  // cursor overshoots by at most one grab per warp.
   bool drained = false;
   while (true) {
     const unsigned idle = __ballot_sync(kFull, !active);
     if (!drained && __popc(idle) >= P.refill) {
       unsigned long long base = 0;
-      if (lane == 0) base = atomicAdd(&c->prim_head, (unsigned long long)__popc(idle));
+      if (lane == 0) base = atomicAdd(head, (unsigned long long)__popc(idle));
       base = __shfl_sync(kFull, base, 0);
       drained = (int64_t)base + __popc(idle) >= total;
+      bool started = false, walk = false;
       if (!active) {
-        const int64_t g = (int64_t)base + __popc(idle & lanemask_lt());
-        if (g < total && prim_locate(P, g, slot, ray)) {
-          prim_init(P.jobs[slot], ray, st, tc);
-          active = true;
-          ++queries;
+        const int64_t i = (int64_t)base + __popc(idle & lanemask_lt());
+        Ray r{};
+        if (kPrim && i >= n && i < total) {
+          int64_t ray = 0;
+          if (prim_locate(P, i - n, slot, ray)) {
+            r = prim_ray(P.jobs[slot], ray);
+            item = -1 - (int)ray;
+            started = true;
+          }
+        }
+        if (kQueue && i < n) {
+          bool ok = true;
+          HPT_DCHECK(&c->err, i < P.capacity, 221, i, ok = false);
+          if (ok) {
+            const float4 o4 = P.R_o[i], d4 = P.R_d[i];
+            slot = __float_as_int(P.R_s[i].w);
+            HPT_DCHECK(&c->err, slot >= 0 && slot < P.num_slots, 222, slot, ok = false);
+            r = Ray{mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z)};
+            item = (int)i;
+            started = ok;
+          }
+        }
+        if (started) {
+          float eps = P.uscene.scene_eps;
+          if (!kUniform) {
+            const DevScene& s = P.jobs[slot].scene;
+            bvh = s.bvh;
+            btris = s.btris;
+            num_bvh = (uint32_t)s.num_bvh;
+            max_steps = s.max_steps;
+            eps = s.scene_eps;
+          }
+          steps = 0;
+          active = bvh_init(eps, r, b);
+          walk = !active;
+        }
+      }
+      queries += __popc(__ballot_sync(kFull, started));
+      const unsigned wm = __ballot_sync(kFull, walk);
+      if (wm) {
+        if (walk) {
+          const int k = n_walk + __popc(wm & lanemask_lt());
+          W.item[k] = item;
+          W.slot[k] = slot;
+        }
+        n_walk += __popc(wm);
+        __syncwarp();
+        if (n_walk >= 32) {
+          n_walk -= 32;
+          walk_rays(P, W, n_walk, 32);
         }
       }
     }
-    if (__ballot_sync(kFull, active) == 0) break;
+    if (__ballot_sync(kFull, active) == 0) {
+      if (drained) break;
+      continue;
+    }
     bool finished = false;
-#if HPT_PHASE_VOTE
-    if constexpr (kStep) {
-      if (P.uniform_scene)
-        finished = vote_units<kMode, kCoopPrimary>(OneScene{P.uscene}, slot, active, st, tc,
-                                         snodes, n_smem, &c->err, cnt, P.trav_steps);
-      else if (P.scene_table)
-        finished = vote_units<kMode, kCoopPrimary>(TableScene{scene_tab}, slot, active, st, tc,
-                                         snodes, n_smem, &c->err, cnt, P.trav_steps);
-      else
-        finished = vote_units<kMode, kCoopPrimary>(JobScene{P.jobs}, slot, active, st, tc,
-                                         snodes, n_smem, &c->err, cnt, P.trav_steps);
-    } else if (active) {
-      finished = trav_leaf(P.jobs[slot].scene, st, tc, snodes, n_smem, &c->err, cnt);
-    }
-#else
-    if (active) {
-      if constexpr (kStep) {
-        if (P.uniform_scene) {
-          for (int u = 0; u < P.trav_steps; ++u)
-            if (trav_step<false, kMode == kTravStepSmem>(P.uscene, st, tc, snodes, n_smem,
-                                                         &c->err, cnt)) {
-              finished = true;
-              break;
-            }
-        } else if (P.scene_table) {
-          const TravScene& sc = scene_tab[slot];
-          for (int u = 0; u < P.trav_steps; ++u)
-            if (trav_step<false, kMode == kTravStepSmem>(sc, st, tc, snodes, n_smem, &c->err,
-                                                         cnt)) {
-              finished = true;
-              break;
-            }
-        } else {
-          const DevScene& sc = P.jobs[slot].scene;
-          for (int u = 0; u < P.trav_steps; ++u)
-            if (trav_step<false, kMode == kTravStepSmem>(sc, st, tc, snodes, n_smem, &c->err,
-                                                         cnt)) {
-              finished = true;
-              break;
-            }
+    for (int u = 0; u < P.rounds; ++u) {
+      const bool go = active && !finished;
+      const unsigned lm = __ballot_sync(kFull, go);
+      if (lm == 0) break;
+      const bool testing = go && b.tri_bits != 0;
+      const unsigned tm = __ballot_sync(kFull, testing);
+      // Every round moves a lane on: a test round needs a testing lane, a
+      // visit round one that is not.
+      if (tm != 0 && 8 * __popc(tm) >= HPT_TEST_EIGHTHS * __popc(lm)) {
+        if (testing) {
+          bvh_test(btris, b);
+          ++steps;
+          finished = b.tri_bits == 0 && (b.node_bits & 255u) == 0 && b.sp == 0;
         }
+        tests += __popc(tm);
       } else {
-        finished = trav_leaf(P.jobs[slot].scene, st, tc, snodes, n_smem, &c->err, cnt);
+        if (go && !testing) {
+          finished = !bvh_visit(bvh, num_bvh, b, stack, &c->err) ||
+                     (b.tri_bits == 0 && (b.node_bits & 255u) == 0 && b.sp == 0);
+          ++steps;
+        }
+        nodes += __popc(lm & ~tm);
+        leaves += __popc(__ballot_sync(kFull, go && !testing && b.tri_bits != 0));
+      }
+      if (go && steps > max_steps) {
+        atomicOr(&c->err.flags, 1u);
+        finished = true;
       }
     }
-#endif
-    if (finished) {
-      prim_finish(P, slot, ray, st, tc);
-      active = false;
+    const unsigned fm = __ballot_sync(kFull, finished);
+    if (fm) {
+      if (finished) {
+        const int k = n_hits + __popc(fm & lanemask_lt());
+        L.item[k] = item;
+        L.slot[k] = slot;
+        L.best[k] = b.best;
+        L.t[k] = b.best_t;
+        active = false;
+      }
+      n_hits += __popc(fm);
+      __syncwarp();
+      if (n_hits >= 32) {
+        n_hits -= 32;
+        n_walk = finish_rays(P, L, n_hits, 32, W, n_walk);
+        if (n_walk >= 32) {
+          n_walk -= 32;
+          walk_rays(P, W, n_walk, 32);
+        }
+        __syncwarp();
+      }
     }
   }
-  flush_counts(c, queries, cnt);
+  if (n_hits) n_walk = finish_rays(P, L, 0, n_hits, W, n_walk);
+  for (; n_walk > 0; n_walk -= min(n_walk, 32)) {
+    const int m = min(n_walk, 32);
+    walk_rays(P, W, n_walk - m, m);
+  }
+  if (lane == 0) add_counts(c, queries, nodes, leaves, tests);
 }
 
 // Sets the path count of primary-pass entry e's slot when the entry
@@ -684,7 +618,7 @@ __global__ void __launch_bounds__(BS, MINB) k_shade(EngineParams P) {
     int slot = 0;
     float4 oo, dd, ss, rr;
     if (i < n_items) {
-      int sample = 0, bounce = 0, tri = -1, hint = -1;
+      int sample = 0, bounce = 0, tri = -1;
       int64_t ray = -1;
       f3 o, d, strength, rad;
       float t = 0.f;
@@ -695,7 +629,6 @@ __global__ void __launch_bounds__(BS, MINB) k_shade(EngineParams P) {
           const float4 ao = P.A_o[par][i], ad = P.A_d[par][i], as = P.A_s[par][i],
                        ar = P.A_r[par][i];
           tri = P.A_tri[par][i];
-          hint = P.A_leaf[par][i];
           o = mk(ao.x, ao.y, ao.z);
           ray = __float_as_int(ao.w);
           d = mk(ad.x, ad.y, ad.z);
@@ -729,7 +662,6 @@ __global__ void __launch_bounds__(BS, MINB) k_shade(EngineParams P) {
             ray = __float_as_int(p0.w);
             tri = __float_as_int(p1.x);
             t = p1.y;
-            hint = __float_as_int(p1.z);
             strength = mk(1.f, 1.f, 1.f);
             rad = mk(0.f, 0.f, 0.f);
           }
@@ -760,7 +692,7 @@ __global__ void __launch_bounds__(BS, MINB) k_shade(EngineParams P) {
             dd = make_float4(no.d.x, no.d.y, no.d.z,
                              __uint_as_float(((uint32_t)sample << 8) | (uint32_t)(bounce + 1)));
             ss = make_float4(no.strength.x, no.strength.y, no.strength.z, __int_as_float(slot));
-            rr = make_float4(rad.x, rad.y, rad.z, __int_as_float(hint));
+            rr = make_float4(rad.x, rad.y, rad.z, 0.f);
           }
         }
         if (!alive) {
@@ -806,178 +738,6 @@ __global__ void __launch_bounds__(BS, MINB) k_shade(EngineParams P) {
 #endif
 }
 
-// ---------------------------------------------------------------------------
-// Intersect queue -> next shade queue, persistent warps with lane refill.
-// ---------------------------------------------------------------------------
-// kMode: kTravStep / kTravStepSmem traverse with trav_step, P.trav_steps
-// calls per lane between refill checks (lanes move to their next leaf
-// independently), reading nodes from global memory only / also from the
-// shared-memory prefix; kTravLeaf: one leaf per lane per round with
-// trav_leaf.
-// kPrim: the launch also traces the camera rays of its primary-pass entries
-// (P.prim_*), after the queue's rays, and records them as k_primary does;
-// k_ctrl then starts the paths of the jobs whose primary pass completed.
-// A serving loop admits requests this way, with no launch of its own.
-template <int BS, int MINB, int kMode, bool kPrim = false>
-__global__ void __launch_bounds__(BS, MINB) k_isect(EngineParams P) {
-  constexpr bool kStep = kMode != kTravLeaf;
-  extern __shared__ uint2 snodes[];
-  const int n_smem = kMode == kTravStep ? 0 : stage_nodes(P, snodes);
-  const TravScene* scene_tab = stage_scenes(P, snodes);
-  DevCtrl* c = P.ctrl;
-  const int n = c->nR;
-  const int64_t total = kPrim ? (int64_t)n + P.prim_prefix[P.prim_n] : (int64_t)n;
-  const int out_par = c->parity ^ 1;
-  const int lane = threadIdx.x & 31;
-  bool active = false;
-  TravState st;
-  __shared__ TravCold cold_sh[BS];
-  __shared__ CountSlot count_sh[BS];
-  TravCold& tc = cold_sh[threadIdx.x];
-  TravCount& cnt = count_sh[threadIdx.x].c;
-  cnt = TravCount{};
-  uint32_t& queries = count_sh[threadIdx.x].queries;
-  queries = 0;
-  // Index in the intersect queue (the payload is reloaded at the end); with
-  // kPrim, -1 - ray for a camera ray. Read when the ray finishes, so it
-  // stays in shared memory.
-  __shared__ int item_sh[BS];
-  int& item = item_sh[threadIdx.x];
-  item = 0;
-  int slot = 0;
-  // As in k_primary: a warp that finds the queue exhausted stops refilling.
-  bool drained = false;
-  while (true) {
-    const unsigned idle = __ballot_sync(kFull, !active);
-    if (!drained && __popc(idle) >= P.refill) {
-      unsigned long long base = 0;
-      if (lane == 0) base = atomicAdd(&c->isect_head, (unsigned long long)__popc(idle));
-      base = __shfl_sync(kFull, base, 0);
-      drained = (int64_t)base + __popc(idle) >= total;
-      if (!active) {
-        const int64_t i = (int64_t)base + __popc(idle & lanemask_lt());
-        if constexpr (kPrim) {
-          int64_t ray = 0;
-          if (i >= n && i < total && prim_locate(P, i - n, slot, ray)) {
-            prim_init(P.jobs[slot], ray, st, tc);
-            item = -1 - (int)ray;
-            active = true;
-            ++queries;
-          }
-        }
-        if (i < n) {
-          bool ok = true;
-          HPT_DCHECK(&c->err, i < P.capacity, 221, i, ok = false);
-          if (ok) {
-            const float4 o4 = P.R_o[i], d4 = P.R_d[i];
-            item = (int)i;
-            slot = __float_as_int(P.R_s[i].w);
-            HPT_DCHECK(&c->err, slot >= 0 && slot < P.num_slots, 222, slot, ok = false);
-            if (ok) {
-              trav_init(P.jobs[slot].scene, Ray{mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z)}, st,
-                        tc, __float_as_int(P.R_r[i].w));
-              active = true;
-              ++queries;
-            }
-          }
-        }
-      }
-    }
-    if (__ballot_sync(kFull, active) == 0) break;
-    bool finished = false;
-#if HPT_PHASE_VOTE
-    if constexpr (kStep) {
-      if (P.uniform_scene)
-        finished = vote_units<kMode, true>(OneScene{P.uscene}, slot, active, st, tc,
-                                         snodes, n_smem, &c->err, cnt, P.trav_steps);
-      else if (P.scene_table)
-        finished = vote_units<kMode, true>(TableScene{scene_tab}, slot, active, st, tc,
-                                         snodes, n_smem, &c->err, cnt, P.trav_steps);
-      else
-        finished = vote_units<kMode, true>(JobScene{P.jobs}, slot, active, st, tc,
-                                         snodes, n_smem, &c->err, cnt, P.trav_steps);
-    } else if (active) {
-      finished = trav_leaf(P.jobs[slot].scene, st, tc, snodes, n_smem, &c->err, cnt);
-    }
-#else
-    if (active) {
-      if constexpr (kStep) {
-        if (P.uniform_scene) {
-          for (int u = 0; u < P.trav_steps; ++u)
-            if (trav_step<false, kMode == kTravStepSmem>(P.uscene, st, tc, snodes, n_smem,
-                                                         &c->err, cnt)) {
-              finished = true;
-              break;
-            }
-        } else if (P.scene_table) {
-          const TravScene& sc = scene_tab[slot];
-          for (int u = 0; u < P.trav_steps; ++u)
-            if (trav_step<false, kMode == kTravStepSmem>(sc, st, tc, snodes, n_smem, &c->err,
-                                                         cnt)) {
-              finished = true;
-              break;
-            }
-        } else {
-          const DevScene& sc = P.jobs[slot].scene;
-          for (int u = 0; u < P.trav_steps; ++u)
-            if (trav_step<false, kMode == kTravStepSmem>(sc, st, tc, snodes, n_smem, &c->err,
-                                                         cnt)) {
-              finished = true;
-              break;
-            }
-        }
-      } else {
-        finished = trav_leaf(P.jobs[slot].scene, st, tc, snodes, n_smem, &c->err, cnt);
-      }
-    }
-#endif
-    // A camera ray (kPrim) goes to its job's primary-hit cache instead.
-    const bool queued = !kPrim || item >= 0;
-    if constexpr (kPrim) {
-      if (finished && !queued) prim_finish(P, slot, -1 - (int64_t)item, st, tc);
-    }
-    const bool hit = finished && queued && st.best.rec >= 0;
-    const unsigned hm = __ballot_sync(kFull, hit);
-    if (hm) {
-      const int leader = __ffs(hm) - 1;
-      int base = 0;
-      if (lane == leader) base = atomicAdd(&c->nA_next, __popc(hm));
-      base = __shfl_sync(kFull, base, leader);
-      if (hit) {
-        const int pos = base + __popc(hm & lanemask_lt());
-        bool ok = true;
-        HPT_DCHECK(&c->err, pos < P.capacity, 223, pos, ok = false);
-        if (ok) {
-          const float4 r4 = P.R_r[item];
-          P.A_o[out_par][pos] = P.R_o[item];
-          P.A_d[out_par][pos] = P.R_d[item];
-          P.A_s[out_par][pos] = P.R_s[item];
-          P.A_r[out_par][pos] = make_float4(r4.x, r4.y, r4.z, st.best.t);
-          P.A_tri[out_par][pos] = st.best.tri;
-          P.A_leaf[out_par][pos] = tc.best_node;
-        }
-      }
-    }
-    const bool missed = finished && queued && !hit;
-    if (missed) {
-      // kernel.cl:195-200: miss adds background * strength (sample_n = 1).
-      const DevJob& J = P.jobs[slot];
-      const float4 s4 = P.R_s[item], r4 = P.R_r[item];
-      const int64_t ray = __float_as_int(P.R_o[item].w);
-      bool ok = true;
-      HPT_DCHECK(&c->err, ray >= 0 && ray < job_rays(J), 224, ray, ok = false);
-      if (ok) {
-        f3 rad = mk(r4.x, r4.y, r4.z);
-        rad = add(rad, mul(mk(J.bg[0], J.bg[1], J.bg[2]), mk(s4.x, s4.y, s4.z)));
-        flush_radiance(J, ray, rad);
-      }
-    }
-    count_done(P.slots, missed, slot);
-    if (finished) active = false;
-  }
-  flush_counts(c, queries, cnt);
-}
-
 // Advances the queues and the path cursors, then grants paths (one thread).
 __global__ void k_ctrl(EngineParams P) {
   DevCtrl* c = P.ctrl;
@@ -1006,35 +766,24 @@ __global__ void k_ctrl(EngineParams P) {
   schedule(P);
 }
 
-// Register budgets for the traversal kernels: (threads per block, blocks
-// per SM the compiler must fit). The natural allocation is ~97 registers;
-// tighter budgets trade spills for resident warps. Chosen by the tuning.
+// Register budgets of the closest-hit kernels: (threads per block, blocks per
+// SM the compiler must fit); more resident warps against spills. Chosen by
+// the tuning.
 struct IsectVariant {
   int block, min_blocks;
-  void (*isect)(EngineParams);            // one leaf per round
-  void (*isect_step)(EngineParams);       // step-at-a-time, nodes from global memory
-  void (*isect_step_smem)(EngineParams);  // step-at-a-time, shared-memory node prefix
-  void (*primary)(EngineParams);
-  void (*primary_step)(EngineParams);
-  void (*primary_step_smem)(EngineParams);
-  void (*isect_step_prim)(EngineParams);  // step-at-a-time with primary-pass entries
-  // The kernel a launch with these tuning values uses (shared-node prefix
-  // only when smem_nodes > 0).
-  void (*isect_kernel(int trav_steps, int smem_nodes) const)(EngineParams) {
-    return trav_steps <= 0 ? isect : (smem_nodes > 0 ? isect_step_smem : isect_step);
-  }
-  void (*primary_kernel(int trav_steps, int smem_nodes) const)(EngineParams) {
-    return trav_steps <= 0 ? primary : (smem_nodes > 0 ? primary_step_smem : primary_step);
-  }
+  // [uniform scene]: queue rays, camera rays, both in one launch.
+  void (*isect[2])(EngineParams);
+  void (*primary[2])(EngineParams);
+  void (*both[2])(EngineParams);
 };
-#define HPT_ISECT_VARIANT(B, M)                                                       \
-  {B, M, k_isect<B, M, kTravLeaf>, k_isect<B, M, kTravStep>,                          \
-   k_isect<B, M, kTravStepSmem>, k_primary<B, M, kTravLeaf>, k_primary<B, M, kTravStep>, \
-   k_primary<B, M, kTravStepSmem>, k_isect<B, M, kTravStep, true>}
+#define HPT_ISECT_VARIANT(B, M)                                                   \
+  {B, M, {k_trace<B, M, false, true, false>, k_trace<B, M, true, true, false>},   \
+   {k_trace<B, M, false, false, true>, k_trace<B, M, true, false, true>},         \
+   {k_trace<B, M, false, true, true>, k_trace<B, M, true, true, true>}}
 const IsectVariant kIsectVariants[] = {
-    HPT_ISECT_VARIANT(128, 5), HPT_ISECT_VARIANT(128, 6), HPT_ISECT_VARIANT(128, 7),
-    HPT_ISECT_VARIANT(128, 8), HPT_ISECT_VARIANT(128, 9), HPT_ISECT_VARIANT(128, 10),
-    HPT_ISECT_VARIANT(256, 2), HPT_ISECT_VARIANT(256, 3),
+    HPT_ISECT_VARIANT(128, 6), HPT_ISECT_VARIANT(128, 7), HPT_ISECT_VARIANT(128, 8),
+    HPT_ISECT_VARIANT(128, 9), HPT_ISECT_VARIANT(128, 10),
+    HPT_ISECT_VARIANT(256, 3), HPT_ISECT_VARIANT(256, 4),
 };
 #undef HPT_ISECT_VARIANT
 constexpr int kNumIsectVariants = sizeof(kIsectVariants) / sizeof(kIsectVariants[0]);
@@ -1127,26 +876,21 @@ void cuda_soft_fail(cudaError_t e, const char* what) {
 hpt_tuning default_tuning() {
   hpt_tuning t;
   memset(&t, 0, sizeof t);
-  // From the tuning sweeps on the 61k-triangle spheres frame (512x512,
-  // 64 spp) and the 2.4M-triangle terrain frame: step-at-a-time traversal
-  // with the phase vote, 48 warp rounds per refill check (16 / 24 / 32 /
-  // 48: spheres 107.0 / 105.7 / 105.0 / 105.0 ms, terrain at 4 spp 79.6 /
-  // 79.0 / 78.7 / 77.7 ms; with cooperative tests 32 / 48 / 64: 92.5 /
-  // 92.3 / 93.0 ms), 9 blocks of 128 per SM (56 registers; with
-  // cooperative tests 8 / 9 / 10 blocks: spheres 94.8 / 92.3 / 101.4 ms,
-  // terrain 74.3 / 70.7 / 81.5 ms - at 10 the 48-register budget spills),
-  // no shared-node prefix, a wavefront of 2^24 paths (2^22 / 2^23 / 2^24 /
-  // 2^25: spheres 92.2 / 88.7 / 87.0 / 87.1 ms, terrain at 16 spp 227.5 /
-  // 223.0 / 220.3 / 218.4 ms; 3.5 GB of queues, allocated only up to the
-  // paths a run has).
+  // From sweeps on the 512x512, 64 spp spheres frame and the 1920x1080, 4 spp
+  // terrain frame: 7 blocks of 128 per SM (72 registers; 6 / 7 / 8 / 9 / 10
+  // blocks: spheres 47.1 / 45.4 / 49.5 / 52.3 / 51.9 ms, terrain 15.6 / 15.1
+  // / 16.1 / 16.4 / 16.2 ms - the tighter budgets spill in the walk's loop),
+  // 16 rounds between refills (2 / 4 / 8 / 16: spheres 52.5 / 49.3 / 46.7 /
+  // 45.4 ms), a wavefront of 2^24 paths (3.5 GB of queues, allocated only up
+  // to the paths a run has).
   t.capacity = 1 << 24;
   t.isect_block = 128;
-  t.isect_min_blocks = 9;
+  t.isect_min_blocks = 7;
   t.shade_block = 256;
   t.refill_chunk = 4;
   t.smem_nodes = 0;
   t.use_graph = 0;
-  t.trav_steps = 48;
+  t.trav_steps = 16;
   // Shading at 4 blocks of 256 per SM (64 registers): 7.0 instead of 8.4 ms
   // per spheres frame at the natural 106-register allocation (2 blocks).
   t.shade_min_blocks = 4;
@@ -1223,7 +967,6 @@ Engine::~Engine() {
     HPT_SOFT(cudaFree(A_s_[p]));
     HPT_SOFT(cudaFree(A_r_[p]));
     HPT_SOFT(cudaFree(A_tri_[p]));
-    HPT_SOFT(cudaFree(A_leaf_[p]));
   }
   HPT_SOFT(cudaFree(R_o_));
   HPT_SOFT(cudaFree(R_d_));
@@ -1270,9 +1013,8 @@ hpt_status Engine::ensure_capacity(int capacity) {
     HPT_SOFT(cudaFree(A_s_[p]));
     HPT_SOFT(cudaFree(A_r_[p]));
     HPT_SOFT(cudaFree(A_tri_[p]));
-    HPT_SOFT(cudaFree(A_leaf_[p]));
     A_o_[p] = A_d_[p] = A_s_[p] = A_r_[p] = nullptr;
-    A_tri_[p] = A_leaf_[p] = nullptr;
+    A_tri_[p] = nullptr;
   }
   HPT_SOFT(cudaFree(R_o_));
   HPT_SOFT(cudaFree(R_d_));
@@ -1287,7 +1029,6 @@ hpt_status Engine::ensure_capacity(int capacity) {
     HPT_CUDA(cudaMalloc(&A_s_[p], n * sizeof(float4)));
     HPT_CUDA(cudaMalloc(&A_r_[p], n * sizeof(float4)));
     HPT_CUDA(cudaMalloc(&A_tri_[p], n * sizeof(int32_t)));
-    HPT_CUDA(cudaMalloc(&A_leaf_[p], n * sizeof(int32_t)));
   }
   HPT_CUDA(cudaMalloc(&R_o_, n * sizeof(float4)));
   HPT_CUDA(cudaMalloc(&R_d_, n * sizeof(float4)));
@@ -1356,41 +1097,12 @@ int Engine::isect_variant() const {
   return 0;
 }
 
-// The dynamic shared-memory limit is an attribute of the kernel function
-// (per device, shared by every engine of the process), so it is raised once
-// to the largest node prefix a tuning may ask for and never lowered.
-static hpt_status raise_smem_limits(int device) {
-  static std::mutex mu;
-  static std::vector<char> done;
-  std::lock_guard<std::mutex> lk(mu);
-  if ((int)done.size() <= device) done.resize(device + 1, 0);
-  if (done[device]) return HPT_OK;
-  const int bytes = kMaxSmemNodes * (int)sizeof(uint2);
-  for (const IsectVariant& v : kIsectVariants) {
-    HPT_CUDA(cudaFuncSetAttribute(v.primary, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    HPT_CUDA(cudaFuncSetAttribute(v.primary_step, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  bytes));
-    HPT_CUDA(cudaFuncSetAttribute(v.isect, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    HPT_CUDA(cudaFuncSetAttribute(v.isect_step, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  bytes));
-    HPT_CUDA(cudaFuncSetAttribute(v.primary_step_smem,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    HPT_CUDA(cudaFuncSetAttribute(v.isect_step_smem,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  }
-  done[device] = 1;
-  return HPT_OK;
-}
-
 hpt_status Engine::query_occupancy() {
   if (occ_done_) return HPT_OK;
-  hpt_status s = raise_smem_limits(device);
-  if (s != HPT_OK) return s;
   const IsectVariant& v = kIsectVariants[isect_variant()];
-  const size_t smem = (size_t)std::max(0, tuning.smem_nodes) * sizeof(uint2);
   int b = 0;
   HPT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      &b, v.isect_kernel(tuning.trav_steps, tuning.smem_nodes), v.block, smem));
+      &b, v.isect[1], v.block, 0));
   occ_isect_ = std::max(1, b);
   HPT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, shade_kernel(tuning), 256, 0));
   occ_shade_ = std::max(1, b);
@@ -1459,15 +1171,11 @@ DevJob Engine::make_job(const JobSpec& js, const JobBuffers& b) const {
   return j;
 }
 
-// Largest per-slot scene table kept in shared memory (102 slots): 10
-// blocks of 128 per SM then still fit beside their static shared memory.
-constexpr size_t kSceneTableBytes = 8192;
-
 static EngineParams make_params(const Engine& e, DevCtrl* ctrl, DevJob* jobs, DevSlot* slots,
                                 int num_slots, const int32_t* order, int32_t* quota_slot,
                                 int32_t* quota_prefix, const int32_t* prim_slot,
                                 const int64_t* prim_prefix, int prim_n, int capacity,
-                                float4* const* A, int32_t* const* Atri, int32_t* const* Aleaf,
+                                float4* const* A, int32_t* const* Atri,
                                 float4* const* R, const DevScene* shared) {
   EngineParams P;
   memset(&P, 0, sizeof P);
@@ -1487,7 +1195,6 @@ static EngineParams make_params(const Engine& e, DevCtrl* ctrl, DevJob* jobs, De
     P.A_s[p] = A[4 * p + 2];
     P.A_r[p] = A[4 * p + 3];
     P.A_tri[p] = Atri[p];
-    P.A_leaf[p] = Aleaf[p];
   }
   P.R_o = R[0];
   P.R_d = R[1];
@@ -1495,24 +1202,12 @@ static EngineParams make_params(const Engine& e, DevCtrl* ctrl, DevJob* jobs, De
   P.R_r = R[3];
   P.capacity = capacity;
   P.refill = std::max(1, std::min(32, e.tuning.refill_chunk));
-  P.trav_steps = std::max(0, e.tuning.trav_steps);
+  P.rounds = e.tuning.trav_steps > 0 ? e.tuning.trav_steps : default_tuning().trav_steps;
   if (shared) {
     P.uniform_scene = 1;
     P.uscene = capped_scene(*shared, e.tuning);
   }
-  if (shared && e.tuning.smem_nodes > 0) {
-    P.smem_nodes = std::min(e.tuning.smem_nodes, shared->num_nodes);
-    P.shared_nodes = shared->nodes;
-  }
-  if (!shared && (size_t)num_slots * sizeof(TravScene) <= kSceneTableBytes) P.scene_table = 1;
   return P;
-}
-
-// Dynamic shared memory of a traversal launch: the node prefix of a
-// one-scene launch, or the per-slot scene table of a several-scene one.
-static size_t launch_smem(const EngineParams& P) {
-  return P.scene_table ? (size_t)P.num_slots * sizeof(TravScene)
-                       : (size_t)P.smem_nodes * sizeof(uint2);
 }
 
 void Engine::reset_ctrl() {
@@ -1567,10 +1262,9 @@ hpt_status Engine::admit(const std::vector<int>& slot_ids, const std::vector<Dev
   float4* R[4] = {R_o_, R_d_, R_s_, R_r_};
   EngineParams P = make_params(*this, ctrl_, jobs_, slot_state_, slots_, order_, quota_slot_,
                                quota_prefix_, prim_slot_, prim_prefix_, n, capacity_, A, A_tri_,
-                               A_leaf_, R, shared_scene);
-  const size_t smem = launch_smem(P);
+                               R, shared_scene);
   const IsectVariant& v = kIsectVariants[isect_variant()];
-  v.primary_kernel(P.trav_steps, P.smem_nodes)<<<num_sms * occ_isect_, v.block, smem, stream>>>(P);
+  v.primary[P.uniform_scene]<<<num_sms * occ_isect_, v.block, 0, stream>>>(P);
   HPT_CUDA(cudaGetLastError());
   hpt_status s = set_order(order);  // synchronises: the staging is free again
   if (s != HPT_OK) return s;
@@ -1674,8 +1368,6 @@ hpt_status Engine::stage_primary(StagingSet& st, int n, const int* slot_ids, con
   return HPT_OK;
 }
 
-bool Engine::fused_primary() const { return tuning.trav_steps > 0; }
-
 hpt_status Engine::queue_primary(int slot, const DevJob& job, int64_t rays, int64_t first,
                                  bool final_part) {
   if (slot < 0 || slot >= slots_ || rays <= 0 || first < 0)
@@ -1706,8 +1398,6 @@ hpt_status Engine::launch_iteration_async() {
     launch_iteration(nullptr);
     return HPT_OK;
   }
-  if (!fused_primary())
-    return fail(HPT_ERR_INVALID_ARGUMENT, "queued primary rays need step-at-a-time traversal");
   hpt_status s = query_occupancy();
   if (s != HPT_OK) return s;
   StagingSet* st = nullptr;
@@ -1726,51 +1416,13 @@ hpt_status Engine::launch_iteration_async() {
   float4* R[4] = {R_o_, R_d_, R_s_, R_r_};
   EngineParams P = make_params(*this, ctrl_, jobs_, slot_state_, slots_, order_, quota_slot_,
                                quota_prefix_, prim_slot_, prim_prefix_, n, capacity_, A, A_tri_,
-                               A_leaf_, R, nullptr);
+                               R, nullptr);
   P.prim_first = prim_first_;
   P.prim_final = prim_final_;
   shade_kernel(tuning)<<<num_sms * occ_shade_, 256, 0, stream>>>(P);
   const IsectVariant& v = kIsectVariants[isect_variant()];
-  v.isect_step_prim<<<num_sms * occ_isect_, v.block, launch_smem(P), stream>>>(P);
+  v.both[0]<<<num_sms * occ_isect_, v.block, 0, stream>>>(P);
   k_ctrl<<<1, 1, 0, stream>>>(P);
-  HPT_CUDA(cudaGetLastError());
-  return HPT_OK;
-}
-
-hpt_status Engine::admit_async(const std::vector<int>& slot_ids, const std::vector<DevJob>& jobs,
-                               const std::vector<int64_t>& rays, const std::vector<int>& order,
-                               const DevScene* shared_scene, const std::vector<int64_t>& first,
-                               const std::vector<int>& final_part) {
-  const int n = (int)slot_ids.size();
-  if (n == 0) return set_order_async(order);
-  hpt_status s = query_occupancy();
-  if (s != HPT_OK) return s;
-  const bool parts = !first.empty();
-  if (parts && ((int)first.size() != n || (int)final_part.size() != n))
-    return fail(HPT_ERR_INVALID_ARGUMENT, "primary parts: %d entries, %d firsts, %d flags", n,
-                (int)first.size(), (int)final_part.size());
-  StagingSet* st = nullptr;
-  s = next_staging(&st);
-  if (s != HPT_OK) return s;
-  s = stage_primary(*st, n, slot_ids.data(), jobs.data(), rays.data(),
-                    parts ? first.data() : nullptr, parts ? final_part.data() : nullptr);
-  if (s != HPT_OK) return s;
-  s = upload_order(order, *st);
-  if (s != HPT_OK) return s;
-  HPT_CUDA(cudaEventRecord(st->ev, stream));
-  float4* A[8] = {A_o_[0], A_d_[0], A_s_[0], A_r_[0], A_o_[1], A_d_[1], A_s_[1], A_r_[1]};
-  float4* R[4] = {R_o_, R_d_, R_s_, R_r_};
-  EngineParams P = make_params(*this, ctrl_, jobs_, slot_state_, slots_, order_, quota_slot_,
-                               quota_prefix_, prim_slot_, prim_prefix_, n, capacity_, A, A_tri_,
-                               A_leaf_, R, shared_scene);
-  if (parts) {
-    P.prim_first = prim_first_;
-    P.prim_final = prim_final_;
-  }
-  const size_t smem = launch_smem(P);
-  const IsectVariant& v = kIsectVariants[isect_variant()];
-  v.primary_kernel(P.trav_steps, P.smem_nodes)<<<num_sms * occ_isect_, v.block, smem, stream>>>(P);
-  k_admit<<<1, 1, 0, stream>>>(P);
   HPT_CUDA(cudaGetLastError());
   return HPT_OK;
 }
@@ -1834,13 +1486,12 @@ void Engine::launch_iteration(const DevScene* shared_scene, cudaEvent_t* ev) {
   float4* R[4] = {R_o_, R_d_, R_s_, R_r_};
   EngineParams P = make_params(*this, ctrl_, jobs_, slot_state_, slots_, order_, quota_slot_,
                                quota_prefix_, prim_slot_, prim_prefix_, 0, capacity_, A, A_tri_,
-                               A_leaf_, R, shared_scene);
+                               R, shared_scene);
   if (ev) HPT_SOFT(cudaEventRecord(ev[0], stream));
   shade_kernel(tuning)<<<num_sms * occ_shade_, 256, 0, stream>>>(P);
   if (ev) HPT_SOFT(cudaEventRecord(ev[1], stream));
-  const size_t smem = launch_smem(P);
   const IsectVariant& v = kIsectVariants[isect_variant()];
-  v.isect_kernel(P.trav_steps, P.smem_nodes)<<<num_sms * occ_isect_, v.block, smem, stream>>>(P);
+  v.isect[P.uniform_scene]<<<num_sms * occ_isect_, v.block, 0, stream>>>(P);
   if (ev) HPT_SOFT(cudaEventRecord(ev[2], stream));
   k_ctrl<<<1, 1, 0, stream>>>(P);
 }

@@ -80,25 +80,14 @@ class Engine {
   // Asynchronous forms for a serving loop: the uploads go through a ring of
   // pinned staging sets and nothing waits for the stream (only, rarely, for
   // a staging set's previous copies to have run).
-  // With `first` and `final_part` (one entry per slot), entry k traces rays
-  // [first[k], first[k] + rays[k]) of its job, and only an entry with
-  // final_part[k] != 0 starts the job's paths: a large job's primary pass
-  // can be split over several calls (same slot, same job, consecutive
-  // ranges, the last one final) so that no single launch stalls the
-  // iterations of the others for long.
-  hpt_status admit_async(const std::vector<int>& slot_ids, const std::vector<DevJob>& jobs,
-                         const std::vector<int64_t>& rays, const std::vector<int>& order,
-                         const DevScene* shared_scene, const std::vector<int64_t>& first = {},
-                         const std::vector<int>& final_part = {});
   hpt_status set_order_async(const std::vector<int>& order);
-  // Serving loop: a newly admitted job's camera rays can instead be traced
-  // inside the next iteration's traversal launch (fused_primary(): the
-  // tuning traverses step at a time), so that admissions add no launch of
-  // their own. queue_primary() records rays [first, first + rays) of the
+  // Serving loop: a newly admitted job's camera rays are traced inside the
+  // next iteration's closest-hit launch, so that admissions add no launch of
+  // their own (and a large job's can be split over several iterations, so
+  // that no launch stalls the others for long). queue_primary() records rays [first, first + rays) of the
   // job in `slot` (parts of one job in order; final_part on the last, which
   // starts its paths); launch_iteration_async() uploads what was queued and
   // launches one iteration that carries it.
-  bool fused_primary() const;
   hpt_status queue_primary(int slot, const DevJob& job, int64_t rays, int64_t first,
                            bool final_part);
   hpt_status launch_iteration_async();
@@ -150,7 +139,6 @@ class Engine {
   float4* A_s_[2] = {nullptr, nullptr};
   float4* A_r_[2] = {nullptr, nullptr};
   int32_t* A_tri_[2] = {nullptr, nullptr};
-  int32_t* A_leaf_[2] = {nullptr, nullptr};
   float4* R_o_ = nullptr;
   float4* R_d_ = nullptr;
   float4* R_s_ = nullptr;

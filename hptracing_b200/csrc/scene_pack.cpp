@@ -20,13 +20,16 @@
 //    that test in the reference's first-hit-wins tie rule (kernel.cl:180),
 //    and one record (a, b - a, c - a) per triangle.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <deque>
 #include <string>
+#include <thread>
 
 #include "device_types.h"
 #include "host.h"
+#include "parallel.h"
 #include "scene_pack.h"
 
 namespace hpt {
@@ -175,39 +178,61 @@ struct Packer {
     return r;
   }
 
+  struct RopeItem {
+    int node;
+    int rope[6];
+    float lo[3], hi[3];
+  };
+
+  // Sets a leaf's ropes, or pushes an inner node's children.
+  void rope_step(RopeItem c, std::vector<RopeItem>& stack) {
+    const TmpNode& n = nodes[c.node];
+    if (n.axis < 0) {
+      DevLeaf& L = leaves[n.leaf];
+      for (int f = 0; f < 6; ++f) L.rope[f] = c.rope[f];
+      return;
+    }
+    for (int f = 0; f < 6; ++f) c.rope[f] = optimize(c.rope[f], f, c.lo, c.hi);
+    RopeItem l = c, r = c;
+    l.node = n.left;
+    r.node = n.right;
+    l.rope[2 * n.axis + 1] = n.right;
+    r.rope[2 * n.axis] = n.left;
+    l.hi[n.axis] = n.split;
+    r.lo[n.axis] = n.split;
+    stack.push_back(r);
+    stack.push_back(l);
+  }
+
   void ropes(int root, const float rlo[3], const float rhi[3]) {
-    struct Item {
-      int node;
-      int rope[6];
-      float lo[3], hi[3];
-    };
-    std::vector<Item> stack;
-    Item it;
+    RopeItem it;
     it.node = root;
     for (int f = 0; f < 6; ++f) it.rope[f] = -1;
     memcpy(it.lo, rlo, sizeof it.lo);
     memcpy(it.hi, rhi, sizeof it.hi);
-    stack.push_back(it);
-    while (!stack.empty()) {
-      Item c = stack.back();
-      stack.pop_back();
-      const TmpNode& n = nodes[c.node];
-      if (n.axis < 0) {
-        DevLeaf& L = leaves[n.leaf];
-        for (int f = 0; f < 6; ++f) L.rope[f] = c.rope[f];
-        continue;
-      }
-      for (int f = 0; f < 6; ++f) c.rope[f] = optimize(c.rope[f], f, c.lo, c.hi);
-      Item l = c, r = c;
-      l.node = n.left;
-      r.node = n.right;
-      l.rope[2 * n.axis + 1] = n.right;
-      r.rope[2 * n.axis] = n.left;
-      l.hi[n.axis] = n.split;
-      r.lo[n.axis] = n.split;
-      stack.push_back(r);
-      stack.push_back(l);
+    // A subtree only writes its own leaves: the top is opened breadth-first
+    // into enough subtrees for all cores (small trees: one thread).
+    const int threads =
+        nodes.size() < 65536 ? 1 : (int)std::max(1u, std::thread::hardware_concurrency());
+    std::vector<RopeItem> top{it}, next;
+    while (threads > 1 && top.size() < 1024 && !top.empty()) {
+      next.clear();
+      for (const RopeItem& c : top) rope_step(c, next);
+      top.swap(next);
     }
+    std::atomic<size_t> cursor{0};
+    auto work = [&] {
+      std::vector<RopeItem> stack;
+      for (size_t k = cursor++; k < top.size(); k = cursor++) {
+        stack.push_back(top[k]);
+        while (!stack.empty()) {
+          const RopeItem c = stack.back();
+          stack.pop_back();
+          rope_step(c, stack);
+        }
+      }
+    };
+    run_threads(threads, work);
   }
 };
 
@@ -224,6 +249,8 @@ hpt_status pack_scene(const hpt_scene_desc& d, int bfs_nodes, PackedScene& out) 
   p.tris = reinterpret_cast<const I4*>(d.triangles);
   p.points = reinterpret_cast<const F4*>(d.points);
   p.nodes.reserve((size_t)d.num_nodes * 5 / 4 + 16);
+  p.leaves.reserve((size_t)d.num_nodes * 5 / 8 + 16);
+  p.refs.reserve((size_t)std::max(0, d.num_leaf_data));
   const hpt_ref_node& r0 = d.nodes[0];
   float lo[3] = {r0.box_start[0], r0.box_start[1], r0.box_start[2]};
   float hi[3] = {r0.box_end[0], r0.box_end[1], r0.box_end[2]};

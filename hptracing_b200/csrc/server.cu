@@ -277,9 +277,9 @@ hpt_status hpt_server::admit_pending() {
   // large request's are traced in parts, at most its in-flight share of the
   // wavefront (large_inflight_pct, else a quarter) of rays per iteration for
   // all large requests together: one panorama's 2M camera rays traced at
-  // once would stall every request in flight for milliseconds. With
-  // step-at-a-time traversal the camera rays ride in the next iteration's
-  // traversal launch (no launch, and no launch tail, of their own).
+  // once would stall every request in flight for milliseconds. The camera
+  // rays ride in the next iteration's closest-hit launch (no launch, and no
+  // launch tail, of their own).
   const int pct = cfg.large_inflight_pct;
   const int64_t share = pct > 0 && pct < 100 ? (int64_t)cfg.capacity * pct / 100
                                              : (int64_t)cfg.capacity / 4;
@@ -402,19 +402,12 @@ hpt_status hpt_server::admit_pending() {
     it = queue.erase(it);
   }
   if (ids.empty()) return HPT_OK;
-  if (engine->fused_primary()) {
-    for (size_t k = 0; k < ids.size(); ++k) {
-      const hpt_status s = engine->queue_primary(ids[k], jobs[k], rays[k], first[k],
-                                                 final_part[k] != 0);
-      if (s != HPT_OK) return s;
-    }
-    return engine->set_order_async(order());
+  for (size_t k = 0; k < ids.size(); ++k) {
+    const hpt_status s = engine->queue_primary(ids[k], jobs[k], rays[k], first[k],
+                                               final_part[k] != 0);
+    if (s != HPT_OK) return s;
   }
-  large_queued = 0;  // traced right now by their own launch
-  HPT_TRACE_BEGIN(admit_async);
-  const hpt_status s = engine->admit_async(ids, jobs, rays, order(), nullptr, first, final_part);
-  HPT_TRACE_END(admit_async);
-  return s;
+  return engine->set_order_async(order());
 }
 
 // Enqueues the resolve and copy-back of a request whose paths all finished.
@@ -540,7 +533,6 @@ hpt_status hpt_server_create(const hpt_server_config* config, hpt_server** out) 
     s->t0 = std::chrono::steady_clock::now();
     s->engine.reset(new Engine(config->device));
     s->engine->tuning.capacity = config->capacity;
-    s->engine->tuning.smem_nodes = 0;  // requests mix scenes
     HPT_CUDA(cudaSetDevice(config->device));
     hpt_status st = s->engine->ensure_capacity(config->capacity);
     if (st == HPT_OK) st = s->engine->ensure_slots(config->max_jobs);
@@ -840,7 +832,9 @@ std::string tune_key(const hpt_scene* scene, const hpt_render_params* p) {
     if (ch == ' ' || ch == '|') ch = '_';
   std::ostringstream k;
   const hpt_scene_info& in = scene->h.scene.info;
-  k << dev << "|tris=" << in.num_triangles << "|nodes=" << in.num_device_nodes
+  // "|bvh": the kernels that walk the hierarchy; entries timed on the tree
+  // walk's kernels (no such mark) do not describe them.
+  k << dev << "|bvh|tris=" << in.num_triangles << "|nodes=" << in.num_device_nodes
     << "|rays=" << (int64_t)p->sample_x * p->supersample_x * p->sample_y * p->supersample_y
     << "|spp=" << p->sample << "|depth=" << p->depth;
   return k.str();
@@ -925,17 +919,15 @@ extern "C" hpt_status hpt_autotune(hpt_scene* scene, const hpt_camera* camera,
     void (*apply)(hpt_tuning&, int, int);
   };
   const Knob knobs[] = {
-      {{{128, 5}, {128, 6}, {128, 7}, {128, 8}, {128, 9}, {128, 10}, {256, 2}, {256, 3}},
+      {{{128, 6}, {128, 7}, {128, 8}, {128, 9}, {128, 10}, {256, 3}, {256, 4}},
        [](hpt_tuning& t, int a, int b) {
          t.isect_block = a;
          t.isect_min_blocks = b;
        }},
-      {{{0, 0}, {16, 0}, {32, 0}, {48, 0}},
+      {{{2, 0}, {4, 0}, {8, 0}, {16, 0}},
        [](hpt_tuning& t, int a, int) { t.trav_steps = a; }},
       {{{2, 0}, {4, 0}, {8, 0}, {16, 0}},
        [](hpt_tuning& t, int a, int) { t.refill_chunk = a; }},
-      {{{0, 0}, {1024, 0}, {2048, 0}, {4096, 0}},
-       [](hpt_tuning& t, int a, int) { t.smem_nodes = a; }},
       {{{1 << 20, 0}, {1 << 21, 0}, {1 << 22, 0}, {1 << 23, 0}, {1 << 24, 0}},
        [](hpt_tuning& t, int a, int) { t.capacity = a; }},
       {{{0, 0}, {1, 0}}, [](hpt_tuning& t, int a, int) { t.use_graph = a; }},

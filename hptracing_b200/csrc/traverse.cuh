@@ -1,5 +1,9 @@
 // Closest-hit query against the rope KD-tree.
 //
+// The kernels answer most rays through the wide hierarchy (bvh.cuh), which
+// has to give this walk's result; the walk takes the rays for which that is
+// not certain.
+//
 // Result contract (src/hp/cl_src/kernel.cl:111-208): the hit is the
 // minimum-t triangle over the leaves whose reference box passes
 // _box_intersect (kernel.cl:56-83), tested with the reference's
@@ -75,8 +79,8 @@ HPT_HD bool mt_test(const Ray& r, const float4 A, const float4 E1,
   return t > 0.f;
 }
 
-// Entries of the per-ray triangle mailbox (a performance knob only: a
-// repeated triangle that misses the mailbox is simply tested again).
+// Entries of the per-ray triangle mailbox (for speed only: a repeated
+// triangle that misses the mailbox is simply tested again).
 #ifndef HPT_MAILBOX
 #define HPT_MAILBOX 1
 #endif
@@ -106,9 +110,7 @@ struct TravState {
 
 // The rest of a ray's traversal state: written when the query starts or a
 // leaf is set up, read at a leaf's exit or when a candidate would win -
-// at most a few times per leaf. The kernels keep it in shared memory
-// (eleven words per lane: an odd stride, free of bank conflicts) so that
-// the registers go to the state every unit touches.
+// at most a few times per leaf.
 struct TravCold {
   f3 inv_d;           // 1 / d (exit distances only; the filter divides)
   float t_end;        // scene exit distance
@@ -126,7 +128,6 @@ struct TravCold {
                       // 3-5: axes on which a descent met such a plane;
                       // 6-8: axes whose planes this walk passes on the right
 };
-static_assert(sizeof(TravCold) == 52, "odd word stride in shared memory");
 
 // A ray with a zero direction component whose coordinate equals a node's
 // split on that axis lies in the plane between the two children, and a
@@ -265,26 +266,6 @@ HPT_HD void trav_init(const Sc& s, const Ray& r, TravState& st, TravCold& tc,
       }
     }
   }
-}
-
-// The traversal's view of a scene (the fields trav_* read).
-HPT_HD TravScene trav_scene(const DevScene& s) {
-  TravScene t;
-  t.nodes = s.nodes;
-  t.leaves = s.leaves;
-  t.leaf_refs = s.leaf_refs;
-  t.tris = s.tris;
-  t.num_nodes = s.num_nodes;
-  t.num_leaves = s.num_leaves;
-  t.num_leaf_tris = s.num_leaf_tris;
-  t.num_triangles = s.num_triangles;
-  for (int a = 0; a < 3; ++a) {
-    t.root_lo[a] = s.root_lo[a];
-    t.root_hi[a] = s.root_hi[a];
-  }
-  t.scene_eps = s.scene_eps;
-  t.max_steps = s.max_steps;
-  return t;
 }
 
 // Node fetch with an optional shared-memory copy of the first n_smem nodes.
@@ -520,11 +501,7 @@ HPT_HD bool trav_setup(const Sc& s, TravState& st, TravCold& tc, DevErr* err, Cn
 // one with the longest triangle list; results are identical to trav_leaf's
 // (same tests in the same order, same termination).
 // A call runs one unit, except that a leaf's last triangle test falls
-// through to the leaf's exit in the same call: the exit needs no load of
-// its own (the ropes are read at set-up), so this saves a call per leaf for
-// a few instructions. Falling through from set-up to the first test as
-// well measured slower (the set-up's loads and the test's loads then
-// chain within one call).
+// through to the leaf's exit in the same call (the ropes are read at set-up).
 
 // Returns true when the ray is finished.
 // kSmem: nodes below n_smem are read from the shared-memory prefix (false:

@@ -254,8 +254,10 @@ typedef struct hpt_render_stats {
   float ms_intersect;         /* -1; ms_loop covers both)                 */
   float ms_resolve;
   float ms_loop;              /* all wavefront iterations                */
-  int64_t nodes_visited;      /* inner nodes descended, all queries      */
-  int64_t leaves_visited;
+  /* Work of all queries' walks (the hierarchy's, and the tree's for the   */
+  /* few rays that need it):                                               */
+  int64_t nodes_visited;      /* eight-child nodes (tree: inner nodes)   */
+  int64_t leaves_visited;     /* nodes with triangles to test (leaves)   */
   int64_t triangle_tests;     /* Moller-Trumbore tests run               */
   int64_t triangle_repeats;   /* leaf references skipped as already tested */
 } hpt_render_stats;
@@ -275,17 +277,16 @@ typedef struct hpt_tuning {
   int32_t capacity;          /* paths in flight (wavefront size); a run's */
                              /* queues hold at most its rays x spp paths; */
                              /* default 2^24 (208 B per path)             */
-  int32_t isect_block;       /* threads per intersect block (128 / 256)   */
+  int32_t isect_block;       /* threads per closest-hit block (128 / 256) */
   int32_t shade_block;       /* threads per shade block                   */
   int32_t refill_chunk;      /* lanes idle before a warp refills          */
-  int32_t smem_nodes;        /* top-of-tree nodes staged in shared memory */
+  int32_t smem_nodes;        /* accepted (0..8192), without effect        */
   int32_t use_graph;         /* capture the bounce loop in a CUDA graph   */
   int32_t profile;           /* time each stage with CUDA events          */
   int32_t isect_min_blocks;  /* register budget: blocks per SM to fit     */
-  int32_t trav_steps;        /* 0: one leaf per lane per round; n > 0:    */
-                             /* n traversal steps (descent step, leaf     */
-                             /* set-up, triangle test or leaf exit) per   */
-                             /* lane between refills                      */
+  int32_t trav_steps;        /* warp rounds (a node visit or a triangle   */
+                             /* test per lane) between refills; 0 = the   */
+                             /* default                                   */
   int32_t max_steps;         /* traversal steps one ray may take before   */
                              /* the walk gives up and the render returns  */
                              /* HPT_ERR_TRAVERSAL_LIMIT; 0 = the scene's  */
