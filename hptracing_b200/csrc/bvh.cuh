@@ -9,14 +9,24 @@
 //     arithmetic. The boxes are grown by what that arithmetic can be off by
 //     (build_bvh), so the tree walk, which tests some of the same triangles,
 //     finds this triangle or none as near.
-//  2. bvh_certain looks the hit up in the tree: it descends to the leaf that
-//     holds the hit point and checks that the leaf lists the triangle and
-//     that the ray runs through the leaf by more than rounding. Then the
-//     leaf passes the reference's filter, and the tree walk, whose leaves
-//     cover the ray up to its best hit, visits it: its answer is this one.
-// A ray for which part 2 fails (hits at a leaf's corner, rays in a split
-// plane) and one with two triangles at exactly the same t are walked through
-// the tree instead.
+//  2. bvh_certain shows that the tree walk tests this triangle in a leaf that
+//     passes the reference's filter; then its answer is this one.
+// A ray for which part 2 fails (mostly rays in a split plane) is walked
+// through the tree instead.
+//
+// Part 2, from the triangle alone. The reference's builder puts a
+// triangle into every leaf its bounds touch (src/hp/scene/kdtree.cpp:145-154),
+// so around a hit point inside the bounds all leaves list it, except a leaf
+// beyond a split just outside the bounds. Where no leaf that lists the
+// triangle ends so (its flags), or the hit point is not at that bound, every
+// leaf within rounding (kCertainRound) of the hit point lists the triangle:
+// the tree walk, whose leaves cover the ray up to its best hit, is in one of
+// them at the hit, and the ray runs through the leaves around it by more than
+// rounding. [A leaf near the hit that does not list it was cut off by a split
+// X beyond the bound m, m < X <= m + 3 roundings; the leaf on the split's near
+// side that holds m lists the triangle and ends in (m, X]: flagged.]
+// What this leaves open, and two triangles at exactly the same t, bvh_resolve
+// looks up in the tree.
 #pragma once
 
 #include "traverse.cuh"
@@ -53,30 +63,87 @@ HPT_HD float plane(uint32_t w) {
   return as_float_u(0x47000000u | (((w >> (8 * k)) & 255u) << 8));
 #endif
 }
+// Three-operand minimum and maximum (one instruction on sm_100).
+HPT_HD float max3(float a, float b, float c) {
+#ifdef __CUDA_ARCH__
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+#else
+  return fmaxf(a, fmaxf(b, c));
+#endif
+}
+HPT_HD float min3(float a, float b, float c) {
+#ifdef __CUDA_ARCH__
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+#else
+  return fminf(a, fminf(b, c));
+#endif
+}
+// Two fused multiply-adds in one instruction.
+struct Pair {
+#ifdef __CUDA_ARCH__
+  unsigned long long v;
+#else
+  float x, y;
+#endif
+};
+HPT_HD Pair pair(float x, float y) {
+#ifdef __CUDA_ARCH__
+  Pair p;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(p.v) : "f"(x), "f"(y));
+  return p;
+#else
+  return Pair{x, y};
+#endif
+}
+HPT_HD void unpair(const Pair& p, float& x, float& y) {
+#ifdef __CUDA_ARCH__
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(p.v));
+#else
+  x = p.x;
+  y = p.y;
+#endif
+}
+HPT_HD Pair fma2(const Pair& a, const Pair& b, const Pair& c) {
+#ifdef __CUDA_ARCH__
+  Pair r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+#else
+  return Pair{fma_rn(a.x, b.x, c.x), fma_rn(a.y, b.y, c.y)};
+#endif
+}
 
 // Walk state of one ray.
 struct BvhRay {
   Ray ray;
   f3 inv;            // 1 / d
   float cull;        // boxes that start beyond it are skipped
-  float slack;       // rounding slack in t units
   float best_t;      // nearest accepted t, +inf = none
   uint32_t best;     // its record in btris, kBvhNone = none; | kBvhTie when
-                     // another triangle was accepted at exactly best_t
-  uint32_t oct;      // bit a: the ray runs toward +a (slot order)
-  uint32_t node_base, node_bits;  // pending children: base, imask << 8 | hits
+                     // another triangle was accepted at exactly best_t,
+                     // | kBvhMany when more than one was
+  uint32_t node_base, node_bits;  // pending children: base; bits 0-7 = slots in
+                                  // visiting order, 8-15 = imask, 16-18 =
+                                  // octant (bit a: the ray runs toward +a)
   uint32_t tri_base, tri_bits;    // pending triangles
-  int32_t sp;        // entries on the stack
+  uint32_t steps;    // bits 0-4 = stack entries, the rest counts node visits
+                     // and triangle tests
 };
-constexpr uint32_t kBvhNone = 0x3FFFFFFFu, kBvhTie = 0x40000000u;
+constexpr uint32_t kBvhStep = 32u;
+static_assert(kBvhStack == 32, "stack entries fit bits 0-4");
+constexpr uint32_t kBvhNone = 0x3FFFFFFFu, kBvhTie = 0x40000000u, kBvhMany = 0x80000000u;
 
 // Starts a walk. Returns false when the ray is to be walked through the tree
 // instead (non-finite rays, directions of extreme length).
-HPT_HD bool bvh_init(float scene_eps, const Ray& r, BvhRay& b) {
+HPT_HD bool bvh_init(const Ray& r, BvhRay& b) {
   b.ray = r;
   b.best = kBvhNone;
   b.best_t = b.cull = as_float(0x7f800000);
-  b.sp = 0;
+  b.steps = 0;
   b.tri_bits = 0;
   b.tri_base = 0;
   const float dmax = fmaxf(fabsf(r.d.x), fmaxf(fabsf(r.d.y), fabsf(r.d.z)));
@@ -89,21 +156,24 @@ HPT_HD bool bvh_init(float scene_eps, const Ray& r, BvhRay& b) {
   b.inv.y = fabsf(r.d.y) > tiny ? rn_rcp(r.d.y) : copysignf(big, r.d.y);
   b.inv.z = fabsf(r.d.z) > tiny ? rn_rcp(r.d.z) : copysignf(big, r.d.z);
   // The root as the only pending child (slot 0).
-  b.oct = (b.inv.x > 0.f ? 1u : 0u) | (b.inv.y > 0.f ? 2u : 0u) | (b.inv.z > 0.f ? 4u : 0u);
+  const uint32_t oct =
+      (b.inv.x > 0.f ? 1u : 0u) | (b.inv.y > 0.f ? 2u : 0u) | (b.inv.z > 0.f ? 4u : 0u);
   b.node_base = 0;
-  b.node_bits = (1u << 8) | (1u << b.oct);
-  b.slack = rn_div(scene_eps, dmax);
+  b.node_bits = (oct << 16) | (1u << 8) | (1u << oct);
   return finite3(r.o) && finite3(r.d) && dmax > 1e-15f && dmax < 1e15f;
 }
 
-// The slots of a node whose boxes the ray enters before b.cull.
+// Bit k, when the ray enters the box of slot k before cull: the planes of
+// four slots are the bytes of near / far words.
 template <int k>
 HPT_HD uint32_t bvh_slot(uint32_t nx, uint32_t ny, uint32_t nz, uint32_t fx, uint32_t fy,
-                         uint32_t fz, const f3& S, const f3& O, float cull) {
-  const float t0 = fmaxf(fmaxf(fma_rn(plane<k & 3>(nx), S.x, O.x), fma_rn(plane<k & 3>(ny), S.y, O.y)),
-                         fmaxf(fma_rn(plane<k & 3>(nz), S.z, O.z), 0.f));
-  const float t1 = fminf(fminf(fma_rn(plane<k & 3>(fx), S.x, O.x), fma_rn(plane<k & 3>(fy), S.y, O.y)),
-                         fminf(fma_rn(plane<k & 3>(fz), S.z, O.z), cull));
+                         uint32_t fz, const Pair& Sxy, const Pair& Oxy, const Pair& Szz,
+                         const Pair& Ozz, float cull) {
+  float x0, y0, z0, x1, y1, z1;
+  unpair(fma2(pair(plane<k & 3>(nx), plane<k & 3>(ny)), Sxy, Oxy), x0, y0);
+  unpair(fma2(pair(plane<k & 3>(fx), plane<k & 3>(fy)), Sxy, Oxy), x1, y1);
+  unpair(fma2(pair(plane<k & 3>(nz), plane<k & 3>(fz)), Szz, Ozz), z0, z1);
+  const float t0 = fmaxf(max3(x0, y0, z0), 0.f), t1 = fminf(min3(x1, y1, z1), cull);
   return t0 <= t1 ? 1u << k : 0u;
 }
 
@@ -118,35 +188,38 @@ HPT_HD void bvh_node(BvhRay& b, const uint4& n0, const uint4& n1, const uint4& n
   O.x = fma_rn(-32768.f, S.x, rn_mul(rn_sub(as_float_u(n0.x), b.ray.o.x), b.inv.x));
   O.y = fma_rn(-32768.f, S.y, rn_mul(rn_sub(as_float_u(n0.y), b.ray.o.y), b.inv.y));
   O.z = fma_rn(-32768.f, S.z, rn_mul(rn_sub(as_float_u(n0.z), b.ray.o.z), b.inv.z));
-  const bool px = b.oct & 1u, py = b.oct & 2u, pz = b.oct & 4u;
+  const Pair Sxy = pair(S.x, S.y), Oxy = pair(O.x, O.y);
+  const Pair Szz = pair(S.z, S.z), Ozz = pair(O.z, O.z);
+  const uint32_t oct = b.node_bits >> 16;
+  const bool px = oct & 1u, py = oct & 2u, pz = oct & 4u;
   uint32_t h = 0;
   // Words: n2 = lo x (2), lo y (2); n3 = lo z, hi x; n4 = hi y, hi z.
   {
     const uint32_t nx = px ? n2.x : n3.z, fx = px ? n3.z : n2.x;
     const uint32_t ny = py ? n2.z : n4.x, fy = py ? n4.x : n2.z;
     const uint32_t nz = pz ? n3.x : n4.z, fz = pz ? n4.z : n3.x;
-    h |= bvh_slot<0>(nx, ny, nz, fx, fy, fz, S, O, b.cull);
-    h |= bvh_slot<1>(nx, ny, nz, fx, fy, fz, S, O, b.cull);
-    h |= bvh_slot<2>(nx, ny, nz, fx, fy, fz, S, O, b.cull);
-    h |= bvh_slot<3>(nx, ny, nz, fx, fy, fz, S, O, b.cull);
+    h |= bvh_slot<0>(nx, ny, nz, fx, fy, fz, Sxy, Oxy, Szz, Ozz, b.cull);
+    h |= bvh_slot<1>(nx, ny, nz, fx, fy, fz, Sxy, Oxy, Szz, Ozz, b.cull);
+    h |= bvh_slot<2>(nx, ny, nz, fx, fy, fz, Sxy, Oxy, Szz, Ozz, b.cull);
+    h |= bvh_slot<3>(nx, ny, nz, fx, fy, fz, Sxy, Oxy, Szz, Ozz, b.cull);
   }
   {
     const uint32_t nx = px ? n2.y : n3.w, fx = px ? n3.w : n2.y;
     const uint32_t ny = py ? n2.w : n4.y, fy = py ? n4.y : n2.w;
     const uint32_t nz = pz ? n3.y : n4.w, fz = pz ? n4.w : n3.y;
-    h |= bvh_slot<4>(nx, ny, nz, fx, fy, fz, S, O, b.cull);
-    h |= bvh_slot<5>(nx, ny, nz, fx, fy, fz, S, O, b.cull);
-    h |= bvh_slot<6>(nx, ny, nz, fx, fy, fz, S, O, b.cull);
-    h |= bvh_slot<7>(nx, ny, nz, fx, fy, fz, S, O, b.cull);
+    h |= bvh_slot<4>(nx, ny, nz, fx, fy, fz, Sxy, Oxy, Szz, Ozz, b.cull);
+    h |= bvh_slot<5>(nx, ny, nz, fx, fy, fz, Sxy, Oxy, Szz, Ozz, b.cull);
+    h |= bvh_slot<6>(nx, ny, nz, fx, fy, fz, Sxy, Oxy, Szz, Ozz, b.cull);
+    h |= bvh_slot<7>(nx, ny, nz, fx, fy, fz, Sxy, Oxy, Szz, Ozz, b.cull);
   }
   const uint32_t imask = e >> 24;
   uint32_t inner = h & imask;
   // Hits by visiting order: slot s goes to bit s ^ oct, the highest first.
-  if (b.oct & 1u) inner = ((inner & 0x55u) << 1) | ((inner >> 1) & 0x55u);
-  if (b.oct & 2u) inner = ((inner & 0x33u) << 2) | ((inner >> 2) & 0x33u);
-  if (b.oct & 4u) inner = ((inner & 0x0Fu) << 4) | (inner >> 4);
+  if (px) inner = ((inner & 0x55u) << 1) | ((inner >> 1) & 0x55u);
+  if (py) inner = ((inner & 0x33u) << 2) | ((inner >> 2) & 0x33u);
+  if (pz) inner = ((inner & 0x0Fu) << 4) | (inner >> 4);
   b.node_base = n1.x;
-  b.node_bits = (imask << 8) | inner;
+  b.node_bits = (oct << 16) | (imask << 8) | inner;
   b.tri_base = n1.y;
   uint32_t tri = 0;
   for (uint32_t l = h & ~imask; l; l &= l - 1) {
@@ -162,132 +235,282 @@ HPT_HD void bvh_node(BvhRay& b, const uint4& n0, const uint4& n1, const uint4& n
 HPT_HD bool bvh_visit(const BvhNode* bvh, uint32_t num_bvh, BvhRay& b, uint2* stack,
                       DevErr* err) {
   if (!(b.node_bits & 255u)) {
-    if (b.sp == 0) return false;
-    const uint2 e = stack[--b.sp];
+    if ((b.steps & 31u) == 0) return false;
+    --b.steps;
+    const uint2 e = stack[b.steps & 31u];
     b.node_base = e.x;
     b.node_bits = e.y;
   }
   const int bit = high_bit(b.node_bits & 255u);
-  const uint32_t slot = (uint32_t)bit ^ b.oct;
+  const uint32_t slot = (uint32_t)bit ^ (b.node_bits >> 16);
   const uint32_t node = b.node_base + popc((b.node_bits >> 8) & ((1u << slot) - 1u));
   b.node_bits &= ~(1u << bit);
   if (b.node_bits & 255u) {
-    HPT_DCHECK(err, b.sp < kBvhStack, 113, b.sp, return false);
-    stack[b.sp].x = b.node_base;
-    stack[b.sp].y = b.node_bits;
-    ++b.sp;
+    HPT_DCHECK(err, (b.steps & 31u) < kBvhStack - 1, 113, b.steps, return false);
+    stack[b.steps & 31u].x = b.node_base;
+    stack[b.steps & 31u].y = b.node_bits;
+    ++b.steps;
   }
   HPT_DCHECK(err, node < num_bvh, 114, node, return false);
   const uint4* n = reinterpret_cast<const uint4*>(bvh + node);
   bvh_node(b, ldg(n), ldg(n + 1), ldg(n + 2), ldg(n + 3), ldg(n + 4));
+  b.steps += kBvhStep;
   return true;
 }
 
 // One triangle test of the pending ones. A winning hit shrinks the cull
 // distance to the tree walk's own stopping rule (best t plus slack).
-HPT_HD void bvh_test(const BvhTri* btris, BvhRay& b) {
+// tie receives the other triangle's record where best gets kBvhTie.
+HPT_HD void bvh_test(const BvhTri* btris, float scene_eps, BvhRay& b, uint32_t& tie) {
   const int k = high_bit(b.tri_bits);
   b.tri_bits &= ~(1u << k);
   const int32_t i = (int32_t)b.tri_base + k;
   const float4* rec = reinterpret_cast<const float4*>(btris + i);
+  b.steps += kBvhStep;
   float t, u, v;
   if (mt_test(b.ray, ldg(rec), ldg(rec + 1), ldg(rec + 2), t, u, v)) {
     if (t < b.best_t) {
       b.best_t = t;
       b.best = (uint32_t)i;
-      b.cull = fma_rn(t, 1.0001f, b.slack);
+      const float per_unit =
+          fminf(fabsf(b.inv.x), fminf(fabsf(b.inv.y), fabsf(b.inv.z)));  // 1 / largest |d|
+      b.cull = fma_rn(t, 1.0001f, rn_mul(scene_eps, per_unit));
     } else if (t == b.best_t) {
-      b.best |= kBvhTie;
+      b.best |= b.best & kBvhTie ? kBvhMany : kBvhTie;
+      tie = (uint32_t)i;
     }
   }
+}
+
+// A ray that meets nothing misses - unless it runs exactly along a triangle's
+// edge e2: then the Moller-Trumbore test divides by zero, its comparisons
+// pass 0 / 0, and the reference "hits" the triangle at t = +inf when there is
+// no other hit. d x e2 is exactly zero only if e2 has d's zero components and
+// the same direction beside them within two roundings. True when the scene
+// has no such edge for a d with one zero component (for one without any such
+// an edge would have to be met by chance; along an axis edges are common).
+template <class Sc>
+HPT_HD bool bvh_no_parallel_edge(const Sc& s, const f3& d) {
+  const int zeros = (d.x == 0.f) + (d.y == 0.f) + (d.z == 0.f);
+  if (zeros != 1) return false;
+  const int a = d.x == 0.f ? 0 : (d.y == 0.f ? 1 : 2);
+  const float b = a == 0 ? d.y : (a == 1 ? d.z : d.x), c = a == 0 ? d.z : (a == 1 ? d.x : d.y);
+  const float key = rn_div(b > 0.f ? c : -c, rn_add(fabsf(b), fabsf(c)));  // edge_key
+  const float* keys = a == 0 ? s.edge_keys[0] : (a == 1 ? s.edge_keys[1] : s.edge_keys[2]);
+  int lo = 0, hi = a == 0 ? s.num_edge_keys[0] : (a == 1 ? s.num_edge_keys[1] : s.num_edge_keys[2]);
+  const int n = hi;
+  // (Near +-1, where the keys of one line wrap around: as if there were one.)
+  if (fabsf(key) > 1.f - 4e-7f) return false;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (ldg(keys + mid) < key - 4e-7f) lo = mid + 1;
+    else hi = mid;
+  }
+  return lo == n || ldg(keys + lo) > key + 4e-7f;
 }
 
 // True when the tree walk's answer for ray r is (best, best_t), the result
-// of its hierarchy walk (see the file comment); kBvhNone without kBvhTie: a
-// miss.
+// of its hierarchy walk (see the file comment); kBvhNone alone: a miss.
 template <class Sc>
 HPT_HD bool bvh_certain(const Sc& s, const Ray& r, uint32_t best, float best_t, DevErr* err) {
-  if (best & kBvhTie) return false;
-  // Nothing accepted: a miss. Along a zero component a triangle with an edge
-  // parallel to the ray can be "hit" at t = +inf (0 / 0 passes the tests),
-  // which the reference reports when there is no other hit.
-  if (best == kBvhNone) return r.d.x != 0.f && r.d.y != 0.f && r.d.z != 0.f;
+  if (best & (kBvhTie | kBvhMany)) return false;
+  const bool axes = r.d.x != 0.f && r.d.y != 0.f && r.d.z != 0.f;
+  if (best == kBvhNone) return axes || bvh_no_parallel_edge(s, r.d);
   HPT_DCHECK(err, best < (uint32_t)s.num_btris, 115, best, return false);
   const float4* rec = reinterpret_cast<const float4*>(s.btris + best);
-  const int32_t id = as_int(ldg(rec).w);
-  int node = as_int(ldg(rec + 1).w);
-  const float px = rn_add(r.o.x, rn_mul(best_t, r.d.x));
-  const float py = rn_add(r.o.y, rn_mul(best_t, r.d.y));
-  const float pz = rn_add(r.o.z, rn_mul(best_t, r.d.z));
-  uint2 nd;
-  while (true) {
-    HPT_DCHECK(err, node >= 0 && node < s.num_nodes, 110, node, return false);
-    nd = ldg(reinterpret_cast<const uint2*>(s.nodes) + node);
-    const uint32_t axis = nd.x >> 30;
-    if (axis == kLeafKind) break;
-    const float split = as_float_u(nd.y);
-    const float p = axis == 0 ? px : (axis == 1 ? py : pz);
-    const float dd = axis == 0 ? r.d.x : (axis == 1 ? r.d.y : r.d.z);
-    // In a split plane of a zero component the tree walk takes both sides.
-    if (p == split && dd == 0.f) return false;
-    node = (int)(nd.x & kIndexMask) + (p > split || (p == split && dd > 0.f) ? 1 : 0);
-  }
-  HPT_DCHECK(err, (int)(nd.x & kIndexMask) < s.num_leaves, 111, nd.x & kIndexMask, return false);
-  const float4* L = reinterpret_cast<const float4*>(s.leaves + (nd.x & kIndexMask));
-  const float4 lo = ldg(L), hi = ldg(L + 1);
-  // Along a zero component the reference's filter wants the origin strictly
-  // between the leaf's faces (0 / 0 on a face).
-  if ((r.d.x == 0.f && !(r.o.x > lo.x && r.o.x < hi.x)) ||
-      (r.d.y == 0.f && !(r.o.y > lo.y && r.o.y < hi.y)) ||
-      (r.d.z == 0.f && !(r.o.z > lo.z && r.o.z < hi.z)))
-    return false;
-  // The ray's interval in the leaf, against rounding: 2e-6 of the scene's
-  // size and 1e-6 of the distance (a face's distance is off by a few 1e-7).
-  float t0 = 0.f, t1 = as_float(0x7f800000);
-  const float o[3] = {r.o.x, r.o.y, r.o.z}, d[3] = {r.d.x, r.d.y, r.d.z};
-  const float l[3] = {lo.x, lo.y, lo.z}, h[3] = {hi.x, hi.y, hi.z};
+  const float4 A = ldg(rec), E1 = ldg(rec + 1), E2 = ldg(rec + 2);
+  const uint32_t flags = (uint32_t)as_int(E2.w);
+  const float p[3] = {rn_add(r.o.x, rn_mul(best_t, r.d.x)), rn_add(r.o.y, rn_mul(best_t, r.d.y)),
+                      rn_add(r.o.z, rn_mul(best_t, r.d.z))};
+  if (axes && !(flags & kTriIrregular)) {
+    const float a[3] = {A.x, A.y, A.z}, e1[3] = {E1.x, E1.y, E1.z}, e2[3] = {E2.x, E2.y, E2.z};
+    const float round = rn_mul(kCertainRound, s.scene_eps);
+    bool ok = true;
 #pragma unroll
-  for (int a = 0; a < 3; ++a)
-    if (d[a] != 0.f) {
-      const float inv = rn_rcp(d[a]);
-      const float x0 = rn_mul(rn_sub(l[a], o[a]), inv), x1 = rn_mul(rn_sub(h[a], o[a]), inv);
-      t0 = fmaxf(t0, fminf(x0, x1));
-      t1 = fminf(t1, fmaxf(x0, x1));
+    for (int k = 0; k < 3; ++k) {
+      const float v1 = rn_add(a[k], e1[k]), v2 = rn_add(a[k], e2[k]);
+      const float lo = fminf(a[k], fminf(v1, v2)), hi = fmaxf(a[k], fmaxf(v1, v2));
+      ok = ok && p[k] > rn_add(lo, flags & (1u << (2 * k)) ? round : -2.f * round) &&
+           p[k] < rn_sub(hi, flags & (2u << (2 * k)) ? round : -2.f * round);
     }
-  const float dmax = fmaxf(fabsf(r.d.x), fmaxf(fabsf(r.d.y), fabsf(r.d.z)));
-  const float tol = fma_rn(best_t, 1e-6f, rn_mul(0.1f, rn_div(s.scene_eps, dmax)));
-  if (!(rn_sub(t1, t0) > tol) || !(best_t > rn_sub(t0, tol)) || !(best_t < rn_add(t1, tol)))
-    return false;
-  const int begin = as_int(lo.w), count = as_int(hi.w);
-  HPT_DCHECK(err, begin >= 0 && count >= 0 && (long long)begin + count <= s.num_leaf_tris, 112,
-             begin, return false);
-  for (int k = 0; k < count; ++k)
-    if (ldg(s.leaf_refs + begin + k) == id) return true;
+    if (ok) return true;
+  }
   return false;
 }
 
+// Looks up a hit in the tree that bvh_certain leaves open: goes through the
+// leaves that list the triangle - of two at the same t, both - along the ray.
+// Returns the record the tree walk would report, or kBvhNone when that is not
+// certain either (a leaf the ray crosses by no more than rounding, or at the
+// walk's end; a ray in a split plane; more than two at one t).
+// Of two triangles at one t the reference keeps the one it meets first, the
+// lowest position in the leaf lists over the leaves that count for either.
+template <class Sc>
+HPT_HD uint32_t bvh_resolve(const Sc& s, const Ray& r, uint32_t best, uint32_t tie, float best_t,
+                            DevErr* err) {
+  const bool two = best & kBvhTie;
+  const uint32_t first = best & kBvhNone;
+  if ((best & kBvhMany) || first == kBvhNone) return kBvhNone;
+  const float o[3] = {r.o.x, r.o.y, r.o.z};
+  // 1 / d; zero stands for a zero component.
+  const float inv[3] = {r.d.x != 0.f ? rn_rcp(r.d.x) : 0.f, r.d.y != 0.f ? rn_rcp(r.d.y) : 0.f,
+                        r.d.z != 0.f ? rn_rcp(r.d.z) : 0.f};
+  const float dmax = fmaxf(fabsf(r.d.x), fmaxf(fabsf(r.d.y), fabsf(r.d.z)));
+  const float slack = rn_div(s.scene_eps, dmax);
+  // A face's distance is off by a few 1e-7 of the scene's size and of itself.
+  const float tol = fma_rn(best_t, 1e-6f, rn_mul(0.1f, slack));
+  // The walk goes on to best_t x 1.0001 + slack.
+  const float last = fma_rn(best_t, 1.0001f, rn_mul(1.5f, slack));
+  // The bounds of the triangle, or of both, and the tree node that holds all
+  // their leaves.
+  float lo[3], hi[3];
+  int32_t id[2] = {-1, -1};
+  int node = 0;
+  for (int k = 0; k < (two ? 2 : 1); ++k) {
+    const uint32_t cand = k ? tie : first;
+    HPT_DCHECK(err, cand < (uint32_t)s.num_btris, 116, cand, return kBvhNone);
+    const float4* rec = reinterpret_cast<const float4*>(s.btris + cand);
+    const float4 A = ldg(rec), E1 = ldg(rec + 1), E2 = ldg(rec + 2);
+    if ((uint32_t)as_int(E2.w) & kTriIrregular) return kBvhNone;
+    id[k] = as_int(A.w);
+    if (!two) node = as_int(E1.w);
+    const float grow = rn_mul(0.1f, s.scene_eps);
+    const float v0[3] = {A.x, A.y, A.z}, e1[3] = {E1.x, E1.y, E1.z}, e2[3] = {E2.x, E2.y, E2.z};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const float v1 = rn_add(v0[a], e1[a]), v2 = rn_add(v0[a], e2[a]);
+      const float l = rn_sub(fminf(v0[a], fminf(v1, v2)), grow);
+      const float h = rn_add(fmaxf(v0[a], fmaxf(v1, v2)), grow);
+      lo[a] = k ? fminf(lo[a], l) : l;
+      hi[a] = k ? fmaxf(hi[a], h) : h;
+    }
+  }
+  // Depth-first over the nodes that the bounds and the ray (up to `last`)
+  // touch.
+  constexpr int kDepth = 64;
+  int node_stack[kDepth];
+  float t0_stack[kDepth], t1_stack[kDepth];
+  int sp = 0, rank = 0x7FFFFFFF;
+  uint32_t winner = kBvhNone;
+  bool reached = false;  // a leaf that counts and begins before the hit
+  float t0 = 0.f, t1 = last;
+  while (true) {
+    HPT_DCHECK(err, node >= 0 && node < s.num_nodes, 110, node, return kBvhNone);
+    const uint2 nd = ldg(reinterpret_cast<const uint2*>(s.nodes) + node);
+    const uint32_t axis = nd.x >> 30;
+    if (axis != kLeafKind) {
+      const float split = as_float_u(nd.y);
+      const float iv = axis == 0 ? inv[0] : (axis == 1 ? inv[1] : inv[2]);
+      const float oa = axis == 0 ? o[0] : (axis == 1 ? o[1] : o[2]);
+      const float la = axis == 0 ? lo[0] : (axis == 1 ? lo[1] : lo[2]);
+      const float ha = axis == 0 ? hi[0] : (axis == 1 ? hi[1] : hi[2]);
+      // Along a zero component the ray stays on the origin's side (in the
+      // split plane itself the tree walk takes both).
+      if (iv == 0.f && oa == split) return kBvhNone;
+      const bool up = iv > 0.f || (iv == 0.f && oa < split);
+      const float ts = iv == 0.f ? as_float(0x7f800000) : rn_mul(rn_sub(split, oa), iv);
+      // The side the ray is on before the split, and the one after it.
+      const bool before = (up ? la <= split : ha >= split) && t0 <= rn_add(ts, tol);
+      const bool after = (up ? ha >= split : la <= split) && t1 >= rn_sub(ts, tol);
+      const int child = (int)(nd.x & kIndexMask);
+      const int near = child + (up ? 0 : 1), far = child + (up ? 1 : 0);
+      if (before && after) {
+        if (sp >= kDepth) return kBvhNone;
+        node_stack[sp] = far;
+        t0_stack[sp] = fmaxf(t0, rn_sub(ts, tol));
+        t1_stack[sp] = t1;
+        ++sp;
+      }
+      if (before) {
+        node = near;
+        t1 = fminf(t1, rn_add(ts, tol));
+        continue;
+      }
+      if (after) {
+        node = far;
+        t0 = fmaxf(t0, rn_sub(ts, tol));
+        continue;
+      }
+    } else {
+      HPT_DCHECK(err, (int)(nd.x & kIndexMask) < s.num_leaves, 111, nd.x & kIndexMask,
+                 return kBvhNone);
+      const float4* L = reinterpret_cast<const float4*>(s.leaves + (nd.x & kIndexMask));
+      const float4 bl = ldg(L), bh = ldg(L + 1);
+      const int begin = as_int(bl.w), count = as_int(bh.w);
+      HPT_DCHECK(err, begin >= 0 && count >= 0 && (long long)begin + count <= s.num_leaf_tris,
+                 112, begin, return kBvhNone);
+      int at = -1;  // the first entry of either
+      uint32_t which = first;
+      for (int k = count - 1; k >= 0; --k) {
+        const int32_t entry = ldg(s.leaf_refs + begin + k);
+        if (entry == id[0] || entry == id[1]) {
+          at = begin + k;
+          which = entry == id[0] ? first : tie;
+        }
+      }
+      if (at >= 0) {
+        const float l[3] = {bl.x, bl.y, bl.z}, h[3] = {bh.x, bh.y, bh.z};
+        float f0 = -as_float(0x7f800000), f1 = as_float(0x7f800000);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          if (inv[a] == 0.f) {
+            // The filter rejects a leaf beside the origin, and on its face.
+            if (!(o[a] > l[a] && o[a] < h[a])) f1 = -as_float(0x7f800000);
+            if (o[a] == l[a] || o[a] == h[a]) return kBvhNone;
+            continue;
+          }
+          const float x0 = rn_mul(rn_sub(l[a], o[a]), inv[a]);
+          const float x1 = rn_mul(rn_sub(h[a], o[a]), inv[a]);
+          f0 = fmaxf(f0, fminf(x0, x1));
+          f1 = fminf(f1, fmaxf(x0, x1));
+        }
+        const float length = rn_sub(f1, fmaxf(f0, 0.f));
+        if (length > tol && f0 < fma_rn(0.5f, slack, best_t)) {
+          // The ray crosses the leaf and the walk comes to it.
+          if (at < rank) {
+            rank = at;
+            winner = which;
+          }
+          reached = reached || f0 < best_t;
+          if (!two && reached) return winner;
+        } else if (two && length >= -tol && f0 <= last) {
+          return kBvhNone;  // it may count or not
+        }
+      }
+    }
+    if (sp == 0) break;
+    --sp;
+    node = node_stack[sp];
+    t0 = t0_stack[sp];
+    t1 = t1_stack[sp];
+  }
+  return reached ? winner : kBvhNone;
+}
+
 // The whole query of one ray; the tree walk's answer (t and triangle id).
-// The nodes, leaf groups and tests of both walks are added to cnt.
+// The work of both walks is added to cnt (leaves: the tree walk's).
 template <class Sc>
 HPT_HD void bvh_query(const Sc& s, const Ray& r, int32_t& tri, float& t, DevErr* err,
                       TravCount& cnt, int* how = nullptr) {
   BvhRay b;
-  bool ok = bvh_init(s.scene_eps, r, b);
-  int steps = 0;
+  bool ok = bvh_init(r, b);
   if (ok) {
     uint2 stack[kBvhStack];
+    uint32_t tie = 0;
     while (true) {
-      for (; b.tri_bits; ++cnt.tris, ++steps) bvh_test(s.btris, b);
-      if (steps > s.max_steps) {
+      for (; b.tri_bits; ++cnt.tris) bvh_test(s.btris, s.scene_eps, b, tie);
+      if (b.steps / kBvhStep > (uint32_t)s.max_steps) {
         hpt_atomic_or(&err->flags, 1u);
         break;
       }
       if (!bvh_visit(s.bvh, (uint32_t)s.num_bvh, b, stack, err)) break;
       ++cnt.nodes;
-      ++steps;
-      if (b.tri_bits) ++cnt.leaves;
     }
     ok = bvh_certain(s, r, b.best, b.best_t, err);
+    if (!ok) {
+      b.best = bvh_resolve(s, r, b.best, tie, b.best_t, err);
+      ok = b.best != kBvhNone;
+    }
   }
   if (how) *how = ok;
   if (ok) {

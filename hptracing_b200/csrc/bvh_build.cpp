@@ -257,6 +257,7 @@ struct Collapser {
   const std::vector<Node2>& in;
   const std::vector<Prim>& prims;
   const PackedScene& scene;
+  const std::vector<uint8_t>& flags;
   PackedBvh& out;
 
   struct Item {
@@ -364,6 +365,7 @@ struct Collapser {
       r.e2[a] = t.e2[a];
     }
     r.tri_id = id;
+    r.flags = flags[(size_t)id];
     return r;
   }
 
@@ -403,23 +405,98 @@ struct Collapser {
 
 }  // namespace
 
-void build_bvh(const PackedScene& scene, float scene_eps, int num_threads, PackedBvh& out) {
+namespace {
+
+// Leaves whose closed box the closed box b touches.
+int64_t touched_leaves(const PackedScene& scene, const Box& b, std::vector<uint32_t>& stack) {
+  int64_t count = 0;
+  stack.assign(1, 0u);
+  while (!stack.empty()) {
+    const DevNode& d = scene.nodes[stack.back()];
+    stack.pop_back();
+    const uint32_t axis = d.meta >> 30, child = d.meta & kIndexMask;
+    if (axis == kLeafKind) {
+      ++count;
+      continue;
+    }
+    if (b.lo[axis] <= d.split) stack.push_back(child);
+    if (b.hi[axis] >= d.split) stack.push_back(child + 1);
+  }
+  return count;
+}
+
+}  // namespace
+
+void build_bvh(const float* points, const int32_t* triangles, const PackedScene& scene,
+               float scene_eps, int num_threads, PackedBvh& out) {
   const size_t n = scene.tris.size();
   // A small scene builds in less than it takes to start a thread.
   const int threads = n <= 8192 ? 1
                       : num_threads > 0
                           ? num_threads
                           : (int)std::max(1u, std::thread::hardware_concurrency());
-  std::vector<Box> boxes(n);
-  for (Box& b : boxes) b.reset();
+  // Per triangle: its bounds, the union of the leaves that list it, how many
+  // do, and its flags.
+  std::vector<Box> bounds(n), boxes(n);
+  std::vector<int32_t> listed(n, 0);
+  std::vector<uint8_t> flags(n, 0);
+  for (size_t i = 0; i < n; ++i) {
+    boxes[i].reset();
+    bounds[i].reset();
+    for (int k = 0; k < 3; ++k) {
+      const float* v = points + 4 * (size_t)triangles[4 * i + k];
+      for (int a = 0; a < 3; ++a) {
+        bounds[i].lo[a] = std::min(bounds[i].lo[a], v[a]);
+        bounds[i].hi[a] = std::max(bounds[i].hi[a], v[a]);
+      }
+    }
+  }
+  const float near = kCertainNear * scene_eps;
   for (const DevLeaf& L : scene.leaves) {
     Box b;
     for (int a = 0; a < 3; ++a) {
       b.lo[a] = L.lo[a];
       b.hi[a] = L.hi[a];
     }
-    for (int32_t k = 0; k < L.tri_count; ++k)
-      boxes[(size_t)scene.refs[(size_t)L.tri_begin + k]].add(b);
+    for (int32_t k = 0; k < L.tri_count; ++k) {
+      const size_t id = (size_t)scene.refs[(size_t)L.tri_begin + k];
+      boxes[id].add(b);
+      ++listed[id];
+      const Box& t = bounds[id];
+      uint32_t f = 0;
+      for (int a = 0; a < 3; ++a) {
+        const float below = t.lo[a] - b.lo[a], above = b.hi[a] - t.hi[a];
+        if (below > 0.f && below < near) f |= 1u << (2 * a);
+        if (above > 0.f && above < near) f |= 2u << (2 * a);
+        if (b.lo[a] > t.hi[a] || b.hi[a] < t.lo[a]) f |= kTriIrregular;
+      }
+      flags[id] |= (uint8_t)f;
+    }
+  }
+  {
+    std::atomic<size_t> cursor{0};
+    run_threads(threads, [&] {
+      std::vector<uint32_t> stack;
+      for (size_t i = cursor.fetch_add(1024); i < n; i = cursor.fetch_add(1024))
+        for (size_t k = i; k < std::min(n, i + 1024); ++k)
+          if (listed[k] != touched_leaves(scene, bounds[k], stack))
+            flags[k] |= (uint8_t)kTriIrregular;
+    });
+  }
+  {
+    std::atomic<int> axis{0};
+    run_threads(std::min(threads, 3), [&] {
+      for (int a = axis++; a < 3; a = axis++) {
+        std::vector<float>& keys = out.edge_keys[a];
+        keys.clear();
+        for (const DevTri& t : scene.tris) {
+          const float b = t.e2[(a + 1) % 3], c = t.e2[(a + 2) % 3];
+          if (t.e2[a] == 0.f && (b != 0.f || c != 0.f)) keys.push_back(edge_key(b, c));
+        }
+        std::sort(keys.begin(), keys.end());
+        keys.erase(std::unique(keys.begin(), keys.end()), keys.end());
+      }
+    });
   }
   const float pad = 0.1f * scene_eps;
   std::vector<Prim> prims;
@@ -434,14 +511,9 @@ void build_bvh(const PackedScene& scene, float scene_eps, int num_threads, Packe
     const float ny = t.e1[2] * t.e2[0] - t.e1[0] * t.e2[2];
     const float nz = t.e1[0] * t.e2[1] - t.e1[1] * t.e2[0];
     const float n[3] = {nx, ny, nz}, nn = nx * nx + ny * ny + nz * nz;
-    Box tb;
+    const Box& tb = bounds[i];
     float extent = 0.f;
-    for (int a = 0; a < 3; ++a) {
-      const float v[3] = {t.a[a], t.a[a] + t.e1[a], t.a[a] + t.e2[a]};
-      tb.lo[a] = std::min(v[0], std::min(v[1], v[2]));
-      tb.hi[a] = std::max(v[0], std::max(v[1], v[2]));
-      extent = std::max(extent, tb.hi[a] - tb.lo[a]);
-    }
+    for (int a = 0; a < 3; ++a) extent = std::max(extent, tb.hi[a] - tb.lo[a]);
     for (int a = 0; a < 3; ++a) {
       const float in_plane = nn > 0.f ? std::sqrt(std::max(0.f, 1.f - n[a] * n[a] / nn)) : 1.f;
       p.b.lo[a] = std::max(p.b.lo[a], tb.lo[a] - kPlaneGrowth * extent * in_plane);
@@ -463,7 +535,7 @@ void build_bvh(const PackedScene& scene, float scene_eps, int num_threads, Packe
     }
     Builder2 b2(prims, median);
     b2.run(threads);
-    Collapser c{b2.nodes, prims, scene, out};
+    Collapser c{b2.nodes, prims, scene, flags, out};
     c.run();
     if (out.max_depth < kBvhStack - 1) break;
   }

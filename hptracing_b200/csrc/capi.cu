@@ -405,10 +405,16 @@ hpt_status upload_scene(const hpt_scene_desc& d, SceneDev& out) {
                       pk.root_hi[a] - pk.root_lo[a]});
   }
   ds.scene_eps = 2e-5f * scale;
-  build_bvh(pk, ds.scene_eps, 0, bvh);
+  build_bvh(d.points, d.triangles, pk, ds.scene_eps, 0, bvh);
   if ((s = dev_upload(out, bvh.nodes.data(), bvh.nodes.size(), &ds.bvh)) != HPT_OK) return s;
   if (bvh.tris.empty()) bvh.tris.emplace_back();
   if ((s = dev_upload(out, bvh.tris.data(), bvh.tris.size(), &ds.btris)) != HPT_OK) return s;
+  for (int a = 0; a < 3; ++a) {
+    if ((s = dev_upload(out, bvh.edge_keys[a].data(), bvh.edge_keys[a].size(), &ds.edge_keys[a])) !=
+        HPT_OK)
+      return s;
+    ds.num_edge_keys[a] = (int32_t)bvh.edge_keys[a].size();
+  }
   ds.num_bvh = (int32_t)bvh.nodes.size();
   ds.num_btris = (int32_t)bvh.tris.size();
   ds.nodes = nodes;

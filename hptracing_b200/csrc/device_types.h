@@ -77,17 +77,28 @@ struct BvhNode {
 };
 static_assert(sizeof(BvhNode) == 80, "80-byte wide node");
 
-// Triangle record in node order: the DevTri values and the lowest tree node
-// that holds every leaf listing the triangle (bvh_certain in bvh.cuh).
+// Triangle record in node order: the DevTri values, and for the certificate
+// (bvh_certain in bvh.cuh) the lowest tree node that holds every leaf listing
+// the triangle, and flags. Bit 2a / 2a + 1 of the flags: one of those leaves
+// ends just outside the triangle's lower / upper bound on axis a, by less
+// than kCertainNear. kTriIrregular: the tree does not list the triangle in
+// exactly the leaves its bounds touch.
 struct BvhTri {
   float a[3];
   int32_t tri_id;
   float e1[3];
   int32_t start_node;
   float e2[3];
-  int32_t pad;
+  uint32_t flags;
 };
 static_assert(sizeof(BvhTri) == 48, "48-byte triangle record");
+constexpr uint32_t kTriIrregular = 64u;
+
+// Distances of the certificate in units of DevScene::scene_eps (2e-5 of the
+// scene's size): the tree walk's rounding, generously (4e-6 of the size), and
+// the leaf faces that count as just outside a triangle's bounds.
+constexpr float kCertainRound = 0.2f;
+constexpr float kCertainNear = 4 * kCertainRound;
 
 // Entries of a ray's node stack; the builder bounds the depth below it (one
 // entry at most per level).
@@ -122,6 +133,10 @@ struct DevScene {
   const BvhNode* bvh;       // wide nodes, root first
   const BvhTri* btris;      // triangle records in node order
   int32_t num_bvh, num_btris;
+  // Directions of the triangle edges e2 that have a zero on axis a, sorted
+  // (edge_key in scene_pack.h; used by bvh_certain).
+  const float* edge_keys[3];
+  int32_t num_edge_keys[3];
 };
 
 // --- Wavefront job table ------------------------------------------------
@@ -195,7 +210,8 @@ struct DevCtrl {
   int32_t chk_shade_items;
   int32_t chk_shade_done;
   int32_t chk_isect_done;
-  int32_t chk_pad;
+  int32_t n_open;           // rays of the intersect queue in the open list
+  int32_t ticket;           // blocks of the control kernel that are done
   // Started-but-unfinished paths all capped slots (max_inflight > 0) may
   // hold together (0 = no shared cap); host-written.
   int64_t capped_budget;

@@ -73,6 +73,9 @@ struct EngineParams {
   float4* R_d;
   float4* R_s;
   float4* R_r;
+  // Rays of the intersect queue whose hits are open after k_trace: (item,
+  // best, tie, t) as OpenList holds them, settled by k_ctrl.
+  uint4* open;
   int capacity;
   int refill;           // idle lanes that make a warp refill
   int rounds;           // warp rounds between refills
@@ -229,16 +232,34 @@ __device__ __forceinline__ Ray prim_ray(const DevJob& J, int64_t ray) {
 
 // Rays a warp has finished walking, waiting to be certified and written out
 // 32 at a time with every lane busy (a lane that finishes takes its next ray
-// at once). item: index in the intersect queue, or -1 - ray for a camera ray.
+// at once). item: index in the intersect queue, or -1 - ray for a camera ray
+// of job slot `slot` (lists of launches with camera rays).
+// The lists are as short as their use allows: what they take of the SM's
+// 256 KB, L1 does not have for nodes.
+template <bool kPrim>
 struct HitList {
-  int32_t item[64], slot[64];
+  int32_t item[64];
   uint32_t best[64];
   float t[64];
+  int32_t slot[kPrim ? 64 : 1];
 };
-// Rays of a warp that need the tree walk.
-struct WalkList {
-  int32_t item[64], slot[64];
+// Rays whose hits bvh_certain leaves open. A launch over the intersect queue
+// alone appends them to P.open for k_ctrl (a call in the walk's loop that
+// settles them costs its registers: 1.84 against 1.30 ms for the first
+// bounce of 4M paths on the spheres scene); one with camera rays, which may
+// outnumber that list, keeps them per warp and settles them itself.
+struct OpenList {
+  int32_t item[32];
+  uint32_t best[32], tie[32];
+  float t[32];
+  int32_t slot[32];
 };
+
+template <bool kPrim>
+__device__ __forceinline__ int list_slot(const EngineParams& P, int item, const int32_t* slots,
+                                         int k) {
+  return kPrim && item < 0 ? slots[kPrim ? k : 0] : __float_as_int(P.R_s[item].w);
+}
 
 __device__ __forceinline__ Ray list_ray(const EngineParams& P, int item, int slot) {
   if (item < 0) return prim_ray(P.jobs[slot], -1 - (int64_t)item);
@@ -320,57 +341,106 @@ __device__ __forceinline__ void write_hits(const EngineParams& P, bool have, int
   }
 }
 
-// Tree walk of the rays [first, first + n) of the list, n <= 32. Not inlined:
-// few rays need it, and its registers must not weigh on the main loop.
-__device__ __noinline__ void walk_rays(const EngineParams& P, const WalkList& W, int first,
-                                       int n) {
+// One open ray per lane (`have`): looks its hit up in the tree, and walks the
+// tree where that does not settle it. Every lane of the warp calls it.
+__device__ __forceinline__ void settle(const EngineParams& P, bool have, int item, int slot,
+                                       uint32_t best, uint32_t tie, float t) {
   DevCtrl* c = P.ctrl;
-  const int lane = threadIdx.x & 31;
-  const bool have = lane < n;
-  int item = 0, slot = 0;
   TravCount cnt{};
-  TravState st;
-  st.best.tri = -1;
-  st.best.t = 0.f;
   Ray r{};
+  int tri = -1;
   if (have) {
-    item = W.item[first + lane];
-    slot = W.slot[first + lane];
     const DevScene& s = P.jobs[slot].scene;
     r = list_ray(P, item, slot);
-    TravCold tc;
-    trav_init(s, r, st, tc);
-    while (!trav_leaf(s, st, tc, nullptr, 0, &c->err, cnt)) {
+    const uint32_t hit = bvh_resolve(s, r, best, tie, t, &c->err);
+    if (hit != kBvhNone) {
+      tri = __float_as_int(__ldg(reinterpret_cast<const float4*>(s.btris + hit)).w);
+    } else {
+      TravState st;
+      TravCold tc;
+      trav_init(s, r, st, tc);
+      while (!trav_leaf(s, st, tc, nullptr, 0, &c->err, cnt)) {
+      }
+      if (st.best.rec >= 0) tri = st.best.tri;
+      t = st.best.t;
     }
   }
   __syncwarp();
-  write_hits(P, have, item, slot, r.d, have && st.best.rec >= 0 ? st.best.tri : -1, st.best.t);
+  write_hits(P, have, item, slot, r.d, tri, t);
   const uint32_t nodes = __reduce_add_sync(kFull, cnt.nodes);
   const uint32_t leaves = __reduce_add_sync(kFull, cnt.leaves);
   const uint32_t tests = __reduce_add_sync(kFull, cnt.tris);
   const uint32_t repeats = __reduce_add_sync(kFull, cnt.repeats);
-  if (lane == 0) {
+  if ((threadIdx.x & 31) == 0) {
     add_counts(c, 0, nodes, leaves, tests);
     if (repeats) atomicAdd(&c->tri_repeats, (unsigned long long)repeats);
   }
 }
 
+__device__ __noinline__ void settle_list(const EngineParams& P, const OpenList& W, int n) {
+  const int lane = threadIdx.x & 31;
+  const bool have = lane < n;
+  const int k = have ? lane : 0;
+  const int item = W.item[k];
+  settle(P, have, item, have ? list_slot<true>(P, item, W.slot, k) : 0, W.best[k], W.tie[k],
+         W.t[k]);
+}
+
+// Appends one ray per lane (`want`) to the open list: the warp's (kPrim; at
+// length n, worked off first when it has no room) or the launch's. Returns
+// the warp's list's new length.
+template <bool kPrim>
+__device__ __forceinline__ int push_open(const EngineParams& P, OpenList* W, int n, bool want,
+                                         int item, int slot, uint32_t best, uint32_t tie,
+                                         float t) {
+  const unsigned m = __ballot_sync(kFull, want);
+  if (m == 0) return n;
+  if constexpr (!kPrim) {
+    int base = 0;
+    const int leader = __ffs(m) - 1;
+    if ((int)(threadIdx.x & 31) == leader) base = atomicAdd(&P.ctrl->n_open, __popc(m));
+    base = __shfl_sync(kFull, base, leader) + __popc(m & lanemask_lt());
+    bool ok = want;
+    HPT_DCHECK(&P.ctrl->err, !want || base < P.capacity, 225, base, ok = false);
+    if (ok) P.open[base] = make_uint4((uint32_t)item, best, tie, __float_as_uint(t));
+    return 0;
+  } else {
+    if (n + __popc(m) > 32) {
+      settle_list(P, *W, n);
+      n = 0;
+      __syncwarp();
+    }
+    if (want) {
+      const int k = n + __popc(m & lanemask_lt());
+      W->item[k] = item;
+      W->best[k] = best;
+      W->tie[k] = tie;
+      W->t[k] = t;
+      W->slot[k] = slot;
+    }
+    __syncwarp();
+    return n + __popc(m);
+  }
+}
+
 // Certifies the finished rays [first, first + n) of the list, n <= 32, and
-// writes them out; those that need the tree walk go to W at n_walk. Returns
-// the new length of W.
-__device__ __noinline__ int finish_rays(const EngineParams& P, const HitList& L, int first, int n,
-                                        WalkList& W, int n_walk) {
+// writes them out; those that stay open go to W at n_open. Returns the new
+// length of W.
+template <bool kPrim>
+__device__ __noinline__ int finish_rays(const EngineParams& P, const HitList<kPrim>& L, int first,
+                                        int n, OpenList* W, int n_open) {
   DevCtrl* c = P.ctrl;
   const int lane = threadIdx.x & 31;
   const bool have = lane < n;
   int item = 0, slot = 0, tri = -1;
+  uint32_t best = kBvhNone;
   float t = 0.f;
   bool certain = false;
   Ray r{};
   if (have) {
     item = L.item[first + lane];
-    slot = L.slot[first + lane];
-    const uint32_t best = L.best[first + lane];
+    slot = list_slot<kPrim>(P, item, L.slot, first + lane);
+    best = L.best[first + lane];
     t = L.t[first + lane];
     const DevScene& s = P.jobs[slot].scene;
     r = list_ray(P, item, slot);
@@ -379,21 +449,14 @@ __device__ __noinline__ int finish_rays(const EngineParams& P, const HitList& L,
       tri = __float_as_int(__ldg(reinterpret_cast<const float4*>(s.btris + best)).w);
   }
   __syncwarp();
-  const unsigned wm = __ballot_sync(kFull, have && !certain);
-  if (have && !certain) {
-    const int k = n_walk + __popc(wm & lanemask_lt());
-    W.item[k] = item;
-    W.slot[k] = slot;
-  }
-  __syncwarp();
   write_hits(P, have && certain, item, slot, r.d, tri, t);
-  return n_walk + __popc(wm);
+  return push_open<kPrim>(P, W, n_open, have && !certain, item, slot, best, 0, t);
 }
 
 // Test rounds run when at least this share (in eighths) of the warp's live
 // lanes hold pending triangles.
 #ifndef HPT_TEST_EIGHTHS
-#define HPT_TEST_EIGHTHS 4
+#define HPT_TEST_EIGHTHS 3
 #endif
 
 // kUniform: every job of the launch renders P.uscene. kQueue: traces the
@@ -406,10 +469,10 @@ __device__ __noinline__ int finish_rays(const EngineParams& P, const HitList& L,
 // pending triangles, or one triangle test for those with some.
 template <int BS, int MINB, bool kUniform, bool kQueue, bool kPrim>
 __global__ void __launch_bounds__(BS, MINB) k_trace(const __grid_constant__ EngineParams P) {
-  __shared__ HitList hit_lists[BS / 32];
-  __shared__ WalkList walk_lists[BS / 32];
-  HitList& L = hit_lists[threadIdx.x >> 5];
-  WalkList& W = walk_lists[threadIdx.x >> 5];
+  __shared__ HitList<kPrim> hit_lists[BS / 32];
+  __shared__ OpenList open_lists[kPrim ? BS / 32 : 1];
+  HitList<kPrim>& L = hit_lists[threadIdx.x >> 5];
+  OpenList* W = open_lists + (kPrim ? threadIdx.x >> 5 : 0);
   DevCtrl* c = P.ctrl;
   const int n = kQueue ? c->nR : 0;
   const int64_t total = kPrim ? (int64_t)n + P.prim_prefix[P.prim_n] : (int64_t)n;
@@ -418,15 +481,22 @@ __global__ void __launch_bounds__(BS, MINB) k_trace(const __grid_constant__ Engi
   bool active = false;
   BvhRay b;
   b.tri_bits = 0;
+  // The node stack (at most kBvhStack - 1 entries); its last word holds the
+  // other triangle of a tie.
   uint2 stack[kBvhStack];
-  int item = 0, slot = 0, steps = 0;
+  // The lane's ray (as HitList), read when it finishes: kept out of the
+  // registers the walk needs.
+  __shared__ int item_sh[BS], slot_sh[kPrim ? BS : 1];
+  int& my_item = item_sh[threadIdx.x];
+  int& my_slot = slot_sh[kPrim ? threadIdx.x : 0];
   const BvhNode* bvh = P.uscene.bvh;
   const BvhTri* btris = P.uscene.btris;
   uint32_t num_bvh = (uint32_t)P.uscene.num_bvh;
-  int max_steps = P.uscene.max_steps;
+  float eps = P.uscene.scene_eps;
+  uint32_t max_steps = (uint32_t)P.uscene.max_steps;
   // The warp's counts and list lengths (the same value in every lane).
-  uint32_t queries = 0, nodes = 0, leaves = 0, tests = 0;
-  int n_hits = 0, n_walk = 0;
+  uint32_t queries = 0, nodes = 0, tests = 0;
+  int n_hits = 0, n_open = 0;
   // Once a refill finds the rays exhausted the warp stops asking, so the
   // cursor overshoots by at most one grab per warp.
   bool drained = false;
@@ -438,6 +508,7 @@ __global__ void __launch_bounds__(BS, MINB) k_trace(const __grid_constant__ Engi
       base = __shfl_sync(kFull, base, 0);
       drained = (int64_t)base + __popc(idle) >= total;
       bool started = false, walk = false;
+      int item = 0, slot = 0;
       if (!active) {
         const int64_t i = (int64_t)base + __popc(idle & lanemask_lt());
         Ray r{};
@@ -462,35 +533,23 @@ __global__ void __launch_bounds__(BS, MINB) k_trace(const __grid_constant__ Engi
           }
         }
         if (started) {
-          float eps = P.uscene.scene_eps;
+          my_item = item;
+          if (kPrim) my_slot = slot;
           if (!kUniform) {
             const DevScene& s = P.jobs[slot].scene;
             bvh = s.bvh;
             btris = s.btris;
             num_bvh = (uint32_t)s.num_bvh;
-            max_steps = s.max_steps;
+            max_steps = (uint32_t)s.max_steps;
             eps = s.scene_eps;
           }
-          steps = 0;
-          active = bvh_init(eps, r, b);
+          active = bvh_init(r, b);
           walk = !active;
         }
       }
       queries += __popc(__ballot_sync(kFull, started));
-      const unsigned wm = __ballot_sync(kFull, walk);
-      if (wm) {
-        if (walk) {
-          const int k = n_walk + __popc(wm & lanemask_lt());
-          W.item[k] = item;
-          W.slot[k] = slot;
-        }
-        n_walk += __popc(wm);
-        __syncwarp();
-        if (n_walk >= 32) {
-          n_walk -= 32;
-          walk_rays(P, W, n_walk, 32);
-        }
-      }
+      // kBvhMany: straight to the tree walk.
+      n_open = push_open<kPrim>(P, W, n_open, walk, item, slot, kBvhMany, 0, 0.f);
     }
     if (__ballot_sync(kFull, active) == 0) {
       if (drained) break;
@@ -506,55 +565,48 @@ __global__ void __launch_bounds__(BS, MINB) k_trace(const __grid_constant__ Engi
       // Every round moves a lane on: a test round needs a testing lane, a
       // visit round one that is not.
       if (tm != 0 && 8 * __popc(tm) >= HPT_TEST_EIGHTHS * __popc(lm)) {
-        if (testing) {
-          bvh_test(btris, b);
-          ++steps;
-          finished = b.tri_bits == 0 && (b.node_bits & 255u) == 0 && b.sp == 0;
-        }
+        if (testing) bvh_test(btris, eps, b, stack[kBvhStack - 1].x);
         tests += __popc(tm);
       } else {
-        if (go && !testing) {
-          finished = !bvh_visit(bvh, num_bvh, b, stack, &c->err) ||
-                     (b.tri_bits == 0 && (b.node_bits & 255u) == 0 && b.sp == 0);
-          ++steps;
-        }
+        if (go && !testing) finished = !bvh_visit(bvh, num_bvh, b, stack, &c->err);
         nodes += __popc(lm & ~tm);
-        leaves += __popc(__ballot_sync(kFull, go && !testing && b.tri_bits != 0));
       }
-      if (go && steps > max_steps) {
-        atomicOr(&c->err.flags, 1u);
-        finished = true;
+      if (go) {
+        if (((b.node_bits & 255u) | b.tri_bits | (b.steps & 31u)) == 0) finished = true;
+        if (b.steps / kBvhStep > max_steps) {
+          atomicOr(&c->err.flags, 1u);
+          finished = true;
+        }
       }
     }
-    const unsigned fm = __ballot_sync(kFull, finished);
-    if (fm) {
-      if (finished) {
+    // A tie goes straight to the open list, the others to the hit list.
+    const bool open = finished && (b.best & (kBvhTie | kBvhMany)) != 0;
+    n_open = push_open<kPrim>(P, W, n_open, open, my_item, kPrim ? my_slot : 0, b.best,
+                              open ? stack[kBvhStack - 1].x : 0u, b.best_t);
+    const unsigned fm = __ballot_sync(kFull, finished && !open);
+    if (finished) {
+      if (!open) {
         const int k = n_hits + __popc(fm & lanemask_lt());
-        L.item[k] = item;
-        L.slot[k] = slot;
+        L.item[k] = my_item;
         L.best[k] = b.best;
         L.t[k] = b.best_t;
-        active = false;
+        if (kPrim) L.slot[kPrim ? k : 0] = my_slot;
       }
-      n_hits += __popc(fm);
+      active = false;
+    }
+    n_hits += __popc(fm);
+    __syncwarp();
+    if (n_hits >= 32) {
+      n_hits -= 32;
+      n_open = finish_rays<kPrim>(P, L, n_hits, 32, W, n_open);
       __syncwarp();
-      if (n_hits >= 32) {
-        n_hits -= 32;
-        n_walk = finish_rays(P, L, n_hits, 32, W, n_walk);
-        if (n_walk >= 32) {
-          n_walk -= 32;
-          walk_rays(P, W, n_walk, 32);
-        }
-        __syncwarp();
-      }
     }
   }
-  if (n_hits) n_walk = finish_rays(P, L, 0, n_hits, W, n_walk);
-  for (; n_walk > 0; n_walk -= min(n_walk, 32)) {
-    const int m = min(n_walk, 32);
-    walk_rays(P, W, n_walk - m, m);
+  if (n_hits) n_open = finish_rays<kPrim>(P, L, 0, n_hits, W, n_open);
+  if constexpr (kPrim) {
+    if (n_open) settle_list(P, *W, n_open);
   }
-  if (lane == 0) add_counts(c, queries, nodes, leaves, tests);
+  if (lane == 0) add_counts(c, queries, nodes, 0, tests);
 }
 
 // Sets the path count of primary-pass entry e's slot when the entry
@@ -738,9 +790,32 @@ __global__ void __launch_bounds__(BS, MINB) k_shade(EngineParams P) {
 #endif
 }
 
-// Advances the queues and the path cursors, then grants paths (one thread).
-__global__ void k_ctrl(EngineParams P) {
+// Settles the open rays of the intersect queue (all blocks), then advances
+// the queues and the path cursors and grants paths (one thread, of the block
+// that finishes last). The rays are dealt out over the warps first, lanes
+// second: they are few and their lookups are chains of loads.
+constexpr int kCtrlThreads = 128;
+__global__ void __launch_bounds__(kCtrlThreads) k_ctrl(const __grid_constant__ EngineParams P) {
   DevCtrl* c = P.ctrl;
+  const int n_open = c->n_open;
+  const int warps = gridDim.x * (kCtrlThreads / 32);
+  const int warp = (int)blockIdx.x + (int)gridDim.x * (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  for (int first = 0; first + warp < n_open; first += 32 * warps) {
+    const int i = first + lane * warps + warp;
+    const bool have = i < n_open;
+    uint4 e = make_uint4(0u, 0u, 0u, 0u);
+    if (have) e = P.open[i];
+    const int item = (int)e.x;
+    settle(P, have, item, have ? __float_as_int(P.R_s[item].w) : 0, e.y, e.z,
+           __uint_as_float(e.w));
+  }
+  // What this block wrote happens before the last block's reads.
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x != 0 || atomicAdd(&c->ticket, 1) != (int)gridDim.x - 1) return;
+  __threadfence();
+  c->ticket = 0;
+  c->n_open = 0;
 #ifdef HPT_DEVICE_CHECKS
   HPT_DCHECK(&c->err, c->chk_shade_done == c->chk_shade_items, 241,
              (long long)c->chk_shade_items * 1000000 + c->chk_shade_done, (void)0);
@@ -876,16 +951,16 @@ void cuda_soft_fail(cudaError_t e, const char* what) {
 hpt_tuning default_tuning() {
   hpt_tuning t;
   memset(&t, 0, sizeof t);
-  // From sweeps on the 512x512, 64 spp spheres frame and the 1920x1080, 4 spp
-  // terrain frame: 7 blocks of 128 per SM (72 registers; 6 / 7 / 8 / 9 / 10
-  // blocks: spheres 47.1 / 45.4 / 49.5 / 52.3 / 51.9 ms, terrain 15.6 / 15.1
-  // / 16.1 / 16.4 / 16.2 ms - the tighter budgets spill in the walk's loop),
-  // 16 rounds between refills (2 / 4 / 8 / 16: spheres 52.5 / 49.3 / 46.7 /
-  // 45.4 ms), a wavefront of 2^24 paths (3.5 GB of queues, allocated only up
-  // to the paths a run has).
+  // From sweeps on the 512x512, 64 spp spheres frame, the 1920x1080, 4 spp
+  // terrain frame and the 256x256, 16 spp box room: 8 blocks of 128 per SM
+  // (64 registers; 6 / 7 / 8 / 9 blocks: spheres 33.8 / 31.7 / 30.7 / 30.1
+  // ms, terrain 10.0 / 9.6 / 9.5 / 9.6 ms, room 1.17 / 1.15 / 1.17 / 1.20
+  // ms), 16 rounds between refills (8 / 16 / 24: spheres 37.6 / 37.2 / 38.1
+  // ms), a wavefront of 2^24 paths (3.8 GB of queues, allocated only up to
+  // the paths a run has).
   t.capacity = 1 << 24;
   t.isect_block = 128;
-  t.isect_min_blocks = 7;
+  t.isect_min_blocks = 8;
   t.shade_block = 256;
   t.refill_chunk = 4;
   t.smem_nodes = 0;
@@ -972,6 +1047,7 @@ Engine::~Engine() {
   HPT_SOFT(cudaFree(R_d_));
   HPT_SOFT(cudaFree(R_s_));
   HPT_SOFT(cudaFree(R_r_));
+  HPT_SOFT(cudaFree(open_));
   HPT_SOFT(cudaFree(ctrl_));
   HPT_SOFT(cudaFree(jobs_));
   HPT_SOFT(cudaFree(slot_state_));
@@ -1020,7 +1096,9 @@ hpt_status Engine::ensure_capacity(int capacity) {
   HPT_SOFT(cudaFree(R_d_));
   HPT_SOFT(cudaFree(R_s_));
   HPT_SOFT(cudaFree(R_r_));
+  HPT_SOFT(cudaFree(open_));
   R_o_ = R_d_ = R_s_ = R_r_ = nullptr;
+  open_ = nullptr;
   capacity_ = 0;
   const size_t n = (size_t)capacity;
   for (int p = 0; p < 2; ++p) {
@@ -1034,6 +1112,7 @@ hpt_status Engine::ensure_capacity(int capacity) {
   HPT_CUDA(cudaMalloc(&R_d_, n * sizeof(float4)));
   HPT_CUDA(cudaMalloc(&R_s_, n * sizeof(float4)));
   HPT_CUDA(cudaMalloc(&R_r_, n * sizeof(float4)));
+  HPT_CUDA(cudaMalloc(&open_, n * sizeof(uint4)));
   capacity_ = capacity;
   return HPT_OK;
 }
@@ -1176,7 +1255,7 @@ static EngineParams make_params(const Engine& e, DevCtrl* ctrl, DevJob* jobs, De
                                 int32_t* quota_prefix, const int32_t* prim_slot,
                                 const int64_t* prim_prefix, int prim_n, int capacity,
                                 float4* const* A, int32_t* const* Atri,
-                                float4* const* R, const DevScene* shared) {
+                                float4* const* R, uint4* open, const DevScene* shared) {
   EngineParams P;
   memset(&P, 0, sizeof P);
   P.jobs = jobs;
@@ -1200,6 +1279,7 @@ static EngineParams make_params(const Engine& e, DevCtrl* ctrl, DevJob* jobs, De
   P.R_d = R[1];
   P.R_s = R[2];
   P.R_r = R[3];
+  P.open = open;
   P.capacity = capacity;
   P.refill = std::max(1, std::min(32, e.tuning.refill_chunk));
   P.rounds = e.tuning.trav_steps > 0 ? e.tuning.trav_steps : default_tuning().trav_steps;
@@ -1262,7 +1342,7 @@ hpt_status Engine::admit(const std::vector<int>& slot_ids, const std::vector<Dev
   float4* R[4] = {R_o_, R_d_, R_s_, R_r_};
   EngineParams P = make_params(*this, ctrl_, jobs_, slot_state_, slots_, order_, quota_slot_,
                                quota_prefix_, prim_slot_, prim_prefix_, n, capacity_, A, A_tri_,
-                               R, shared_scene);
+                               R, open_, shared_scene);
   const IsectVariant& v = kIsectVariants[isect_variant()];
   v.primary[P.uniform_scene]<<<num_sms * occ_isect_, v.block, 0, stream>>>(P);
   HPT_CUDA(cudaGetLastError());
@@ -1416,13 +1496,13 @@ hpt_status Engine::launch_iteration_async() {
   float4* R[4] = {R_o_, R_d_, R_s_, R_r_};
   EngineParams P = make_params(*this, ctrl_, jobs_, slot_state_, slots_, order_, quota_slot_,
                                quota_prefix_, prim_slot_, prim_prefix_, n, capacity_, A, A_tri_,
-                               R, nullptr);
+                               R, open_, nullptr);
   P.prim_first = prim_first_;
   P.prim_final = prim_final_;
   shade_kernel(tuning)<<<num_sms * occ_shade_, 256, 0, stream>>>(P);
   const IsectVariant& v = kIsectVariants[isect_variant()];
   v.both[0]<<<num_sms * occ_isect_, v.block, 0, stream>>>(P);
-  k_ctrl<<<1, 1, 0, stream>>>(P);
+  k_ctrl<<<4 * num_sms, kCtrlThreads, 0, stream>>>(P);
   HPT_CUDA(cudaGetLastError());
   return HPT_OK;
 }
@@ -1486,14 +1566,14 @@ void Engine::launch_iteration(const DevScene* shared_scene, cudaEvent_t* ev) {
   float4* R[4] = {R_o_, R_d_, R_s_, R_r_};
   EngineParams P = make_params(*this, ctrl_, jobs_, slot_state_, slots_, order_, quota_slot_,
                                quota_prefix_, prim_slot_, prim_prefix_, 0, capacity_, A, A_tri_,
-                               R, shared_scene);
+                               R, open_, shared_scene);
   if (ev) HPT_SOFT(cudaEventRecord(ev[0], stream));
   shade_kernel(tuning)<<<num_sms * occ_shade_, 256, 0, stream>>>(P);
   if (ev) HPT_SOFT(cudaEventRecord(ev[1], stream));
   const IsectVariant& v = kIsectVariants[isect_variant()];
   v.isect[P.uniform_scene]<<<num_sms * occ_isect_, v.block, 0, stream>>>(P);
   if (ev) HPT_SOFT(cudaEventRecord(ev[2], stream));
-  k_ctrl<<<1, 1, 0, stream>>>(P);
+  k_ctrl<<<4 * num_sms, kCtrlThreads, 0, stream>>>(P);
 }
 
 void Engine::launch_resolve(int slot, const JobSpec& js, const JobBuffers& b, float samples) {

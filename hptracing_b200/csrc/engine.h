@@ -143,6 +143,7 @@ class Engine {
   float4* R_d_ = nullptr;
   float4* R_s_ = nullptr;
   float4* R_r_ = nullptr;
+  uint4* open_ = nullptr;  // rays whose hits are open (k_ctrl settles them)
   cudaEvent_t ev_[6];
   cudaEvent_t ev_done_[2] = {nullptr, nullptr};
   std::vector<cudaEvent_t> pev_;  // profiling events, created on first use

@@ -343,10 +343,12 @@ HPT_HD bool trav_leaf(const Sc& s, TravState& st, TravCold& tc, const uint2* sme
   ++cnt.leaves;
   HPT_DCHECK(err, begin >= 0 && count >= 0 && (long long)begin + count <= s.num_leaf_tris, 103,
              begin, { st.node = -1; return true; });
-  if (count > 0) {
-    // The reference only considers triangles of leaves whose box passes
-    // _box_intersect; evaluated once, when a candidate would win.
-    int pierced = -1;
+  // The reference only considers triangles of leaves whose box passes
+  // _box_intersect; evaluated once, when a candidate would win (at once for a
+  // ray with a zero component: in a split plane it fails in most leaves).
+  int pierced = -1;
+  if (count > 0 && (tc.ties & 7)) pierced = ref_box_test(r, L0, L1) ? 1 : 0;
+  if (count > 0 && pierced != 0) {
     const int32_t* ids = s.leaf_refs + begin;
     const float4* recs = reinterpret_cast<const float4*>(s.tris);
     for (int k = 0; k < count; ++k) {
@@ -480,14 +482,14 @@ HPT_HD bool trav_setup(const Sc& s, TravState& st, TravCold& tc, DevErr* err, Cn
   // trav_leaf adds the leaf's cost when it leaves it; every comparison with
   // max_steps comes later in both orders, so adding it here is equivalent.
   st.steps += 1 + count;
+  tc.pierced = count > 0 && (tc.ties & 7) ? (ref_box_test(r, L0, L1) ? 1 : 0) : -1;
   st.k = begin;
-  st.end = begin + count;
+  st.end = tc.pierced == 0 ? begin : begin + count;  // as trav_leaf: nothing counts here
   tc.leaf = leaf;
   tc.leaf_node = st.node;
   tc.rope = face == 0 ? R03.x : face == 1 ? R03.y : face == 2 ? R03.z
           : face == 3 ? R03.w : face == 4 ? R45.x : face == 5 ? R45.y : -1;
   tc.t_exit = t_exit;
-  tc.pierced = -1;
   st.phase = kStepTest;
   return false;
 }

@@ -257,7 +257,7 @@ typedef struct hpt_render_stats {
   /* Work of all queries' walks (the hierarchy's, and the tree's for the   */
   /* few rays that need it):                                               */
   int64_t nodes_visited;      /* eight-child nodes (tree: inner nodes)   */
-  int64_t leaves_visited;     /* nodes with triangles to test (leaves)   */
+  int64_t leaves_visited;     /* tree leaves walked                      */
   int64_t triangle_tests;     /* Moller-Trumbore tests run               */
   int64_t triangle_repeats;   /* leaf references skipped as already tested */
 } hpt_render_stats;
@@ -276,7 +276,7 @@ hpt_status hpt_render_stats_get(const hpt_scene* scene, hpt_render_stats* out);
 typedef struct hpt_tuning {
   int32_t capacity;          /* paths in flight (wavefront size); a run's */
                              /* queues hold at most its rays x spp paths; */
-                             /* default 2^24 (208 B per path)             */
+                             /* default 2^24 (216 B per path)             */
   int32_t isect_block;       /* threads per closest-hit block (128 / 256) */
   int32_t shade_block;       /* threads per shade block                   */
   int32_t refill_chunk;      /* lanes idle before a warp refills          */

@@ -37,7 +37,7 @@ void* bvhemu_create(const hpt_scene_desc* d) {
   }
   s.scene_eps = 2e-5f * scale;
   s.max_steps = 1 << 30;
-  build_bvh(e->pk, s.scene_eps, 0, e->bvh);
+  build_bvh(d->points, d->triangles, e->pk, s.scene_eps, 0, e->bvh);
   s.nodes = e->pk.nodes.data();
   s.leaves = e->pk.leaves.data();
   s.leaf_refs = e->pk.refs.data();
@@ -50,6 +50,10 @@ void* bvhemu_create(const hpt_scene_desc* d) {
   s.btris = e->bvh.tris.data();
   s.num_bvh = (int32_t)e->bvh.nodes.size();
   s.num_btris = (int32_t)e->bvh.tris.size();
+  for (int a = 0; a < 3; ++a) {
+    s.edge_keys[a] = e->bvh.edge_keys[a].data();
+    s.num_edge_keys[a] = (int32_t)e->bvh.edge_keys[a].size();
+  }
   return e;
 }
 
