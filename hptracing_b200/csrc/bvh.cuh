@@ -25,7 +25,7 @@
 // rounding. [A leaf near the hit that does not list it was cut off by a split
 // X beyond the bound m, m < X <= m + 3 roundings; the leaf on the split's near
 // side that holds m lists the triangle and ends in (m, X]: flagged.]
-// What this leaves open, and two triangles at exactly the same t, bvh_resolve
+// What this leaves open, and two triangles at exactly the same t, bvh_settle
 // looks up in the tree.
 #pragma once
 
@@ -338,19 +338,23 @@ HPT_HD bool bvh_certain(const Sc& s, const Ray& r, uint32_t best, float best_t, 
   return false;
 }
 
-// Looks up a hit in the tree that bvh_certain leaves open: goes through the
+// Looks up in the tree a hit that bvh_certain leaves open: goes through the
 // leaves that list the triangle - of two at the same t, both - along the ray.
-// Returns the record the tree walk would report, or kBvhNone when that is not
-// certain either (a leaf the ray crosses by no more than rounding, or at the
-// walk's end; a ray in a split plane; more than two at one t).
-// Of two triangles at one t the reference keeps the one it meets first, the
-// lowest position in the leaf lists over the leaves that count for either.
+// kLookupHit: the tree walk tests it in a leaf that counts, and `winner` is
+// the record it would report: of two triangles at one t the reference keeps
+// the one it meets first, the lowest position in the leaf lists over the
+// leaves that count for either. kLookupNone: no leaf that lists it counts.
+// kLookupOpen: a leaf may count or not (the ray crosses it by no more than
+// rounding, or it lies at the walk's end), or the tree is irregular there.
+enum Lookup : int { kLookupOpen = 0, kLookupHit = 1, kLookupNone = 2 };
+// Not inlined (two call sites: its code is mostly run cold).
 template <class Sc>
-HPT_HD uint32_t bvh_resolve(const Sc& s, const Ray& r, uint32_t best, uint32_t tie, float best_t,
-                            DevErr* err) {
+__host__ __device__ __noinline__ Lookup bvh_lookup(const Sc& s, const Ray& r, uint32_t best, uint32_t tie, float best_t,
+                         uint32_t& winner, DevErr* err) {
   const bool two = best & kBvhTie;
   const uint32_t first = best & kBvhNone;
-  if ((best & kBvhMany) || first == kBvhNone) return kBvhNone;
+  if ((best & kBvhMany) || first == kBvhNone || !(best_t < as_float(0x7f800000)))
+    return kLookupOpen;
   const float o[3] = {r.o.x, r.o.y, r.o.z};
   // 1 / d; zero stands for a zero component.
   const float inv[3] = {r.d.x != 0.f ? rn_rcp(r.d.x) : 0.f, r.d.y != 0.f ? rn_rcp(r.d.y) : 0.f,
@@ -359,8 +363,8 @@ HPT_HD uint32_t bvh_resolve(const Sc& s, const Ray& r, uint32_t best, uint32_t t
   const float slack = rn_div(s.scene_eps, dmax);
   // A face's distance is off by a few 1e-7 of the scene's size and of itself.
   const float tol = fma_rn(best_t, 1e-6f, rn_mul(0.1f, slack));
-  // The walk goes on to best_t x 1.0001 + slack.
-  const float last = fma_rn(best_t, 1.0001f, rn_mul(1.5f, slack));
+  // The walk visits the leaves that begin before this.
+  const float stop = fma_rn(best_t, 1.0001f, slack);
   // The bounds of the triangle, or of both, and the tree node that holds all
   // their leaves.
   float lo[3], hi[3];
@@ -368,10 +372,10 @@ HPT_HD uint32_t bvh_resolve(const Sc& s, const Ray& r, uint32_t best, uint32_t t
   int node = 0;
   for (int k = 0; k < (two ? 2 : 1); ++k) {
     const uint32_t cand = k ? tie : first;
-    HPT_DCHECK(err, cand < (uint32_t)s.num_btris, 116, cand, return kBvhNone);
+    HPT_DCHECK(err, cand < (uint32_t)s.num_btris, 116, cand, return kLookupOpen);
     const float4* rec = reinterpret_cast<const float4*>(s.btris + cand);
     const float4 A = ldg(rec), E1 = ldg(rec + 1), E2 = ldg(rec + 2);
-    if ((uint32_t)as_int(E2.w) & kTriIrregular) return kBvhNone;
+    if ((uint32_t)as_int(E2.w) & kTriIrregular) return kLookupOpen;
     id[k] = as_int(A.w);
     if (!two) node = as_int(E1.w);
     const float grow = rn_mul(0.1f, s.scene_eps);
@@ -385,17 +389,20 @@ HPT_HD uint32_t bvh_resolve(const Sc& s, const Ray& r, uint32_t best, uint32_t t
       hi[a] = k ? fmaxf(hi[a], h) : h;
     }
   }
-  // Depth-first over the nodes that the bounds and the ray (up to `last`)
-  // touch.
+  // Depth-first over the nodes that the bounds and the ray touch: of two
+  // triangles up to the walk's end, of one all along the ray (until a leaf
+  // counts the walk has no end there).
   constexpr int kDepth = 64;
   int node_stack[kDepth];
   float t0_stack[kDepth], t1_stack[kDepth];
   int sp = 0, rank = 0x7FFFFFFF;
-  uint32_t winner = kBvhNone;
   bool reached = false;  // a leaf that counts and begins before the hit
-  float t0 = 0.f, t1 = last;
+  // Leaves that may count: the lowest entry of each triangle in them.
+  int open_first = 0x7FFFFFFF, open_tie = 0x7FFFFFFF;
+  float t0 = 0.f, t1 = two ? rn_add(stop, tol) : as_float(0x7f800000);
+  winner = kBvhNone;
   while (true) {
-    HPT_DCHECK(err, node >= 0 && node < s.num_nodes, 110, node, return kBvhNone);
+    HPT_DCHECK(err, node >= 0 && node < s.num_nodes, 110, node, return kLookupOpen);
     const uint2 nd = ldg(reinterpret_cast<const uint2*>(s.nodes) + node);
     const uint32_t axis = nd.x >> 30;
     if (axis != kLeafKind) {
@@ -404,20 +411,22 @@ HPT_HD uint32_t bvh_resolve(const Sc& s, const Ray& r, uint32_t best, uint32_t t
       const float oa = axis == 0 ? o[0] : (axis == 1 ? o[1] : o[2]);
       const float la = axis == 0 ? lo[0] : (axis == 1 ? lo[1] : lo[2]);
       const float ha = axis == 0 ? hi[0] : (axis == 1 ? hi[1] : hi[2]);
-      // Along a zero component the ray stays on the origin's side (in the
-      // split plane itself the tree walk takes both).
-      if (iv == 0.f && oa == split) return kBvhNone;
-      const bool up = iv > 0.f || (iv == 0.f && oa < split);
-      const float ts = iv == 0.f ? as_float(0x7f800000) : rn_mul(rn_sub(split, oa), iv);
-      // The side the ray is on before the split, and the one after it.
+      // The side the ray is on before the split, and the one after it. Along
+      // a zero component it stays on the origin's side, in the split plane
+      // itself it touches both.
+      const bool up = iv > 0.f || (iv == 0.f && oa <= split);
+      const bool flat = iv == 0.f;
+      const float ts = flat ? as_float(0x7f800000) : rn_mul(rn_sub(split, oa), iv);
       const bool before = (up ? la <= split : ha >= split) && t0 <= rn_add(ts, tol);
-      const bool after = (up ? ha >= split : la <= split) && t1 >= rn_sub(ts, tol);
+      const bool after = (up ? ha >= split : la <= split) &&
+                         (flat ? oa == split : t1 >= rn_sub(ts, tol));
       const int child = (int)(nd.x & kIndexMask);
       const int near = child + (up ? 0 : 1), far = child + (up ? 1 : 0);
+      const float far_t0 = flat ? t0 : fmaxf(t0, rn_sub(ts, tol));
       if (before && after) {
-        if (sp >= kDepth) return kBvhNone;
+        if (sp >= kDepth) return kLookupOpen;
         node_stack[sp] = far;
-        t0_stack[sp] = fmaxf(t0, rn_sub(ts, tol));
+        t0_stack[sp] = far_t0;
         t1_stack[sp] = t1;
         ++sp;
       }
@@ -428,19 +437,20 @@ HPT_HD uint32_t bvh_resolve(const Sc& s, const Ray& r, uint32_t best, uint32_t t
       }
       if (after) {
         node = far;
-        t0 = fmaxf(t0, rn_sub(ts, tol));
+        t0 = far_t0;
         continue;
       }
     } else {
       HPT_DCHECK(err, (int)(nd.x & kIndexMask) < s.num_leaves, 111, nd.x & kIndexMask,
-                 return kBvhNone);
+                 return kLookupOpen);
       const float4* L = reinterpret_cast<const float4*>(s.leaves + (nd.x & kIndexMask));
       const float4 bl = ldg(L), bh = ldg(L + 1);
       const int begin = as_int(bl.w), count = as_int(bh.w);
       HPT_DCHECK(err, begin >= 0 && count >= 0 && (long long)begin + count <= s.num_leaf_tris,
-                 112, begin, return kBvhNone);
+                 112, begin, return kLookupOpen);
       int at = -1;  // the first entry of either
       uint32_t which = first;
+#pragma unroll 4
       for (int k = count - 1; k >= 0; --k) {
         const int32_t entry = ldg(s.leaf_refs + begin + k);
         if (entry == id[0] || entry == id[1]) {
@@ -451,12 +461,13 @@ HPT_HD uint32_t bvh_resolve(const Sc& s, const Ray& r, uint32_t best, uint32_t t
       if (at >= 0) {
         const float l[3] = {bl.x, bl.y, bl.z}, h[3] = {bh.x, bh.y, bh.z};
         float f0 = -as_float(0x7f800000), f1 = as_float(0x7f800000);
+        bool inside = true, face = false;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
+          inside = inside && o[a] >= l[a] && o[a] <= h[a];
           if (inv[a] == 0.f) {
-            // The filter rejects a leaf beside the origin, and on its face.
-            if (!(o[a] > l[a] && o[a] < h[a])) f1 = -as_float(0x7f800000);
-            if (o[a] == l[a] || o[a] == h[a]) return kBvhNone;
+            if (!(o[a] >= l[a] && o[a] <= h[a])) f1 = -as_float(0x7f800000);
+            face = face || o[a] == l[a] || o[a] == h[a];
             continue;
           }
           const float x0 = rn_mul(rn_sub(l[a], o[a]), inv[a]);
@@ -465,16 +476,24 @@ HPT_HD uint32_t bvh_resolve(const Sc& s, const Ray& r, uint32_t best, uint32_t t
           f1 = fminf(f1, fmaxf(x0, x1));
         }
         const float length = rn_sub(f1, fmaxf(f0, 0.f));
-        if (length > tol && f0 < fma_rn(0.5f, slack, best_t)) {
+        if (face && !inside) {
+          // The filter's slab of the face the ray lies in is 0 / 0: rejected
+          // (see tie_goes_right).
+        } else if (face) {
+          return kLookupOpen;  // the origin's own leaves: left to the walk
+        } else if (length > tol && f0 < rn_sub(stop, tol)) {
           // The ray crosses the leaf and the walk comes to it.
           if (at < rank) {
             rank = at;
             winner = which;
           }
           reached = reached || f0 < best_t;
-          if (!two && reached) return winner;
-        } else if (two && length >= -tol && f0 <= last) {
-          return kBvhNone;  // it may count or not
+          if (!two && reached) return kLookupHit;
+        } else if (length >= -tol && !(two && f0 > rn_add(stop, tol))) {
+          if (ref_box_test(r, bl, bh)) {
+            if (which == first) open_first = at < open_first ? at : open_first;
+            else open_tie = at < open_tie ? at : open_tie;
+          }
         }
       }
     }
@@ -484,7 +503,176 @@ HPT_HD uint32_t bvh_resolve(const Sc& s, const Ray& r, uint32_t best, uint32_t t
     t0 = t0_stack[sp];
     t1 = t1_stack[sp];
   }
-  return reached ? winner : kBvhNone;
+  // They matter when they could bring in the other triangle, or any.
+  if (reached) return (winner == first ? open_tie : open_first) < rank ? kLookupOpen : kLookupHit;
+  return winner == kBvhNone && open_first == 0x7FFFFFFF && open_tie == 0x7FFFFFFF ? kLookupNone
+                                                                                  : kLookupOpen;
+}
+
+// The tree walk for one triangle, or two at the same t, known to be nearest of
+// all that are accepted: the same leaves in the same order, but only those
+// entries of their lists are looked at, with the known t. True with the record
+// of the one the walk reports, false when it passes the hit without one (the
+// walk may then report another triangle).
+template <class Sc>
+__host__ __device__ __noinline__ bool walk_for(const Sc& s, const Ray& r, uint32_t first,
+                                               uint32_t tie, float best_t, uint32_t& winner,
+                                               DevErr* err) {
+  TravState st;
+  TravCold tc;
+  trav_init(s, r, st, tc);
+  if (tc.ties) return false;  // zero components: walks on several sides
+  const int32_t id0 = as_int(ldg(reinterpret_cast<const float4*>(s.btris + first)).w);
+  const int32_t id1 =
+      tie == kBvhNone ? -1 : as_int(ldg(reinterpret_cast<const float4*>(s.btris + tie)).w);
+  const float stop = rn_add(best_t, rn_add(rn_mul(best_t, 1e-4f), tc.slack));
+  int rank = 0x7FFFFFFF;
+  while (st.node >= 0) {
+    const float px = rn_add(r.o.x, rn_mul(st.t_entry, r.d.x));
+    const float py = rn_add(r.o.y, rn_mul(st.t_entry, r.d.y));
+    const float pz = rn_add(r.o.z, rn_mul(st.t_entry, r.d.z));
+    int node = st.node;
+    uint2 nd = ldg(reinterpret_cast<const uint2*>(s.nodes) + node);
+    while ((nd.x >> 30) != kLeafKind) {
+      const uint32_t axis = nd.x >> 30;
+      const float split = as_float_u(nd.y);
+      const float p = axis == 0 ? px : (axis == 1 ? py : pz);
+      const float dd = axis == 0 ? r.d.x : (axis == 1 ? r.d.y : r.d.z);
+      node = (int)(nd.x & kIndexMask) + (p > split || (p == split && dd > 0.f) ? 1 : 0);
+      HPT_DCHECK(err, node < s.num_nodes, 106, node, return false);
+      nd = ldg(reinterpret_cast<const uint2*>(s.nodes) + node);
+      if (++st.steps > s.max_steps) return false;
+    }
+    HPT_DCHECK(err, (int)(nd.x & kIndexMask) < s.num_leaves, 102, nd.x & kIndexMask,
+               return false);
+    const DevLeaf* L = s.leaves + (nd.x & kIndexMask);
+    const float4 L0 = ldg(reinterpret_cast<const float4*>(L));
+    const float4 L1 = ldg(reinterpret_cast<const float4*>(L) + 1);
+    const int4 R03 = ldg(reinterpret_cast<const int4*>(L) + 2);
+    const int2 R45 = ldg(reinterpret_cast<const int2*>(L) + 6);
+    const int begin = as_int(L0.w), count = as_int(L1.w);
+    HPT_DCHECK(err, begin >= 0 && count >= 0 && (long long)begin + count <= s.num_leaf_tris, 103,
+               begin, return false);
+    int at = -1;
+    uint32_t which = first;
+#pragma unroll 4
+    for (int k = count - 1; k >= 0; --k) {
+      const int32_t entry = ldg(s.leaf_refs + begin + k);
+      if (entry == id0 || entry == id1) {
+        at = begin + k;
+        which = entry == id0 ? first : tie;
+      }
+    }
+    if (at >= 0 && at < rank && ref_box_test(r, L0, L1)) {
+      rank = at;
+      winner = which;
+    }
+    float t_exit = as_float(0x7f800000);
+    int rope = -1;
+    const float tx = rn_mul(rn_sub(r.d.x > 0.f ? L1.x : L0.x, r.o.x), tc.inv_d.x);
+    const float ty = rn_mul(rn_sub(r.d.y > 0.f ? L1.y : L0.y, r.o.y), tc.inv_d.y);
+    const float tz = rn_mul(rn_sub(r.d.z > 0.f ? L1.z : L0.z, r.o.z), tc.inv_d.z);
+    if (tx < t_exit) {
+      t_exit = tx;
+      rope = r.d.x > 0.f ? R03.y : R03.x;
+    }
+    if (ty < t_exit) {
+      t_exit = ty;
+      rope = r.d.y > 0.f ? R03.w : R03.z;
+    }
+    if (tz < t_exit) {
+      t_exit = tz;
+      rope = r.d.z > 0.f ? R45.y : R45.x;
+    }
+    // Before the hit is found the walk goes on at least this far, after it no
+    // further.
+    if (!(t_exit < tc.t_end) || rope < 0 || t_exit > stop) break;
+    HPT_DCHECK(err, rope < s.num_nodes, 105, rope, return false);
+    if (++st.steps > s.max_steps) return false;
+    st.node = rope;
+    st.t_entry = fmaxf(st.t_entry, t_exit);
+  }
+  return rank != 0x7FFFFFFF;
+}
+
+// Settles an open hit: sets the triangle's record (kBvhNone: a miss) and t of
+// the tree walk's answer and returns true, or returns false when the tree has
+// to be walked. A hit in leaves that do not count (the ray lies in a split
+// plane) makes it search the hierarchy again for the nearest one that does.
+template <class Sc>
+HPT_HD bool bvh_settle(const Sc& s, const Ray& r, uint32_t& best, uint32_t tie, float& t,
+                       DevErr* err) {
+  uint32_t winner;
+  const Lookup l = bvh_lookup(s, r, best, tie, t, winner, err);
+  if (l == kLookupHit) {
+    best = winner;
+    return true;
+  }
+  if (l == kLookupOpen) {
+    if ((best & kBvhMany) || (best & kBvhNone) == kBvhNone || !(t < as_float(0x7f800000)) ||
+        !walk_for(s, r, best & kBvhNone, best & kBvhTie ? tie : kBvhNone, t, winner, err))
+      return false;
+    best = winner;
+    return true;
+  }
+  BvhRay b;
+  bvh_init(r, b);
+  uint2 stack[kBvhStack];
+  while (true) {
+    while (b.tri_bits) {
+      const uint32_t before = b.best;
+      const float before_t = b.best_t, before_cull = b.cull;
+      uint32_t other = 0;
+      bvh_test(s.btris, s.scene_eps, b, other);
+      if (b.best == before) continue;
+      if (b.best & (kBvhTie | kBvhMany)) return false;
+      const Lookup c = bvh_lookup(s, r, b.best, 0u, b.best_t, winner, err);
+      if (c == kLookupOpen) return false;
+      if (c == kLookupNone) {
+        b.best = before;
+        b.best_t = before_t;
+        b.cull = before_cull;
+      }
+    }
+    if (!bvh_visit(s.bvh, (uint32_t)s.num_bvh, b, stack, err)) break;
+  }
+  best = b.best;
+  t = b.best_t;
+  return best != kBvhNone || bvh_no_parallel_edge(s, r.d);
+}
+
+// Of two triangles at the same t (best with kBvhTie, second), the record of the one the tree walk reports
+// wherever it accepts it: when one's bounds hold the other's, every leaf that
+// lists the inner one lists the outer one too, and with the smaller id the
+// outer one stands before it there. kBvhNone when that does not settle it.
+template <class Sc>
+HPT_HD uint32_t bvh_outer(const Sc& s, uint32_t best, uint32_t second, DevErr* err) {
+  const uint32_t first = best & kBvhNone;
+  if ((best & kBvhMany) || first == kBvhNone) return kBvhNone;
+  HPT_DCHECK(err, first < (uint32_t)s.num_btris && second < (uint32_t)s.num_btris, 117, second,
+             return kBvhNone);
+  float lo[2][3], hi[2][3];
+  int32_t id[2];
+  for (int k = 0; k < 2; ++k) {
+    const float4* rec = reinterpret_cast<const float4*>(s.btris + (k ? second : first));
+    const float4 A = ldg(rec), E1 = ldg(rec + 1), E2 = ldg(rec + 2);
+    if ((uint32_t)as_int(E2.w) & (kTriIrregular | kTriUnordered)) return kBvhNone;
+    id[k] = as_int(A.w);
+    const float a[3] = {A.x, A.y, A.z}, e1[3] = {E1.x, E1.y, E1.z}, e2[3] = {E2.x, E2.y, E2.z};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const float v1 = rn_add(a[c], e1[c]), v2 = rn_add(a[c], e2[c]);
+      lo[k][c] = fminf(a[c], fminf(v1, v2));
+      hi[k][c] = fmaxf(a[c], fmaxf(v1, v2));
+    }
+  }
+  bool first_holds = id[0] < id[1], second_holds = id[1] < id[0];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    first_holds = first_holds && lo[0][c] <= lo[1][c] && hi[0][c] >= hi[1][c];
+    second_holds = second_holds && lo[1][c] <= lo[0][c] && hi[1][c] >= hi[0][c];
+  }
+  return first_holds ? first : (second_holds ? second : kBvhNone);
 }
 
 // The whole query of one ray; the tree walk's answer (t and triangle id).
@@ -507,10 +695,14 @@ HPT_HD void bvh_query(const Sc& s, const Ray& r, int32_t& tri, float& t, DevErr*
       ++cnt.nodes;
     }
     ok = bvh_certain(s, r, b.best, b.best_t, err);
-    if (!ok) {
-      b.best = bvh_resolve(s, r, b.best, tie, b.best_t, err);
-      ok = b.best != kBvhNone;
+    if (b.best & kBvhTie) {
+      const uint32_t outer = bvh_outer(s, b.best, tie, err);
+      if (outer != kBvhNone && bvh_certain(s, r, outer, b.best_t, err)) {
+        b.best = outer;
+        ok = true;
+      }
     }
+    if (!ok) ok = bvh_settle(s, r, b.best, tie, b.best_t, err);
   }
   if (how) *how = ok;
   if (ok) {

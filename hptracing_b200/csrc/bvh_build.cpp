@@ -458,12 +458,16 @@ void build_bvh(const float* points, const int32_t* triangles, const PackedScene&
       b.lo[a] = L.lo[a];
       b.hi[a] = L.hi[a];
     }
+    bool ascending = true;
+    for (int32_t k = 1; k < L.tri_count; ++k)
+      ascending = ascending && scene.refs[(size_t)L.tri_begin + k - 1] <
+                                   scene.refs[(size_t)L.tri_begin + k];
     for (int32_t k = 0; k < L.tri_count; ++k) {
       const size_t id = (size_t)scene.refs[(size_t)L.tri_begin + k];
       boxes[id].add(b);
       ++listed[id];
       const Box& t = bounds[id];
-      uint32_t f = 0;
+      uint32_t f = ascending ? 0u : kTriUnordered;
       for (int a = 0; a < 3; ++a) {
         const float below = t.lo[a] - b.lo[a], above = b.hi[a] - t.hi[a];
         if (below > 0.f && below < near) f |= 1u << (2 * a);

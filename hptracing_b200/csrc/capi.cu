@@ -415,6 +415,13 @@ hpt_status upload_scene(const hpt_scene_desc& d, SceneDev& out) {
       return s;
     ds.num_edge_keys[a] = (int32_t)bvh.edge_keys[a].size();
   }
+  ds.finite_shading = 1;
+  for (int m = 0; m < d.num_materials; ++m)
+    for (int k = 0; k < 3; ++k)
+      if (!std::isfinite(d.materials[m].emission[k]) || !std::isfinite(d.materials[m].ambient[k]))
+        ds.finite_shading = 0;
+  for (int64_t k = 0; k < 4 * (int64_t)d.num_normals; ++k)
+    if ((k & 3) != 3 && !std::isfinite(d.normals[k])) ds.finite_shading = 0;
   ds.num_bvh = (int32_t)bvh.nodes.size();
   ds.num_btris = (int32_t)bvh.tris.size();
   ds.nodes = nodes;

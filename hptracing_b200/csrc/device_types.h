@@ -82,7 +82,8 @@ static_assert(sizeof(BvhNode) == 80, "80-byte wide node");
 // the triangle, and flags. Bit 2a / 2a + 1 of the flags: one of those leaves
 // ends just outside the triangle's lower / upper bound on axis a, by less
 // than kCertainNear. kTriIrregular: the tree does not list the triangle in
-// exactly the leaves its bounds touch.
+// exactly the leaves its bounds touch. kTriUnordered: in one of them the
+// entries are not in ascending order.
 struct BvhTri {
   float a[3];
   int32_t tri_id;
@@ -92,7 +93,7 @@ struct BvhTri {
   uint32_t flags;
 };
 static_assert(sizeof(BvhTri) == 48, "48-byte triangle record");
-constexpr uint32_t kTriIrregular = 64u;
+constexpr uint32_t kTriIrregular = 64u, kTriUnordered = 128u;
 
 // Distances of the certificate in units of DevScene::scene_eps (2e-5 of the
 // scene's size): the tree walk's rounding, generously (4e-6 of the size), and
@@ -135,6 +136,9 @@ struct DevScene {
   int32_t num_bvh, num_btris;
   // Directions of the triangle edges e2 that have a zero on axis a, sorted
   // (edge_key in scene_pack.h; used by bvh_certain).
+  // Emission, ambient colours and normals are finite: a ray of zero strength
+  // adds zero wherever it hits.
+  int32_t finite_shading;
   const float* edge_keys[3];
   int32_t num_edge_keys[3];
 };
@@ -183,10 +187,10 @@ struct DevErr {
 
 // Wavefront control block (device memory, updated by the control kernel).
 struct DevCtrl {
-  int32_t nA;               // paths in the current shade queue
-  int32_t nR;               // rays in the intersect queue
-  int32_t nA_next;          // hits appended by the intersect kernel
-  int32_t parity;           // which shade buffer is current
+  int32_t nQ;               // paths in the queue the coming shade pass reads
+  int32_t nR;               // survivors it wrote to the other queue
+  int32_t shade_head;       // the shade pass's item cursor
+  int32_t parity;           // which queue the coming shade pass reads
   int32_t n_new;            // new paths granted to the coming shade pass
   int32_t done;             // no queued path and nothing left to issue
   int32_t n_quota;          // slots with a grant (quota_slot / quota_prefix)
@@ -210,8 +214,9 @@ struct DevCtrl {
   int32_t chk_shade_items;
   int32_t chk_shade_done;
   int32_t chk_isect_done;
-  int32_t n_open;           // rays of the intersect queue in the open list
-  int32_t ticket;           // blocks of the control kernel that are done
+  int32_t chk_pad;
+  // Per queue, after it was traced: rays in the hit list and the open list.
+  int32_t n_hit[2], n_open[2];
   // Started-but-unfinished paths all capped slots (max_inflight > 0) may
   // hold together (0 = no shared cap); host-written.
   int64_t capped_budget;

@@ -8,19 +8,20 @@
 //
 // Here the same per-path arithmetic runs as a regenerating wavefront over
 // job slots (one job = one frame of one scene):
-//   k_primary  - ray generation + closest hit for the primary rays of newly
-//                admitted jobs; hits go to a per-job cache, misses write
+//   k_trace    - closest hit for the queue's rays, or for the camera rays of
+//                newly admitted jobs, or both, with persistent warps that
+//                refill idle lanes (ballot + one atomic per warp). A queue
+//                ray's hit goes to the hit list, its miss adds background *
+//                strength; camera hits go to a per-job cache, misses add
 //                background * sample.
 //   k_admit    - sets each new job's path count and grants paths.
-//   k_shade    - for each pending hit: self-emission, normal / UV / texture,
-//                branch choice and next direction (s1_run + s2_*_run fused);
-//                new (primary hit, sample) paths are started in the same
-//                pass from the grants. Survivors are compacted (warp ballot
-//                + block scan, one atomic per block) into the intersect
-//                queue; finished paths flush their radiance.
-//   k_isect    - closest hit for the intersect queue with persistent warps
-//                that refill idle lanes from the queue (ballot + one atomic
-//                per warp); hits are appended to the next shade queue.
+//   k_shade    - for each hit: self-emission, normal / UV / texture, branch
+//                choice and next direction (s1_run + s2_*_run fused); new
+//                (primary hit, sample) paths are started in the same pass
+//                from the grants. Survivors are compacted (warp ballot +
+//                block scan, one atomic per block) into the other queue;
+//                finished paths flush their radiance. Hits that k_trace
+//                leaves open are settled here first.
 //   k_ctrl     - advances queue counters and path cursors and grants the
 //                free wavefront capacity to the active jobs in priority
 //                order (the host never reads stage sizes).
@@ -64,17 +65,15 @@ struct EngineParams {
   const int64_t* prim_first;
   const int32_t* prim_final;
   int prim_n;
-  float4* A_o[2];
-  float4* A_d[2];
-  float4* A_s[2];
-  float4* A_r[2];
-  int32_t* A_tri[2];
-  float4* R_o;
-  float4* R_d;
-  float4* R_s;
-  float4* R_r;
-  // Rays of the intersect queue whose hits are open after k_trace: (item,
-  // best, tie, t) as OpenList holds them, settled by k_ctrl.
+  // The queue of paths, double-buffered: k_shade reads queue c->parity and
+  // writes the survivors to the other one, whose rays k_trace then traces.
+  float4* Q_o[2];       // origin, ray index
+  float4* Q_d[2];       // direction, sample << 8 | bounce
+  float4* Q_s[2];       // strength, job slot
+  float4* Q_r[2];       // radiance so far
+  uint4* hits;          // rays that hit: (item, triangle, t bits, -)
+  // Rays whose hits k_trace leaves open: (item, best, tie, t bits) as
+  // bvh_settle takes them; the next k_shade settles them.
   uint4* open;
   int capacity;
   int refill;           // idle lanes that make a warp refill
@@ -134,7 +133,7 @@ __device__ __forceinline__ void count_done(DevSlot* slots, bool done, int slot) 
     atomicAdd(&slots[slot].done, (unsigned long long)__popc(same & m));
 }
 
-// Counts the paths each slot sends to the intersect queue (one atomic per
+// Counts the paths each slot sends on to be traced (one atomic per
 // (warp, slot)).
 __device__ __forceinline__ void count_queries(DevSlot* slots, bool alive, int slot) {
   const unsigned m = __ballot_sync(kFull, alive);
@@ -160,7 +159,7 @@ __device__ __forceinline__ void add_counts(DevCtrl* c, uint32_t queries, uint32_
 // (one thread). A slot with nothing left to issue no longer needs grants.
 __device__ void schedule(const EngineParams& P) {
   DevCtrl* c = P.ctrl;
-  const int budget = P.capacity - c->nA;
+  const int budget = P.capacity - (c->n_hit[c->parity] + c->n_open[c->parity]);
   int n_new = 0, nq = 0;
   bool remaining = false;
   // Paths the capped slots hold now, against their shared budget.
@@ -201,7 +200,7 @@ __device__ void schedule(const EngineParams& P) {
   P.quota_prefix[nq] = n_new;
   c->n_quota = nq;
   c->n_new = n_new;
-  c->done = (c->nA == 0 && !remaining) ? 1 : 0;
+  c->done = (budget == P.capacity && !remaining) ? 1 : 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -232,225 +231,238 @@ __device__ __forceinline__ Ray prim_ray(const DevJob& J, int64_t ray) {
 
 // Rays a warp has finished walking, waiting to be certified and written out
 // 32 at a time with every lane busy (a lane that finishes takes its next ray
-// at once). item: index in the intersect queue, or -1 - ray for a camera ray
-// of job slot `slot` (lists of launches with camera rays).
-// The lists are as short as their use allows: what they take of the SM's
-// 256 KB, L1 does not have for nodes.
+// at once). item: index in the queue, or -1 - ray for a camera ray of job slot
+// `slot` (launches with camera rays). The lists are as short as their use
+// allows: what they take of the SM's 256 KB, L1 does not have for nodes.
 template <bool kPrim>
 struct HitList {
   int32_t item[64];
-  uint32_t best[64];
+  uint32_t best[64], tie[64];
   float t[64];
   int32_t slot[kPrim ? 64 : 1];
 };
-// Rays whose hits bvh_certain leaves open. A launch over the intersect queue
-// alone appends them to P.open for k_ctrl (a call in the walk's loop that
-// settles them costs its registers: 1.84 against 1.30 ms for the first
-// bounce of 4M paths on the spheres scene); one with camera rays, which may
-// outnumber that list, keeps them per warp and settles them itself.
+// Camera rays of a warp whose hits bvh_certain leaves open. Queue rays go to
+// P.open for the next k_shade instead: a call in the walk's loop that settles
+// them costs its registers (1.84 against 1.30 ms for the first bounce of 4M
+// paths on the spheres scene), and one ray's tree walk at the end of a launch
+// takes up to 0.65 ms, which k_shade has other work to hide behind.
 struct OpenList {
-  int32_t item[32];
+  int32_t item[32], slot[32];
   uint32_t best[32], tie[32];
   float t[32];
-  int32_t slot[32];
 };
 
-template <bool kPrim>
-__device__ __forceinline__ int list_slot(const EngineParams& P, int item, const int32_t* slots,
-                                         int k) {
-  return kPrim && item < 0 ? slots[kPrim ? k : 0] : __float_as_int(P.R_s[item].w);
+// An open hit: looked up in the tree, and by the tree walk where that does not
+// settle it. tri: -1 for a miss. Not inlined: few rays need it, and its
+// registers must not weigh on the callers.
+__device__ __noinline__ void settle(const DevScene& s, const Ray& r, uint32_t best, uint32_t tie,
+                                    DevCtrl* c, int& tri, float& t) {
+  if (bvh_settle(s, r, best, tie, t, &c->err)) {
+    tri = best == kBvhNone
+              ? -1
+              : __float_as_int(__ldg(reinterpret_cast<const float4*>(s.btris + best)).w);
+    return;
+  }
+  TravState st;
+  TravCold tc;
+  TravCount cnt{};
+  trav_init(s, r, st, tc);
+  while (!trav_leaf(s, st, tc, nullptr, 0, &c->err, cnt)) {
+  }
+  tri = st.best.rec >= 0 ? st.best.tri : -1;
+  t = st.best.t;
+  add_counts(c, 0, cnt.nodes, cnt.leaves, cnt.tris);
+  if (cnt.repeats) atomicAdd(&c->tri_repeats, (unsigned long long)cnt.repeats);
 }
 
-__device__ __forceinline__ Ray list_ray(const EngineParams& P, int item, int slot) {
-  if (item < 0) return prim_ray(P.jobs[slot], -1 - (int64_t)item);
-  const float4 o = P.R_o[item], d = P.R_d[item];
-  return Ray{mk(o.x, o.y, o.z), mk(d.x, d.y, d.z)};
-}
-
-// Writes out one finished ray per lane (`have`): a hit goes to the next shade
-// queue (or, for a camera ray, to its job's primary-hit cache), a miss adds
-// the background. Every lane of the warp calls it.
-__device__ __forceinline__ void write_hits(const EngineParams& P, bool have, int item, int slot,
-                                           const f3& dir, int tri, float t) {
-  DevCtrl* c = P.ctrl;
+// Writes out one camera ray per lane (`have`): a hit goes to its job's
+// primary-hit cache; a miss adds the background (kernel.cl:193-206: the first
+// pass assigns background * strength * sample_n with strength (1,1,1)). Every
+// lane of the warp calls it.
+__device__ __forceinline__ void write_camera(const EngineParams& P, bool have, int ray, int slot,
+                                             const f3& dir, int tri, float t) {
   const int lane = threadIdx.x & 31;
-  const int out_par = c->parity ^ 1;
-  const bool queued = have && item >= 0, camera = have && item < 0;
-  const bool hit = queued && tri >= 0;
+  const bool hit = have && tri >= 0;
   const unsigned hm = __ballot_sync(kFull, hit);
   if (hm) {
-    const int leader = __ffs(hm) - 1;
+    const unsigned same = __match_any_sync(kFull, hit ? slot : -1) & hm;
+    const int leader = hit ? __ffs(same) - 1 : 0;
     int base = 0;
-    if (lane == leader) base = atomicAdd(&c->nA_next, __popc(hm));
+    if (hit && lane == leader) base = atomicAdd(P.jobs[slot].prim_count, __popc(same));
     base = __shfl_sync(kFull, base, leader);
     if (hit) {
-      const int pos = base + __popc(hm & lanemask_lt());
-      bool ok = true;
-      HPT_DCHECK(&c->err, pos < P.capacity, 223, pos, ok = false);
-      if (ok) {
-        const float4 r4 = P.R_r[item];
-        P.A_o[out_par][pos] = P.R_o[item];
-        P.A_d[out_par][pos] = P.R_d[item];
-        P.A_s[out_par][pos] = P.R_s[item];
-        P.A_r[out_par][pos] = make_float4(r4.x, r4.y, r4.z, t);
-        P.A_tri[out_par][pos] = tri;
-      }
-    }
-  }
-  const bool missed = queued && !hit;
-  if (missed) {
-    // kernel.cl:195-200: miss adds background * strength (sample_n = 1).
-    const DevJob& J = P.jobs[slot];
-    const float4 s4 = P.R_s[item], r4 = P.R_r[item];
-    const int64_t ray = __float_as_int(P.R_o[item].w);
-    bool ok = true;
-    HPT_DCHECK(&c->err, ray >= 0 && ray < job_rays(J), 224, ray, ok = false);
-    if (ok) {
-      f3 rad = mk(r4.x, r4.y, r4.z);
-      rad = add(rad, mul(mk(J.bg[0], J.bg[1], J.bg[2]), mk(s4.x, s4.y, s4.z)));
-      flush_radiance(J, ray, rad);
-    }
-  }
-  count_done(P.slots, missed, slot);
-  // Camera rays: a hit goes to the job's primary-hit cache; a miss adds the
-  // background (kernel.cl:193-206: the first pass assigns background *
-  // strength * sample_n with strength (1,1,1)).
-  const unsigned cm = __ballot_sync(kFull, camera && tri >= 0);
-  if (cm) {
-    const unsigned same = __match_any_sync(kFull, camera && tri >= 0 ? slot : -1) & cm;
-    int base = 0;
-    const int leader = __ffs(same) - 1;
-    if (camera && tri >= 0 && lane == leader)
-      base = atomicAdd(P.jobs[slot].prim_count, __popc(same));
-    base = __shfl_sync(kFull, base, leader < 0 ? 0 : leader);
-    if (camera && tri >= 0) {
       const DevJob& J = P.jobs[slot];
       int k = base + __popc(same & lanemask_lt());
-      HPT_DCHECK(&c->err, k < job_rays(J), 203, k, k = -1);
+      HPT_DCHECK(&P.ctrl->err, k < job_rays(J), 203, k, k = -1);
       if (k >= 0) {
         float4* dst = reinterpret_cast<float4*>(J.prim) + 2 * (size_t)k;
-        dst[0] = make_float4(dir.x, dir.y, dir.z, __int_as_float(-1 - item));
+        dst[0] = make_float4(dir.x, dir.y, dir.z, __int_as_float(ray));
         dst[1] = make_float4(__int_as_float(tri), t, 0.f, 0.f);
       }
     }
   }
-  if (camera && tri < 0) {
+  if (have && !hit) {
     const DevJob& J = P.jobs[slot];
     const f3 val = scale((float)J.spp, mul(mk(J.bg[0], J.bg[1], J.bg[2]), mk(1.f, 1.f, 1.f)));
-    flush_radiance(J, -1 - (int64_t)item, val);
+    flush_radiance(J, ray, val);
   }
 }
 
-// One open ray per lane (`have`): looks its hit up in the tree, and walks the
-// tree where that does not settle it. Every lane of the warp calls it.
-__device__ __forceinline__ void settle(const EngineParams& P, bool have, int item, int slot,
-                                       uint32_t best, uint32_t tie, float t) {
-  DevCtrl* c = P.ctrl;
-  TravCount cnt{};
-  Ray r{};
-  int tri = -1;
-  if (have) {
-    const DevScene& s = P.jobs[slot].scene;
-    r = list_ray(P, item, slot);
-    const uint32_t hit = bvh_resolve(s, r, best, tie, t, &c->err);
-    if (hit != kBvhNone) {
-      tri = __float_as_int(__ldg(reinterpret_cast<const float4*>(s.btris + hit)).w);
-    } else {
-      TravState st;
-      TravCold tc;
-      trav_init(s, r, st, tc);
-      while (!trav_leaf(s, st, tc, nullptr, 0, &c->err, cnt)) {
-      }
-      if (st.best.rec >= 0) tri = st.best.tri;
-      t = st.best.t;
-    }
-  }
-  __syncwarp();
-  write_hits(P, have, item, slot, r.d, tri, t);
-  const uint32_t nodes = __reduce_add_sync(kFull, cnt.nodes);
-  const uint32_t leaves = __reduce_add_sync(kFull, cnt.leaves);
-  const uint32_t tests = __reduce_add_sync(kFull, cnt.tris);
-  const uint32_t repeats = __reduce_add_sync(kFull, cnt.repeats);
-  if ((threadIdx.x & 31) == 0) {
-    add_counts(c, 0, nodes, leaves, tests);
-    if (repeats) atomicAdd(&c->tri_repeats, (unsigned long long)repeats);
-  }
-}
-
-__device__ __noinline__ void settle_list(const EngineParams& P, const OpenList& W, int n) {
+__device__ __noinline__ void settle_camera(const EngineParams& P, const OpenList& W, int n) {
   const int lane = threadIdx.x & 31;
   const bool have = lane < n;
-  const int k = have ? lane : 0;
-  const int item = W.item[k];
-  settle(P, have, item, have ? list_slot<true>(P, item, W.slot, k) : 0, W.best[k], W.tie[k],
-         W.t[k]);
+  int ray = 0, slot = 0, tri = -1;
+  float t = 0.f;
+  Ray r{};
+  if (have) {
+    ray = -1 - W.item[lane];
+    slot = W.slot[lane];
+    t = W.t[lane];
+    const DevJob& J = P.jobs[slot];
+    r = prim_ray(J, ray);
+    settle(J.scene, r, W.best[lane], W.tie[lane], P.ctrl, tri, t);
+  }
+  __syncwarp();
+  write_camera(P, have, ray, slot, r.d, tri, t);
 }
 
-// Appends one ray per lane (`want`) to the open list: the warp's (kPrim; at
-// length n, worked off first when it has no room) or the launch's. Returns
-// the warp's list's new length.
-template <bool kPrim>
+// Hands over one open ray per lane (`want`); W / n: the warp's list of camera
+// rays, worked off when it has no room. Returns its new length.
+template <bool kQueue, bool kPrim>
 __device__ __forceinline__ int push_open(const EngineParams& P, OpenList* W, int n, bool want,
                                          int item, int slot, uint32_t best, uint32_t tie,
                                          float t) {
-  const unsigned m = __ballot_sync(kFull, want);
+  unsigned m = __ballot_sync(kFull, want);
   if (m == 0) return n;
-  if constexpr (!kPrim) {
-    int base = 0;
-    const int leader = __ffs(m) - 1;
-    if ((int)(threadIdx.x & 31) == leader) base = atomicAdd(&P.ctrl->n_open, __popc(m));
-    base = __shfl_sync(kFull, base, leader) + __popc(m & lanemask_lt());
-    bool ok = want;
-    HPT_DCHECK(&P.ctrl->err, !want || base < P.capacity, 225, base, ok = false);
-    if (ok) P.open[base] = make_uint4((uint32_t)item, best, tie, __float_as_uint(t));
-    return 0;
-  } else {
-    if (n + __popc(m) > 32) {
-      settle_list(P, *W, n);
-      n = 0;
-      __syncwarp();
+  if constexpr (kQueue) {
+    const bool queued = want && (!kPrim || item >= 0);
+    const unsigned qm = __ballot_sync(kFull, queued);
+    if (qm) {
+      int base = 0;
+      const int leader = __ffs(qm) - 1;
+      if ((int)(threadIdx.x & 31) == leader) base = atomicAdd(&P.ctrl->n_open[P.ctrl->parity ^ 1], __popc(qm));
+      base = __shfl_sync(kFull, base, leader) + __popc(qm & lanemask_lt());
+      bool ok = queued;
+      HPT_DCHECK(&P.ctrl->err, !queued || base < P.capacity, 225, base, ok = false);
+      if (ok) P.open[base] = make_uint4((uint32_t)item, best, tie, __float_as_uint(t));
     }
-    if (want) {
-      const int k = n + __popc(m & lanemask_lt());
-      W->item[k] = item;
-      W->best[k] = best;
-      W->tie[k] = tie;
-      W->t[k] = t;
-      W->slot[k] = slot;
-    }
-    __syncwarp();
-    return n + __popc(m);
+    m &= ~qm;
+    want = want && !queued;
   }
+  if constexpr (kPrim) {
+    if (m) {
+      if (n + __popc(m) > 32) {
+        settle_camera(P, *W, n);
+        n = 0;
+        __syncwarp();
+      }
+      if (want) {
+        const int k = n + __popc(m & lanemask_lt());
+        W->item[k] = item;
+        W->slot[k] = slot;
+        W->best[k] = best;
+        W->tie[k] = tie;
+        W->t[k] = t;
+      }
+      __syncwarp();
+      n += __popc(m);
+    }
+  }
+  return n;
+}
+
+// True when the ray's strength is zero and its hit, whichever it is, adds zero
+// to its path and ends it (a light sampled along the surface it lies in: the
+// ray runs in a split plane, where a certain hit would take a look at the
+// tree). `s`: its scene.
+__device__ __forceinline__ bool no_strength(const EngineParams& P, const DevScene& s, const Ray& r,
+                                            int item) {
+  const float4 w = P.Q_s[P.ctrl->parity ^ 1][item];
+  return w.x == 0.f && w.y == 0.f && w.z == 0.f && s.finite_shading &&
+         bvh_no_parallel_edge(s, r.d);
+}
+
+// Writes out one ray of the queue per lane (`have`): a hit goes to the hit
+// list, a miss adds background * strength (kernel.cl:195-200, sample_n = 1)
+// and ends its path. Every lane of the warp calls it.
+__device__ __forceinline__ void write_queue(const EngineParams& P, bool have, int item, int tri,
+                                            float t) {
+  DevCtrl* c = P.ctrl;
+  const int lane = threadIdx.x & 31;
+  const int q = c->parity ^ 1;
+  const bool hit = have && tri >= 0;
+  const unsigned hm = __ballot_sync(kFull, hit);
+  if (hm) {
+    int base = 0;
+    const int leader = __ffs(hm) - 1;
+    if (lane == leader) base = atomicAdd(&c->n_hit[q], __popc(hm));
+    base = __shfl_sync(kFull, base, leader) + __popc(hm & lanemask_lt());
+    bool ok = hit;
+    HPT_DCHECK(&c->err, !hit || base < P.capacity, 223, base, ok = false);
+    if (ok) P.hits[base] = make_uint4((uint32_t)item, (uint32_t)tri, __float_as_uint(t), 0u);
+  }
+  const bool missed = have && tri < 0;
+  int slot = 0;
+  if (missed) {
+    const float4 s4 = P.Q_s[q][item], r4 = P.Q_r[q][item];
+    const int64_t ray = __float_as_int(P.Q_o[q][item].w);
+    slot = __float_as_int(s4.w);
+    bool ok = true;
+    HPT_DCHECK(&c->err, slot >= 0 && slot < P.num_slots, 222, slot, ok = false);
+    HPT_DCHECK(&c->err, !ok || (ray >= 0 && ray < job_rays(P.jobs[slot])), 224, ray, ok = false);
+    if (ok) {
+      const DevJob& J = P.jobs[slot];
+      const f3 rad = mk(r4.x, r4.y, r4.z);
+      flush_radiance(J, ray, add(rad, mul(mk(J.bg[0], J.bg[1], J.bg[2]), mk(s4.x, s4.y, s4.z))));
+    }
+  }
+  count_done(P.slots, missed, slot);
 }
 
 // Certifies the finished rays [first, first + n) of the list, n <= 32, and
-// writes them out; those that stay open go to W at n_open. Returns the new
-// length of W.
-template <bool kPrim>
+// writes them out, or hands them over as open. Returns W's new length.
+template <bool kUniform, bool kQueue, bool kPrim>
 __device__ __noinline__ int finish_rays(const EngineParams& P, const HitList<kPrim>& L, int first,
                                         int n, OpenList* W, int n_open) {
   DevCtrl* c = P.ctrl;
   const int lane = threadIdx.x & 31;
   const bool have = lane < n;
   int item = 0, slot = 0, tri = -1;
-  uint32_t best = kBvhNone;
+  uint32_t best = kBvhNone, tie = 0;
   float t = 0.f;
-  bool certain = false;
+  bool certain = false, camera = false;
   Ray r{};
   if (have) {
     item = L.item[first + lane];
-    slot = list_slot<kPrim>(P, item, L.slot, first + lane);
     best = L.best[first + lane];
     t = L.t[first + lane];
-    const DevScene& s = P.jobs[slot].scene;
-    r = list_ray(P, item, slot);
+    camera = kPrim && (!kQueue || item < 0);
+    if (camera) {
+      slot = L.slot[kPrim ? first + lane : 0];
+      r = prim_ray(P.jobs[slot], -1 - (int64_t)item);
+    } else {
+      const int q = c->parity ^ 1;
+      const float4 o4 = P.Q_o[q][item], d4 = P.Q_d[q][item];
+      r = Ray{mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z)};
+      if (!kUniform) slot = __float_as_int(P.Q_s[q][item].w);
+    }
+    const DevScene& s = kUniform ? P.uscene : P.jobs[slot].scene;
+    if (best & kBvhTie) {
+      tie = L.tie[first + lane];
+      const uint32_t outer = bvh_outer(s, best, tie, &c->err);
+      if (outer != kBvhNone) best = outer;
+    }
     certain = bvh_certain(s, r, best, t, &c->err);
+    if (!certain && kQueue && !camera && best < kBvhNone && no_strength(P, s, r, item))
+      certain = true;
     if (certain && best != kBvhNone)
       tri = __float_as_int(__ldg(reinterpret_cast<const float4*>(s.btris + best)).w);
   }
   __syncwarp();
-  write_hits(P, have && certain, item, slot, r.d, tri, t);
-  return push_open<kPrim>(P, W, n_open, have && !certain, item, slot, best, 0, t);
+  if (kQueue) write_queue(P, have && certain && !camera, item, tri, t);
+  if (kPrim)
+    write_camera(P, have && certain && camera, -1 - item, slot, r.d, tri, t);
+  return push_open<kQueue, kPrim>(P, W, n_open, have && !certain, item, slot, best, tie, t);
 }
 
 // Test rounds run when at least this share (in eighths) of the warp's live
@@ -460,7 +472,7 @@ __device__ __noinline__ int finish_rays(const EngineParams& P, const HitList<kPr
 #endif
 
 // kUniform: every job of the launch renders P.uscene. kQueue: traces the
-// intersect queue; kPrim: traces the camera rays of the launch's primary-pass
+// queue; kPrim: traces the camera rays of the launch's primary-pass
 // entries (P.prim_*), after the queue's; k_admit (or, with kQueue, k_ctrl)
 // then starts the paths of the jobs whose primary pass completed. A serving
 // loop admits requests with both, with no launch of its own.
@@ -474,6 +486,7 @@ __global__ void __launch_bounds__(BS, MINB) k_trace(const __grid_constant__ Engi
   HitList<kPrim>& L = hit_lists[threadIdx.x >> 5];
   OpenList* W = open_lists + (kPrim ? threadIdx.x >> 5 : 0);
   DevCtrl* c = P.ctrl;
+  const int q = c->parity ^ 1;
   const int n = kQueue ? c->nR : 0;
   const int64_t total = kPrim ? (int64_t)n + P.prim_prefix[P.prim_n] : (int64_t)n;
   unsigned long long* head = kQueue ? &c->isect_head : &c->prim_head;
@@ -524,9 +537,11 @@ __global__ void __launch_bounds__(BS, MINB) k_trace(const __grid_constant__ Engi
           bool ok = true;
           HPT_DCHECK(&c->err, i < P.capacity, 221, i, ok = false);
           if (ok) {
-            const float4 o4 = P.R_o[i], d4 = P.R_d[i];
-            slot = __float_as_int(P.R_s[i].w);
-            HPT_DCHECK(&c->err, slot >= 0 && slot < P.num_slots, 222, slot, ok = false);
+            const float4 o4 = P.Q_o[q][i], d4 = P.Q_d[q][i];
+            if (!kUniform) {
+              slot = __float_as_int(P.Q_s[q][i].w);
+              HPT_DCHECK(&c->err, slot >= 0 && slot < P.num_slots, 222, slot, ok = false);
+            }
             r = Ray{mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z)};
             item = (int)i;
             started = ok;
@@ -549,7 +564,7 @@ __global__ void __launch_bounds__(BS, MINB) k_trace(const __grid_constant__ Engi
       }
       queries += __popc(__ballot_sync(kFull, started));
       // kBvhMany: straight to the tree walk.
-      n_open = push_open<kPrim>(P, W, n_open, walk, item, slot, kBvhMany, 0, 0.f);
+      n_open = push_open<kQueue, kPrim>(P, W, n_open, walk, item, slot, kBvhMany, 0, 0.f);
     }
     if (__ballot_sync(kFull, active) == 0) {
       if (drained) break;
@@ -579,32 +594,27 @@ __global__ void __launch_bounds__(BS, MINB) k_trace(const __grid_constant__ Engi
         }
       }
     }
-    // A tie goes straight to the open list, the others to the hit list.
-    const bool open = finished && (b.best & (kBvhTie | kBvhMany)) != 0;
-    n_open = push_open<kPrim>(P, W, n_open, open, my_item, kPrim ? my_slot : 0, b.best,
-                              open ? stack[kBvhStack - 1].x : 0u, b.best_t);
-    const unsigned fm = __ballot_sync(kFull, finished && !open);
+    const unsigned fm = __ballot_sync(kFull, finished);
     if (finished) {
-      if (!open) {
-        const int k = n_hits + __popc(fm & lanemask_lt());
-        L.item[k] = my_item;
-        L.best[k] = b.best;
-        L.t[k] = b.best_t;
-        if (kPrim) L.slot[kPrim ? k : 0] = my_slot;
-      }
+      const int k = n_hits + __popc(fm & lanemask_lt());
+      L.item[k] = my_item;
+      L.best[k] = b.best;
+      if (b.best & kBvhTie) L.tie[k] = stack[kBvhStack - 1].x;
+      L.t[k] = b.best_t;
+      if (kPrim) L.slot[kPrim ? k : 0] = my_slot;
       active = false;
     }
     n_hits += __popc(fm);
     __syncwarp();
     if (n_hits >= 32) {
       n_hits -= 32;
-      n_open = finish_rays<kPrim>(P, L, n_hits, 32, W, n_open);
+      n_open = finish_rays<kUniform, kQueue, kPrim>(P, L, n_hits, 32, W, n_open);
       __syncwarp();
     }
   }
-  if (n_hits) n_open = finish_rays<kPrim>(P, L, 0, n_hits, W, n_open);
+  if (n_hits) n_open = finish_rays<kUniform, kQueue, kPrim>(P, L, 0, n_hits, W, n_open);
   if constexpr (kPrim) {
-    if (n_open) settle_list(P, *W, n_open);
+    if (n_open) settle_camera(P, *W, n_open);
   }
   if (lane == 0) add_counts(c, queries, nodes, 0, tests);
 }
@@ -626,7 +636,7 @@ __device__ void activate_slot(const EngineParams& P, int e) {
   S.active = 1;
 }
 
-// After k_primary: starts the paths of the slots whose primary pass
+// After a pass of camera rays: starts the paths of the slots whose primary pass
 // completed and grants paths (one thread).
 __global__ void k_admit(EngineParams P) {
 #ifdef HPT_DEVICE_CHECKS
@@ -639,6 +649,25 @@ __global__ void k_admit(EngineParams P) {
   schedule(P);
 }
 
+// Settles open ray i of the queue of nQ paths with parity par: its hit as
+// P.hits would hold it, with triangle -1 for a miss. Called before anything of
+// the item is loaded: what is live across the call is spilled.
+__device__ __noinline__ void settle_queued(const EngineParams& P, int i, int par, int nQ,
+                                           uint4& hit) {
+  const uint4 e = P.open[i];
+  const int item = (int)e.x;
+  hit = make_uint4(e.x, 0xFFFFFFFFu, 0u, 0u);
+  if (item < 0 || item >= nQ) return;  // the caller's check 211
+  const float4 o = P.Q_o[par][item], d = P.Q_d[par][item];
+  const int slot = __float_as_int(P.Q_s[par][item].w);
+  HPT_DCHECK(&P.ctrl->err, slot >= 0 && slot < P.num_slots, 212, slot, return);
+  int tri = -1;
+  float t = __uint_as_float(e.w);
+  settle(P.jobs[slot].scene, Ray{mk(o.x, o.y, o.z), mk(d.x, d.y, d.z)}, e.y, e.z, P.ctrl, tri, t);
+  hit.y = (uint32_t)tri;
+  hit.z = __float_as_uint(t);
+}
+
 // ---------------------------------------------------------------------------
 // Shade + next direction (+ new paths), compacting survivors into R.
 // ---------------------------------------------------------------------------
@@ -647,21 +676,27 @@ __global__ void k_admit(EngineParams P) {
 // kernel is bound by gather latency, so resident warps can pay for a few
 // spills; the tuning chooses.
 template <int BS, int MINB>
-__global__ void __launch_bounds__(BS, MINB) k_shade(EngineParams P) {
+__global__ void __launch_bounds__(BS, MINB) k_shade(const __grid_constant__ EngineParams P) {
   __shared__ int warp_counts[BS / 32];
   __shared__ int block_base;
   DevCtrl* c = P.ctrl;
   const int par = c->parity;
-  const int nA = c->nA;
+  const int n_open = c->n_open[par], n_hit = c->n_hit[par], nQ = c->nQ;
   const int n_new = c->n_new, n_quota = c->n_quota;
-  const int n_items = nA + n_new;
+  const int n_items = n_open + n_hit + n_new;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned long long shades = 0;
 #ifdef HPT_DEVICE_CHECKS
   if (blockIdx.x == 0 && threadIdx.x == 0) c->chk_shade_items = n_items;
   int chk_items = 0;
 #endif
-  for (int base = blockIdx.x * BS; base < n_items; base += gridDim.x * BS) {
+  // The open hits come first (one may take a tree walk), and blocks take their
+  // next items from a cursor, so the others go on meanwhile.
+  while (true) {
+    if (threadIdx.x == 0) block_base = atomicAdd(&c->shade_head, BS);
+    __syncthreads();
+    const int base = block_base;
+    if (base >= n_items) break;
     const int i = base + threadIdx.x;
 #ifdef HPT_DEVICE_CHECKS
     if (i < n_items) ++chk_items;
@@ -675,25 +710,38 @@ __global__ void __launch_bounds__(BS, MINB) k_shade(EngineParams P) {
       f3 o, d, strength, rad;
       float t = 0.f;
       bool ok = true;
-      if (i < nA) {
-        HPT_DCHECK(&c->err, i < P.capacity, 211, i, ok = false);
+      if (i < n_open + n_hit) {
+        uint4 h;
+        if (i < n_open) settle_queued(P, i, par, nQ, h);
+        else h = P.hits[i - n_open];
+        const int item = (int)h.x;
+        HPT_DCHECK(&c->err, item >= 0 && item < nQ, 211, item, ok = false);
         if (ok) {
-          const float4 ao = P.A_o[par][i], ad = P.A_d[par][i], as = P.A_s[par][i],
-                       ar = P.A_r[par][i];
-          tri = P.A_tri[par][i];
-          o = mk(ao.x, ao.y, ao.z);
-          ray = __float_as_int(ao.w);
-          d = mk(ad.x, ad.y, ad.z);
-          const uint32_t meta = __float_as_uint(ad.w);
+          const float4 qo = P.Q_o[par][item], qd = P.Q_d[par][item], qs = P.Q_s[par][item],
+                       qr = P.Q_r[par][item];
+          tri = (int)h.y;
+          t = __uint_as_float(h.z);
+          o = mk(qo.x, qo.y, qo.z);
+          ray = __float_as_int(qo.w);
+          d = mk(qd.x, qd.y, qd.z);
+          const uint32_t meta = __float_as_uint(qd.w);
           sample = (int)(meta >> 8);
           bounce = (int)(meta & 0xFF);
-          strength = mk(as.x, as.y, as.z);
-          slot = __float_as_int(as.w);
-          rad = mk(ar.x, ar.y, ar.z);
-          t = ar.w;
+          strength = mk(qs.x, qs.y, qs.z);
+          slot = __float_as_int(qs.w);
+          rad = mk(qr.x, qr.y, qr.z);
+          HPT_DCHECK(&c->err, slot >= 0 && slot < P.num_slots, 212, slot, ok = false);
+          if (ok && tri < 0) {
+            // kernel.cl:195-200: miss adds background * strength (sample_n = 1).
+            const DevJob& J = P.jobs[slot];
+            HPT_DCHECK(&c->err, ray >= 0 && ray < job_rays(J), 224, ray, ok = false);
+            if (ok) flush_radiance(J, ray, add(rad, mul(mk(J.bg[0], J.bg[1], J.bg[2]), strength)));
+            ended = ok;
+            ok = false;
+          }
         }
       } else {
-        const int off = i - nA;
+        const int off = i - n_open - n_hit;
         const int e = find_prefix(P.quota_prefix, n_quota, off);
         slot = P.quota_slot[e];
         HPT_DCHECK(&c->err, slot >= 0 && slot < P.num_slots, 212, slot, ok = false);
@@ -774,10 +822,10 @@ __global__ void __launch_bounds__(BS, MINB) k_shade(EngineParams P) {
       bool ok = true;
       HPT_DCHECK(&c->err, pos < P.capacity, 216, pos, ok = false);
       if (ok) {
-        P.R_o[pos] = oo;
-        P.R_d[pos] = dd;
-        P.R_s[pos] = ss;
-        P.R_r[pos] = rr;
+        P.Q_o[par ^ 1][pos] = oo;
+        P.Q_d[par ^ 1][pos] = dd;
+        P.Q_s[par ^ 1][pos] = ss;
+        P.Q_r[par ^ 1][pos] = rr;
       }
     }
     __syncthreads();
@@ -790,32 +838,9 @@ __global__ void __launch_bounds__(BS, MINB) k_shade(EngineParams P) {
 #endif
 }
 
-// Settles the open rays of the intersect queue (all blocks), then advances
-// the queues and the path cursors and grants paths (one thread, of the block
-// that finishes last). The rays are dealt out over the warps first, lanes
-// second: they are few and their lookups are chains of loads.
-constexpr int kCtrlThreads = 128;
-__global__ void __launch_bounds__(kCtrlThreads) k_ctrl(const __grid_constant__ EngineParams P) {
+// Advances the queues and the path cursors, then grants paths (one thread).
+__global__ void k_ctrl(EngineParams P) {
   DevCtrl* c = P.ctrl;
-  const int n_open = c->n_open;
-  const int warps = gridDim.x * (kCtrlThreads / 32);
-  const int warp = (int)blockIdx.x + (int)gridDim.x * (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  for (int first = 0; first + warp < n_open; first += 32 * warps) {
-    const int i = first + lane * warps + warp;
-    const bool have = i < n_open;
-    uint4 e = make_uint4(0u, 0u, 0u, 0u);
-    if (have) e = P.open[i];
-    const int item = (int)e.x;
-    settle(P, have, item, have ? __float_as_int(P.R_s[item].w) : 0, e.y, e.z,
-           __uint_as_float(e.w));
-  }
-  // What this block wrote happens before the last block's reads.
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x != 0 || atomicAdd(&c->ticket, 1) != (int)gridDim.x - 1) return;
-  __threadfence();
-  c->ticket = 0;
-  c->n_open = 0;
 #ifdef HPT_DEVICE_CHECKS
   HPT_DCHECK(&c->err, c->chk_shade_done == c->chk_shade_items, 241,
              (long long)c->chk_shade_items * 1000000 + c->chk_shade_done, (void)0);
@@ -830,13 +855,15 @@ __global__ void __launch_bounds__(kCtrlThreads) k_ctrl(const __grid_constant__ E
     S.cursor += S.alloc;
     S.alloc = 0;
   }
-  c->nA = c->nA_next;
-  c->nA_next = 0;
+  c->nQ = c->nR;
   c->nR = 0;
+  c->shade_head = 0;
   c->isect_head = 0;
+  c->n_open[c->parity] = 0;
+  c->n_hit[c->parity] = 0;
   c->parity ^= 1;
   c->iterations += 1;
-  // Jobs whose primary pass the iteration's k_isect completed (kPrim).
+  // Jobs whose primary pass the iteration's k_trace completed (kPrim).
   for (int e = 0; e < P.prim_n; ++e) activate_slot(P, e);
   schedule(P);
 }
@@ -1036,18 +1063,7 @@ hpt_status Engine::init() {
 Engine::~Engine() {
   HPT_SOFT(cudaSetDevice(device));
   if (stream) HPT_SOFT(cudaStreamSynchronize(stream));
-  for (int p = 0; p < 2; ++p) {
-    HPT_SOFT(cudaFree(A_o_[p]));
-    HPT_SOFT(cudaFree(A_d_[p]));
-    HPT_SOFT(cudaFree(A_s_[p]));
-    HPT_SOFT(cudaFree(A_r_[p]));
-    HPT_SOFT(cudaFree(A_tri_[p]));
-  }
-  HPT_SOFT(cudaFree(R_o_));
-  HPT_SOFT(cudaFree(R_d_));
-  HPT_SOFT(cudaFree(R_s_));
-  HPT_SOFT(cudaFree(R_r_));
-  HPT_SOFT(cudaFree(open_));
+  free_queues();
   HPT_SOFT(cudaFree(ctrl_));
   HPT_SOFT(cudaFree(jobs_));
   HPT_SOFT(cudaFree(slot_state_));
@@ -1080,38 +1096,33 @@ Engine::~Engine() {
   if (stream) HPT_SOFT(cudaStreamDestroy(stream));
 }
 
+void Engine::free_queues() {
+  for (int p = 0; p < 2; ++p) {
+    HPT_SOFT(cudaFree(Q_o_[p]));
+    HPT_SOFT(cudaFree(Q_d_[p]));
+    HPT_SOFT(cudaFree(Q_s_[p]));
+    HPT_SOFT(cudaFree(Q_r_[p]));
+    Q_o_[p] = Q_d_[p] = Q_s_[p] = Q_r_[p] = nullptr;
+  }
+  HPT_SOFT(cudaFree(hits_));
+  HPT_SOFT(cudaFree(open_));
+  hits_ = nullptr;
+  open_ = nullptr;
+  capacity_ = 0;
+}
+
 hpt_status Engine::ensure_capacity(int capacity) {
   if (capacity <= capacity_) return HPT_OK;
   HPT_SOFT(cudaStreamSynchronize(stream));
-  for (int p = 0; p < 2; ++p) {
-    HPT_SOFT(cudaFree(A_o_[p]));
-    HPT_SOFT(cudaFree(A_d_[p]));
-    HPT_SOFT(cudaFree(A_s_[p]));
-    HPT_SOFT(cudaFree(A_r_[p]));
-    HPT_SOFT(cudaFree(A_tri_[p]));
-    A_o_[p] = A_d_[p] = A_s_[p] = A_r_[p] = nullptr;
-    A_tri_[p] = nullptr;
-  }
-  HPT_SOFT(cudaFree(R_o_));
-  HPT_SOFT(cudaFree(R_d_));
-  HPT_SOFT(cudaFree(R_s_));
-  HPT_SOFT(cudaFree(R_r_));
-  HPT_SOFT(cudaFree(open_));
-  R_o_ = R_d_ = R_s_ = R_r_ = nullptr;
-  open_ = nullptr;
-  capacity_ = 0;
+  free_queues();
   const size_t n = (size_t)capacity;
   for (int p = 0; p < 2; ++p) {
-    HPT_CUDA(cudaMalloc(&A_o_[p], n * sizeof(float4)));
-    HPT_CUDA(cudaMalloc(&A_d_[p], n * sizeof(float4)));
-    HPT_CUDA(cudaMalloc(&A_s_[p], n * sizeof(float4)));
-    HPT_CUDA(cudaMalloc(&A_r_[p], n * sizeof(float4)));
-    HPT_CUDA(cudaMalloc(&A_tri_[p], n * sizeof(int32_t)));
+    HPT_CUDA(cudaMalloc(&Q_o_[p], n * sizeof(float4)));
+    HPT_CUDA(cudaMalloc(&Q_d_[p], n * sizeof(float4)));
+    HPT_CUDA(cudaMalloc(&Q_s_[p], n * sizeof(float4)));
+    HPT_CUDA(cudaMalloc(&Q_r_[p], n * sizeof(float4)));
   }
-  HPT_CUDA(cudaMalloc(&R_o_, n * sizeof(float4)));
-  HPT_CUDA(cudaMalloc(&R_d_, n * sizeof(float4)));
-  HPT_CUDA(cudaMalloc(&R_s_, n * sizeof(float4)));
-  HPT_CUDA(cudaMalloc(&R_r_, n * sizeof(float4)));
+  HPT_CUDA(cudaMalloc(&hits_, n * sizeof(uint4)));
   HPT_CUDA(cudaMalloc(&open_, n * sizeof(uint4)));
   capacity_ = capacity;
   return HPT_OK;
@@ -1254,8 +1265,8 @@ static EngineParams make_params(const Engine& e, DevCtrl* ctrl, DevJob* jobs, De
                                 int num_slots, const int32_t* order, int32_t* quota_slot,
                                 int32_t* quota_prefix, const int32_t* prim_slot,
                                 const int64_t* prim_prefix, int prim_n, int capacity,
-                                float4* const* A, int32_t* const* Atri,
-                                float4* const* R, uint4* open, const DevScene* shared) {
+                                float4* const* Q, uint4* hits, uint4* open,
+                                const DevScene* shared) {
   EngineParams P;
   memset(&P, 0, sizeof P);
   P.jobs = jobs;
@@ -1269,16 +1280,12 @@ static EngineParams make_params(const Engine& e, DevCtrl* ctrl, DevJob* jobs, De
   P.prim_prefix = prim_prefix;
   P.prim_n = prim_n;
   for (int p = 0; p < 2; ++p) {
-    P.A_o[p] = A[4 * p + 0];
-    P.A_d[p] = A[4 * p + 1];
-    P.A_s[p] = A[4 * p + 2];
-    P.A_r[p] = A[4 * p + 3];
-    P.A_tri[p] = Atri[p];
+    P.Q_o[p] = Q[4 * p + 0];
+    P.Q_d[p] = Q[4 * p + 1];
+    P.Q_s[p] = Q[4 * p + 2];
+    P.Q_r[p] = Q[4 * p + 3];
   }
-  P.R_o = R[0];
-  P.R_d = R[1];
-  P.R_s = R[2];
-  P.R_r = R[3];
+  P.hits = hits;
   P.open = open;
   P.capacity = capacity;
   P.refill = std::max(1, std::min(32, e.tuning.refill_chunk));
@@ -1338,11 +1345,10 @@ hpt_status Engine::admit(const std::vector<int>& slot_ids, const std::vector<Dev
                            stream));
   HPT_CUDA(cudaMemcpyAsync(prim_prefix_, host_i64_, (n + 1) * sizeof(int64_t),
                            cudaMemcpyHostToDevice, stream));
-  float4* A[8] = {A_o_[0], A_d_[0], A_s_[0], A_r_[0], A_o_[1], A_d_[1], A_s_[1], A_r_[1]};
-  float4* R[4] = {R_o_, R_d_, R_s_, R_r_};
+  float4* Q[8] = {Q_o_[0], Q_d_[0], Q_s_[0], Q_r_[0], Q_o_[1], Q_d_[1], Q_s_[1], Q_r_[1]};
   EngineParams P = make_params(*this, ctrl_, jobs_, slot_state_, slots_, order_, quota_slot_,
-                               quota_prefix_, prim_slot_, prim_prefix_, n, capacity_, A, A_tri_,
-                               R, open_, shared_scene);
+                               quota_prefix_, prim_slot_, prim_prefix_, n, capacity_, Q, hits_,
+                               open_, shared_scene);
   const IsectVariant& v = kIsectVariants[isect_variant()];
   v.primary[P.uniform_scene]<<<num_sms * occ_isect_, v.block, 0, stream>>>(P);
   HPT_CUDA(cudaGetLastError());
@@ -1492,17 +1498,16 @@ hpt_status Engine::launch_iteration_async() {
   pend_rays_.clear();
   pend_first_.clear();
   pend_final_.clear();
-  float4* A[8] = {A_o_[0], A_d_[0], A_s_[0], A_r_[0], A_o_[1], A_d_[1], A_s_[1], A_r_[1]};
-  float4* R[4] = {R_o_, R_d_, R_s_, R_r_};
+  float4* Q[8] = {Q_o_[0], Q_d_[0], Q_s_[0], Q_r_[0], Q_o_[1], Q_d_[1], Q_s_[1], Q_r_[1]};
   EngineParams P = make_params(*this, ctrl_, jobs_, slot_state_, slots_, order_, quota_slot_,
-                               quota_prefix_, prim_slot_, prim_prefix_, n, capacity_, A, A_tri_,
-                               R, open_, nullptr);
+                               quota_prefix_, prim_slot_, prim_prefix_, n, capacity_, Q, hits_,
+                               open_, nullptr);
   P.prim_first = prim_first_;
   P.prim_final = prim_final_;
   shade_kernel(tuning)<<<num_sms * occ_shade_, 256, 0, stream>>>(P);
   const IsectVariant& v = kIsectVariants[isect_variant()];
   v.both[0]<<<num_sms * occ_isect_, v.block, 0, stream>>>(P);
-  k_ctrl<<<4 * num_sms, kCtrlThreads, 0, stream>>>(P);
+  k_ctrl<<<1, 1, 0, stream>>>(P);
   HPT_CUDA(cudaGetLastError());
   return HPT_OK;
 }
@@ -1562,18 +1567,17 @@ hpt_status Engine::ensure_graph(const DevScene* shared_scene, int iterations) {
 }
 
 void Engine::launch_iteration(const DevScene* shared_scene, cudaEvent_t* ev) {
-  float4* A[8] = {A_o_[0], A_d_[0], A_s_[0], A_r_[0], A_o_[1], A_d_[1], A_s_[1], A_r_[1]};
-  float4* R[4] = {R_o_, R_d_, R_s_, R_r_};
+  float4* Q[8] = {Q_o_[0], Q_d_[0], Q_s_[0], Q_r_[0], Q_o_[1], Q_d_[1], Q_s_[1], Q_r_[1]};
   EngineParams P = make_params(*this, ctrl_, jobs_, slot_state_, slots_, order_, quota_slot_,
-                               quota_prefix_, prim_slot_, prim_prefix_, 0, capacity_, A, A_tri_,
-                               R, open_, shared_scene);
+                               quota_prefix_, prim_slot_, prim_prefix_, 0, capacity_, Q, hits_,
+                               open_, shared_scene);
   if (ev) HPT_SOFT(cudaEventRecord(ev[0], stream));
   shade_kernel(tuning)<<<num_sms * occ_shade_, 256, 0, stream>>>(P);
   if (ev) HPT_SOFT(cudaEventRecord(ev[1], stream));
   const IsectVariant& v = kIsectVariants[isect_variant()];
   v.isect[P.uniform_scene]<<<num_sms * occ_isect_, v.block, 0, stream>>>(P);
   if (ev) HPT_SOFT(cudaEventRecord(ev[2], stream));
-  k_ctrl<<<4 * num_sms, kCtrlThreads, 0, stream>>>(P);
+  k_ctrl<<<1, 1, 0, stream>>>(P);
 }
 
 void Engine::launch_resolve(int slot, const JobSpec& js, const JobBuffers& b, float samples) {

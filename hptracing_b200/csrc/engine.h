@@ -133,17 +133,14 @@ class Engine {
   int64_t* host_i64_ = nullptr;
   DevJob* host_jobs_ = nullptr;
   DevSlot* slots_host_ = nullptr;  // pinned mirror for read_slots
-  // Shade queues (double-buffered) and the intersect queue.
-  float4* A_o_[2] = {nullptr, nullptr};
-  float4* A_d_[2] = {nullptr, nullptr};
-  float4* A_s_[2] = {nullptr, nullptr};
-  float4* A_r_[2] = {nullptr, nullptr};
-  int32_t* A_tri_[2] = {nullptr, nullptr};
-  float4* R_o_ = nullptr;
-  float4* R_d_ = nullptr;
-  float4* R_s_ = nullptr;
-  float4* R_r_ = nullptr;
-  uint4* open_ = nullptr;  // rays whose hits are open (k_ctrl settles them)
+  // The queue of paths (double-buffered) and what its rays hit.
+  float4* Q_o_[2] = {nullptr, nullptr};
+  float4* Q_d_[2] = {nullptr, nullptr};
+  float4* Q_s_[2] = {nullptr, nullptr};
+  float4* Q_r_[2] = {nullptr, nullptr};
+  uint4* hits_ = nullptr;
+  uint4* open_ = nullptr;  // rays whose hits are open (k_shade settles them)
+  void free_queues();
   cudaEvent_t ev_[6];
   cudaEvent_t ev_done_[2] = {nullptr, nullptr};
   std::vector<cudaEvent_t> pev_;  // profiling events, created on first use
