@@ -214,7 +214,7 @@ struct DevCtrl {
   int32_t chk_shade_items;
   int32_t chk_shade_done;
   int32_t chk_isect_done;
-  int32_t chk_pad;
+  int32_t ticket;           // blocks of the running launch that are done
   // Per queue, after it was traced: rays in the hit list and the open list.
   int32_t n_hit[2], n_open[2];
   // Started-but-unfinished paths all capped slots (max_inflight > 0) may

@@ -14,7 +14,6 @@
 //                ray's hit goes to the hit list, its miss adds background *
 //                strength; camera hits go to a per-job cache, misses add
 //                background * sample.
-//   k_admit    - sets each new job's path count and grants paths.
 //   k_shade    - for each hit: self-emission, normal / UV / texture, branch
 //                choice and next direction (s1_run + s2_*_run fused); new
 //                (primary hit, sample) paths are started in the same pass
@@ -22,9 +21,10 @@
 //                block scan, one atomic per block) into the other queue;
 //                finished paths flush their radiance. Hits that k_trace
 //                leaves open are settled here first.
-//   k_ctrl     - advances queue counters and path cursors and grants the
-//                free wavefront capacity to the active jobs in priority
-//                order (the host never reads stage sizes).
+//                The last block advances queue counters and path cursors,
+//                sets new jobs' path counts and grants the free wavefront
+//                capacity to the active jobs in priority order (the host never
+//                reads stage sizes).
 //   k_resolve  - fixed-point accumulators -> get_image's tone map.
 // Every random number is drawn from a stream keyed by (job, ray, sample,
 // bounce) and radiance is summed in 2^-32 fixed point, so a job's image does
@@ -159,7 +159,9 @@ __device__ __forceinline__ void add_counts(DevCtrl* c, uint32_t queries, uint32_
 // (one thread). A slot with nothing left to issue no longer needs grants.
 __device__ void schedule(const EngineParams& P) {
   DevCtrl* c = P.ctrl;
-  const int budget = P.capacity - (c->n_hit[c->parity] + c->n_open[c->parity]);
+  // Counts that other blocks of this launch added to are read past L1.
+  const int budget =
+      P.capacity - (__ldcg(&c->n_hit[c->parity]) + __ldcg(&c->n_open[c->parity]));
   int n_new = 0, nq = 0;
   bool remaining = false;
   // Paths the capped slots hold now, against their shared budget.
@@ -169,7 +171,7 @@ __device__ void schedule(const EngineParams& P) {
       const int s = P.order[k];
       if (s < 0 || s >= P.num_slots) continue;
       const DevSlot& S = P.slots[s];
-      if (S.active && S.max_inflight > 0) capped += S.cursor - (int64_t)S.done;
+      if (S.active && S.max_inflight > 0) capped += S.cursor - (int64_t)__ldcg(&S.done);
     }
   for (int k = 0; k < c->n_order; ++k) {
     const int s = P.order[k];
@@ -185,7 +187,7 @@ __device__ void schedule(const EngineParams& P) {
     // latency-sensitive ones behind it) keeps at most max_inflight paths
     // started and unfinished.
     if (S.max_inflight > 0) {
-      grant = min(grant, S.max_inflight - (S.cursor - (int64_t)S.done));
+      grant = min(grant, S.max_inflight - (S.cursor - (int64_t)__ldcg(&S.done)));
       if (c->capped_budget > 0) grant = min(grant, c->capped_budget - capped);
     }
     const int a = (int)grant;
@@ -465,6 +467,82 @@ __device__ __noinline__ int finish_rays(const EngineParams& P, const HitList<kPr
   return push_open<kQueue, kPrim>(P, W, n_open, have && !certain, item, slot, best, tie, t);
 }
 
+// Sets the path count of primary-pass entry e's slot when the entry
+// completes its job's primary pass. A slot whose primary pass is still
+// partial stays as it was: inactive, or finished with nothing left to issue.
+__device__ void activate_slot(const EngineParams& P, int e) {
+  const int s = P.prim_slot[e];
+  HPT_DCHECK(&P.ctrl->err, s >= 0 && s < P.num_slots, 232, s, return);
+  if (P.prim_final && !P.prim_final[e]) return;
+  DevSlot& S = P.slots[s];
+  S.num_paths = (int64_t)__ldcg(P.jobs[s].prim_count) * P.jobs[s].spp;
+  S.cursor = 0;
+  S.done = 0;
+  S.queries = 0;
+  S.max_inflight = P.jobs[s].max_inflight;
+  S.alloc = 0;
+  S.active = 1;
+}
+
+// After a pass of camera rays: starts the paths of the slots whose primary
+// pass completed and grants paths (one thread).
+__device__ void admit(const EngineParams& P) {
+#ifdef HPT_DEVICE_CHECKS
+  HPT_DCHECK(&P.ctrl->err, __ldcg(&P.ctrl->chk_isect_done) == P.prim_prefix[P.prim_n], 243,
+             P.ctrl->chk_isect_done, (void)0);
+  P.ctrl->chk_isect_done = 0;
+#endif
+  for (int e = 0; e < P.prim_n; ++e) activate_slot(P, e);
+  P.ctrl->prim_head = 0;
+  schedule(P);
+}
+
+// Advances the queues and the path cursors, then grants paths (one thread).
+__device__ void control(const EngineParams& P) {
+  DevCtrl* c = P.ctrl;
+#ifdef HPT_DEVICE_CHECKS
+  HPT_DCHECK(&c->err, c->chk_shade_done == c->chk_shade_items, 241,
+             (long long)c->chk_shade_items * 1000000 + c->chk_shade_done, (void)0);
+  const int traced = __ldcg(&c->chk_isect_done);
+  HPT_DCHECK(&c->err, traced == c->nR + (P.prim_n ? P.prim_prefix[P.prim_n] : 0), 242,
+             (long long)c->nR * 1000000 + traced, (void)0);
+  c->chk_shade_items = 0;
+  c->chk_shade_done = 0;
+  c->chk_isect_done = 0;
+#endif
+  for (int k = 0; k < c->n_quota; ++k) {
+    DevSlot& S = P.slots[P.quota_slot[k]];
+    S.cursor += S.alloc;
+    S.alloc = 0;
+  }
+  c->nQ = c->nR;
+  c->nR = 0;
+  c->shade_head = 0;
+  c->isect_head = 0;
+  c->n_open[c->parity] = 0;
+  c->n_hit[c->parity] = 0;
+  c->parity ^= 1;
+  c->iterations += 1;
+  // Jobs whose primary pass the iteration's k_trace completed (kPrim).
+  for (int e = 0; e < P.prim_n; ++e) activate_slot(P, e);
+  schedule(P);
+}
+
+// The end of a launch's last block (one thread of it, after every block is
+// done): a launch that ends with it needs none of its own for it.
+__device__ __forceinline__ bool last_block(DevCtrl* c) {
+  // What this block wrote happens before the last block's reads.
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x != 0 || atomicAdd(&c->ticket, 1) != (int)gridDim.x - 1) return false;
+  __threadfence();
+  c->ticket = 0;
+  return true;
+}
+
+// An iteration's control without a trace (the run's last).
+__global__ void k_ctrl(EngineParams P) { control(P); }
+
 // Test rounds run when at least this share (in eighths) of the warp's live
 // lanes hold pending triangles.
 #ifndef HPT_TEST_EIGHTHS
@@ -473,9 +551,9 @@ __device__ __noinline__ int finish_rays(const EngineParams& P, const HitList<kPr
 
 // kUniform: every job of the launch renders P.uscene. kQueue: traces the
 // queue; kPrim: traces the camera rays of the launch's primary-pass
-// entries (P.prim_*), after the queue's; k_admit (or, with kQueue, k_ctrl)
-// then starts the paths of the jobs whose primary pass completed. A serving
-// loop admits requests with both, with no launch of its own.
+// entries (P.prim_*), after the queue's. The last block to finish advances the
+// queues, starts the paths of the jobs whose primary pass completed and grants
+// paths. A serving loop admits requests with both, with no launch of its own.
 //
 // A round of the warp runs one code path: a node visit for the lanes without
 // pending triangles, or one triangle test for those with some.
@@ -617,36 +695,10 @@ __global__ void __launch_bounds__(BS, MINB) k_trace(const __grid_constant__ Engi
     if (n_open) settle_camera(P, *W, n_open);
   }
   if (lane == 0) add_counts(c, queries, nodes, 0, tests);
-}
-
-// Sets the path count of primary-pass entry e's slot when the entry
-// completes its job's primary pass. A slot whose primary pass is still
-// partial stays as it was: inactive, or finished with nothing left to issue.
-__device__ void activate_slot(const EngineParams& P, int e) {
-  const int s = P.prim_slot[e];
-  HPT_DCHECK(&P.ctrl->err, s >= 0 && s < P.num_slots, 232, s, return);
-  if (P.prim_final && !P.prim_final[e]) return;
-  DevSlot& S = P.slots[s];
-  S.num_paths = (int64_t)(*P.jobs[s].prim_count) * P.jobs[s].spp;
-  S.cursor = 0;
-  S.done = 0;
-  S.queries = 0;
-  S.max_inflight = P.jobs[s].max_inflight;
-  S.alloc = 0;
-  S.active = 1;
-}
-
-// After a pass of camera rays: starts the paths of the slots whose primary pass
-// completed and grants paths (one thread).
-__global__ void k_admit(EngineParams P) {
-#ifdef HPT_DEVICE_CHECKS
-  HPT_DCHECK(&P.ctrl->err, P.ctrl->chk_isect_done == P.prim_prefix[P.prim_n], 243,
-             P.ctrl->chk_isect_done, (void)0);
-  P.ctrl->chk_isect_done = 0;
-#endif
-  for (int e = 0; e < P.prim_n; ++e) activate_slot(P, e);
-  P.ctrl->prim_head = 0;
-  schedule(P);
+  if (last_block(c)) {
+    if (kQueue) control(P);
+    else admit(P);
+  }
 }
 
 // Settles open ray i of the queue of nQ paths with parity par: its hit as
@@ -836,36 +888,6 @@ __global__ void __launch_bounds__(BS, MINB) k_shade(const __grid_constant__ Engi
   for (int o = 16; o > 0; o >>= 1) chk_items += __shfl_down_sync(kFull, chk_items, o);
   if (lane == 0 && chk_items) atomicAdd(&c->chk_shade_done, chk_items);
 #endif
-}
-
-// Advances the queues and the path cursors, then grants paths (one thread).
-__global__ void k_ctrl(EngineParams P) {
-  DevCtrl* c = P.ctrl;
-#ifdef HPT_DEVICE_CHECKS
-  HPT_DCHECK(&c->err, c->chk_shade_done == c->chk_shade_items, 241,
-             (long long)c->chk_shade_items * 1000000 + c->chk_shade_done, (void)0);
-  HPT_DCHECK(&c->err, c->chk_isect_done == c->nR + (P.prim_n ? P.prim_prefix[P.prim_n] : 0),
-             242, (long long)c->nR * 1000000 + c->chk_isect_done, (void)0);
-  c->chk_shade_items = 0;
-  c->chk_shade_done = 0;
-  c->chk_isect_done = 0;
-#endif
-  for (int k = 0; k < c->n_quota; ++k) {
-    DevSlot& S = P.slots[P.quota_slot[k]];
-    S.cursor += S.alloc;
-    S.alloc = 0;
-  }
-  c->nQ = c->nR;
-  c->nR = 0;
-  c->shade_head = 0;
-  c->isect_head = 0;
-  c->n_open[c->parity] = 0;
-  c->n_hit[c->parity] = 0;
-  c->parity ^= 1;
-  c->iterations += 1;
-  // Jobs whose primary pass the iteration's k_trace completed (kPrim).
-  for (int e = 0; e < P.prim_n; ++e) activate_slot(P, e);
-  schedule(P);
 }
 
 // Register budgets of the closest-hit kernels: (threads per block, blocks per
@@ -1204,29 +1226,36 @@ hpt_status Engine::alloc_job(const JobSpec& js, bool want_accum, JobBuffers& b) 
   const hpt_render_params& p = js.params;
   const int64_t nx = (int64_t)p.sample_x * p.supersample_x, ny = (int64_t)p.sample_y * p.supersample_y;
   b.rays = nx * ny;
-  auto take = [&](auto** ptr, size_t bytes) {
-    return cudaMallocFromPoolAsync(reinterpret_cast<void**>(ptr), bytes, pool_, stream);
+  // One allocation and one clear: accumulators, flags and hit count first.
+  size_t size = 0;
+  auto part = [&](size_t bytes) {
+    const size_t at = size;
+    size += (bytes + 255) & ~(size_t)255;
+    return at;
   };
-  HPT_CUDA(take(&b.accum, (size_t)b.rays * 3 * sizeof(unsigned long long)));
-  HPT_CUDA(take(&b.flags, (size_t)b.rays * sizeof(uint32_t)));
-  HPT_CUDA(take(&b.prim, (size_t)b.rays * 8 * sizeof(float)));
-  HPT_CUDA(take(&b.prim_count, sizeof(int32_t)));
-  HPT_CUDA(take(&b.rgba, (size_t)p.sample_x * p.sample_y * 4));
-  if (want_accum) HPT_CUDA(take(&b.accum_f, (size_t)b.rays * 3 * sizeof(float)));
-  HPT_CUDA(cudaMemsetAsync(b.accum, 0, (size_t)b.rays * 3 * sizeof(unsigned long long), stream));
-  HPT_CUDA(cudaMemsetAsync(b.flags, 0, (size_t)b.rays * sizeof(uint32_t), stream));
-  HPT_CUDA(cudaMemsetAsync(b.prim_count, 0, sizeof(int32_t), stream));
+  const size_t accum = part((size_t)b.rays * 3 * sizeof(unsigned long long));
+  const size_t flags = part((size_t)b.rays * sizeof(uint32_t));
+  const size_t count = part(sizeof(int32_t));
+  const size_t cleared = size;
+  const size_t prim = part((size_t)b.rays * 8 * sizeof(float));
+  const size_t rgba = part((size_t)p.sample_x * p.sample_y * 4);
+  const size_t accum_f = want_accum ? part((size_t)b.rays * 3 * sizeof(float)) : 0;
+  void* mem = nullptr;
+  HPT_CUDA(cudaMallocFromPoolAsync(&mem, size, pool_, stream));
+  b.base = static_cast<uint8_t*>(mem);
+  b.accum = reinterpret_cast<unsigned long long*>(b.base + accum);
+  b.flags = reinterpret_cast<uint32_t*>(b.base + flags);
+  b.prim_count = reinterpret_cast<int32_t*>(b.base + count);
+  b.prim = reinterpret_cast<float*>(b.base + prim);
+  b.rgba = b.base + rgba;
+  if (want_accum) b.accum_f = reinterpret_cast<float*>(b.base + accum_f);
+  HPT_CUDA(cudaMemsetAsync(b.base, 0, cleared, stream));
   b.bytes = job_footprint(p, want_accum);
   return HPT_OK;
 }
 
 void Engine::free_job(JobBuffers& b) {
-  HPT_SOFT(cudaFreeAsync(b.accum, stream));
-  HPT_SOFT(cudaFreeAsync(b.flags, stream));
-  HPT_SOFT(cudaFreeAsync(b.prim, stream));
-  HPT_SOFT(cudaFreeAsync(b.prim_count, stream));
-  HPT_SOFT(cudaFreeAsync(b.rgba, stream));
-  if (b.accum_f) HPT_SOFT(cudaFreeAsync(b.accum_f, stream));
+  if (b.base) HPT_SOFT(cudaFreeAsync(b.base, stream));
   b = JobBuffers();
 }
 
@@ -1302,11 +1331,18 @@ void Engine::reset_ctrl() {
   if (slots_ > 0) HPT_SOFT(cudaMemsetAsync(slot_state_, 0, (size_t)slots_ * sizeof(DevSlot), stream));
 }
 
-hpt_status Engine::set_order(const std::vector<int>& order) {
+// The run's uploads go through pinned staging that is free again when run()
+// has synchronised: [0, slots] prim_slot, [slots + 1, 2 slots + 1] order,
+// [2 slots + 2] n_order.
+hpt_status Engine::admit(const std::vector<int>& slot_ids, const std::vector<DevJob>& jobs,
+                         const std::vector<int64_t>& rays, const std::vector<int>& order,
+                         const DevScene* shared_scene) {
+  const int n = (int)slot_ids.size();
+  {
+    hpt_status qs = query_occupancy();
+    if (qs != HPT_OK) return qs;
+  }
   if ((int)order.size() > slots_) return fail(HPT_ERR_INVALID_ARGUMENT, "order larger than slots");
-  // Pinned staging: [0, slots] prim_slot (admit), [slots + 1, 2 slots + 1]
-  // order, [2 slots + 2] n_order. Regions never overlap, so a copy still
-  // queued behind a kernel reads what was written for it.
   int32_t* stage = host_i32_ + (slots_ + 1);
   for (size_t k = 0; k < order.size(); ++k) stage[k] = order[k];
   if (!order.empty())
@@ -1315,20 +1351,6 @@ hpt_status Engine::set_order(const std::vector<int>& order) {
   stage[slots_ + 1] = (int32_t)order.size();
   HPT_CUDA(cudaMemcpyAsync(&ctrl_->n_order, &stage[slots_ + 1], sizeof(int32_t),
                            cudaMemcpyHostToDevice, stream));
-  // The pinned staging is reused by the next call: wait for these copies.
-  HPT_CUDA(cudaStreamSynchronize(stream));
-  return HPT_OK;
-}
-
-hpt_status Engine::admit(const std::vector<int>& slot_ids, const std::vector<DevJob>& jobs,
-                         const std::vector<int64_t>& rays, const std::vector<int>& order,
-                         const DevScene* shared_scene) {
-  const int n = (int)slot_ids.size();
-  if (n == 0) return set_order(order);
-  {
-    hpt_status qs = query_occupancy();
-    if (qs != HPT_OK) return qs;
-  }
   for (int k = 0; k < n; ++k) {
     if (slot_ids[k] < 0 || slot_ids[k] >= slots_)
       return fail(HPT_ERR_INVALID_ARGUMENT, "slot %d out of range", slot_ids[k]);
@@ -1350,13 +1372,15 @@ hpt_status Engine::admit(const std::vector<int>& slot_ids, const std::vector<Dev
                                quota_prefix_, prim_slot_, prim_prefix_, n, capacity_, Q, hits_,
                                open_, shared_scene);
   const IsectVariant& v = kIsectVariants[isect_variant()];
-  v.primary[P.uniform_scene]<<<num_sms * occ_isect_, v.block, 0, stream>>>(P);
-  HPT_CUDA(cudaGetLastError());
-  hpt_status s = set_order(order);  // synchronises: the staging is free again
-  if (s != HPT_OK) return s;
-  k_admit<<<1, 1, 0, stream>>>(P);
+  v.primary[P.uniform_scene]<<<trace_grid(host_i64_[n]), v.block, 0, stream>>>(P);
   HPT_CUDA(cudaGetLastError());
   return HPT_OK;
+}
+
+// Blocks of a launch over at most `items` rays: all that fit, or for few rays
+// one per warp's worth, so that they spread over the SMs.
+int Engine::trace_grid(int64_t items) const {
+  return (int)std::max<int64_t>(1, std::min<int64_t>(num_sms * occ_isect_, (items + 31) / 32));
 }
 
 // --- Asynchronous uploads (serving loop) ------------------------------------
@@ -1481,7 +1505,7 @@ hpt_status Engine::queue_primary(int slot, const DevJob& job, int64_t rays, int6
 hpt_status Engine::launch_iteration_async() {
   const int n = (int)pend_slot_.size();
   if (n == 0) {
-    launch_iteration(nullptr);
+    launch_iteration(nullptr, nullptr, capacity_, false);
     return HPT_OK;
   }
   hpt_status s = query_occupancy();
@@ -1507,7 +1531,6 @@ hpt_status Engine::launch_iteration_async() {
   shade_kernel(tuning)<<<num_sms * occ_shade_, 256, 0, stream>>>(P);
   const IsectVariant& v = kIsectVariants[isect_variant()];
   v.both[0]<<<num_sms * occ_isect_, v.block, 0, stream>>>(P);
-  k_ctrl<<<1, 1, 0, stream>>>(P);
   HPT_CUDA(cudaGetLastError());
   return HPT_OK;
 }
@@ -1541,7 +1564,8 @@ hpt_status Engine::ensure_graph(const DevScene* shared_scene, int iterations) {
   }
   cudaGraph_t g = nullptr;
   HPT_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-  for (int k = 0; k < iterations; ++k) launch_iteration(shared_scene, nullptr);
+  for (int k = 0; k < iterations; ++k)
+    launch_iteration(shared_scene, nullptr, capacity_, false);
   const cudaError_t launch = cudaGetLastError();
   const cudaError_t end = cudaStreamEndCapture(stream, &g);
   if (launch != cudaSuccess) {
@@ -1566,18 +1590,20 @@ hpt_status Engine::ensure_graph(const DevScene* shared_scene, int iterations) {
   return HPT_OK;
 }
 
-void Engine::launch_iteration(const DevScene* shared_scene, cudaEvent_t* ev) {
+void Engine::launch_iteration(const DevScene* shared_scene, cudaEvent_t* ev, int64_t paths,
+                              bool last) {
   float4* Q[8] = {Q_o_[0], Q_d_[0], Q_s_[0], Q_r_[0], Q_o_[1], Q_d_[1], Q_s_[1], Q_r_[1]};
   EngineParams P = make_params(*this, ctrl_, jobs_, slot_state_, slots_, order_, quota_slot_,
                                quota_prefix_, prim_slot_, prim_prefix_, 0, capacity_, Q, hits_,
                                open_, shared_scene);
   if (ev) HPT_SOFT(cudaEventRecord(ev[0], stream));
-  shade_kernel(tuning)<<<num_sms * occ_shade_, 256, 0, stream>>>(P);
+  const int64_t shade_blocks = std::min<int64_t>(num_sms * occ_shade_, (paths + 255) / 256);
+  shade_kernel(tuning)<<<(int)std::max<int64_t>(1, shade_blocks), 256, 0, stream>>>(P);
   if (ev) HPT_SOFT(cudaEventRecord(ev[1], stream));
   const IsectVariant& v = kIsectVariants[isect_variant()];
-  v.isect[P.uniform_scene]<<<num_sms * occ_isect_, v.block, 0, stream>>>(P);
+  if (last) k_ctrl<<<1, 1, 0, stream>>>(P);
+  else v.isect[P.uniform_scene]<<<trace_grid(paths), v.block, 0, stream>>>(P);
   if (ev) HPT_SOFT(cudaEventRecord(ev[2], stream));
-  k_ctrl<<<1, 1, 0, stream>>>(P);
 }
 
 void Engine::launch_resolve(int slot, const JobSpec& js, const JobBuffers& b, float samples) {
@@ -1693,23 +1719,30 @@ hpt_status Engine::run(const std::vector<JobSpec>& jobs, hpt_render_stats* stats
   // Iterate until the device says the wavefront is drained. Batches of
   // iterations are queued ahead; the done flag of batch k is checked while
   // batch k+1 runs (extra iterations after completion are empty launches).
+  // When the queue holds every path of the run, all start in the first
+  // iteration and each has ended after as many as its depth: those are
+  // launched, and no others.
   const int kBatch = 4;
   const bool prof = tuning.profile != 0;
+  const bool at_once = paths <= capacity_ && (tuning.use_graph == 0 || prof);
+  int max_depth = 1;
+  for (const JobSpec& js : jobs) max_depth = std::max(max_depth, js.params.depth);
   int32_t* done_host = done_host_;
   done_host[0] = done_host[1] = 0;
   cudaEvent_t* ev_done = ev_done_;
   std::vector<cudaEvent_t>& pev = pev_;
-  if (prof && pev.empty()) {
-    pev.resize(2 * kBatch * 3);
-    for (auto& e : pev) HPT_CUDA(cudaEventCreate(&e));
-  }
+  if (prof)
+    while ((int)pev.size() < 3 * std::max(2 * kBatch, at_once ? max_depth : 0)) {
+      cudaEvent_t e = nullptr;
+      HPT_CUDA(cudaEventCreate(&e));
+      pev.push_back(e);
+    }
   float ms_shade = 0.f, ms_isect = 0.f;
-  auto harvest = [&](int sl) {
-    for (int k = 0; k < kBatch; ++k) {
-      cudaEvent_t* e = &pev[(sl * kBatch + k) * 3];
+  auto harvest = [&](int first, int count) {
+    for (int k = first; k < first + count; ++k) {
       float a = 0.f, b = 0.f;
-      HPT_SOFT(cudaEventElapsedTime(&a, e[0], e[1]));
-      HPT_SOFT(cudaEventElapsedTime(&b, e[1], e[2]));
+      HPT_SOFT(cudaEventElapsedTime(&a, pev[3 * k], pev[3 * k + 1]));
+      HPT_SOFT(cudaEventElapsedTime(&b, pev[3 * k + 1], pev[3 * k + 2]));
       ms_shade += a;
       ms_isect += b;
     }
@@ -1718,12 +1751,10 @@ hpt_status Engine::run(const std::vector<JobSpec>& jobs, hpt_render_stats* stats
   // iteration, so the wavefront drains within paths * depth / capacity
   // iterations plus one path lifetime; 2x that plus slack is the cap.
   int64_t work = 0;
-  int max_depth = 1;
   for (const JobSpec& js : jobs) {
     const hpt_render_params& p = js.params;
     work += (int64_t)p.sample_x * p.supersample_x * p.sample_y * p.supersample_y * p.sample *
             p.depth;
-    max_depth = std::max(max_depth, p.depth);
   }
   const int64_t max_batches = (2 * (work / std::max(1, capacity_) + max_depth) + 64) / kBatch + 4;
   // With use_graph, the kBatch iterations are replayed from one CUDA graph
@@ -1743,18 +1774,21 @@ hpt_status Engine::run(const std::vector<JobSpec>& jobs, hpt_render_stats* stats
   bool drained = false;
   int slot = 0;
   bool pending = false;
-  while (true) {
+  for (int k = 0; at_once && k < max_depth; ++k)
+    launch_iteration(shared_dev, prof ? &pev[3 * k] : nullptr, paths, k == max_depth - 1);
+  while (!at_once) {
     if (use_graph) {
       HPT_CUDA(cudaGraphLaunch(graph_exec_, stream));
     } else {
       for (int k = 0; k < kBatch; ++k)
-        launch_iteration(shared_dev, prof ? &pev[(slot * kBatch + k) * 3] : nullptr);
+        launch_iteration(shared_dev, prof ? &pev[(slot * kBatch + k) * 3] : nullptr, capacity_,
+                         false);
     }
     HPT_SOFT(cudaMemcpyAsync(&done_host[slot], &ctrl_->done, sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
     HPT_SOFT(cudaEventRecord(ev_done[slot], stream));
     if (pending) {
       HPT_SOFT(cudaEventSynchronize(ev_done[slot ^ 1]));
-      if (prof) harvest(slot ^ 1);
+      if (prof) harvest((slot ^ 1) * kBatch, kBatch);
       if (done_host[slot ^ 1]) {
         drained = true;
         break;
@@ -1775,9 +1809,11 @@ hpt_status Engine::run(const std::vector<JobSpec>& jobs, hpt_render_stats* stats
       HPT_SOFT(cudaMemcpyAsync(jobs[j].accum_out, bufs[j].accum_f, (size_t)bufs[j].rays * 3 * sizeof(float), cudaMemcpyDeviceToHost, stream));
   }
   HPT_SOFT(cudaMemcpyAsync(ctrl_host_, ctrl_, sizeof(DevCtrl), cudaMemcpyDeviceToHost, stream));
+  HPT_SOFT(cudaMemcpyAsync(slots_host_, slot_state_, n * sizeof(DevSlot), cudaMemcpyDeviceToHost,
+                           stream));
   for (auto& b : bufs) free_job(b);
   cudaError_t e = cudaStreamSynchronize(stream);
-  if (prof) harvest(slot);
+  if (prof) harvest(at_once ? 0 : slot * kBatch, at_once ? max_depth : kBatch);
   if (e != cudaSuccess) return cuda_fail(e, "render");
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "render launch");
@@ -1800,15 +1836,7 @@ hpt_status Engine::run(const std::vector<JobSpec>& jobs, hpt_render_stats* stats
     stats->leaves_visited = (int64_t)ctrl_host_->leaves_visited;
     stats->triangle_tests = (int64_t)ctrl_host_->tri_tests;
     stats->triangle_repeats = (int64_t)ctrl_host_->tri_repeats;
-    std::vector<DevSlot> st(n);
-    const cudaError_t ce =
-        cudaMemcpy(st.data(), slot_state_, n * sizeof(DevSlot), cudaMemcpyDeviceToHost);
-    if (ce != cudaSuccess) cuda_soft_fail(ce, "slot state read-back");
-    if (ce == cudaSuccess) {
-      int64_t paths = 0;
-      for (const DevSlot& x : st) paths += x.num_paths;
-      stats->paths = paths;
-    }
+    for (int j = 0; j < n; ++j) stats->paths += slots_host_[j].num_paths;
   }
   if (ctrl_host_->err.flags & 2u)
     return fail(HPT_ERR_INVALID_SCENE, "device self-check %d failed (value %lld)",

@@ -36,6 +36,7 @@ struct JobSpec {
 
 // Per-job device buffers (owned by the engine while the job runs).
 struct JobBuffers {
+  uint8_t* base = nullptr;  // the one allocation the others point into
   unsigned long long* accum = nullptr;  // 3 per ray, fixed point
   uint32_t* flags = nullptr;            // non-finite markers per ray
   float* prim = nullptr;                // primary hit cache
@@ -76,7 +77,6 @@ class Engine {
   hpt_status admit(const std::vector<int>& slot_ids, const std::vector<DevJob>& jobs,
                    const std::vector<int64_t>& rays, const std::vector<int>& order,
                    const DevScene* shared_scene);
-  hpt_status set_order(const std::vector<int>& order);
   // Asynchronous forms for a serving loop: the uploads go through a ring of
   // pinned staging sets and nothing waits for the stream (only, rarely, for
   // a staging set's previous copies to have run).
@@ -84,9 +84,9 @@ class Engine {
   // Serving loop: a newly admitted job's camera rays are traced inside the
   // next iteration's closest-hit launch, so that admissions add no launch of
   // their own (and a large job's can be split over several iterations, so
-  // that no launch stalls the others for long). queue_primary() records rays [first, first + rays) of the
-  // job in `slot` (parts of one job in order; final_part on the last, which
-  // starts its paths); launch_iteration_async() uploads what was queued and
+  // that no launch stalls the others for long). queue_primary() records rays
+  // [first, first + rays) of the job in `slot` (parts of one job in order;
+  // final_part on the last, which starts its paths); launch_iteration_async() uploads what was queued and
   // launches one iteration that carries it.
   hpt_status queue_primary(int slot, const DevJob& job, int64_t rays, int64_t first,
                            bool final_part);
@@ -94,7 +94,10 @@ class Engine {
   // Enqueues a copy of the slot table and control block into pinned host
   // memory and records ev after it.
   hpt_status read_state_async(DevSlot* slots, DevCtrl* ctrl, cudaEvent_t ev);
-  void launch_iteration(const DevScene* shared_scene, cudaEvent_t* ev3 = nullptr);
+  // One iteration over a queue of at most `paths` paths; `last`: the run's last,
+  // after which nothing is left to trace.
+  void launch_iteration(const DevScene* shared_scene, cudaEvent_t* ev3, int64_t paths,
+                        bool last);
   // Captures `iterations` consecutive iterations into graph_exec_ (kept
   // until the queues, slots, shared scene or tuning change).
   hpt_status ensure_graph(const DevScene* shared_scene, int iterations);
@@ -173,6 +176,7 @@ class Engine {
   hpt_status init_status_ = HPT_OK;
   hpt_status init();
   int occ_isect_ = 1, occ_shade_ = 1;
+  int trace_grid(int64_t items) const;
   bool occ_done_ = false;
   hpt_status query_occupancy();
 };
