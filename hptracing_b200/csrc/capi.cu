@@ -63,6 +63,72 @@ struct DBuf {
   }
 };
 
+// One stage call on a scene: its buffers are parts of one allocation from the
+// scene's own stream-ordered pool, and everything runs on the scene's stage
+// stream. (A cudaMalloc and cudaFree per buffer took 8 to 60 ms of a call on
+// 1M rays; the pool keeps up to kStagePoolKeep mapped and goes with the
+// scene.)
+constexpr uint64_t kStagePoolKeep = 256ull << 20;
+class StageCall {
+ public:
+  explicit StageCall(SceneHandle& h) : h_(h) {}
+  ~StageCall() {
+    if (base_) HPT_SOFT(cudaFreeAsync(base_, h_.stage_stream));
+    if (h_.stage_stream) HPT_SOFT(cudaStreamSynchronize(h_.stage_stream));
+  }
+  // Reserves a buffer; returns its number.
+  int add(size_t bytes) {
+    at_.push_back(size_);
+    bytes_.push_back(bytes);
+    size_ += (bytes + 255) & ~(size_t)255;
+    return (int)at_.size() - 1;
+  }
+  // Allocates what was reserved.
+  hpt_status begin() {
+    HPT_CUDA(cudaSetDevice(h_.scene.device));
+    if (!h_.stage_stream) {
+      HPT_CUDA(cudaStreamCreateWithFlags(&h_.stage_stream, cudaStreamNonBlocking));
+      cudaMemPoolProps props;
+      memset(&props, 0, sizeof props);
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = h_.scene.device;
+      HPT_CUDA(cudaMemPoolCreate(&h_.stage_pool, &props));
+      uint64_t keep = kStagePoolKeep;
+      HPT_CUDA(cudaMemPoolSetAttribute(h_.stage_pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    }
+    void* p = nullptr;
+    HPT_CUDA(cudaMallocFromPoolAsync(&p, size_, h_.stage_pool, h_.stage_stream));
+    base_ = static_cast<uint8_t*>(p);
+    return HPT_OK;
+  }
+  template <typename T>
+  T* ptr(int k) const {
+    return reinterpret_cast<T*>(base_ + at_[k]);
+  }
+  hpt_status up(int k, const void* host) {
+    HPT_CUDA(cudaMemcpyAsync(base_ + at_[k], host, bytes_[k], cudaMemcpyHostToDevice,
+                             h_.stage_stream));
+    return HPT_OK;
+  }
+  hpt_status down(int k, void* host) {
+    HPT_CUDA(cudaMemcpyAsync(host, base_ + at_[k], bytes_[k], cudaMemcpyDeviceToHost,
+                             h_.stage_stream));
+    return HPT_OK;
+  }
+  hpt_status wait() {
+    HPT_CUDA(cudaStreamSynchronize(h_.stage_stream));
+    return HPT_OK;
+  }
+  cudaStream_t stream() const { return h_.stage_stream; }
+
+ private:
+  SceneHandle& h_;
+  uint8_t* base_ = nullptr;
+  size_t size_ = 0;
+  std::vector<size_t> at_, bytes_;
+};
+
 // ---------------------------------------------------------------------------
 // Stage kernels (one thread per element).
 // ---------------------------------------------------------------------------
@@ -570,6 +636,8 @@ void hpt_scene_destroy(hpt_scene* scene) {
     std::lock_guard<std::mutex> lk(scene->h.mu);
     scene->h.engine.reset();
     release_scene(scene->h.scene);
+    if (scene->h.stage_stream) HPT_SOFT(cudaStreamDestroy(scene->h.stage_stream));
+    if (scene->h.stage_pool) HPT_SOFT(cudaMemPoolDestroy(scene->h.stage_pool));
   }
   delete scene;
 }
@@ -648,22 +716,20 @@ hpt_status hpt_intersect(hpt_scene* scene, int32_t n, const float* origins,
   if (n == 0) return HPT_OK;
   return guarded([&]() -> hpt_status {
     std::lock_guard<std::mutex> lk(scene->h.mu);
-    HPT_CUDA(cudaSetDevice(scene->h.scene.device));
-    DBuf o, d, tri, t, u, v, err;
-    hpt_status s;
     const size_t b3 = (size_t)n * 3 * sizeof(float), b1 = (size_t)n * 4;
-    if ((s = o.up(origins, b3)) || (s = d.up(directions, b3)) || (s = tri.alloc(b1)) ||
-        (s = t.alloc(b1)) || (s = u.alloc(b1)) || (s = v.alloc(b1)) ||
-        (s = err.alloc(sizeof(DevErr))))
-      return s;
-    HPT_CUDA(cudaMemset(err.p, 0, sizeof(DevErr)));
-    k_stage_intersect<<<blocks_for(n, 128), 128>>>(scene->h.scene.d_scene, n, o.as<float>(),
-                                                   d.as<float>(), tri.as<int32_t>(), t.as<float>(),
-                                                   u.as<float>(), v.as<float>(), err.as<DevErr>());
+    StageCall c(scene->h);
+    const int o = c.add(b3), d = c.add(b3), tri = c.add(b1), t = c.add(b1), u = c.add(b1),
+              v = c.add(b1), err = c.add(sizeof(DevErr));
+    hpt_status s;
+    if ((s = c.begin()) || (s = c.up(o, origins)) || (s = c.up(d, directions))) return s;
+    HPT_CUDA(cudaMemsetAsync(c.ptr<DevErr>(err), 0, sizeof(DevErr), c.stream()));
+    k_stage_intersect<<<blocks_for(n, 128), 128, 0, c.stream()>>>(
+        scene->h.scene.d_scene, n, c.ptr<float>(o), c.ptr<float>(d), c.ptr<int32_t>(tri),
+        c.ptr<float>(t), c.ptr<float>(u), c.ptr<float>(v), c.ptr<DevErr>(err));
     HPT_CUDA(cudaGetLastError());
     DevErr e;
-    if ((s = tri.down(tri_out)) || (s = t.down(t_out)) || (s = u.down(u_out)) || (s = v.down(v_out)) ||
-        (s = err.down(&e)))
+    if ((s = c.down(tri, tri_out)) || (s = c.down(t, t_out)) || (s = c.down(u, u_out)) ||
+        (s = c.down(v, v_out)) || (s = c.down(err, &e)) || (s = c.wait()))
       return s;
     if (e.flags & 2u)
       return fail(HPT_ERR_INVALID_SCENE, "device self-check %d failed (value %lld)", e.site,
@@ -687,25 +753,27 @@ hpt_status hpt_shade(hpt_scene* scene, int32_t n, const float* origins, const fl
       return fail(HPT_ERR_INVALID_ARGUMENT, "shade: triangle id %d out of range", tris[i]);
   return guarded([&]() -> hpt_status {
     std::lock_guard<std::mutex> lk(scene->h.mu);
-    HPT_CUDA(cudaSetDevice(scene->h.scene.device));
     const size_t b3 = (size_t)n * 3 * sizeof(float), b1 = (size_t)n * 4, b8 = (size_t)n * 8;
-    DBuf o, d, st, tri, t, sd, co, br, hp, nm, so, pa;
+    StageCall c(scene->h);
+    const int o = c.add(b3), d = c.add(b3), st = c.add(b3), tri = c.add(b1), t = c.add(b1),
+              sd = c.add(b8), co = c.add(b3), br = c.add(b1), hp = c.add(b3), nm = c.add(b3),
+              so = c.add(b3), pa = c.add(b1);
     hpt_status s;
-    if ((s = o.up(origins, b3)) || (s = d.up(directions, b3)) || (s = st.up(strengths, b3)) ||
-        (s = tri.up(tris, b1)) || (s = t.up(ts, b1)) || (s = sd.up(seeds, b8)) ||
-        (s = co.alloc(b3)) || (s = br.alloc(b1)) || (s = hp.alloc(b3)) || (s = nm.alloc(b3)) ||
-        (s = so.alloc(b3)) || (s = pa.alloc(b1)))
+    if ((s = c.begin()) || (s = c.up(o, origins)) || (s = c.up(d, directions)) ||
+        (s = c.up(st, strengths)) || (s = c.up(tri, tris)) || (s = c.up(t, ts)) ||
+        (s = c.up(sd, seeds)))
       return s;
-    k_stage_shade<<<blocks_for(n, 128), 128>>>(
-        scene->h.scene.d_scene, n, o.as<float>(), d.as<float>(), st.as<float>(), tri.as<int32_t>(),
-        t.as<float>(), sd.as<uint64_t>(), disable_diffuse, co.as<float>(), br.as<int32_t>(),
-        hp.as<float>(), nm.as<float>(), so.as<float>(), pa.as<float>());
+    k_stage_shade<<<blocks_for(n, 128), 128, 0, c.stream()>>>(
+        scene->h.scene.d_scene, n, c.ptr<float>(o), c.ptr<float>(d), c.ptr<float>(st),
+        c.ptr<int32_t>(tri), c.ptr<float>(t), c.ptr<uint64_t>(sd), disable_diffuse,
+        c.ptr<float>(co), c.ptr<int32_t>(br), c.ptr<float>(hp), c.ptr<float>(nm),
+        c.ptr<float>(so), c.ptr<float>(pa));
     HPT_CUDA(cudaGetLastError());
-    if ((s = sd.down(seeds)) || (s = co.down(contrib)) || (s = br.down(branch)) ||
-        (s = hp.down(hit_p)) || (s = nm.down(normal)) || (s = so.down(strength_out)) ||
-        (s = pa.down(param)))
+    if ((s = c.down(sd, seeds)) || (s = c.down(co, contrib)) || (s = c.down(br, branch)) ||
+        (s = c.down(hp, hit_p)) || (s = c.down(nm, normal)) || (s = c.down(so, strength_out)) ||
+        (s = c.down(pa, param)))
       return s;
-    return HPT_OK;
+    return c.wait();
   });
 }
 
@@ -721,25 +789,26 @@ hpt_status hpt_next_dir(hpt_scene* scene, int32_t n, const int32_t* branch,
   if (n == 0) return HPT_OK;
   return guarded([&]() -> hpt_status {
     std::lock_guard<std::mutex> lk(scene->h.mu);
-    HPT_CUDA(cudaSetDevice(scene->h.scene.device));
     const size_t b3 = (size_t)n * 3 * sizeof(float), b1 = (size_t)n * 4, b8 = (size_t)n * 8;
-    DBuf br, d, hp, nm, st, pa, sd, oo, dd, so, al;
+    StageCall c(scene->h);
+    const int br = c.add(b1), d = c.add(b3), hp = c.add(b3), nm = c.add(b3), st = c.add(b3),
+              pa = c.add(b1), sd = c.add(b8), oo = c.add(b3), dd = c.add(b3), so = c.add(b3),
+              al = c.add(b1);
     hpt_status s;
-    if ((s = br.up(branch, b1)) || (s = d.up(directions, b3)) || (s = hp.up(hit_p, b3)) ||
-        (s = nm.up(normal, b3)) || (s = st.up(strengths, b3)) || (s = pa.up(param, b1)) ||
-        (s = sd.up(seeds, b8)) || (s = oo.alloc(b3)) || (s = dd.alloc(b3)) || (s = so.alloc(b3)) ||
-        (s = al.alloc(b1)))
+    if ((s = c.begin()) || (s = c.up(br, branch)) || (s = c.up(d, directions)) ||
+        (s = c.up(hp, hit_p)) || (s = c.up(nm, normal)) || (s = c.up(st, strengths)) ||
+        (s = c.up(pa, param)) || (s = c.up(sd, seeds)))
       return s;
-    k_stage_next<<<blocks_for(n, 128), 128>>>(scene->h.scene.d_scene, n, br.as<int32_t>(),
-                                              d.as<float>(), hp.as<float>(), nm.as<float>(),
-                                              st.as<float>(), pa.as<float>(), sd.as<uint64_t>(),
-                                              oo.as<float>(), dd.as<float>(), so.as<float>(),
-                                              al.as<int32_t>());
+    k_stage_next<<<blocks_for(n, 128), 128, 0, c.stream()>>>(
+        scene->h.scene.d_scene, n, c.ptr<int32_t>(br), c.ptr<float>(d), c.ptr<float>(hp),
+        c.ptr<float>(nm), c.ptr<float>(st), c.ptr<float>(pa), c.ptr<uint64_t>(sd),
+        c.ptr<float>(oo), c.ptr<float>(dd), c.ptr<float>(so), c.ptr<int32_t>(al));
     HPT_CUDA(cudaGetLastError());
-    if ((s = sd.down(seeds)) || (s = oo.down(origins_out)) || (s = dd.down(directions_out)) ||
-        (s = so.down(strength_out)) || (s = al.down(alive_out)))
+    if ((s = c.down(sd, seeds)) || (s = c.down(oo, origins_out)) ||
+        (s = c.down(dd, directions_out)) || (s = c.down(so, strength_out)) ||
+        (s = c.down(al, alive_out)))
       return s;
-    return HPT_OK;
+    return c.wait();
   });
 }
 

@@ -185,6 +185,8 @@ struct SceneHandle {
   SceneDev scene;
   std::mutex mu;
   std::unique_ptr<Engine> engine;
+  cudaStream_t stage_stream = nullptr;  // stage entry points (created on first use)
+  cudaMemPool_t stage_pool = nullptr;
   hpt_render_stats last_stats{};
   hpt_tuning tuning{};
 };
