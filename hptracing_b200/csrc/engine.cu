@@ -143,6 +143,43 @@ __device__ __forceinline__ void count_queries(DevSlot* slots, bool alive, int sl
     atomicAdd(&slots[slot].queries, (unsigned long long)__popc(same & m));
 }
 
+// A warp's counts for one slot, kept in shared memory by its lane 0 and added
+// to the slot when another slot comes up and at the end of the kernel: one
+// atomic on a slot's counter per 32 paths is what the warps would queue for
+// when all paths are of one job.
+struct Tally {
+  int slot;
+  uint32_t done, queries;
+};
+
+__device__ __forceinline__ void flush_tally(DevSlot* slots, Tally& w) {
+  if ((threadIdx.x & 31) == 0) {
+    if (w.done) atomicAdd(&slots[w.slot].done, (unsigned long long)w.done);
+    if (w.queries) atomicAdd(&slots[w.slot].queries, (unsigned long long)w.queries);
+    w.slot = 0;
+    w.done = w.queries = 0;
+  }
+}
+
+// Counts finished and surviving paths of the warp's lanes by slot.
+__device__ __forceinline__ void count_paths(DevSlot* slots, Tally& w, bool done, bool alive,
+                                            int slot) {
+  const unsigned dm = __ballot_sync(kFull, done), am = __ballot_sync(kFull, alive);
+  if (!(dm | am)) return;
+  const int s = __shfl_sync(kFull, slot, __ffs(dm | am) - 1);
+  if (__ballot_sync(kFull, (done || alive) && slot != s) == 0) {
+    if ((threadIdx.x & 31) == 0) {
+      if (w.slot != s) flush_tally(slots, w);
+      w.slot = s;
+      w.done += __popc(dm);
+      w.queries += __popc(am);
+    }
+  } else {
+    count_done(slots, done, slot);
+    count_queries(slots, alive, slot);
+  }
+}
+
 // Adds a warp's query and work counts to the control block (lane 0 calls).
 __device__ __forceinline__ void add_counts(DevCtrl* c, uint32_t queries, uint32_t nodes,
                                            uint32_t leaves, uint32_t tests) {
@@ -723,20 +760,28 @@ __device__ __noinline__ void settle_queued(const EngineParams& P, int i, int par
 // ---------------------------------------------------------------------------
 // Shade + next direction (+ new paths), compacting survivors into R.
 // ---------------------------------------------------------------------------
-// MINB: blocks of BS threads per SM the register budget must fit (1 leaves
-// the compiler's natural allocation, ~106 registers = 2 blocks of 256). The
-// kernel is bound by gather latency, so resident warps can pay for a few
-// spills; the tuning chooses.
-template <int BS, int MINB>
+// Bound by gather latency with half of its lanes idle (the four kinds of next
+// ray; DRAM at 18 % of its rate): hence the one copy of the random direction
+// for two of them (shading.cuh), no atomic that all warps queue for (count_paths,
+// the block's one cursor step and one queue step for BS items - one of each per
+// warp costs 5 % more), and 32 warps per SM against a few spills. Over the 58 M
+// paths of 512x512x64 on 100 K triangles: 6.94 ms before these three, 6.26 now.
+// MINB: blocks of BS threads per SM the register budget must fit (1 leaves the
+// compiler's natural allocation of ~150); the tuning chooses.
+// kUniform: every job renders P.uscene, whose pointers are constant operands.
+template <int BS, int MINB, bool kUniform>
 __global__ void __launch_bounds__(BS, MINB) k_shade(const __grid_constant__ EngineParams P) {
   __shared__ int warp_counts[BS / 32];
   __shared__ int block_base;
+  __shared__ Tally tallies[BS / 32];
   DevCtrl* c = P.ctrl;
   const int par = c->parity;
   const int n_open = c->n_open[par], n_hit = c->n_hit[par], nQ = c->nQ;
   const int n_new = c->n_new, n_quota = c->n_quota;
   const int n_items = n_open + n_hit + n_new;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  Tally& tally = tallies[warp];
+  if (lane == 0) tally = Tally{0, 0, 0};
   unsigned long long shades = 0;
 #ifdef HPT_DEVICE_CHECKS
   if (blockIdx.x == 0 && threadIdx.x == 0) c->chk_shade_items = n_items;
@@ -804,8 +849,8 @@ __global__ void __launch_bounds__(BS, MINB) k_shade(const __grid_constant__ Engi
           HPT_DCHECK(&c->err, nh > 0 && q < (int64_t)nh * J.spp, 213, q, ok = false);
           HPT_DCHECK(&c->err, !ok || nh <= job_rays(J), 217, nh, ok = false);
           if (ok) {
-            const int64_t k = q % nh;
-            sample = (int)(q / nh);
+            sample = q <= 0xFFFFFFFFll ? (int)((uint32_t)q / (uint32_t)nh) : (int)(q / nh);
+            const int64_t k = q - (int64_t)sample * nh;
             bounce = 0;
             const float4* src = reinterpret_cast<const float4*>(J.prim) + 2 * k;
             const float4 p0 = src[0], p1 = src[1];
@@ -825,18 +870,19 @@ __global__ void __launch_bounds__(BS, MINB) k_shade(const __grid_constant__ Engi
       HPT_DCHECK(&c->err, !ok || (ray >= 0 && ray < job_rays(P.jobs[slot])), 215, ray, ok = false);
       if (ok) {
         const DevJob& J = P.jobs[slot];
+        const DevScene& sc = kUniform ? P.uscene : J.scene;
         // The frame's sample index keys the random stream, so a render of
         // samples [first_sample, first_sample + spp) traces the same paths
         // as those samples of one whole-frame render.
         uint64_t seed = path_seed(J.seed, (uint32_t)ray, (uint32_t)(J.first_sample + sample),
                                   (uint32_t)bounce);
         const Ray r{o, d};
-        const ShadeOut so = shade_hit(J.scene, r, strength, tri, t, J.disable_diffuse, seed,
+        const ShadeOut so = shade_hit(sc, r, strength, tri, t, J.disable_diffuse, seed,
                                       &c->err);
         ++shades;
         rad = add(rad, so.contrib);
         if (so.branch != kDead && bounce + 1 < J.depth) {
-          const NextOut no = next_direction(J.scene, so.branch, d, so.hit_p, so.normal,
+          const NextOut no = next_direction(sc, so.branch, d, so.hit_p, so.normal,
                                             so.strength, so.param, seed, &c->err);
           if (no.alive) {
             alive = true;
@@ -853,8 +899,7 @@ __global__ void __launch_bounds__(BS, MINB) k_shade(const __grid_constant__ Engi
         }
       }
     }
-    count_done(P.slots, ended, slot);
-    count_queries(P.slots, alive, slot);
+    count_paths(P.slots, tally, ended, alive, slot);
     // Block-level stable compaction: ballot per warp, scan over warps.
     const unsigned m = __ballot_sync(kFull, alive);
     if (lane == 0) warp_counts[warp] = __popc(m);
@@ -882,6 +927,7 @@ __global__ void __launch_bounds__(BS, MINB) k_shade(const __grid_constant__ Engi
     }
     __syncthreads();
   }
+  flush_tally(P.slots, tally);
   for (int o = 16; o > 0; o >>= 1) shades += __shfl_down_sync(kFull, shades, o);
   if (lane == 0 && shades) atomicAdd(&c->shades, shades);
 #ifdef HPT_DEVICE_CHECKS
@@ -914,10 +960,10 @@ constexpr int kNumIsectVariants = sizeof(kIsectVariants) / sizeof(kIsectVariants
 
 // The shading kernel for a tuning's register budget (shade_min_blocks 3 or
 // 4 blocks of 256 per SM; anything else: the natural allocation).
-void (*shade_kernel(const hpt_tuning& t))(EngineParams) {
-  if (t.shade_min_blocks == 3) return k_shade<256, 3>;
-  if (t.shade_min_blocks == 4) return k_shade<256, 4>;
-  return k_shade<256, 1>;
+void (*shade_kernel(const hpt_tuning& t, bool uniform))(EngineParams) {
+  if (t.shade_min_blocks == 3) return uniform ? k_shade<256, 3, true> : k_shade<256, 3, false>;
+  if (t.shade_min_blocks == 4) return uniform ? k_shade<256, 4, true> : k_shade<256, 4, false>;
+  return uniform ? k_shade<256, 1, true> : k_shade<256, 1, false>;
 }
 
 __device__ __forceinline__ float ray_value(const unsigned long long* acc, const uint32_t* flags,
@@ -1216,7 +1262,7 @@ hpt_status Engine::query_occupancy() {
   HPT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
       &b, v.isect[1], v.block, 0));
   occ_isect_ = std::max(1, b);
-  HPT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, shade_kernel(tuning), 256, 0));
+  HPT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, shade_kernel(tuning, false), 256, 0));
   occ_shade_ = std::max(1, b);
   occ_done_ = true;
   return HPT_OK;
@@ -1528,7 +1574,7 @@ hpt_status Engine::launch_iteration_async() {
                                open_, nullptr);
   P.prim_first = prim_first_;
   P.prim_final = prim_final_;
-  shade_kernel(tuning)<<<num_sms * occ_shade_, 256, 0, stream>>>(P);
+  shade_kernel(tuning, P.uniform_scene)<<<num_sms * occ_shade_, 256, 0, stream>>>(P);
   const IsectVariant& v = kIsectVariants[isect_variant()];
   v.both[0]<<<num_sms * occ_isect_, v.block, 0, stream>>>(P);
   HPT_CUDA(cudaGetLastError());
@@ -1598,7 +1644,7 @@ void Engine::launch_iteration(const DevScene* shared_scene, cudaEvent_t* ev, int
                                open_, shared_scene);
   if (ev) HPT_SOFT(cudaEventRecord(ev[0], stream));
   const int64_t shade_blocks = std::min<int64_t>(num_sms * occ_shade_, (paths + 255) / 256);
-  shade_kernel(tuning)<<<(int)std::max<int64_t>(1, shade_blocks), 256, 0, stream>>>(P);
+  shade_kernel(tuning, P.uniform_scene)<<<(int)std::max<int64_t>(1, shade_blocks), 256, 0, stream>>>(P);
   if (ev) HPT_SOFT(cudaEventRecord(ev[1], stream));
   const IsectVariant& v = kIsectVariants[isect_variant()];
   if (last) k_ctrl<<<1, 1, 0, stream>>>(P);

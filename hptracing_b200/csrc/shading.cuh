@@ -222,28 +222,28 @@ HPT_HD NextOut next_direction(const DevScene& s, int branch, f3 in_dir,
     } else {
       dir = add(add(in_dir, p), p);
     }
-  } else if (branch == kSpecular) {
-    f3 rv = randf3(seed);
-    rv = divs(divs(rv, 2.0f), param);
+  } else if (branch == kSpecular || branch == kDiffuse) {
+    // One copy of the draw for both: a warp with lanes of either kind runs
+    // its four trigonometric calls once.
+    const f3 rv = randf3(seed);
     const float d_ = dot(in_dir, normal);
-    const f3 projection = scale(d_, normal);
-    dir = sub(in_dir, scale(2.0f, projection));
-    dir = add(dir, rv);
-  } else if (branch == kDiffuse) {
-    const bool front = dot(in_dir, normal) < 0.f;
-    f3 p = randf3(seed);
-    float dn = dot(p, normal);
-    if (dn < 0.f) {
-      dn = -dn;
-      if (front) p = neg(p);
+    if (branch == kSpecular) {
+      const f3 projection = scale(d_, normal);
+      dir = add(sub(in_dir, scale(2.0f, projection)), divs(divs(rv, 2.0f), param));
+    } else {
+      float dn = dot(rv, normal);
+      dir = rv;
+      if (dn < 0.f) {
+        dn = -dn;
+        if (d_ < 0.f) dir = neg(rv);
+      }
+      out.strength = scale(dn, strength);
     }
-    out.strength = scale(dn, strength);
-    dir = p;
   } else if (branch == kLight) {
     if (s.num_lights == 0) return out;
     const bool front = dot(in_dir, normal) < 0.f;
     const uint32_t ri = lcg_next(seed);
-    const int li = (int)((int64_t)ri % (int64_t)s.num_lights);
+    const int li = (int)(ri % (uint32_t)s.num_lights);
     HPT_DCHECK(err, li >= 0 && li < s.num_lights, 307, li, return out);
     const int4 light = ldg(reinterpret_cast<const int4*>(s.lights) + li);
     HPT_DCHECK(err, light.x >= 0 && light.x < s.num_points && light.y >= 0 &&
