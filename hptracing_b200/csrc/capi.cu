@@ -231,160 +231,158 @@ __global__ void k_stage_resolve(const float* accum, int W, int H, int ssx, int s
   out[3] = 0;
 }
 
-// --- Stream compaction: per-tile counts, then a stable scatter. ----------
-// A tile is 4096 flags: 256 threads x 16 consecutive flags, read as four
-// 16-byte loads where the flag array is 16-byte aligned and the tile is
-// whole. The flags are read once: the count pass also stores each thread's
-// 16 flags as a 16-bit mask (n / 8 bytes in all), which the scatter pass
-// reads instead of the flags. Tiles are grouped into superblocks of
-// 2^shift tiles with shift = ceil(log2(tiles) / 2); the count pass adds
-// each tile's count to its superblock's total, and the scatter pass finds a
-// tile's output offset by summing at most 2^shift superblock totals and
-// 2^shift tile counts (L2-resident) instead of waiting for a scan. No
+// --- Stream compaction: per-warp counts, then a stable scatter. ----------
+// The flags are split into rows of 32, and the rows into one contiguous share
+// per warp of at most kCompactMaxWarps (8 blocks of 8 warps on each of 148
+// SMs: what is resident at once, so large arrays run as one full wave). The
+// count pass reads the flags once and stores each row as a 32-bit mask
+// (n / 8 bytes in all) and the survivors of each warp's share and of each
+// block's; the scatter pass, with the same shares, finds a warp's output
+// position by summing the earlier blocks' and warps' counts (L2-resident)
+// instead of waiting for a scan, and reads the masks instead of the flags. No
 // kernel waits on another block: the two passes are ordered by the stream.
+// At n = 2^25, half of them set, the passes read 134 MB and write 67 MB, 31 us
+// at the copy rate, in 48.7 us (27 us counting, bound by DRAM; the scatter by
+// its instructions per row). One 4,096-flag tile per block, with a memset and
+// atomics for the tiles' totals: 55.3 us. At n <= 300,000, where launches
+// count, 9.1 us against 12.2.
 constexpr int kCompactThreads = 256;
-constexpr int kCompactItems = 16;
-constexpr int kCompactTile = kCompactThreads * kCompactItems;
+constexpr int kCompactWarps = kCompactThreads / 32;
+constexpr int kCompactMaxBlocks = 148 * 8;
+constexpr int kCompactMaxWarps = kCompactMaxBlocks * kCompactWarps;
+constexpr int kCompactBatch = 16;  // rows a warp has in flight
 
-inline int compact_super_shift(int tiles) {
-  int s = 0;
-  while ((int64_t)1 << (2 * s) < tiles) ++s;
-  return s;
-}
-inline int compact_supers(int tiles, int shift) { return (tiles + (1 << shift) - 1) >> shift; }
-
-// This thread's 16 flags as a bit mask (bit k: flag i0 + k nonzero).
-__device__ __forceinline__ uint32_t load_flags16(const uint32_t* flags, int64_t i0, int n,
-                                                 bool vec) {
-  uint32_t m = 0;
-  if (vec && i0 + kCompactItems <= n) {
-    const uint4* p = reinterpret_cast<const uint4*>(flags + i0);
-    const uint4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2), d = __ldg(p + 3);
-    m = (a.x != 0) | (a.y != 0) << 1 | (a.z != 0) << 2 | (a.w != 0) << 3 | (b.x != 0) << 4 |
-        (b.y != 0) << 5 | (b.z != 0) << 6 | (b.w != 0) << 7 | (c.x != 0) << 8 |
-        (c.y != 0) << 9 | (c.z != 0) << 10 | (c.w != 0) << 11 | (d.x != 0) << 12 |
-        (d.y != 0) << 13 | (d.z != 0) << 14 | (d.w != 0) << 15;
-  } else {
-    for (int k = 0; k < kCompactItems; ++k)
-      if (i0 + k < n && __ldg(flags + i0 + k) != 0) m |= 1u << k;
-  }
-  return m;
-}
-
-// Exclusive scan of one value per thread over a block of BS threads;
-// *total receives the block's sum. Two barriers.
-template <int BS>
-__device__ __forceinline__ int block_exclusive_scan(int v, int* total) {
-  __shared__ int warp_tot[BS / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int inc = v;
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xFFFFFFFFu, inc, o);
-    if (lane >= o) inc += y;
-  }
-  if (lane == 31) warp_tot[warp] = inc;
-  __syncthreads();
-  if (warp == 0) {
-    int t = lane < BS / 32 ? warp_tot[lane] : 0;
-    int ti = t;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xFFFFFFFFu, ti, o);
-      if (lane >= o) ti += y;
-    }
-    if (lane < BS / 32) warp_tot[lane] = ti - t;  // exclusive warp offsets
-    const int all = __shfl_sync(0xFFFFFFFFu, ti, 31);
-    if (lane == 0) *total = all;
-  }
-  __syncthreads();
-  return warp_tot[warp] + inc - v;
+struct CompactShape {
+  int64_t rows;  // of 32 flags
+  int share;     // rows per warp, a multiple of kCompactBatch
+  int blocks;
+};
+inline CompactShape compact_shape(int64_t n) {
+  CompactShape c;
+  c.rows = (n + 31) / 32;
+  const int64_t per = (c.rows + kCompactMaxWarps - 1) / kCompactMaxWarps;
+  c.share = (int)((per + kCompactBatch - 1) / kCompactBatch * kCompactBatch);
+  c.blocks = (int)((c.rows + (int64_t)c.share * kCompactWarps - 1) / ((int64_t)c.share * kCompactWarps));
+  return c;
 }
 
 __global__ void __launch_bounds__(kCompactThreads)
-    k_compact_count(const uint32_t* flags, int n, int shift, int* tile_counts, int* super_counts,
-                    uint16_t* masks) {
-  __shared__ int warp_sum[kCompactThreads / 32];
-  const bool vec = (reinterpret_cast<uintptr_t>(flags) & 15) == 0;
-  const int64_t i0 = (int64_t)blockIdx.x * kCompactTile + (int64_t)threadIdx.x * kCompactItems;
-  const uint32_t m = load_flags16(flags, i0, n, vec);
-  masks[(int64_t)blockIdx.x * kCompactThreads + threadIdx.x] = (uint16_t)m;
-  const int w = __reduce_add_sync(0xFFFFFFFFu, __popc(m));
-  if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = w;
+    k_compact_count(const uint32_t* flags, int n, int64_t rows, int share, uint32_t* masks,
+                    int* warp_counts, int* block_counts) {
+  __shared__ int sums[kCompactWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t g = (int64_t)blockIdx.x * kCompactWarps + warp;
+  const int64_t end = min(rows, (g + 1) * share);
+  int count = 0;
+  for (int64_t r = g * share; r < end; r += kCompactBatch) {
+    const int64_t i = r * 32 + lane;
+    uint32_t v[kCompactBatch];
+    if ((r + kCompactBatch) * 32 <= n) {
+#pragma unroll
+      for (int k = 0; k < kCompactBatch; ++k) v[k] = __ldcs(flags + i + 32 * k);
+    } else {
+#pragma unroll
+      for (int k = 0; k < kCompactBatch; ++k) v[k] = i + 32 * k < n ? __ldcs(flags + i + 32 * k) : 0u;
+    }
+    uint32_t word = 0;
+#pragma unroll
+    for (int k = 0; k < kCompactBatch; ++k) {
+      const uint32_t bits = __ballot_sync(0xFFFFFFFFu, v[k] != 0);
+      if (lane == k) word = bits;
+    }
+    if (lane < kCompactBatch && r + lane < end) masks[r + lane] = word;
+    count += __popc(word);
+  }
+  count = __reduce_add_sync(0xFFFFFFFFu, count);
+  if (lane == 0) {
+    warp_counts[g] = count;
+    sums[warp] = count;
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
     int sum = 0;
-    for (int k = 0; k < kCompactThreads / 32; ++k) sum += warp_sum[k];
-    tile_counts[blockIdx.x] = sum;
-    if (sum) atomicAdd(&super_counts[blockIdx.x >> shift], sum);
+    for (int k = 0; k < kCompactWarps; ++k) sum += sums[k];
+    block_counts[blockIdx.x] = sum;
   }
 }
 
-// One tile per block, no staging: the 16-bit masks of lanes 2r and 2r + 1
-// of a warp, read as one 32-bit word, are the survivor bits of the 32
-// consecutive flags w * 512 + r * 32 + [0, 32) of its tile, lane l's flag
-// in bit l. So for each of its 16 rows a warp writes the row's survivors
-// to consecutive slots with one coalesced store (position: the popcount of
-// the row's bits below the lane). Mask bits of flags at or past n are zero
-// (the count pass bounds-checks), so the scatter needs no n. The block of
-// the last tile writes the survivor total.
+// A warp's lanes write a row's survivors to consecutive slots with one
+// coalesced store: the row's place comes from a scan of 32 rows' counts, a
+// lane's in the row is the number of the row's bits below it. (Places and bits
+// go through shared memory, two rows per 16-byte broadcast: 2 us less than
+// shuffles at n = 2^25. Staging the survivors for 16-byte stores: no gain.)
+// The last block writes the total.
 __global__ void __launch_bounds__(kCompactThreads)
-    k_compact_scatter(const uint32_t* rows, int tiles, int shift, const int* tile_counts,
-                      const int* super_counts, int* out, int* total) {
-  constexpr int kWarps = kCompactThreads / 32;
-  constexpr int kRows = kCompactItems;  // 32-flag rows per warp
-  __shared__ int before[kWarps], warp_count[kWarps];
+    k_compact_scatter(const uint32_t* masks, int64_t rows, int share, const int* warp_counts,
+                      const int* block_counts, int* out, int* total) {
+  __shared__ int before[kCompactWarps];
+  __shared__ __align__(16) uint2 row_sh[kCompactWarps][32];  // a row's place and bits
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int b = blockIdx.x;
-  const uint32_t word = lane < kRows ? rows[((int64_t)b * kWarps + warp) * kRows + lane] : 0u;
-  const int wcount = __reduce_add_sync(0xFFFFFFFFu, __popc(word));
-  // Survivors of the earlier superblocks, then of this superblock's earlier
-  // tiles (each warp sums a share).
-  const int sb = b >> shift;
+  uint2* row = row_sh[warp];
+  cudaGridDependencySynchronize();  // the count pass is done
   int acc = 0;
-  for (int i = threadIdx.x; i < sb; i += kCompactThreads) acc += super_counts[i];
-  for (int i = (sb << shift) + threadIdx.x; i < b; i += kCompactThreads) acc += tile_counts[i];
+  for (int i = threadIdx.x; i < (int)blockIdx.x; i += kCompactThreads) acc += block_counts[i];
   acc = __reduce_add_sync(0xFFFFFFFFu, acc);
-  if (lane == 0) {
-    before[warp] = acc;
-    warp_count[warp] = wcount;
-  }
+  const int own = lane < kCompactWarps ? warp_counts[blockIdx.x * kCompactWarps + lane] : 0;
+  int o = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? own : 0);
+  if (lane == 0) before[warp] = acc;
   __syncthreads();
-  int base = 0, offset = 0, count = 0;
 #pragma unroll
-  for (int k = 0; k < kWarps; ++k) {
-    base += before[k];
-    offset += k < warp ? warp_count[k] : 0;
-    count += warp_count[k];
-  }
-  int o = base + offset;
-  const int f0 = (int)((int64_t)b * kCompactTile) + warp * (kRows * 32) + lane;
+  for (int k = 0; k < kCompactWarps; ++k) o += before[k];
+  const int64_t g = (int64_t)blockIdx.x * kCompactWarps + warp;
+  const int64_t end = min(rows, (g + 1) * share);
   const uint32_t below = (1u << lane) - 1u;  // lanes below this one
+  uint32_t next = g * share + lane < end ? masks[g * share + lane] : 0u;
+  for (int64_t r = g * share; r < end; r += 32) {
+    const uint32_t word = next;
+    next = r + 32 + lane < end ? masks[r + 32 + lane] : 0u;
+    const int c = __popc(word);
+    int inc = c;
 #pragma unroll
-  for (int r = 0; r < kRows; ++r) {
-    const uint32_t bits = __shfl_sync(0xFFFFFFFFu, word, r);
-    if ((bits >> lane) & 1u) out[o + __popc(bits & below)] = f0 + r * 32;
-    o += __popc(bits);
+    for (int d = 1; d < 32; d <<= 1) {
+      const int y = __shfl_up_sync(0xFFFFFFFFu, inc, d);
+      if (lane >= d) inc += y;
+    }
+    const int m = __shfl_sync(0xFFFFFFFFu, inc, 31);
+    row[lane] = make_uint2((uint32_t)(o + inc - c), word);
+    __syncwarp();
+    const uint32_t i = (uint32_t)(r * 32) + lane;
+#pragma unroll 8
+    for (int k = 0; k < 32; k += 2) {
+      const uint4 two = *reinterpret_cast<const uint4*>(row + k);
+      if ((two.y >> lane) & 1u) out[two.x + __popc(two.y & below)] = (int)(i + 32u * k);
+      if ((two.w >> lane) & 1u) out[two.z + __popc(two.w & below)] = (int)(i + 32u * k + 32u);
+    }
+    o += m;
+    __syncwarp();
   }
-  if (b == tiles - 1 && threadIdx.x == 0) *total = base + count;
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == kCompactThreads - 32) *total = o;
 }
 
 inline int blocks_for(int64_t n, int bs) { return (int)((n + bs - 1) / bs); }
 
-// Enqueues the two compaction passes on `st`. Scratch: tile_counts (tiles
-// ints), super_counts (compact_supers(tiles, shift) ints, zeroed here) and
-// masks (tiles * 256 16-bit masks); the survivor count goes to *total.
-cudaError_t launch_compact(const uint32_t* flags, int n, int* tile_counts, int* super_counts,
-                           uint16_t* masks, int* out, int* total, cudaStream_t st) {
-  const int tiles = blocks_for(n, kCompactTile);
-  const int shift = compact_super_shift(tiles);
-  cudaError_t e = cudaMemsetAsync(super_counts, 0,
-                                  (size_t)compact_supers(tiles, shift) * sizeof(int), st);
+// Enqueues the two compaction passes on `st` for n > 0 flags. Scratch:
+// compact_shape(n)'s rows masks, kCompactMaxWarps and kCompactMaxBlocks counts;
+// the survivor count goes to *total. The scatter pass is launched while the
+// count pass drains and waits for it on the device.
+cudaError_t launch_compact(const uint32_t* flags, int n, uint32_t* masks, int* warp_counts,
+                           int* block_counts, int* out, int* total, cudaStream_t st) {
+  const CompactShape c = compact_shape(n);
+  k_compact_count<<<c.blocks, kCompactThreads, 0, st>>>(flags, n, c.rows, c.share, masks,
+                                                        warp_counts, block_counts);
+  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_compact_count<<<tiles, kCompactThreads, 0, st>>>(flags, n, shift, tile_counts, super_counts,
-                                                     masks);
-  k_compact_scatter<<<tiles, kCompactThreads, 0, st>>>(reinterpret_cast<const uint32_t*>(masks),
-                                                       tiles, shift, tile_counts, super_counts,
-                                                       out, total);
-  return cudaGetLastError();
+  cudaLaunchAttribute early{};
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(c.blocks);
+  cfg.blockDim = dim3(kCompactThreads);
+  cfg.stream = st;
+  cfg.attrs = &early;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_compact_scatter, (const uint32_t*)masks, c.rows, c.share,
+                            (const int*)warp_counts, (const int*)block_counts, out, total);
 }
 
 hpt_status check_scene_desc(const hpt_scene_desc& d) {
@@ -819,15 +817,14 @@ hpt_status hpt_compact(const uint32_t* flags, int32_t n, int32_t* out, int32_t* 
   if (n == 0) return HPT_OK;
   if (hpt_device_count() == 0) return fail(HPT_ERR_CUDA, "no CUDA device");
   return guarded([&]() -> hpt_status {
-    const int nb = blocks_for(n, kCompactTile);
-    const int ns = compact_supers(nb, compact_super_shift(nb));
-    DBuf f, o, bc, sc, tot, mk;
+    DBuf f, o, mk, wc, bc, tot;
     hpt_status s;
     if ((s = f.up(flags, (size_t)n * 4)) || (s = o.alloc((size_t)n * 4)) ||
-        (s = bc.alloc((size_t)nb * 4)) || (s = sc.alloc((size_t)ns * 4)) ||
-        (s = tot.alloc(4)) || (s = mk.alloc((size_t)nb * kCompactThreads * 2)))
+        (s = mk.alloc((size_t)compact_shape(n).rows * 4)) ||
+        (s = wc.alloc(kCompactMaxWarps * 4)) || (s = bc.alloc(kCompactMaxBlocks * 4)) ||
+        (s = tot.alloc(4)))
       return s;
-    HPT_CUDA(launch_compact(f.as<uint32_t>(), n, bc.as<int>(), sc.as<int>(), mk.as<uint16_t>(),
+    HPT_CUDA(launch_compact(f.as<uint32_t>(), n, mk.as<uint32_t>(), wc.as<int>(), bc.as<int>(),
                             o.as<int>(), tot.as<int>(), 0));
     int total = 0;
     if ((s = tot.down(&total))) return s;
@@ -931,30 +928,23 @@ void hpt_batch_destroy(hpt_batch* batch) { delete batch; }
 
 // ---------------------------------------------------------------------------
 // hpt_compact_noalloc: the compaction kernels over caller-owned device
-// buffers, with the per-block counts and the mask bytes in static device
-// arrays instead of cudaMalloc'd ones. For callers that cannot allocate device memory where
+// buffers, with the counts and the masks in static device arrays instead of
+// cudaMalloc'd ones. For callers that cannot allocate device memory where
 // they call it (allocation synchronises the device and would stall their
 // stream; a fixed memory budget leaves nothing to allocate).
 // ---------------------------------------------------------------------------
 namespace {
 
-// One count per 4096-flag tile (32 KB per device), one total per
-// superblock of at most 128 tiles (8,192 tiles need 64), and 16-bit masks,
-// one per 16 flags (4 MiB per device).
-constexpr int kNoallocMaxBlocks = HPT_COMPACT_NOALLOC_MAX_N / kCompactTile;
-static_assert(kNoallocMaxBlocks * kCompactTile == HPT_COMPACT_NOALLOC_MAX_N,
-              "the limit is a whole number of tiles");
-constexpr int kNoallocMaxSupers = 128;
-static_assert(kNoallocMaxBlocks <= kNoallocMaxSupers * kNoallocMaxSupers,
-              "superblocks of at most 128 tiles cover the limit");
-static __device__ __align__(256) int g_noalloc_block_counts[kNoallocMaxBlocks];
-static __device__ __align__(256) int g_noalloc_super_counts[kNoallocMaxSupers];
-static __device__ __align__(256) uint16_t g_noalloc_masks[kNoallocMaxBlocks * kCompactThreads];
+// A mask bit per flag (4 MiB per device) and the counts of the warps' and the
+// blocks' shares (42 KB).
+static __device__ __align__(256) uint32_t g_noalloc_masks[HPT_COMPACT_NOALLOC_MAX_N / 32];
+static __device__ __align__(256) int g_noalloc_warp_counts[kCompactMaxWarps];
+static __device__ __align__(256) int g_noalloc_block_counts[kCompactMaxBlocks];
 
 struct NoallocScratch {
-  int* counts = nullptr;
-  int* supers = nullptr;
-  uint16_t* masks = nullptr;
+  uint32_t* masks = nullptr;
+  int* warps = nullptr;
+  int* blocks = nullptr;
 };
 
 // Device addresses of the static scratch arrays, looked up once per device
@@ -967,16 +957,16 @@ hpt_status noalloc_scratch(int device, NoallocScratch* out) {
   static std::vector<NoallocScratch> addr;
   std::lock_guard<std::mutex> lk(mu);
   if ((int)addr.size() <= device) addr.resize(device + 1);
-  if (!addr[device].counts) {
-    void* c = nullptr;
-    void* sc = nullptr;
+  if (!addr[device].masks) {
     void* m = nullptr;
-    HPT_CUDA(cudaGetSymbolAddress(&c, g_noalloc_block_counts));
-    HPT_CUDA(cudaGetSymbolAddress(&sc, g_noalloc_super_counts));
+    void* w = nullptr;
+    void* b = nullptr;
     HPT_CUDA(cudaGetSymbolAddress(&m, g_noalloc_masks));
-    addr[device].counts = static_cast<int*>(c);
-    addr[device].supers = static_cast<int*>(sc);
-    addr[device].masks = static_cast<uint16_t*>(m);
+    HPT_CUDA(cudaGetSymbolAddress(&w, g_noalloc_warp_counts));
+    HPT_CUDA(cudaGetSymbolAddress(&b, g_noalloc_block_counts));
+    addr[device].masks = static_cast<uint32_t*>(m);
+    addr[device].warps = static_cast<int*>(w);
+    addr[device].blocks = static_cast<int*>(b);
   }
   *out = addr[device];
   return HPT_OK;
@@ -1003,9 +993,8 @@ extern "C" hpt_status hpt_compact_noalloc(const uint32_t* flags, int32_t n, int3
     HPT_CUDA(cudaMemsetAsync(count, 0, sizeof(int32_t), st));
     return HPT_OK;
   }
-  // Every tile count is written by the count pass before the scatter reads
-  // it; the total goes straight to the caller's counter.
-  HPT_CUDA(launch_compact(flags, n, scratch.counts, scratch.supers, scratch.masks, out, count,
-                          st));
+  // Every scratch entry the scatter reads is written by the count pass; the
+  // total goes straight to the caller's counter.
+  HPT_CUDA(launch_compact(flags, n, scratch.masks, scratch.warps, scratch.blocks, out, count, st));
   return HPT_OK;
 }

@@ -349,7 +349,7 @@ hpt_status hpt_next_dir(hpt_scene* scene, int32_t n, const int32_t* branch,
                         float* origins_out, float* directions_out,
                         float* strength_out, int32_t* alive_out);
 
-/* Stable stream compaction (warp ballot + block scan): out receives the
+/* Stable stream compaction (warp ballots): out receives the
  * indices i with flags[i] != 0 in increasing order, *count their number.
  * Replaces the atomic_inc appends of kernel.cl (e.g. :188-189). */
 hpt_status hpt_compact(const uint32_t* flags, int32_t n, int32_t* out,
@@ -363,16 +363,15 @@ hpt_status hpt_compact(const uint32_t* flags, int32_t n, int32_t* out,
  * out and count are device pointers; the work is enqueued on `stream`
  * (a cudaStream_t, NULL = legacy default stream) and the call returns
  * without waiting: *count is valid once the stream reaches that point.
- * The scratch (tile counts, superblock totals, one mask bit per flag:
+ * The scratch (one mask bit per flag, counts per share of the flags:
  * 4.1 MiB) is fixed static device arrays, so n is limited to
  * HPT_COMPACT_NOALLOC_MAX_N flags (larger n: HPT_ERR_INVALID_ARGUMENT,
  * nothing enqueued). The first call on each device looks up those arrays'
  * addresses (set-up, with the device current). Every call shares the one
  * set of arrays: calls whose
  * work overlaps on the GPU (different streams, or host threads) race on it
- * and must be serialised by the caller. Each call overwrites (or zeroes,
- * with cudaMemsetAsync on `stream`) every scratch entry it reads, so no
- * state carries over between calls. The addresses are cached per device:
+ * and must be serialised by the caller. Each call overwrites every
+ * scratch entry it reads, so no state carries over between calls. The addresses are cached per device:
  * after cudaDeviceReset this entry point must not be called again in the
  * same process. */
 #define HPT_COMPACT_NOALLOC_MAX_N (8192 * 4096)
