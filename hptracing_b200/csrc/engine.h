@@ -103,8 +103,7 @@ class Engine {
   hpt_status ensure_graph(const DevScene* shared_scene, int iterations);
   // samples: the divisor of the accumulated radiance (<= 0: params.sample).
   void launch_resolve(int slot, const JobSpec& js, const JobBuffers& b, float samples = 0.f);
-  // Synchronous read-back of the slot table / control block.
-  hpt_status read_slots(std::vector<DevSlot>& out);
+  // Synchronous read-back of the control block.
   hpt_status read_ctrl(DevCtrl* out);
   // Maps `bytes` of device memory into the job-buffer pool now and keeps
   // it there, so later job allocations do not map memory (which blocks the
@@ -112,7 +111,6 @@ class Engine {
   hpt_status reserve_pool(size_t bytes);
   // Shared in-flight budget of the capped slots (reset_ctrl clears it).
   hpt_status set_capped_budget(int64_t paths);
-  hpt_status read_state(std::vector<DevSlot>& slots, DevCtrl* ctrl);  // one sync
   void reset_ctrl();
   DevCtrl* ctrl_dev() const { return ctrl_; }
   DevSlot* slots_dev() const { return slot_state_; }
@@ -135,7 +133,7 @@ class Engine {
   int32_t* host_i32_ = nullptr;   // pinned staging for small uploads
   int64_t* host_i64_ = nullptr;
   DevJob* host_jobs_ = nullptr;
-  DevSlot* slots_host_ = nullptr;  // pinned mirror for read_slots
+  DevSlot* slots_host_ = nullptr;  // pinned mirror of the slot table
   // The queue of paths (double-buffered) and what its rays hit.
   float4* Q_o_[2] = {nullptr, nullptr};
   float4* Q_d_[2] = {nullptr, nullptr};
