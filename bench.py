@@ -180,9 +180,9 @@ def measured_peak():
 
 
 def profiled_traffic():
-    """DRAM bytes (read + write) of one k_isect launch of this workload, from
+    """DRAM bytes (read + write) of one k_trace launch of this workload, from
     the committed ncu summary (None when the summary is absent)."""
-    path = os.path.join(ROOT, "profiles", "k_isect_spheres64_512x512_spp64_d8.md")
+    path = os.path.join(ROOT, "profiles", "k_trace_spheres64_512x512_spp64_d8.md")
     try:
         with open(path) as f:
             for line in f:
@@ -274,15 +274,12 @@ def reference_scene():
 
 
 def isect_bytes(stats):
-    """Algorithmic bytes of all intersect-kernel work in one frame:
-    per query 64 B (origin+direction in, strength+radiance carried) and
-    72 B written per hit (next shade record) -- approximated with the hit
-    count = shade calls; per inner node visited 8 B; per leaf visited 36 B
-    (box + exit rope); per triangle test 48 B (a, b-a, c-a)."""
+    """Algorithmic bytes of all closest-hit work in one frame: per query 32 B
+    (origin, direction), per hit 16 B written, per hierarchy node visited 80 B,
+    per triangle test 48 B."""
     q = stats["intersect_queries"] - stats["primary_rays"]
-    hits = max(0, stats["shade_calls"] - stats["paths"])  # hits found by k_isect
-    return (64 * q + 72 * hits + 8 * stats["nodes_visited"] + 36 * stats["leaves_visited"] +
-            48 * stats["triangle_tests"])
+    hits = max(0, stats["shade_calls"] - stats["paths"])  # hits found by k_trace
+    return 32 * q + 16 * hits + 80 * stats["nodes_visited"] + 48 * stats["triangle_tests"]
 
 
 def cpu_baseline(mesh, nodes, leaf, cam, kind, samples=1):
@@ -380,7 +377,8 @@ def serve_summary(line, cpu):
 
 
 def serve_cpu_baseline(scene_arrays, cam):
-    """The reference kernels on the host cores rendering one pose request of
+    """The reference kernels (where they are not built, the oracle's
+    restatement) on the host cores rendering one pose request of
     the spheres scene (512 x 512, depth 6) at 1 of its 4 samples: the pose
     latency a CPU host would give, scaled to 4 samples."""
     import oracle as O
@@ -388,11 +386,16 @@ def serve_cpu_baseline(scene_arrays, cam):
     cs = O.CpuScene(mesh, nodes, leaf)
     threads = os.cpu_count() or 1
     t0 = time.perf_counter()
-    _, _, counts = cs.refcl_render(cam, 512, 512, 1, 1, (0.05, 0.05, 0.05), 1, 6, 0, 1.0,
-                                   seed=3, threads=threads)
+    kind = "reference" if O.refcl_lib() is not None else "port"
+    if kind == "reference":
+        _, _, counts = cs.refcl_render(cam, 512, 512, 1, 1, (0.05, 0.05, 0.05), 1, 6, 0, 1.0,
+                                       seed=3, threads=threads)
+    else:
+        _, _, counts = cs.render(cam, 512, 512, 1, 1, (0.05, 0.05, 0.05), 1, 6, 0, seed=3,
+                                 threads=threads)
     dt = time.perf_counter() - t0
     return {"pose_latency_ms": dt * 4 * 1e3, "value": counts[0] / dt / 1e6, "unit": "Mrays/s",
-            "cores": threads, "kind": "reference",
+            "cores": threads, "kind": kind,
             "sample": "one 512x512 pose request of the spheres scene at 1 of 4 spp "
                       "(%d queries, %.2f s), latency scaled x4" % (int(counts[0]), dt)}
 
@@ -909,7 +912,9 @@ def main():
     dev_ms = sum(s["ms_total"] for s in stats)
     queries = sum(s["intersect_queries"] for s in stats)
     isect_ms = sum(s["ms_intersect"] for s in stats)
-    launches = sum(3 * s["iterations"] + 3 for s in stats)
+    # Per frame: the camera rays' pass, a shading and a closest-hit pass per
+    # iteration (the last one's is the control kernel), the resolve.
+    launches = sum(2 * s["iterations"] + 2 for s in stats)
     wall_s = sum(walls)
     tot_q = allreduce_sum(float(queries), world)
     max_ms = allreduce_max(dev_ms, world)
@@ -942,7 +947,7 @@ def main():
             "e2e": {"value": e2e, "unit": "Mrays/s", "h2d_bytes_per_step": 320,
                     "d2h_bytes_per_step": W_RES * H_RES * 4 + 256},
             "gpu_launches": launches,
-            "roofline": {"bound": "hbm", "kernel": "k_isect", "achieved": achieved,
+            "roofline": {"bound": "hbm", "kernel": "k_trace", "achieved": achieved,
                          "peak": peak, "unit": "GB/s",
                          "frac": (achieved / peak) if achieved else None,
                          "peak_kind": peak_kind,
