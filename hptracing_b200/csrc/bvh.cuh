@@ -3,12 +3,13 @@
 // The result is that of the tree walk in traverse.cuh, bit for bit: the
 // minimum-t triangle over the tree leaves that pass the reference's box
 // filter. A query runs in two parts:
-//  1. The hierarchy's walk finds the nearest triangle of all the
-//     Moller-Trumbore test accepts. Every triangle is tested once (the tree
-//     lists it in every leaf it touches, ~50 times), with the same FP32
-//     arithmetic. The boxes are grown by what that arithmetic can be off by
-//     (build_bvh), so the tree walk, which tests some of the same triangles,
-//     finds this triangle or none as near.
+//  1. The hierarchy's walk finds the nearest triangle of all that the
+//     Moller-Trumbore test accepts in a leaf the ray crosses. Every triangle
+//     is tested once (the tree lists it in every leaf it touches, ~50 times),
+//     with the same FP32 arithmetic. A child's boxes hold every ray for which
+//     that arithmetic can accept a triangle below it, by an error bound
+//     derived in bvh_build.cpp, so the tree walk, which tests some of the same
+//     triangles, finds this triangle or none as near.
 //  2. bvh_certain shows that the tree walk tests this triangle in a leaf that
 //     passes the reference's filter; then its answer is this one.
 // A ray for which part 2 fails (mostly rays in a split plane) is walked
@@ -117,10 +118,35 @@ HPT_HD Pair fma2(const Pair& a, const Pair& b, const Pair& c) {
 #endif
 }
 
+// acc + the dot product of four signed bytes.
+HPT_HD int dot4(uint32_t a, uint32_t b, int acc) {
+#ifdef __CUDA_ARCH__
+  int r;
+  asm("dp4a.s32.s32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(acc));
+  return r;
+#else
+  for (int k = 0; k < 32; k += 8) acc += (int)(int8_t)(a >> k) * (int)(int8_t)(b >> k);
+  return acc;
+#endif
+}
+// mask << 1, with x's sign as the new bit.
+HPT_HD uint32_t push_sign(uint32_t mask, int x) {
+#ifdef __CUDA_ARCH__
+  return __funnelshift_l((uint32_t)x, mask, 1);
+#else
+  return (mask << 1) | ((uint32_t)x >> 31);
+#endif
+}
+// Bytes 0xFF for the low four bits of m.
+HPT_HD uint32_t byte_mask(uint32_t m) { return (((m & 15u) * 0x00204081u) & 0x01010101u) * 255u; }
+// Bytes of b where mask is set, of a elsewhere.
+HPT_HD uint32_t pick(uint32_t a, uint32_t b, uint32_t mask) { return a ^ ((a ^ b) & mask); }
+
 // Walk state of one ray.
 struct BvhRay {
   Ray ray;
   f3 inv;            // 1 / d
+  uint32_t q, nq;    // d / |d| and its opposite in 127ths, bytes 0-2; byte 3 = -127
   float cull;        // boxes that start beyond it are skipped
   float best_t;      // nearest accepted t, +inf = none
   uint32_t best;     // its record in btris, kBvhNone = none; | kBvhTie when
@@ -136,6 +162,14 @@ struct BvhRay {
 constexpr uint32_t kBvhStep = 32u;
 static_assert(kBvhStack == 32, "stack entries fit bits 0-4");
 constexpr uint32_t kBvhNone = 0x3FFFFFFFu, kBvhTie = 0x40000000u, kBvhMany = 0x80000000u;
+
+// d / |d| as bytes, for the test against a child's cone (BvhNode).
+HPT_HD uint32_t direction_bytes(const f3& d, float scale127) {
+  const uint32_t x = (uint32_t)(int)rintf(rn_mul(d.x, scale127)) & 255u;
+  const uint32_t y = (uint32_t)(int)rintf(rn_mul(d.y, scale127)) & 255u;
+  const uint32_t z = (uint32_t)(int)rintf(rn_mul(d.z, scale127)) & 255u;
+  return x | (y << 8) | (z << 16) | (0x81u << 24);
+}
 
 // Starts a walk. Returns false when the ray is to be walked through the tree
 // instead (non-finite rays, directions of extreme length).
@@ -160,36 +194,80 @@ HPT_HD bool bvh_init(const Ray& r, BvhRay& b) {
       (b.inv.x > 0.f ? 1u : 0u) | (b.inv.y > 0.f ? 2u : 0u) | (b.inv.z > 0.f ? 4u : 0u);
   b.node_base = 0;
   b.node_bits = (oct << 16) | (1u << 8) | (1u << oct);
-  return finite3(r.o) && finite3(r.d) && dmax > 1e-15f && dmax < 1e15f;
+  if (!(finite3(r.o) && finite3(r.d) && dmax > 1e-15f && dmax < 1e15f)) return false;
+  const float len127 = rn_div(127.f, length(r.d));
+  b.q = direction_bytes(r.d, len127);
+  b.nq = direction_bytes(r.d, -len127);
+  return true;
 }
 
 // Bit k, when the ray enters the box of slot k before cull: the planes of
-// four slots are the bytes of near / far words.
+// four slots are the bytes of near / far words. N / F: the node's offsets of
+// near and far planes.
 template <int k>
 HPT_HD uint32_t bvh_slot(uint32_t nx, uint32_t ny, uint32_t nz, uint32_t fx, uint32_t fy,
-                         uint32_t fz, const Pair& Sxy, const Pair& Oxy, const Pair& Szz,
-                         const Pair& Ozz, float cull) {
+                         uint32_t fz, const Pair& Sxy, const Pair& Nxy, const Pair& Fxy,
+                         const Pair& Szz, const Pair& NFz, float cull) {
   float x0, y0, z0, x1, y1, z1;
-  unpair(fma2(pair(plane<k & 3>(nx), plane<k & 3>(ny)), Sxy, Oxy), x0, y0);
-  unpair(fma2(pair(plane<k & 3>(fx), plane<k & 3>(fy)), Sxy, Oxy), x1, y1);
-  unpair(fma2(pair(plane<k & 3>(nz), plane<k & 3>(fz)), Szz, Ozz), z0, z1);
+  unpair(fma2(pair(plane<k & 3>(nx), plane<k & 3>(ny)), Sxy, Nxy), x0, y0);
+  unpair(fma2(pair(plane<k & 3>(fx), plane<k & 3>(fy)), Sxy, Fxy), x1, y1);
+  unpair(fma2(pair(plane<k & 3>(nz), plane<k & 3>(fz)), Szz, NFz), z0, z1);
   const float t0 = fmaxf(max3(x0, y0, z0), 0.f), t1 = fminf(min3(x1, y1, z1), cull);
   return t0 <= t1 ? 1u << k : 0u;
 }
 
 // Visits a node: sets the pending children and triangles.
-HPT_HD void bvh_node(BvhRay& b, const uint4& n0, const uint4& n1, const uint4& n2,
-                     const uint4& n3, const uint4& n4) {
+HPT_HD void bvh_node(BvhRay& b, const uint4* node) {
+  const uint4 n0 = ldg(node), n1 = ldg(node + 1);
+  uint4 n2 = ldg(node + 2), n3 = ldg(node + 3), n4 = ldg(node + 4);
+  {
+    // The slots whose wide box counts.
+    const uint4 c0 = ldg(node + 8), c1 = ldg(node + 9);
+    uint32_t r = 0;
+    r = push_sign(r, dot4(c1.w, b.q, -1) & dot4(c1.w, b.nq, -1));
+    r = push_sign(r, dot4(c1.z, b.q, -1) & dot4(c1.z, b.nq, -1));
+    r = push_sign(r, dot4(c1.y, b.q, -1) & dot4(c1.y, b.nq, -1));
+    r = push_sign(r, dot4(c1.x, b.q, -1) & dot4(c1.x, b.nq, -1));
+    r = push_sign(r, dot4(c0.w, b.q, -1) & dot4(c0.w, b.nq, -1));
+    r = push_sign(r, dot4(c0.z, b.q, -1) & dot4(c0.z, b.nq, -1));
+    r = push_sign(r, dot4(c0.y, b.q, -1) & dot4(c0.y, b.nq, -1));
+    r = push_sign(r, dot4(c0.x, b.q, -1) & dot4(c0.x, b.nq, -1));
+    const uint4 w2 = ldg(node + 5), w3 = ldg(node + 6), w4 = ldg(node + 7);
+    const uint32_t m0 = byte_mask(r), m1 = byte_mask(r >> 4);
+    n2.x = pick(n2.x, w2.x, m0);
+    n2.y = pick(n2.y, w2.y, m1);
+    n2.z = pick(n2.z, w2.z, m0);
+    n2.w = pick(n2.w, w2.w, m1);
+    n3.x = pick(n3.x, w3.x, m0);
+    n3.y = pick(n3.y, w3.y, m1);
+    n3.z = pick(n3.z, w3.z, m0);
+    n3.w = pick(n3.w, w3.w, m1);
+    n4.x = pick(n4.x, w4.x, m0);
+    n4.y = pick(n4.y, w4.y, m1);
+    n4.z = pick(n4.z, w4.z, m0);
+    n4.w = pick(n4.w, w4.w, m1);
+  }
   const uint32_t e = n0.w;
-  f3 S, O;
-  S.x = rn_mul(as_float_u((e & 255u) << 23), b.inv.x);
-  S.y = rn_mul(as_float_u(((e >> 8) & 255u) << 23), b.inv.y);
-  S.z = rn_mul(as_float_u(((e >> 16) & 255u) << 23), b.inv.z);
-  O.x = fma_rn(-32768.f, S.x, rn_mul(rn_sub(as_float_u(n0.x), b.ray.o.x), b.inv.x));
-  O.y = fma_rn(-32768.f, S.y, rn_mul(rn_sub(as_float_u(n0.y), b.ray.o.y), b.inv.y));
-  O.z = fma_rn(-32768.f, S.z, rn_mul(rn_sub(as_float_u(n0.z), b.ray.o.z), b.inv.z));
-  const Pair Sxy = pair(S.x, S.y), Oxy = pair(O.x, O.y);
-  const Pair Szz = pair(S.z, S.z), Ozz = pair(O.z, O.z);
+  const float sx = as_float_u((e & 255u) << 23), sy = as_float_u(((e >> 8) & 255u) << 23),
+              sz = as_float_u(((e >> 16) & 255u) << 23);
+  const float rx = rn_sub(as_float_u(n0.x), b.ray.o.x), ry = rn_sub(as_float_u(n0.y), b.ray.o.y),
+              rz = rn_sub(as_float_u(n0.z), b.ray.o.z);
+  // The planes move outward by kBoxGrowth of the distance to the node's far
+  // side.
+  const float far_side =
+      fma_rn(256.f, max3(sx, sy, sz), max3(fabsf(rx), fabsf(ry), fabsf(rz)));
+  const float grow = rn_mul(kBoxGrowth, far_side);
+  f3 S;
+  S.x = rn_mul(sx, b.inv.x);
+  S.y = rn_mul(sy, b.inv.y);
+  S.z = rn_mul(sz, b.inv.z);
+  const float ox = fma_rn(-32768.f, S.x, rn_mul(rx, b.inv.x));
+  const float oy = fma_rn(-32768.f, S.y, rn_mul(ry, b.inv.y));
+  const float oz = fma_rn(-32768.f, S.z, rn_mul(rz, b.inv.z));
+  const Pair Oxy = pair(ox, oy), Axy = pair(fabsf(b.inv.x), fabsf(b.inv.y));
+  const Pair Sxy = pair(S.x, S.y), Szz = pair(S.z, S.z);
+  const Pair Nxy = fma2(pair(-grow, -grow), Axy, Oxy), Fxy = fma2(pair(grow, grow), Axy, Oxy);
+  const Pair NFz = fma2(pair(-grow, grow), pair(fabsf(b.inv.z), fabsf(b.inv.z)), pair(oz, oz));
   const uint32_t oct = b.node_bits >> 16;
   const bool px = oct & 1u, py = oct & 2u, pz = oct & 4u;
   uint32_t h = 0;
@@ -198,19 +276,19 @@ HPT_HD void bvh_node(BvhRay& b, const uint4& n0, const uint4& n1, const uint4& n
     const uint32_t nx = px ? n2.x : n3.z, fx = px ? n3.z : n2.x;
     const uint32_t ny = py ? n2.z : n4.x, fy = py ? n4.x : n2.z;
     const uint32_t nz = pz ? n3.x : n4.z, fz = pz ? n4.z : n3.x;
-    h |= bvh_slot<0>(nx, ny, nz, fx, fy, fz, Sxy, Oxy, Szz, Ozz, b.cull);
-    h |= bvh_slot<1>(nx, ny, nz, fx, fy, fz, Sxy, Oxy, Szz, Ozz, b.cull);
-    h |= bvh_slot<2>(nx, ny, nz, fx, fy, fz, Sxy, Oxy, Szz, Ozz, b.cull);
-    h |= bvh_slot<3>(nx, ny, nz, fx, fy, fz, Sxy, Oxy, Szz, Ozz, b.cull);
+    h |= bvh_slot<0>(nx, ny, nz, fx, fy, fz, Sxy, Nxy, Fxy, Szz, NFz, b.cull);
+    h |= bvh_slot<1>(nx, ny, nz, fx, fy, fz, Sxy, Nxy, Fxy, Szz, NFz, b.cull);
+    h |= bvh_slot<2>(nx, ny, nz, fx, fy, fz, Sxy, Nxy, Fxy, Szz, NFz, b.cull);
+    h |= bvh_slot<3>(nx, ny, nz, fx, fy, fz, Sxy, Nxy, Fxy, Szz, NFz, b.cull);
   }
   {
     const uint32_t nx = px ? n2.y : n3.w, fx = px ? n3.w : n2.y;
     const uint32_t ny = py ? n2.w : n4.y, fy = py ? n4.y : n2.w;
     const uint32_t nz = pz ? n3.y : n4.w, fz = pz ? n4.w : n3.y;
-    h |= bvh_slot<4>(nx, ny, nz, fx, fy, fz, Sxy, Oxy, Szz, Ozz, b.cull);
-    h |= bvh_slot<5>(nx, ny, nz, fx, fy, fz, Sxy, Oxy, Szz, Ozz, b.cull);
-    h |= bvh_slot<6>(nx, ny, nz, fx, fy, fz, Sxy, Oxy, Szz, Ozz, b.cull);
-    h |= bvh_slot<7>(nx, ny, nz, fx, fy, fz, Sxy, Oxy, Szz, Ozz, b.cull);
+    h |= bvh_slot<4>(nx, ny, nz, fx, fy, fz, Sxy, Nxy, Fxy, Szz, NFz, b.cull);
+    h |= bvh_slot<5>(nx, ny, nz, fx, fy, fz, Sxy, Nxy, Fxy, Szz, NFz, b.cull);
+    h |= bvh_slot<6>(nx, ny, nz, fx, fy, fz, Sxy, Nxy, Fxy, Szz, NFz, b.cull);
+    h |= bvh_slot<7>(nx, ny, nz, fx, fy, fz, Sxy, Nxy, Fxy, Szz, NFz, b.cull);
   }
   const uint32_t imask = e >> 24;
   uint32_t inner = h & imask;
@@ -252,14 +330,14 @@ HPT_HD bool bvh_visit(const BvhNode* bvh, uint32_t num_bvh, BvhRay& b, uint2* st
     ++b.steps;
   }
   HPT_DCHECK(err, node < num_bvh, 114, node, return false);
-  const uint4* n = reinterpret_cast<const uint4*>(bvh + node);
-  bvh_node(b, ldg(n), ldg(n + 1), ldg(n + 2), ldg(n + 3), ldg(n + 4));
+  bvh_node(b, reinterpret_cast<const uint4*>(bvh + node));
   b.steps += kBvhStep;
   return true;
 }
 
 // One triangle test of the pending ones. A winning hit shrinks the cull
-// distance to the tree walk's own stopping rule (best t plus slack).
+// distance to the tree walk's own stopping rule (1.0001 times the best t plus
+// slack), or a little beyond it: what the computed t can be off by.
 // tie receives the other triangle's record where best gets kBvhTie.
 HPT_HD void bvh_test(const BvhTri* btris, float scene_eps, BvhRay& b, uint32_t& tie) {
   const int k = high_bit(b.tri_bits);
@@ -274,7 +352,7 @@ HPT_HD void bvh_test(const BvhTri* btris, float scene_eps, BvhRay& b, uint32_t& 
       b.best = (uint32_t)i;
       const float per_unit =
           fminf(fabsf(b.inv.x), fminf(fabsf(b.inv.y), fabsf(b.inv.z)));  // 1 / largest |d|
-      b.cull = fma_rn(t, 1.0001f, rn_mul(scene_eps, per_unit));
+      b.cull = fma_rn(t, kCullFactor, rn_mul(scene_eps, per_unit));
     } else if (t == b.best_t) {
       b.best |= b.best & kBvhTie ? kBvhMany : kBvhTie;
       tie = (uint32_t)i;

@@ -1,25 +1,53 @@
 // Builder of the 8-wide hierarchy of the closest-hit kernels.
 //
-// Boxes. A triangle's box is its bounds, grown
-//  - by 2e-6 of the scene's size, for the rounding of box and hit distances;
-//  - by a fiftieth of its extent within its plane. For a ray almost in that
-//    plane (cosine c) the Moller-Trumbore test is off by some 5e-8 / c of the
-//    distance and can accept a ray that passes beside the triangle; the tree
-//    walk (traverse.cuh) would then report it, so the hierarchy has to test
-//    it too. Such a ray has to lie within rounding of the triangle's plane:
-//    in 1.5e9 queries (bounces on the 61k-triangle spheres and on the
-//    2.4M-triangle terrain) plain bounds grown by 4e-7 of the scene's size
-//    alone gave the tree walk's answer every time, and this growth is about
-//    50 times that.
-//    The growth stays inside the union of the leaves that list the triangle:
-//    outside of it the tree walk never tests it. (That union alone as the
-//    box costs 27 node visits and 51 tests a ray on the spheres against 12
-//    and 7, and 67 and 180 against 13 and 6 on a terrain.)
+// Boxes. A ray has to visit every triangle that the tree walk (traverse.cuh)
+// would accept, and the FP32 Moller-Trumbore test accepts rays that pass
+// beside the triangle. How far beside? With u = 2^-24, T = o - a, n = e1 x e2,
+// S = |e1||e2|, det = -n.d = -c |n||d| (c: sine of the angle between ray and
+// plane), the computed T.(d x e2) and d.(T x e1) are off by at most 7u
+// |T||d||e|, the computed det by 6u |d| S, the reciprocal and the products by
+// 2u more. Let X = a + u e1 + v e2 for the computed u, v: an accepted X is a
+// point of the triangle, and
+//     (o - X) det = -d (n.T) + E,   |E| <= u |d| S (14 |T| + 8 max|e|).
+// (1) So X is within W = u (14 |T| + 8 max|e|) / (c s) of the ray's line, s =
+//     |n| / S, the sine of the angle at vertex a, and by the same steps the
+//     computed t is off by no more than u (15 |T| + 8 max|e|) / (c s |d|). If c
+//     s >= kGrazing, the ray meets a box around the triangle that is grown by
+//     u (36 max-norm |T| + 40 max|e|) / kGrazing (the rest beyond W: where the
+//     line's nearest point lies behind the origin). The walk grows boxes by the
+//     first term (kBoxGrowth), the second is part of the box; kCullFactor
+//     covers the error of t. [The first term is what makes origins far away
+//     and triangles of any size come out right.]
+// (2) If c s < kGrazing, the ray runs almost in the plane, and W is no bound.
+//     But |n.(x - X)| <= |n| c |x - X| + |E| / |d| for every point x of the
+//     ray: it stays within a thin slab around the plane, of height h = c |x -
+//     X| + u (14 |T| + 8 max|e|) / s, and the tree walk only tests the triangle
+//     in a leaf that lists it. So the ray meets the part of such a leaf that
+//     lies in the slab. The wide box of a triangle holds these parts; it is
+//     used for rays that are within kGrazing of the plane (a cone per child,
+//     device_types.h). If s < kGrazing (slivers, no area), the leaves count
+//     whole, for all rays.
+//     A triangle with e1 and e2 exactly zero on one axis needs no wide box:
+//     every rounded term of the test then carries d's component on that axis
+//     or the distance along it, and (1) holds without c.
+// A box kept in a node also covers the walk's own rounding (8 u of its largest
+// coordinate; the leaf it is in is found by the rounded o + t d).
+// What it costs: 14.6 node visits and 6.6 tests a ray on the 61k-triangle
+// spheres and 19 and 7 on an 842k-triangle terrain, against 11.7 and 6.4, and
+// 12.6 and 5.3 with boxes grown by a fiftieth of a triangle, which lost hits.
+// (Wide boxes for all rays: 20 and 18, and 30 and 37. kGrazing 0.003 / 0.004 /
+// 0.006 / 0.008: 18.4 / 18.4 / 19.3 / 20.5 visits and 7.3 / 7.2 / 7.2 / 7.3
+// tests for the terrain's bounces, 7.2 / 5.4 / 4.5 / 4.2 for its camera rays.)
+// Not covered: an accepted t = +inf, which takes a det of exactly zero: see
+// bvh_no_parallel_edge.
 //
 // Tree. A binary tree by binned SAH (16 bins on three axes, object median
 // where bins fail or the tree gets deep), opened greedily by surface area
 // into nodes of up to eight children; children are placed in slots so that
 // visiting slots in the order of the ray's octant runs roughly front to back.
+// Splits are chosen for boxes 0.6 of the way from the triangle to its wide
+// box. (Own bounds / 0.6 / wide boxes: 15.6 / 14.0 / 15.6 visits on the spheres,
+// 18.1 / 17.8 / 19.0 on a terrain.)
 #include "bvh_build.h"
 
 #include <algorithm>
@@ -52,7 +80,13 @@ struct Box {
       hi[a] = std::max(hi[a], b.hi[a]);
     }
   }
+  bool holds(const Box& b) const {
+    for (int a = 0; a < 3; ++a)
+      if (b.lo[a] < lo[a] || b.hi[a] > hi[a]) return false;
+    return true;
+  }
   float half_area() const {
+    if (!(lo[0] <= hi[0])) return 0.f;
     const float x = hi[0] - lo[0], y = hi[1] - lo[1], z = hi[2] - lo[2];
     return x * y + y * z + z * x;
   }
@@ -63,6 +97,19 @@ struct Prim {
   int32_t tri;
 };
 
+// A triangle's boxes (see the file comment).
+struct TriBoxes {
+  Box own, wide;
+  float normal[3];   // unit, zero without area
+  float graze;       // sine below which a ray counts as in the plane; >= 1: all
+};
+
+// What a child of a wide node stores.
+struct ChildBoxes {
+  Box own, wide;
+  int8_t cone[4];
+};
+
 struct Node2 {
   Box b;
   int32_t left = -1, right = -1;  // -1: leaf
@@ -71,11 +118,18 @@ struct Node2 {
 
 constexpr int kBins = 16;
 constexpr int kLeafTris = 3;
-// Cost of a node visit over a triangle test (per-lane instruction counts of
-// the walk: about 230 per eight-child node, 60 per test).
-constexpr float kNodeCost = 1.0f;
+// Cost of a binary split over a triangle test: a visit of an eight-child node
+// stands for up to seven splits. (0.25 / 0.5 / 1 / 2: 14.9 visits and 6.2 tests
+// / 14.6, 6.6 / 14.4, 7.5 / 14.3, 8.0 a ray on the spheres.)
+constexpr float kNodeCost = 0.5f;
 constexpr int kMedianDepth = 40;
-constexpr float kPlaneGrowth = 0.02f;
+constexpr float kSplitBlend = 0.6f;
+constexpr double kUlp = 1.0 / (1 << 24);
+// Bounds of ray origins, in units of the scene's size, for which the slabs are
+// thick enough (a triangle is at most kMaxDistance away): bvh_init.
+constexpr double kMaxDistance = 16;
+// Subtrees above this size take their wide box for all rays.
+constexpr int32_t kMaxCone = 32768;
 
 class Builder2 {
  public:
@@ -258,7 +312,12 @@ struct Collapser {
   const std::vector<Prim>& prims;
   const PackedScene& scene;
   const std::vector<uint8_t>& flags;
+  const std::vector<TriBoxes>& boxes;
   PackedBvh& out;
+  struct Kids {
+    int32_t slot[8];   // binary node of each slot, -1: free
+  };
+  std::vector<Kids> kids_of;
 
   struct Item {
     int32_t src;    // binary node
@@ -266,19 +325,27 @@ struct Collapser {
     int depth;
   };
 
-  void run() {
+  // The nodes' structure in a fixed order, then their boxes on all threads.
+  void run(int threads) {
     out.nodes.clear();
     out.nodes.reserve(prims.size() / 3 + 16);
     out.tris.clear();
     out.tris.reserve(prims.size());
     out.max_depth = 0;
+    kids_of.clear();
     out.nodes.push_back(BvhNode());
+    kids_of.push_back(Kids());
     std::vector<Item> todo{{0, 0, 0}};
     while (!todo.empty()) {
       const Item it = todo.back();
       todo.pop_back();
       emit(it, todo);
     }
+    std::atomic<size_t> cursor{0};
+    run_threads(threads, [&] {
+      for (size_t k = cursor.fetch_add(64); k < out.nodes.size(); k = cursor.fetch_add(64))
+        for (size_t i = k; i < std::min(out.nodes.size(), k + 64); ++i) fill(i);
+    });
   }
 
   bool leaf(int32_t n) const { return in[n].left < 0; }
@@ -304,8 +371,8 @@ struct Collapser {
     // Slots: bit a of a slot set = far side along axis a. Greedy assignment
     // of the child whose centre lies furthest out in some free slot's
     // direction.
-    int slot_kid[8];
-    std::fill(slot_kid, slot_kid + 8, -1);
+    Kids& w = kids_of[it.dst];
+    std::fill(w.slot, w.slot + 8, -1);
     bool placed[8] = {};
     for (int k = 0; k < n; ++k) {
       float best = -FLT_MAX;
@@ -316,7 +383,7 @@ struct Collapser {
         float d[3];
         for (int a = 0; a < 3; ++a) d[a] = (b.lo[a] + b.hi[a]) - (nb.lo[a] + nb.hi[a]);
         for (int s = 0; s < 8; ++s) {
-          if (slot_kid[s] >= 0) continue;
+          if (w.slot[s] >= 0) continue;
           float v = 0.f;
           for (int a = 0; a < 3; ++a) v += (s >> a & 1) ? d[a] : -d[a];
           if (v > best) {
@@ -327,32 +394,134 @@ struct Collapser {
         }
       }
       if (bc < 0) break;  // not reached: a free slot and child remain
-      slot_kid[bs] = kids[bc];
+      w.slot[bs] = kids[bc];
       placed[bc] = true;
     }
-    BvhNode w;
-    memset(&w, 0, sizeof w);
-    quantise(nb, slot_kid, w);
-    w.child_base = (uint32_t)out.nodes.size();
-    w.tri_base = (uint32_t)out.tris.size();
+    BvhNode node;
+    memset(&node, 0, sizeof node);
+    node.child_base = (uint32_t)out.nodes.size();
+    node.tri_base = (uint32_t)out.tris.size();
     int inner = 0, tris = 0;
+    uint32_t next = node.child_base;
     for (int s = 0; s < 8; ++s) {
-      if (slot_kid[s] < 0) continue;
-      const Node2& c = in[slot_kid[s]];
-      if (!leaf(slot_kid[s])) {
-        w.imask |= (uint8_t)(1u << s);
+      const int32_t src = w.slot[s];
+      if (src < 0) continue;
+      const Node2& c = in[src];
+      if (!leaf(src)) {
+        node.imask |= (uint8_t)(1u << s);
         ++inner;
+        todo.push_back({src, next++, it.depth + 1});
         continue;
       }
-      w.meta[s] = (uint8_t)((((1u << c.count) - 1u) << 5) | (uint32_t)tris);
+      node.meta[s] = (uint8_t)((((1u << c.count) - 1u) << 5) | (uint32_t)tris);
       for (int32_t i = 0; i < c.count; ++i) out.tris.push_back(record(prims[c.begin + i].tri));
       tris += c.count;
     }
+    out.nodes[it.dst] = node;
     out.nodes.resize(out.nodes.size() + inner);
-    uint32_t next = w.child_base;
-    for (int s = 0; s < 8; ++s)
-      if (slot_kid[s] >= 0 && !leaf(slot_kid[s])) todo.push_back({slot_kid[s], next++, it.depth + 1});
-    out.nodes[it.dst] = w;
+    kids_of.resize(out.nodes.size());
+  }
+
+  // The boxes and planes of wide node i.
+  void fill(size_t i) {
+    ChildBoxes kids[8];
+    Box all;
+    all.reset();
+    for (int s = 0; s < 8; ++s) {
+      if (kids_of[i].slot[s] < 0) continue;
+      kids[s] = child_boxes(in[kids_of[i].slot[s]]);
+      all.add(kids[s].wide);
+    }
+    quantise(all, kids_of[i].slot, kids, out.nodes[i]);
+  }
+
+  // A subtree's box may be grown so that it holds the wide boxes of some of
+  // its triangles; the others' wide boxes, and the cone around their normals,
+  // make up the child's wide box. Of a few growths, the one with the smallest
+  // expected area.
+  ChildBoxes child_boxes(const Node2& c) const {
+    ChildBoxes r;
+    Box own, wide;
+    own.reset();
+    wide.reset();
+    for (int32_t i = c.begin; i < c.begin + c.count; ++i) {
+      own.add(boxes[(size_t)prims[i].tri].own);
+      wide.add(boxes[(size_t)prims[i].tri].wide);
+    }
+    const int8_t never[4] = {0, 0, 0, -1};
+    r.own = wide;
+    r.wide = wide;
+    memcpy(r.cone, never, 4);
+    if (c.count > kMaxCone) return r;
+    float extent = 0.f, best = wide.half_area();
+    for (int a = 0; a < 3; ++a) extent = std::max(extent, own.hi[a] - own.lo[a]);
+    for (const float g : {0.f, 0.02f, 0.07f, 0.2f}) {
+      Box b;
+      for (int a = 0; a < 3; ++a) {
+        const float by = g * std::max(0.3f * extent, own.hi[a] - own.lo[a]);
+        b.lo[a] = std::max(wide.lo[a], own.lo[a] - by);
+        b.hi[a] = std::min(wide.hi[a], own.hi[a] + by);
+      }
+      Box w = b;
+      int8_t around[4];
+      const float part = cone(c, b, w, around);
+      const float cost = b.half_area() + part * (w.half_area() - b.half_area());
+      if (cost < best) {
+        best = cost;
+        r.own = b;
+        r.wide = w;
+        memcpy(r.cone, around, 4);
+      }
+      if (part == 0.f) break;  // b holds all: the larger ones cost more
+    }
+    return r;
+  }
+
+  // The cone for those of c's triangles whose wide boxes b does not hold;
+  // adds these boxes to w. Returns the share of all directions it takes.
+  float cone(const Node2& c, const Box& b, Box& w, int8_t around[4]) const {
+    double axis[3] = {0, 0, 0}, length = 0;
+    bool any = false, all = false;
+    for (int32_t i = c.begin; i < c.begin + c.count; ++i) {
+      const TriBoxes& t = boxes[(size_t)prims[i].tri];
+      if (b.holds(t.wide)) continue;
+      any = true;
+      w.add(t.wide);
+      all = all || t.graze >= 1.f;
+      const double side =
+          axis[0] * t.normal[0] + axis[1] * t.normal[1] + axis[2] * t.normal[2] < 0 ? -1 : 1;
+      for (int a = 0; a < 3; ++a) axis[a] += side * t.normal[a];
+    }
+    const int8_t never[4] = {0, 0, 0, -1}, always[4] = {0, 0, 0, 1};
+    memcpy(around, any ? always : never, 4);
+    if (!any) return 0.f;
+    for (int a = 0; a < 3; ++a) length += axis[a] * axis[a];
+    length = std::sqrt(length);
+    if (all || !(length > 1e-6)) return 1.f;
+    // The axis in 127ths, and the largest |axis . d| of a direction within
+    // some triangle's grazing angle of its plane; d's own bytes are off by up
+    // to half a 127th.
+    double q[3], norm = 0, off = 0, sine = 0;
+    for (int a = 0; a < 3; ++a) {
+      q[a] = std::nearbyint(127 * axis[a] / length);
+      norm += q[a] * q[a];
+      off += 0.501 * std::fabs(q[a]);
+    }
+    norm = std::sqrt(norm);
+    for (int32_t i = c.begin; i < c.begin + c.count && sine < 1; ++i) {
+      const TriBoxes& t = boxes[(size_t)prims[i].tri];
+      if (b.holds(t.wide)) continue;
+      const double dot = std::min(
+          1.0, std::fabs(q[0] * t.normal[0] + q[1] * t.normal[1] + q[2] * t.normal[2]) / norm);
+      // asin(graze) + the angle between normal and axis.
+      const double angle = std::asin((double)t.graze) + std::acos(dot);
+      sine = angle < 1.570 ? std::max(sine, std::sin(angle)) : 1;
+    }
+    const double s = std::ceil((127 * norm * sine + off) / 127 + 1e-3);
+    if (sine >= 1 || s >= 127) return 1.f;
+    for (int a = 0; a < 3; ++a) around[a] = (int8_t)q[a];
+    around[3] = (int8_t)s;
+    return (float)(s / 127);
   }
 
   BvhTri record(int32_t id) const {
@@ -371,7 +540,12 @@ struct Collapser {
 
   // Child planes rounded outward by at least 1/64 of a step, which covers the
   // walk's decoding error (1/512 of a step).
-  void quantise(const Box& nb, const int slot_kid[8], BvhNode& w) const {
+  static void quantise(const Box& nb, const int32_t slot[8], const ChildBoxes kids[8],
+                       BvhNode& w) {
+    for (int k = 0; k < 8; ++k) {
+      const int8_t never[4] = {0, 0, 0, -1};
+      memcpy(w.cone[k], slot[k] < 0 ? never : kids[k].cone, 4);
+    }
     for (int a = 0; a < 3; ++a) {
       int e = -100;
       const double ext = (double)nb.hi[a] - nb.lo[a];
@@ -387,17 +561,24 @@ struct Collapser {
         if (((double)nb.hi[a] - p) / s + 1.0 / 64 <= 255.0) break;
       }
       w.e[a] = (uint8_t)(e + 127);
+      auto low = [&](double x) {
+        return (uint8_t)std::min(255.0, std::max(0.0, std::floor((x - p) / s - 1.0 / 64)));
+      };
+      auto high = [&](double x) {
+        return (uint8_t)std::min(255.0, std::max(0.0, std::ceil((x - p) / s + 1.0 / 64)));
+      };
       for (int k = 0; k < 8; ++k) {
-        if (slot_kid[k] < 0) {
-          w.qlo[a][k] = 255;  // an empty slot: lower plane above the upper one
-          w.qhi[a][k] = 0;
+        if (slot[k] < 0) {
+          // An empty slot: lower plane above the upper one (and a hit of it
+          // adds no child).
+          w.qlo[a][k] = w.wlo[a][k] = 255;
+          w.qhi[a][k] = w.whi[a][k] = 0;
           continue;
         }
-        const Box& b = in[slot_kid[k]].b;
-        const double lo = std::floor(((double)b.lo[a] - p) / s - 1.0 / 64);
-        const double hi = std::ceil(((double)b.hi[a] - p) / s + 1.0 / 64);
-        w.qlo[a][k] = (uint8_t)std::min(255.0, std::max(0.0, lo));
-        w.qhi[a][k] = (uint8_t)std::min(255.0, std::max(0.0, hi));
+        w.qlo[a][k] = low(kids[k].own.lo[a]);
+        w.qhi[a][k] = high(kids[k].own.hi[a]);
+        w.wlo[a][k] = low(kids[k].wide.lo[a]);
+        w.whi[a][k] = high(kids[k].wide.hi[a]);
       }
     }
   }
@@ -425,6 +606,92 @@ int64_t touched_leaves(const PackedScene& scene, const Box& b, std::vector<uint3
   return count;
 }
 
+// Bounds that several threads grow.
+struct SharedBox {
+  std::atomic<float> lo[3], hi[3];
+  void set(const Box& b) {
+    for (int a = 0; a < 3; ++a) {
+      lo[a].store(b.lo[a], std::memory_order_relaxed);
+      hi[a].store(b.hi[a], std::memory_order_relaxed);
+    }
+  }
+  Box get() const {
+    Box b;
+    for (int a = 0; a < 3; ++a) {
+      b.lo[a] = lo[a].load(std::memory_order_relaxed);
+      b.hi[a] = hi[a].load(std::memory_order_relaxed);
+    }
+    return b;
+  }
+  void add(const Box& b) {
+    for (int a = 0; a < 3; ++a) {
+      for (float x = lo[a].load(std::memory_order_relaxed);
+           b.lo[a] < x && !lo[a].compare_exchange_weak(x, b.lo[a], std::memory_order_relaxed);) {
+      }
+      for (float x = hi[a].load(std::memory_order_relaxed);
+           b.hi[a] > x && !hi[a].compare_exchange_weak(x, b.hi[a], std::memory_order_relaxed);) {
+      }
+    }
+  }
+};
+
+// What the wide boxes need to know of a triangle.
+struct Plane {
+  double n[3];       // unit normal
+  double graze;      // TriBoxes::graze
+  double thickness;  // the slab's, beside graze times the distance
+  bool wide;         // has a wide box
+};
+Plane plane_of(const DevTri& t, double scene_size) {
+  Plane p;
+  memset(&p, 0, sizeof p);
+  double l1 = 0, l2 = 0, l = 0;
+  bool flat = false;
+  for (int a = 0; a < 3; ++a) {
+    const int b = (a + 1) % 3, c = (a + 2) % 3;
+    p.n[a] = (double)t.e1[b] * t.e2[c] - (double)t.e1[c] * t.e2[b];
+    l1 += (double)t.e1[a] * t.e1[a];
+    l2 += (double)t.e2[a] * t.e2[a];
+    l += p.n[a] * p.n[a];
+    flat = flat || (t.e1[a] == 0.f && t.e2[a] == 0.f);
+  }
+  l = std::sqrt(l);
+  const double s = l1 > 0 && l2 > 0 ? l / std::sqrt(l1 * l2) : 0;
+  for (int a = 0; a < 3; ++a) p.n[a] = l > 0 ? p.n[a] / l : 0;
+  p.graze = s > kGrazing ? kGrazing / s : 1;
+  p.thickness = s > kGrazing ? 14 * kUlp * kMaxDistance * scene_size / s : 0;
+  p.wide = p.graze >= 1 || !flat;
+  return p;
+}
+
+// Narrows leaf box b to where the slab of triangle t (bounds tb, plane p)
+// passes. False when it does not.
+bool clip_to_slab(const DevTri& t, const Box& tb, const Plane& p, Box& b) {
+  if (p.graze >= 1) return true;
+  double lo[3], hi[3], reach = 0, round = 0;
+  for (int a = 0; a < 3; ++a) {
+    const double x = p.n[a] * ((double)b.lo[a] - t.a[a]), y = p.n[a] * ((double)b.hi[a] - t.a[a]);
+    lo[a] = std::min(x, y);
+    hi[a] = std::max(x, y);
+    const double far_off =
+        std::max((double)b.hi[a] - tb.lo[a], (double)tb.hi[a] - b.lo[a]);
+    reach += far_off * far_off;
+    round = std::max({round, std::fabs((double)b.lo[a]), std::fabs((double)b.hi[a])});
+  }
+  // n.(x - a) within [-h, h] (the floats of a box are rounded outward).
+  const double h = p.graze * std::sqrt(reach) + p.thickness + 4 * kUlp * round;
+  for (int a = 0; a < 3; ++a) {
+    const int c = (a + 1) % 3, d = (a + 2) % 3;
+    const double l = -h - hi[c] - hi[d], m = h - lo[c] - lo[d];
+    if (std::max(l, lo[a]) > std::min(m, hi[a])) return false;
+    if (std::fabs(p.n[a]) < 1e-9) continue;
+    const double x = t.a[a] + l / p.n[a], y = t.a[a] + m / p.n[a];
+    b.lo[a] = std::max(b.lo[a], std::nextafterf((float)std::min(x, y), -INFINITY));
+    b.hi[a] = std::min(b.hi[a], std::nextafterf((float)std::max(x, y), INFINITY));
+  }
+  return true;
+}
+
 }  // namespace
 
 void build_bvh(const float* points, const int32_t* triangles, const PackedScene& scene,
@@ -436,12 +703,16 @@ void build_bvh(const float* points, const int32_t* triangles, const PackedScene&
                           ? num_threads
                           : (int)std::max(1u, std::thread::hardware_concurrency());
   // Per triangle: its bounds, the union of the leaves that list it, how many
-  // do, and its flags.
-  std::vector<Box> bounds(n), boxes(n);
+  // do, its flags and its boxes.
+  std::vector<Box> bounds(n), leaves(n);
   std::vector<int32_t> listed(n, 0);
   std::vector<uint8_t> flags(n, 0);
+  std::vector<Plane> planes(n);
+  std::vector<SharedBox> wide(n);
+  // (scene_eps is 2e-5 of the scene's size.)
+  const double scene_size = scene_eps / 2e-5;
   for (size_t i = 0; i < n; ++i) {
-    boxes[i].reset();
+    leaves[i].reset();
     bounds[i].reset();
     for (int k = 0; k < 3; ++k) {
       const float* v = points + 4 * (size_t)triangles[4 * i + k];
@@ -450,6 +721,30 @@ void build_bvh(const float* points, const int32_t* triangles, const PackedScene&
         bounds[i].hi[a] = std::max(bounds[i].hi[a], v[a]);
       }
     }
+    planes[i] = plane_of(scene.tris[i], scene_size);
+    wide[i].set(bounds[i]);
+  }
+  {
+    std::atomic<size_t> cursor{0};
+    run_threads(threads, [&] {
+      const size_t count = scene.leaves.size(), step = 256;
+      for (size_t i = cursor.fetch_add(step); i < count; i = cursor.fetch_add(step))
+        for (size_t l = i; l < std::min(count, i + step); ++l) {
+          const DevLeaf& L = scene.leaves[l];
+          Box b;
+          for (int a = 0; a < 3; ++a) {
+            b.lo[a] = L.lo[a];
+            b.hi[a] = L.hi[a];
+          }
+          for (int32_t k = 0; k < L.tri_count; ++k) {
+            const size_t id = (size_t)scene.refs[(size_t)L.tri_begin + k];
+            Box part = b;
+            if (planes[id].wide && !wide[id].get().holds(b) &&
+                clip_to_slab(scene.tris[id], bounds[id], planes[id], part))
+              wide[id].add(part);
+          }
+        }
+    });
   }
   const float near = kCertainNear * scene_eps;
   for (const DevLeaf& L : scene.leaves) {
@@ -464,7 +759,7 @@ void build_bvh(const float* points, const int32_t* triangles, const PackedScene&
                                    scene.refs[(size_t)L.tri_begin + k];
     for (int32_t k = 0; k < L.tri_count; ++k) {
       const size_t id = (size_t)scene.refs[(size_t)L.tri_begin + k];
-      boxes[id].add(b);
+      leaves[id].add(b);
       ++listed[id];
       const Box& t = bounds[id];
       uint32_t f = ascending ? 0u : kTriUnordered;
@@ -502,30 +797,34 @@ void build_bvh(const float* points, const int32_t* triangles, const PackedScene&
       }
     });
   }
-  const float pad = 0.1f * scene_eps;
+  std::vector<TriBoxes> boxes(n);
   std::vector<Prim> prims;
   prims.reserve(n);
   for (size_t i = 0; i < n; ++i) {
-    Prim p;
-    p.b = boxes[i];
-    p.tri = (int32_t)i;
-    if (p.b.lo[0] > p.b.hi[0]) continue;  // no leaf lists it: never tested
-    const DevTri& t = scene.tris[i];
-    const float nx = t.e1[1] * t.e2[2] - t.e1[2] * t.e2[1];
-    const float ny = t.e1[2] * t.e2[0] - t.e1[0] * t.e2[2];
-    const float nz = t.e1[0] * t.e2[1] - t.e1[1] * t.e2[0];
-    const float n[3] = {nx, ny, nz}, nn = nx * nx + ny * ny + nz * nz;
-    const Box& tb = bounds[i];
-    float extent = 0.f;
-    for (int a = 0; a < 3; ++a) extent = std::max(extent, tb.hi[a] - tb.lo[a]);
+    if (!listed[i]) continue;  // no leaf lists it: never tested
+    TriBoxes& t = boxes[i];
+    t.own = bounds[i];
+    t.wide = wide[i].get();
+    t.graze = (float)planes[i].graze;
+    double edge = 0, coordinate = 0;
     for (int a = 0; a < 3; ++a) {
-      const float in_plane = nn > 0.f ? std::sqrt(std::max(0.f, 1.f - n[a] * n[a] / nn)) : 1.f;
-      p.b.lo[a] = std::max(p.b.lo[a], tb.lo[a] - kPlaneGrowth * extent * in_plane);
-      p.b.hi[a] = std::min(p.b.hi[a], tb.hi[a] + kPlaneGrowth * extent * in_plane);
+      t.normal[a] = (float)planes[i].n[a];
+      edge = std::max({edge, std::fabs((double)scene.tris[i].e1[a]),
+                       std::fabs((double)scene.tris[i].e2[a])});
+      coordinate = std::max({coordinate, std::fabs((double)t.wide.lo[a]),
+                             std::fabs((double)t.wide.hi[a])});
     }
+    // (max|e| is at most sqrt 3 times the largest component.)
+    const double pad = kUlp * (8 * coordinate + 70 * edge / kGrazing);
+    Prim p;
+    p.tri = (int32_t)i;
     for (int a = 0; a < 3; ++a) {
-      p.b.lo[a] -= pad;
-      p.b.hi[a] += pad;
+      t.own.lo[a] = std::nextafterf((float)(t.own.lo[a] - pad), -INFINITY);
+      t.own.hi[a] = std::nextafterf((float)(t.own.hi[a] + pad), INFINITY);
+      t.wide.lo[a] = std::nextafterf((float)(t.wide.lo[a] - pad), -INFINITY);
+      t.wide.hi[a] = std::nextafterf((float)(t.wide.hi[a] + pad), INFINITY);
+      p.b.lo[a] = t.own.lo[a] + kSplitBlend * (t.wide.lo[a] - t.own.lo[a]);
+      p.b.hi[a] = t.own.hi[a] + kSplitBlend * (t.wide.hi[a] - t.own.hi[a]);
     }
     prims.push_back(p);
   }
@@ -535,18 +834,19 @@ void build_bvh(const float* points, const int32_t* triangles, const PackedScene&
       out.nodes.assign(1, BvhNode());
       memset(&out.nodes[0], 0, sizeof(BvhNode));
       memset(out.nodes[0].qlo, 255, sizeof out.nodes[0].qlo);
+      memset(out.nodes[0].wlo, 255, sizeof out.nodes[0].wlo);
       break;
     }
     Builder2 b2(prims, median);
     b2.run(threads);
-    Collapser c{b2.nodes, prims, scene, flags, out};
-    c.run();
+    Collapser c{b2.nodes, prims, scene, flags, boxes, out, {}};
+    c.run(threads);
     if (out.max_depth < kBvhStack - 1) break;
   }
   // Where the certificate's descent starts: the lowest tree node that holds
   // every leaf listing the triangle.
   for (BvhTri& t : out.tris) {
-    const Box& b = boxes[(size_t)t.tri_id];
+    const Box& b = leaves[(size_t)t.tri_id];
     uint32_t node = 0;
     while (true) {
       const DevNode& d = scene.nodes[node];

@@ -57,14 +57,17 @@ struct DevTri {
 static_assert(sizeof(DevTri) == 48, "48-byte triangle record");
 
 // --- Bounding volume hierarchy ---------------------------------------------
-// 8-wide node with child boxes quantised to 8 bits per plane (the published
-// compressed wide layout of Ylitie, Karras and Laine, "Efficient Incoherent
-// Ray Traversal on GPUs Through Compressed Wide BVHs", 2017), 80 bytes
-// (5 x 16 B). A child's plane q on axis a lies at p[a] + q * 2^e[a].
+// 8-wide node with child boxes quantised to 8 bits per plane (after the
+// published compressed wide layout of Ylitie, Karras and Laine, "Efficient
+// Incoherent Ray Traversal on GPUs Through Compressed Wide BVHs", 2017), 160
+// bytes (10 x 16 B). A child's plane q on axis a lies at p[a] + q * 2^e[a].
 //  slot i is an inner child when bit i of imask is set: its node is
 //  child_base + popcount(imask & ((1 << i) - 1)). Otherwise meta[i] is 0 (no
 //  child) or a leaf: bits 0-4 = first triangle relative to tri_base, bits
 //  5-7 = one bit per triangle (1 to 3 triangles).
+// A child has two boxes. A ray of direction d (d / |d| in 127ths) visits it
+// by its wide box when it may run almost in the plane of a triangle below
+// that the other box does not cover (bvh_build.cpp): |cone . d| <= 127 cone_s.
 struct BvhNode {
   float p[3];
   uint8_t e[3];             // biased exponents (float bits e << 23)
@@ -74,8 +77,11 @@ struct BvhNode {
   uint8_t meta[8];
   uint8_t qlo[3][8];        // x, y, z lower planes of the 8 slots
   uint8_t qhi[3][8];        // upper planes
+  uint8_t wlo[3][8];        // the same of the wide boxes
+  uint8_t whi[3][8];
+  int8_t cone[8][4];        // x, y, z, cone_s
 };
-static_assert(sizeof(BvhNode) == 80, "80-byte wide node");
+static_assert(sizeof(BvhNode) == 160, "160-byte wide node");
 
 // Triangle record in node order: the DevTri values, and for the certificate
 // (bvh_certain in bvh.cuh) the lowest tree node that holds every leaf listing
@@ -100,6 +106,16 @@ constexpr uint32_t kTriIrregular = 64u, kTriUnordered = 128u;
 // the leaf faces that count as just outside a triangle's bounds.
 constexpr float kCertainRound = 0.2f;
 constexpr float kCertainNear = 4 * kCertainRound;
+
+// Boxes of the hierarchy (derived in bvh_build.cpp): the sine of the angle to a
+// triangle's plane, times the sine of its angle at vertex a, below which a ray
+// counts as running in the plane; and what the walk grows boxes by, per
+// distance from the ray's origin (37 roundings of 2^-24 over kGrazing). Boxes
+// that begin beyond kCullFactor times the best t so far (16 such roundings
+// beyond it), plus the slack of the tree walk's stopping rule, are not visited.
+constexpr float kGrazing = 0.005f;
+constexpr float kBoxGrowth = 2.2e-6f / kGrazing;
+constexpr float kCullFactor = 1.0001f + 1e-6f / kGrazing;
 
 // Entries of a ray's node stack; the builder bounds the depth below it (one
 // entry at most per level).

@@ -1,0 +1,69 @@
+"""CPU test of the rays for which the hierarchy's boxes have to be larger than
+its triangles: the triangle test's rounding accepts rays that pass beside a
+triangle, and the answer is still the tree walk's bit for bit."""
+import numpy as np
+import pytest
+
+import hptracing_b200 as H
+from tests.test_bvh import _check, _mesh, _scene, emu
+
+
+def _turn(mesh):
+    """The mesh turned, so that no plane of it is along an axis."""
+    q, _ = np.linalg.qr(np.random.default_rng(1).normal(size=(3, 3)))
+    m = _mesh((mesh.points[:, :3] - 0.5) @ q.T, mesh.triangles[:, :3])
+    return (m, *H.build_kdtree(m.points, m.triangles))
+
+
+def _plane(n=40):
+    """A tessellated unit square."""
+    g = np.stack(np.meshgrid(*2 * [np.linspace(0, 1, n + 1)], indexing="ij"), -1).reshape(-1, 2)
+    i = (np.arange(n)[:, None] * (n + 1) + np.arange(n)).ravel()
+    return _mesh(np.concatenate([g, np.full((len(g), 1), 0.5)], 1),
+                 np.concatenate([np.stack([i, i + 1, i + n + 2], 1), np.stack([i, i + n + 2, i + n + 1], 1)]))
+
+
+def _corners(mesh, k):
+    p = mesh.points[:, :3].astype(np.float64)
+    return [p[mesh.triangles[k, j]] for j in range(3)]
+
+
+def _unit(v):
+    return v / np.maximum(np.linalg.norm(v, axis=1, keepdims=True), 1e-30)
+
+
+def _in_plane(mesh, n, seed):
+    """Rays through two points of a triangle's plane: the origin up to a scene
+    size away, the other point within three edges."""
+    rng = np.random.default_rng(seed)
+    a, b, c = _corners(mesh, rng.integers(0, len(mesh.triangles), n))
+    p = mesh.points[:, :3].astype(np.float64)
+    u = _unit(b - a)
+    w = _unit((c - a) - ((c - a) * u).sum(1, keepdims=True) * u)
+    away = np.linalg.norm(p.max(0) - p.min(0)) * 10.0 ** rng.uniform(-3, 0, (n, 1))
+    x = rng.uniform(-1, 1, (2, n, 1)) * away
+    y = rng.uniform(-3, 3, (2, n, 1)) * np.linalg.norm(b - a, axis=1, keepdims=True)
+    o = (a + b + c) / 3 + x[0] * u + x[1] * w
+    return o, _unit((a + b + c) / 3 + y[0] * u + y[1] * w - o)
+
+
+def _along_surface(mesh, n, seed):
+    """From a point of a triangle towards another of the same one, as a light
+    that samples itself."""
+    rng = np.random.default_rng(seed)
+    tri = _corners(mesh, rng.integers(0, len(mesh.triangles), n))
+    o, q = (sum(w[:, None] * v for w, v in zip(rng.dirichlet([1, 1, 1], n).T, tri)).astype(np.float32)
+            for _ in range(2))
+    d = _unit((q - o).astype(np.float64)).astype(np.float32)
+    return o + np.float32(1e-5) * d, d
+
+
+@pytest.mark.parametrize("name", ["room", "turned room", "plane", "turned plane", "soup", "degenerate", "spheres",
+                                  "terrain"])
+def test_rays_in_a_triangles_plane(name):
+    scene = {"turned room": lambda: _turn(_scene("room")[0]), "turned plane": lambda: _turn(_plane()),
+             "plane": lambda: (lambda m: (m, *H.build_kdtree(m.points, m.triangles)))(_plane())}
+    mesh, nodes, leaf = scene.get(name, lambda: _scene(name))()
+    e = emu.BvhEmu(mesh, nodes, leaf)
+    _check(e.query(*_in_plane(mesh, 40000, 5)))
+    _check(e.query(*_along_surface(mesh, 30000, 6)))
