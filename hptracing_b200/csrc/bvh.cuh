@@ -642,6 +642,9 @@ __host__ __device__ __noinline__ bool walk_for(const Sc& s, const Ray& r, uint32
       }
     }
     if (at >= 0 && at < rank && ref_box_test(r, L0, L1)) {
+      // A t before the first leaf that has the triangle (a ray in its plane):
+      // the hierarchy left out what begins behind that t, the walk does not.
+      if (st.t_entry > stop) return false;
       rank = at;
       winner = which;
     }

@@ -67,3 +67,23 @@ def test_rays_in_a_triangles_plane(name):
     e = emu.BvhEmu(mesh, nodes, leaf)
     _check(e.query(*_in_plane(mesh, 40000, 5)))
     _check(e.query(*_along_surface(mesh, 30000, 6)))
+
+
+def test_hit_before_its_leaf():
+    """In a triangle's plane the computed t may lie before every leaf that has
+    the triangle; in the first of them another one may be nearer still."""
+    g = _plane(60)
+    q, _ = np.linalg.qr(np.random.default_rng(1).normal(size=(3, 3)))
+    m = _mesh((g.points[:, :3] - np.float32([0, 0, 0.5])) @ q.T, g.triangles[:, :3])
+    e = emu.BvhEmu(m, *H.build_kdtree(m.points, m.triangles))
+    o = [[0.05844295769929886, 0.13787004351615906, 0.07542713731527328],
+         [-2.018704652786255, 0.4258774518966675, -0.19801566004753113],
+         [-1.3616396188735962, -1.131714105606079, -0.7919849753379822],
+         [1.0416405200958252, 0.9955244064331055, 0.6660779118537903],
+         [0.4593617916107178, 0.31658682227134705, 0.23692654073238373]]
+    d = [[-0.5454838275909424, -0.7143399715423584, -0.43836721777915955],
+         [0.8948383927345276, 0.31137898564338684, 0.3198552131652832],
+         [0.34956181049346924, 0.8218493461608887, 0.4498557448387146],
+         [-0.7876143455505371, -0.48537158966064453, -0.3795762062072754],
+         [-0.7643405795097351, -0.5145841836929321, -0.3885699212551117]]
+    _check(e.query(np.float32(o), np.float32(d)))
