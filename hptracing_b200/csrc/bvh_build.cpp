@@ -747,18 +747,26 @@ void build_bvh(const float* points, const int32_t* triangles, const PackedScene&
     });
   }
   const float near = kCertainNear * scene_eps;
+  std::vector<int32_t> unique;
   for (const DevLeaf& L : scene.leaves) {
     Box b;
     for (int a = 0; a < 3; ++a) {
       b.lo[a] = L.lo[a];
       b.hi[a] = L.hi[a];
     }
+    const int32_t* ids = scene.refs.data() + L.tri_begin;
+    int32_t count = L.tri_count;
     bool ascending = true;
-    for (int32_t k = 1; k < L.tri_count; ++k)
-      ascending = ascending && scene.refs[(size_t)L.tri_begin + k - 1] <
-                                   scene.refs[(size_t)L.tri_begin + k];
-    for (int32_t k = 0; k < L.tri_count; ++k) {
-      const size_t id = (size_t)scene.refs[(size_t)L.tri_begin + k];
+    for (int32_t k = 1; k < count; ++k) ascending = ascending && ids[k - 1] < ids[k];
+    if (!ascending) {  // a triangle may be there twice: it counts once
+      unique.assign(ids, ids + count);
+      std::sort(unique.begin(), unique.end());
+      unique.erase(std::unique(unique.begin(), unique.end()), unique.end());
+      ids = unique.data();
+      count = (int32_t)unique.size();
+    }
+    for (int32_t k = 0; k < count; ++k) {
+      const size_t id = (size_t)ids[k];
       leaves[id].add(b);
       ++listed[id];
       const Box& t = bounds[id];

@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 import hptracing_b200 as H
+from tests import scenes as S
 from tests.test_bvh import _check, _mesh, _scene, emu
 
 
@@ -87,3 +88,35 @@ def test_hit_before_its_leaf():
          [-0.7876143455505371, -0.48537158966064453, -0.3795762062072754],
          [-0.7643405795097351, -0.5145841836929321, -0.3885699212551117]]
     _check(e.query(np.float32(o), np.float32(d)))
+
+
+def _other_tree(nodes, leaf, count, drop, add, seed):
+    """The leaf lists with a share of the entries dropped and some triangles
+    added, most of which the leaf does not touch; some entries twice."""
+    rng = np.random.default_rng(seed)
+    lists, at, used = [], {}, 0
+    for off in nodes["data"][(nodes["child"] < 0) & (nodes["data"] >= 0)]:
+        ids = leaf[off + 1:off + 1 + leaf[off]]
+        ids = ids[rng.random(len(ids)) >= drop]
+        more = rng.integers(0, count, rng.binomial(4, add))
+        twice = ids[:1] if rng.random() < add else ids[:0]
+        ids = np.concatenate([ids, more, twice])
+        at[int(off)] = used
+        lists.append(np.concatenate([[len(ids)], ids]))
+        used += 1 + len(ids)
+    nodes = nodes.copy()
+    has = (nodes["child"] < 0) & (nodes["data"] >= 0)
+    nodes["data"][has] = [at[int(x)] for x in nodes["data"][has]]
+    return nodes, np.concatenate(lists).astype(np.int32)
+
+
+@pytest.mark.parametrize("name", ["nine", "soup", "room", "flat"])
+@pytest.mark.parametrize("drop,add", [(0.1, 0), (0.5, 0), (0.9, 0), (0, 0.5), (0.3, 0.2)])
+def test_tree_with_other_lists(name, drop, add):
+    """A caller's tree need not list a triangle in the leaves it touches, and
+    may list it in others: the answer is that tree's."""
+    mesh, nodes, leaf = _scene(name)
+    nodes, leaf = _other_tree(nodes, leaf, len(mesh.triangles), drop, add, 3)
+    e = emu.BvhEmu(mesh, nodes, leaf)
+    _check(e.query(*S.aabb_random_rays(mesh, 20000, 3)))
+    _check(e.query(*_in_plane(mesh, 5000, 4)))
