@@ -172,8 +172,9 @@ HPT_HD uint32_t direction_bytes(const f3& d, float scale127) {
 }
 
 // Starts a walk. Returns false when the ray is to be walked through the tree
-// instead (non-finite rays, directions of extreme length).
-HPT_HD bool bvh_init(const Ray& r, BvhRay& b) {
+// instead (non-finite rays, directions of extreme length, origins so far away
+// that the roundings outgrow what the boxes and the certificate allow for).
+HPT_HD bool bvh_init(const Ray& r, float scene_eps, BvhRay& b) {
   b.ray = r;
   b.best = kBvhNone;
   b.best_t = b.cull = as_float(0x7f800000);
@@ -194,7 +195,10 @@ HPT_HD bool bvh_init(const Ray& r, BvhRay& b) {
       (b.inv.x > 0.f ? 1u : 0u) | (b.inv.y > 0.f ? 2u : 0u) | (b.inv.z > 0.f ? 4u : 0u);
   b.node_base = 0;
   b.node_bits = (oct << 16) | (1u << 8) | (1u << oct);
-  if (!(finite3(r.o) && finite3(r.d) && dmax > 1e-15f && dmax < 1e15f)) return false;
+  const float omax = fmaxf(fabsf(r.o.x), fmaxf(fabsf(r.o.y), fabsf(r.o.z)));
+  if (!(finite3(r.o) && finite3(r.d) && dmax > 1e-15f && dmax < 1e15f &&
+        omax <= rn_mul(kMaxOrigin, scene_eps)))
+    return false;
   const float len127 = rn_div(127.f, length(r.d));
   b.q = direction_bytes(r.d, len127);
   b.nq = direction_bytes(r.d, -len127);
@@ -697,7 +701,7 @@ HPT_HD bool bvh_settle(const Sc& s, const Ray& r, uint32_t& best, uint32_t tie, 
     return true;
   }
   BvhRay b;
-  bvh_init(r, b);
+  if (!bvh_init(r, s.scene_eps, b)) return false;
   uint2 stack[kBvhStack];
   while (true) {
     while (b.tri_bits) {
@@ -762,7 +766,7 @@ template <class Sc>
 HPT_HD void bvh_query(const Sc& s, const Ray& r, int32_t& tri, float& t, DevErr* err,
                       TravCount& cnt, int* how = nullptr) {
   BvhRay b;
-  bool ok = bvh_init(r, b);
+  bool ok = bvh_init(r, s.scene_eps, b);
   if (ok) {
     uint2 stack[kBvhStack];
     uint32_t tie = 0;

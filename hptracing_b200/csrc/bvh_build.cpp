@@ -125,9 +125,6 @@ constexpr float kNodeCost = 0.5f;
 constexpr int kMedianDepth = 40;
 constexpr float kSplitBlend = 0.6f;
 constexpr double kUlp = 1.0 / (1 << 24);
-// Bounds of ray origins, in units of the scene's size, for which the slabs are
-// thick enough (a triangle is at most kMaxDistance away): bvh_init.
-constexpr double kMaxDistance = 16;
 // Subtrees above this size take their wide box for all rays.
 constexpr int32_t kMaxCone = 32768;
 

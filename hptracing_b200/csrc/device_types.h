@@ -107,6 +107,13 @@ constexpr uint32_t kTriIrregular = 64u, kTriUnordered = 128u;
 constexpr float kCertainRound = 0.2f;
 constexpr float kCertainNear = 4 * kCertainRound;
 
+// Origins beyond 4 times the scene's size (in units of scene_eps; a coordinate)
+// are walked through the tree: 16 roundings of such a coordinate are
+// kCertainRound, and the slabs of the wide boxes are as thick as a distance of
+// kMaxDistance sizes asks for.
+constexpr float kMaxOrigin = 4 / 2e-5f;
+constexpr double kMaxDistance = 5 * 1.7320508;
+
 // Boxes of the hierarchy (derived in bvh_build.cpp): the sine of the angle to a
 // triangle's plane, times the sine of its angle at vertex a, below which a ray
 // counts as running in the plane; and what the walk grows boxes by, per

@@ -671,7 +671,7 @@ __global__ void __launch_bounds__(BS, MINB) k_trace(const __grid_constant__ Engi
             max_steps = (uint32_t)s.max_steps;
             eps = s.scene_eps;
           }
-          active = bvh_init(r, b);
+          active = bvh_init(r, eps, b);
           walk = !active;
         }
       }

@@ -48,6 +48,17 @@ def _in_plane(mesh, n, seed):
     return o, _unit((a + b + c) / 3 + y[0] * u + y[1] * w - o)
 
 
+def _from_afar(mesh, n, seed, sizes):
+    """Rays from that many scene sizes away towards points of triangles."""
+    rng = np.random.default_rng(seed)
+    tri = _corners(mesh, rng.integers(0, len(mesh.triangles), n))
+    q = sum(w[:, None] * v for w, v in zip(rng.dirichlet([1, 1, 1], n).T, tri))
+    p = mesh.points[:, :3].astype(np.float64)
+    o = (0.5 * (p.min(0) + p.max(0)) + _unit(rng.normal(size=(n, 3))) * sizes * (p.max(0) - p.min(0)).max())
+    o = o.astype(np.float32)
+    return o, _unit(q - o)
+
+
 def _along_surface(mesh, n, seed):
     """From a point of a triangle towards another of the same one, as a light
     that samples itself."""
@@ -68,6 +79,17 @@ def test_rays_in_a_triangles_plane(name):
     e = emu.BvhEmu(mesh, nodes, leaf)
     _check(e.query(*_in_plane(mesh, 40000, 5)))
     _check(e.query(*_along_surface(mesh, 30000, 6)))
+
+
+@pytest.mark.parametrize("name", ["terrain", "spheres", "room", "degenerate"])
+def test_origins_far_away(name):
+    """The roundings of boxes, test and certificate grow with the distance."""
+    mesh, nodes, leaf = _scene(name)
+    e = emu.BvhEmu(mesh, nodes, leaf)
+    for sizes in (1.5, 3, 4.2, 10, 100, 1000, 4000, 10000):
+        _check(e.query(*_from_afar(mesh, 10000, 7, sizes)))
+    # Most rays from a few sizes away do not need the tree.
+    assert e.query(*_from_afar(mesh, 4000, 8, 1.5))["certain"].mean() > 0.98
 
 
 def test_hit_before_its_leaf():
