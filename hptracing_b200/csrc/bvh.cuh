@@ -367,28 +367,24 @@ HPT_HD void bvh_test(const BvhTri* btris, float scene_eps, BvhRay& b, uint32_t& 
 // A ray that meets nothing misses - unless it runs exactly along a triangle's
 // edge e2: then the Moller-Trumbore test divides by zero, its comparisons
 // pass 0 / 0, and the reference "hits" the triangle at t = +inf when there is
-// no other hit. d x e2 is exactly zero only if e2 has d's zero components and
-// the same direction beside them within two roundings. True when the scene
-// has no such edge for a d with one zero component (for one without any such
-// an edge would have to be met by chance; along an axis edges are common).
+// no other hit. d x e2 comes out as exactly zero only if d has e2's direction
+// within two roundings per component. True when the scene has no such edge.
+// (A det of exactly zero with d x e2 not zero leaves the tested products +-inf
+// or NaN and is rejected, but for rounded sums that cancel by chance for a ray
+// in the triangle's plane.)
 template <class Sc>
 HPT_HD bool bvh_no_parallel_edge(const Sc& s, const f3& d) {
-  const int zeros = (d.x == 0.f) + (d.y == 0.f) + (d.z == 0.f);
-  if (zeros != 1) return false;
-  const int a = d.x == 0.f ? 0 : (d.y == 0.f ? 1 : 2);
-  const float b = a == 0 ? d.y : (a == 1 ? d.z : d.x), c = a == 0 ? d.z : (a == 1 ? d.x : d.y);
-  const float key = rn_div(b > 0.f ? c : -c, rn_add(fabsf(b), fabsf(c)));  // edge_key
+  const float x = fabsf(d.x), y = fabsf(d.y), z = fabsf(d.z);
+  const int a = x >= y && x >= z ? 0 : (y >= z ? 1 : 2);
+  const uint32_t n = (uint32_t)(a == 0 ? s.num_edge_keys[0] : (a == 1 ? s.num_edge_keys[1] : s.num_edge_keys[2]));
+  if (n == 0) return true;
   const float* keys = a == 0 ? s.edge_keys[0] : (a == 1 ? s.edge_keys[1] : s.edge_keys[2]);
-  int lo = 0, hi = a == 0 ? s.num_edge_keys[0] : (a == 1 ? s.num_edge_keys[1] : s.num_edge_keys[2]);
-  const int n = hi;
-  // (Near +-1, where the keys of one line wrap around: as if there were one.)
-  if (fabsf(key) > 1.f - 4e-7f) return false;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (ldg(keys + mid) < key - 4e-7f) lo = mid + 1;
-    else hi = mid;
-  }
-  return lo == n || ldg(keys + lo) > key + 4e-7f;
+  const float da = a == 0 ? d.x : (a == 1 ? d.y : d.z);
+  const float r1 = rn_div(a == 0 ? d.y : (a == 1 ? d.z : d.x), da);
+  const float r2 = rn_div(a == 0 ? d.z : (a == 1 ? d.x : d.y), da);
+  const uint32_t c1 = edge_cell(r1), c2 = edge_cell(r2), tag = edge_tag(c1, c2);
+  const uint4 k = ldg(reinterpret_cast<const uint4*>(keys) + edge_bucket(c1, c2, n >> 2));
+  return k.x != kEdgeAny && k.x != tag && k.y != tag && k.z != tag && k.w != tag;
 }
 
 // True when the tree walk's answer for ray r is (best, best_t), the result
@@ -397,7 +393,7 @@ template <class Sc>
 HPT_HD bool bvh_certain(const Sc& s, const Ray& r, uint32_t best, float best_t, DevErr* err) {
   if (best & (kBvhTie | kBvhMany)) return false;
   const bool axes = r.d.x != 0.f && r.d.y != 0.f && r.d.z != 0.f;
-  if (best == kBvhNone) return axes || bvh_no_parallel_edge(s, r.d);
+  if (best == kBvhNone) return bvh_no_parallel_edge(s, r.d);
   HPT_DCHECK(err, best < (uint32_t)s.num_btris, 115, best, return false);
   const float4* rec = reinterpret_cast<const float4*>(s.btris + best);
   const float4 A = ldg(rec), E1 = ldg(rec + 1), E2 = ldg(rec + 2);

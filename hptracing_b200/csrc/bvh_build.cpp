@@ -38,8 +38,8 @@
 // (Wide boxes for all rays: 20 and 18, and 30 and 37. kGrazing 0.003 / 0.004 /
 // 0.006 / 0.008: 18.4 / 18.4 / 19.3 / 20.5 visits and 7.3 / 7.2 / 7.2 / 7.3
 // tests for the terrain's bounces, 7.2 / 5.4 / 4.5 / 4.2 for its camera rays.)
-// Not covered: an accepted t = +inf, which takes a det of exactly zero: see
-// bvh_no_parallel_edge.
+// Not covered: an accepted t = +inf (the answer where nothing else is hit),
+// which takes a computed det of exactly zero: see bvh_no_parallel_edge.
 //
 // Tree. A binary tree by binned SAH (16 bins on three axes, object median
 // where bins fail or the tree gets deep), opened greedily by surface area
@@ -603,6 +603,48 @@ int64_t touched_leaves(const PackedScene& scene, const Box& b, std::vector<uint3
   return count;
 }
 
+// DevScene::edge_keys of axis a, of a size at which few buckets overflow (a
+// regular mesh has far fewer directions than edges).
+void edge_table(const std::vector<DevTri>& tris, int a, std::vector<float>& keys) {
+  const int b = (a + 1) % 3, c = (a + 2) % 3;
+  auto largest = [&](const DevTri& t) {
+    // Within rounding: a direction as good as the edge's may have another
+    // largest component.
+    const double x = 1.000001 * std::fabs((double)t.e2[a]);
+    return x > 0 && x >= std::fabs(t.e2[b]) && x >= std::fabs(t.e2[c]);
+  };
+  auto cell = [](double r) { return edge_cell((float)std::min(1.0, std::max(-1.0, r))); };
+  size_t count = 0;
+  for (const DevTri& t : tris) count += largest(t);
+  keys.clear();
+  if (count == 0) return;
+  std::vector<uint32_t> table;
+  uint32_t buckets = 1;
+  while (buckets < count / 2 && buckets < (1u << 27)) buckets *= 2;
+  for (;; buckets *= 2) {
+    size_t full = 0;
+    table.assign(4 * (size_t)buckets, 0u);
+    for (const DevTri& t : tris) {
+      if (!largest(t)) continue;
+      const double r1 = (double)t.e2[b] / t.e2[a], r2 = (double)t.e2[c] / t.e2[a];
+      for (uint32_t i = cell(r1 - kEdgeTolerance); i <= cell(r1 + kEdgeTolerance); ++i)
+        for (uint32_t j = cell(r2 - kEdgeTolerance); j <= cell(r2 + kEdgeTolerance); ++j) {
+          uint32_t* slot = table.data() + 4 * (size_t)edge_bucket(i, j, buckets);
+          const uint32_t tag = edge_tag(i, j);
+          int k = 0;
+          while (k < 4 && slot[k] != 0 && slot[k] != tag && slot[k] != kEdgeAny) ++k;
+          if (k < 4 && slot[k] == 0) slot[k] = tag;
+          if (k < 4) continue;
+          slot[0] = kEdgeAny;
+          ++full;
+        }
+    }
+    if (full <= buckets / 1024 || buckets > 4 * count) break;
+  }
+  keys.resize(table.size());
+  memcpy(keys.data(), table.data(), table.size() * sizeof(uint32_t));
+}
+
 // Bounds that several threads grow.
 struct SharedBox {
   std::atomic<float> lo[3], hi[3];
@@ -790,16 +832,7 @@ void build_bvh(const float* points, const int32_t* triangles, const PackedScene&
   {
     std::atomic<int> axis{0};
     run_threads(std::min(threads, 3), [&] {
-      for (int a = axis++; a < 3; a = axis++) {
-        std::vector<float>& keys = out.edge_keys[a];
-        keys.clear();
-        for (const DevTri& t : scene.tris) {
-          const float b = t.e2[(a + 1) % 3], c = t.e2[(a + 2) % 3];
-          if (t.e2[a] == 0.f && (b != 0.f || c != 0.f)) keys.push_back(edge_key(b, c));
-        }
-        std::sort(keys.begin(), keys.end());
-        keys.erase(std::unique(keys.begin(), keys.end()), keys.end());
-      }
+      for (int a = axis++; a < 3; a = axis++) edge_table(scene.tris, a, out.edge_keys[a]);
     });
   }
   std::vector<TriBoxes> boxes(n);

@@ -134,6 +134,26 @@ struct DevTexInfo {
   int32_t w, h;
 };
 
+// Hash of edge directions. The other two components over the largest one, r1
+// and r2 in [-1, 1], give a cell of 2^-16 by 2^-16; a bucket of four words holds
+// the tags of the cells that edges are in, within kEdgeTolerance (0: no entry;
+// first one kEdgeAny: more than four).
+#ifdef __CUDACC__
+#define HPT_SHARED __host__ __device__ __forceinline__
+#else
+#define HPT_SHARED inline
+#endif
+constexpr uint32_t kEdgeAny = 0xFFFFFFFFu;
+constexpr double kEdgeTolerance = 2e-6;
+HPT_SHARED uint32_t edge_cell(float r) { return (uint32_t)((r + 1.f) * 65536.f); }
+HPT_SHARED uint32_t edge_bucket(uint32_t cell1, uint32_t cell2, uint32_t buckets) {
+  const uint32_t h = cell1 * 0x9E3779B1u ^ cell2 * 0x85EBCA77u;
+  return (h ^ (h >> 15)) & (buckets - 1u);
+}
+HPT_SHARED uint32_t edge_tag(uint32_t cell1, uint32_t cell2) {
+  return (cell1 * 0xC2B2AE3Du + cell2 * 0x27D4EB2Fu) | 1u;
+}
+
 // Pointers of one device-resident scene (all device addresses).
 struct DevScene {
   const DevNode* nodes;
@@ -157,11 +177,12 @@ struct DevScene {
   const BvhNode* bvh;       // wide nodes, root first
   const BvhTri* btris;      // triangle records in node order
   int32_t num_bvh, num_btris;
-  // Directions of the triangle edges e2 that have a zero on axis a, sorted
-  // (edge_key in scene_pack.h; used by bvh_certain).
   // Emission, ambient colours and normals are finite: a ray of zero strength
   // adds zero wherever it hits.
   int32_t finite_shading;
+  // Directions of the triangle edges e2 whose largest component is on axis a
+  // (see edge_bucket; used by bvh_no_parallel_edge): the bits of four words a
+  // bucket, a power of two of buckets, or none.
   const float* edge_keys[3];
   int32_t num_edge_keys[3];
 };

@@ -1,20 +1,12 @@
 // Host packer: reference KD-tree + triangles -> traversal layout.
 #pragma once
 
-#include <cmath>
 #include <vector>
 
 #include "device_types.h"
 #include "host.h"
 
 namespace hpt {
-
-// The direction of the line along (b, c) as one number in (-1, 1]: c over
-// |b| + |c|, of the two opposite directions the one with b > 0.
-inline float edge_key(float b, float c) {
-  const float sum = std::fabs(b) + std::fabs(c);
-  return b == 0.f ? 1.f : (b > 0.f ? c : -c) / sum;
-}
 
 struct PackedScene {
   std::vector<DevNode> nodes;

@@ -142,3 +142,28 @@ def test_tree_with_other_lists(name, drop, add):
     e = emu.BvhEmu(mesh, nodes, leaf)
     _check(e.query(*S.aabb_random_rays(mesh, 20000, 3)))
     _check(e.query(*_in_plane(mesh, 5000, 4)))
+
+
+@pytest.mark.parametrize("name", ["soup", "degenerate", "room", "turned room", "spheres", "flat"])
+def test_directions_along_edges(name):
+    """Along a triangle's edge e2 the test divides zero by zero, and where
+    nothing else is hit the tree walk answers t = +inf."""
+    mesh, nodes, leaf = _turn(_scene("room")[0]) if name == "turned room" else _scene(name)
+    e = emu.BvhEmu(mesh, nodes, leaf)
+    rng = np.random.default_rng(8)
+    p = mesh.points[:, :3]
+    k = rng.integers(0, len(mesh.triangles), 20000)
+    along = (p[mesh.triangles[k, 2]] - p[mesh.triangles[k, 0]]).astype(np.float32)
+    o = rng.uniform(p.min(0), p.max(0), (20000, 3)).astype(np.float32)
+    for d in (along, along * np.float32(0.5), -along, _unit(along.astype(np.float64))):
+        _check(e.query(o, d))
+
+
+def test_axis_rays_that_miss_do_not_need_the_tree():
+    mesh, nodes, leaf = _scene("soup")
+    e = emu.BvhEmu(mesh, nodes, leaf)
+    rng = np.random.default_rng(3)
+    p = mesh.points[:, :3]
+    q = e.query(rng.uniform(p.min(0), p.max(0), (5000, 3)), np.eye(3)[rng.integers(0, 3, 5000)])
+    _check(q)
+    assert q["certain"][q["tri"] < 0].mean() > 0.99
