@@ -20,12 +20,16 @@
 // so around a hit point inside the bounds all leaves list it, except a leaf
 // beyond a split just outside the bounds. Where no leaf that lists the
 // triangle ends so (its flags), or the hit point is not at that bound, every
-// leaf within rounding (kCertainRound) of the hit point lists the triangle:
-// the tree walk, whose leaves cover the ray up to its best hit, is in one of
-// them at the hit, and the ray runs through the leaves around it by more than
-// rounding. [A leaf near the hit that does not list it was cut off by a split
-// X beyond the bound m, m < X <= m + 3 roundings; the leaf on the split's near
-// side that holds m lists the triangle and ends in (m, X]: flagged.]
+// leaf within `round` of the hit point lists the triangle. [A leaf near the hit
+// that does not list it was cut off by a split X beyond the bound m, m < X <= m
+// + 3 round; the leaf on the split's near side that holds m lists the triangle
+// and ends in (m, X]: flagged.]
+// The tree walk has to be in one of these leaves that the ray truly crosses
+// (the filter rejects others). It finds its leaf by the rounded point o + t d,
+// so within e = u (4 t |d| + |o + t d|) of a split, on that axis, it may be on
+// the wrong side, for as long as the ray takes to move away: a ray almost along
+// the split stays there. Of the stretch within `round` of the hit, that is at
+// most 2 e / |d| in t per axis; round is twice what the three need together.
 // What this leaves open, and two triangles at exactly the same t, bvh_settle
 // looks up in the tree.
 #pragma once
@@ -402,14 +406,21 @@ HPT_HD bool bvh_certain(const Sc& s, const Ray& r, uint32_t best, float best_t, 
                       rn_add(r.o.z, rn_mul(best_t, r.d.z))};
   if (axes && !(flags & kTriIrregular)) {
     const float a[3] = {A.x, A.y, A.z}, e1[3] = {E1.x, E1.y, E1.z}, e2[3] = {E2.x, E2.y, E2.z};
-    const float round = rn_mul(kCertainRound, s.scene_eps);
+    const float dmax = fmaxf(fabsf(r.d.x), fmaxf(fabsf(r.d.y), fabsf(r.d.z)));
+    const float along = rn_add(rn_mul(1.5e-6f, best_t),
+                               rn_mul(1.2e-7f, rn_add(fabsf(rn_div(p[0], r.d.x)),
+                                                      rn_add(fabsf(rn_div(p[1], r.d.y)),
+                                                             fabsf(rn_div(p[2], r.d.z))))));
     bool ok = true;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       const float v1 = rn_add(a[k], e1[k]), v2 = rn_add(a[k], e2[k]);
       const float lo = fminf(a[k], fminf(v1, v2)), hi = fmaxf(a[k], fmaxf(v1, v2));
-      ok = ok && p[k] > rn_add(lo, flags & (1u << (2 * k)) ? round : -2.f * round) &&
-           p[k] < rn_sub(hi, flags & (2u << (2 * k)) ? round : -2.f * round);
+      const float round = fma_rn(along, dmax, rn_mul(2.4e-7f, fmaxf(fabsf(lo), fabsf(hi))));
+      // The flags are of leaves that end within kCertainNear.
+      const uint32_t at = 3.f * round > rn_mul(kCertainNear, s.scene_eps) ? 3u : flags >> (2 * k);
+      ok = ok && p[k] > rn_add(lo, at & 1u ? round : -2.f * round) &&
+           p[k] < rn_sub(hi, at & 2u ? round : -2.f * round);
     }
     if (ok) return true;
   }
@@ -538,28 +549,33 @@ __host__ __device__ __noinline__ Lookup bvh_lookup(const Sc& s, const Ray& r, ui
       }
       if (at >= 0) {
         const float l[3] = {bl.x, bl.y, bl.z}, h[3] = {bh.x, bh.y, bh.z};
-        float f0 = -as_float(0x7f800000), f1 = as_float(0x7f800000);
+        // The stretch of the ray that is in the leaf by more than the walk's
+        // rounding (see part 2), and the one that is not outside by more.
+        float f0 = 0.f, f1 = as_float(0x7f800000), g0 = 0.f, g1 = as_float(0x7f800000);
         bool inside = true, face = false;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
           inside = inside && o[a] >= l[a] && o[a] <= h[a];
           if (inv[a] == 0.f) {
-            if (!(o[a] >= l[a] && o[a] <= h[a])) f1 = -as_float(0x7f800000);
+            if (!(o[a] >= l[a] && o[a] <= h[a])) f1 = g1 = -as_float(0x7f800000);
             face = face || o[a] == l[a] || o[a] == h[a];
             continue;
           }
           const float x0 = rn_mul(rn_sub(l[a], o[a]), inv[a]);
           const float x1 = rn_mul(rn_sub(h[a], o[a]), inv[a]);
-          f0 = fmaxf(f0, fminf(x0, x1));
-          f1 = fminf(f1, fmaxf(x0, x1));
+          const float off =
+              fma_rn(rn_mul(1.2e-7f, fmaxf(fabsf(l[a]), fabsf(h[a]))), fabsf(inv[a]), tol);
+          f0 = fmaxf(f0, rn_add(fminf(x0, x1), off));
+          f1 = fminf(f1, rn_sub(fmaxf(x0, x1), off));
+          g0 = fmaxf(g0, rn_sub(fminf(x0, x1), off));
+          g1 = fminf(g1, rn_add(fmaxf(x0, x1), off));
         }
-        const float length = rn_sub(f1, fmaxf(f0, 0.f));
         if (face && !inside) {
           // The filter's slab of the face the ray lies in is 0 / 0: rejected
           // (see tie_goes_right).
         } else if (face) {
           return kLookupOpen;  // the origin's own leaves: left to the walk
-        } else if (length > tol && f0 < rn_sub(stop, tol)) {
+        } else if (f0 < f1 && f0 < rn_sub(stop, tol)) {
           // The ray crosses the leaf and the walk comes to it.
           if (at < rank) {
             rank = at;
@@ -567,7 +583,7 @@ __host__ __device__ __noinline__ Lookup bvh_lookup(const Sc& s, const Ray& r, ui
           }
           reached = reached || f0 < best_t;
           if (!two && reached) return kLookupHit;
-        } else if (length >= -tol && !(two && f0 > rn_add(stop, tol))) {
+        } else if (g0 <= g1 && !(two && g0 > rn_add(stop, tol))) {
           if (ref_box_test(r, bl, bh)) {
             if (which == first) open_first = at < open_first ? at : open_first;
             else open_tie = at < open_tie ? at : open_tie;

@@ -101,16 +101,13 @@ struct BvhTri {
 static_assert(sizeof(BvhTri) == 48, "48-byte triangle record");
 constexpr uint32_t kTriIrregular = 64u, kTriUnordered = 128u;
 
-// Distances of the certificate in units of DevScene::scene_eps (2e-5 of the
-// scene's size): the tree walk's rounding, generously (4e-6 of the size), and
-// the leaf faces that count as just outside a triangle's bounds.
-constexpr float kCertainRound = 0.2f;
-constexpr float kCertainNear = 4 * kCertainRound;
+// Leaf faces that count as just outside a triangle's bounds, in units of
+// DevScene::scene_eps (2e-5 of the scene's size).
+constexpr float kCertainNear = 0.8f;
 
 // Origins beyond 4 times the scene's size (in units of scene_eps; a coordinate)
-// are walked through the tree: 16 roundings of such a coordinate are
-// kCertainRound, and the slabs of the wide boxes are as thick as a distance of
-// kMaxDistance sizes asks for.
+// are walked through the tree: the slabs of the wide boxes are as thick as a
+// distance of kMaxDistance sizes asks for.
 constexpr float kMaxOrigin = 4 / 2e-5f;
 constexpr double kMaxDistance = 5 * 1.7320508;
 

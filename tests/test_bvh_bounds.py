@@ -167,3 +167,25 @@ def test_axis_rays_that_miss_do_not_need_the_tree():
     q = e.query(rng.uniform(p.min(0), p.max(0), (5000, 3)), np.eye(3)[rng.integers(0, 3, 5000)])
     _check(q)
     assert q["certain"][q["tri"] < 0].mean() > 0.99
+
+
+@pytest.mark.parametrize("name", ["far", "soup", "spheres", "terrain", "room", "flat"])
+def test_rays_almost_along_a_split_plane(name):
+    """The tree walk finds its leaves by rounded points: within rounding of a
+    split plane it may go along its other side, where the filter rejects."""
+    mesh, nodes, leaf = _scene(name)
+    rng = np.random.default_rng(0)
+    n, p = 60000, mesh.points[:, :3]
+    faces = np.concatenate([nodes["box_start"].reshape(len(nodes), -1)[:, :3],
+                            nodes["box_end"].reshape(len(nodes), -1)[:, :3]]).astype(np.float32)
+    axis = rng.integers(0, 3, n)
+    x, ulps = faces[rng.integers(0, len(faces), n), axis], rng.integers(-3, 4, n)
+    for k in range(3):
+        to = np.where(ulps > k, np.inf, np.where(ulps < -k, -np.inf, x)).astype(np.float32)
+        x = np.nextafter(x, to)
+    grow = 0.2 * (p.max(0) - p.min(0))
+    o = rng.uniform(p.min(0) - grow, p.max(0) + grow, (n, 3)).astype(np.float32)
+    o[np.arange(n), axis] = x
+    d = rng.normal(size=(n, 3))
+    d[np.arange(n), axis] *= 10.0 ** rng.uniform(-8, -1, n)
+    _check(emu.BvhEmu(mesh, nodes, leaf).query(o, _unit(d)))
