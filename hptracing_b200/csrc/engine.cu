@@ -1742,9 +1742,10 @@ hpt_status Engine::run(const std::vector<JobSpec>& jobs, hpt_render_stats* stats
   // iterations are queued ahead; the done flag of batch k is checked while
   // batch k+1 runs (extra iterations after completion are empty launches).
   // When the queue holds every path of the run, all start in the first
-  // iteration and each has ended after as many as its depth: those are
-  // launched, and no others.
-  const int kBatch = 4;
+  // iteration and each has ended after as many as its depth: no more than
+  // those are launched, and beyond kAhead, where most paths have long ended
+  // (depths go up to 255), batches as long as the flag is not set.
+  const int kBatch = 4, kAhead = 16;
   const bool prof = tuning.profile != 0;
   const bool at_once = paths <= capacity_ && (tuning.use_graph == 0 || prof);
   int max_depth = 1;
@@ -1796,8 +1797,25 @@ hpt_status Engine::run(const std::vector<JobSpec>& jobs, hpt_render_stats* stats
   bool drained = false;
   int slot = 0;
   bool pending = false;
-  for (int k = 0; at_once && k < max_depth; ++k)
-    launch_iteration(shared_dev, prof ? &pev[3 * k] : nullptr, paths, k == max_depth - 1);
+  auto ask = [&](int k) {
+    HPT_SOFT(cudaMemcpyAsync(&done_host[k], &ctrl_->done, sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
+    HPT_SOFT(cudaEventRecord(ev_done[k], stream));
+  };
+  int launched = 0;  // at_once
+  while (at_once && launched < max_depth && !drained) {
+    const int upto = std::min(max_depth, launched == 0 ? kAhead : launched + kBatch);
+    for (; launched < upto; ++launched)
+      launch_iteration(shared_dev, prof ? &pev[3 * launched] : nullptr, paths,
+                       launched == max_depth - 1);
+    if (max_depth <= kAhead) break;
+    ask(slot);
+    if (pending) {
+      HPT_SOFT(cudaEventSynchronize(ev_done[slot ^ 1]));
+      drained = done_host[slot ^ 1] != 0;
+    }
+    pending = true;
+    slot ^= 1;
+  }
   while (!at_once) {
     if (use_graph) {
       HPT_CUDA(cudaGraphLaunch(graph_exec_, stream));
@@ -1806,8 +1824,7 @@ hpt_status Engine::run(const std::vector<JobSpec>& jobs, hpt_render_stats* stats
         launch_iteration(shared_dev, prof ? &pev[(slot * kBatch + k) * 3] : nullptr, capacity_,
                          false);
     }
-    HPT_SOFT(cudaMemcpyAsync(&done_host[slot], &ctrl_->done, sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
-    HPT_SOFT(cudaEventRecord(ev_done[slot], stream));
+    ask(slot);
     if (pending) {
       HPT_SOFT(cudaEventSynchronize(ev_done[slot ^ 1]));
       if (prof) harvest((slot ^ 1) * kBatch, kBatch);
@@ -1835,7 +1852,7 @@ hpt_status Engine::run(const std::vector<JobSpec>& jobs, hpt_render_stats* stats
                            stream));
   for (auto& b : bufs) free_job(b);
   cudaError_t e = cudaStreamSynchronize(stream);
-  if (prof) harvest(at_once ? 0 : slot * kBatch, at_once ? max_depth : kBatch);
+  if (prof) harvest(at_once ? 0 : slot * kBatch, at_once ? launched : kBatch);
   if (e != cudaSuccess) return cuda_fail(e, "render");
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "render launch");
