@@ -19,17 +19,20 @@
 // triangle into every leaf its bounds touch (src/hp/scene/kdtree.cpp:145-154),
 // so around a hit point inside the bounds all leaves list it, except a leaf
 // beyond a split just outside the bounds. Where no leaf that lists the
-// triangle ends so (its flags), or the hit point is not at that bound, every
-// leaf within `round` of the hit point lists the triangle. [A leaf near the hit
-// that does not list it was cut off by a split X beyond the bound m, m < X <= m
-// + 3 round; the leaf on the split's near side that holds m lists the triangle
-// and ends in (m, X]: flagged.]
+// triangle ends within 3 `round` of a bound (its flags say how far the first
+// one is), or the hit point is not at that bound, every leaf within `round` of
+// the hit point lists the triangle. [A leaf near the hit that does not list it
+// was cut off by a split X beyond the bound m, m < X <= m + 3 round; the leaf
+// on the split's near side that holds m lists the triangle and ends in (m, X].]
 // The tree walk has to be in one of these leaves that the ray truly crosses
 // (the filter rejects others). It finds its leaf by the rounded point o + t d,
 // so within e = u (4 t |d| + |o + t d|) of a split, on that axis, it may be on
 // the wrong side, for as long as the ray takes to move away: a ray almost along
 // the split stays there. Of the stretch within `round` of the hit, that is at
 // most 2 e / |d| in t per axis; round is twice what the three need together.
+// Besides, the leaf where the walk starts holds the origin, unrounded, and
+// passes the filter by that: it is enough that it lists the triangle (a light
+// that samples a point of its own plane).
 // What this leaves open, and two triangles at exactly the same t, bvh_settle
 // looks up in the tree.
 #pragma once
@@ -43,6 +46,14 @@ HPT_HD float fma_rn(float a, float b, float c) {
   return __fmaf_rn(a, b, c);
 #else
   return std::fmaf(a, b, c);
+#endif
+}
+// a / b within 2 ulp.
+HPT_HD float near_div(float a, float b) {
+#ifdef __CUDA_ARCH__
+  return __fdividef(a, b);
+#else
+  return a / b;
 #endif
 }
 HPT_HD uint32_t popc(uint32_t x) {
@@ -384,11 +395,25 @@ HPT_HD bool bvh_no_parallel_edge(const Sc& s, const f3& d) {
   if (n == 0) return true;
   const float* keys = a == 0 ? s.edge_keys[0] : (a == 1 ? s.edge_keys[1] : s.edge_keys[2]);
   const float da = a == 0 ? d.x : (a == 1 ? d.y : d.z);
-  const float r1 = rn_div(a == 0 ? d.y : (a == 1 ? d.z : d.x), da);
-  const float r2 = rn_div(a == 0 ? d.z : (a == 1 ? d.x : d.y), da);
+  const float r1 = near_div(a == 0 ? d.y : (a == 1 ? d.z : d.x), da);
+  const float r2 = near_div(a == 0 ? d.z : (a == 1 ? d.x : d.y), da);
   const uint32_t c1 = edge_cell(r1), c2 = edge_cell(r2), tag = edge_tag(c1, c2);
-  const uint4 k = ldg(reinterpret_cast<const uint4*>(keys) + edge_bucket(c1, c2, n >> 2));
-  return k.x != kEdgeAny && k.x != tag && k.y != tag && k.z != tag && k.w != tag;
+  // Entries of a bucket are filled from the first; the table is not full.
+  const uint32_t buckets = n >> 2;
+  for (uint32_t b = edge_bucket(c1, c2, buckets), left = buckets; left != 0; --left) {
+    const uint4 k = ldg(reinterpret_cast<const uint4*>(keys) + b);
+    if (k.x == tag || k.y == tag || k.z == tag || k.w == tag) return false;
+    if (k.w == 0) break;
+    b = b + 1 < buckets ? b + 1 : 0;
+  }
+  return true;
+}
+
+// At least this far from a triangle's bound (face 2a: lower on axis a, 2a + 1:
+// upper) ends the first leaf that lists it and ends beyond (BvhTri::flags).
+HPT_HD float leaf_gap(uint32_t flags, int face, float scene_eps) {
+  const uint32_t c = (flags >> (8 + 4 * face)) & 15u;
+  return c == 0 ? 0.f : rn_mul(rn_mul(kGapUnit, scene_eps), as_float_u((126u + c) << 23));
 }
 
 // True when the tree walk's answer for ray r is (best, best_t), the result
@@ -402,29 +427,37 @@ HPT_HD bool bvh_certain(const Sc& s, const Ray& r, uint32_t best, float best_t, 
   const float4* rec = reinterpret_cast<const float4*>(s.btris + best);
   const float4 A = ldg(rec), E1 = ldg(rec + 1), E2 = ldg(rec + 2);
   const uint32_t flags = (uint32_t)as_int(E2.w);
+  if (flags & kTriIrregular) return false;
+  const float o[3] = {r.o.x, r.o.y, r.o.z}, d[3] = {r.d.x, r.d.y, r.d.z};
   const float p[3] = {rn_add(r.o.x, rn_mul(best_t, r.d.x)), rn_add(r.o.y, rn_mul(best_t, r.d.y)),
                       rn_add(r.o.z, rn_mul(best_t, r.d.z))};
-  if (axes && !(flags & kTriIrregular)) {
-    const float a[3] = {A.x, A.y, A.z}, e1[3] = {E1.x, E1.y, E1.z}, e2[3] = {E2.x, E2.y, E2.z};
-    const float dmax = fmaxf(fabsf(r.d.x), fmaxf(fabsf(r.d.y), fabsf(r.d.z)));
-    const float along = rn_add(rn_mul(1.5e-6f, best_t),
-                               rn_mul(1.2e-7f, rn_add(fabsf(rn_div(p[0], r.d.x)),
-                                                      rn_add(fabsf(rn_div(p[1], r.d.y)),
-                                                             fabsf(rn_div(p[2], r.d.z))))));
-    bool ok = true;
+  const float a[3] = {A.x, A.y, A.z}, e1[3] = {E1.x, E1.y, E1.z}, e2[3] = {E2.x, E2.y, E2.z};
+  const float along = fma_rn(1.5e-6f, best_t,
+                             rn_mul(1.2e-7f, rn_add(fabsf(near_div(p[0], d[0])),
+                                                    rn_add(fabsf(near_div(p[1], d[1])),
+                                                           fabsf(near_div(p[2], d[2]))))));
+  float lo[3], hi[3], below[3], above[3], exact[3];
+  bool ok = axes;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const float v1 = rn_add(a[k], e1[k]), v2 = rn_add(a[k], e2[k]);
-      const float lo = fminf(a[k], fminf(v1, v2)), hi = fmaxf(a[k], fmaxf(v1, v2));
-      const float round = fma_rn(along, dmax, rn_mul(2.4e-7f, fmaxf(fabsf(lo), fabsf(hi))));
-      // The flags are of leaves that end within kCertainNear.
-      const uint32_t at = 3.f * round > rn_mul(kCertainNear, s.scene_eps) ? 3u : flags >> (2 * k);
-      ok = ok && p[k] > rn_add(lo, at & 1u ? round : -2.f * round) &&
-           p[k] < rn_sub(hi, at & 2u ? round : -2.f * round);
-    }
-    if (ok) return true;
+  for (int k = 0; k < 3; ++k) {
+    const float v1 = rn_add(a[k], e1[k]), v2 = rn_add(a[k], e2[k]);
+    lo[k] = min3(a[k], v1, v2);
+    hi[k] = max3(a[k], v1, v2);
+    exact[k] = rn_mul(2.4e-7f, fmaxf(fabsf(lo[k]), fabsf(hi[k])));
+    below[k] = leaf_gap(flags, 2 * k, s.scene_eps);
+    above[k] = leaf_gap(flags, 2 * k + 1, s.scene_eps);
+    const float round = fma_rn(along, fabsf(d[k]), exact[k]);
+    ok = ok && p[k] > rn_add(lo[k], 3.f * round <= below[k] ? -2.f * round : round) &&
+         p[k] < rn_sub(hi[k], 3.f * round <= above[k] ? -2.f * round : round);
   }
-  return false;
+  if (ok) return true;
+  ok = true;
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    ok = ok && o[k] >= s.root_lo[k] && o[k] <= s.root_hi[k] &&
+         o[k] > rn_add(rn_sub(lo[k], below[k]), exact[k]) &&
+         o[k] < rn_sub(rn_add(hi[k], above[k]), exact[k]);
+  return ok;
 }
 
 // Looks up in the tree a hit that bvh_certain leaves open: goes through the
@@ -454,6 +487,11 @@ __host__ __device__ __noinline__ Lookup bvh_lookup(const Sc& s, const Ray& r, ui
   const float tol = fma_rn(best_t, 1e-6f, rn_mul(0.1f, slack));
   // The walk visits the leaves that begin before this.
   const float stop = fma_rn(best_t, 1.0001f, slack);
+  // A ray that stays within rounding of its place on some axis all the way up
+  // to the hit: no leaf holds it by more.
+  if (!two)
+    for (int a = 0; a < 3; ++a)
+      if (rn_mul(2.4e-7f, rn_mul(fabsf(o[a]), fabsf(inv[a]))) > best_t) return kLookupOpen;
   // The bounds of the triangle, or of both, and the tree node that holds all
   // their leaves.
   float lo[3], hi[3];

@@ -66,6 +66,17 @@ namespace hpt {
 
 namespace {
 
+// f(i) for i below count, on up to `threads` threads.
+template <class F>
+void for_all(int threads, size_t count, F&& f) {
+  const size_t step = std::max<size_t>(1, std::min<size_t>(256, count / (4 * (size_t)threads)));
+  std::atomic<size_t> cursor{0};
+  run_threads((int)std::min<size_t>(threads, count), [&] {
+    for (size_t i = cursor.fetch_add(step); i < count; i = cursor.fetch_add(step))
+      for (size_t k = i; k < std::min(count, i + step); ++k) f(k);
+  });
+}
+
 struct Box {
   float lo[3], hi[3];
   void reset() {
@@ -125,6 +136,8 @@ constexpr float kNodeCost = 0.5f;
 constexpr int kMedianDepth = 40;
 constexpr float kSplitBlend = 0.6f;
 constexpr double kUlp = 1.0 / (1 << 24);
+// Leaf entries and triangles per thread (about 2 ms of work).
+constexpr size_t kWorkPerThread = 32768;
 // Subtrees above this size take their wide box for all rays.
 constexpr int32_t kMaxCone = 32768;
 
@@ -308,7 +321,7 @@ struct Collapser {
   const std::vector<Node2>& in;
   const std::vector<Prim>& prims;
   const PackedScene& scene;
-  const std::vector<uint8_t>& flags;
+  const std::vector<std::atomic<uint32_t>>& flags;
   const std::vector<TriBoxes>& boxes;
   PackedBvh& out;
   struct Kids {
@@ -338,11 +351,7 @@ struct Collapser {
       todo.pop_back();
       emit(it, todo);
     }
-    std::atomic<size_t> cursor{0};
-    run_threads(threads, [&] {
-      for (size_t k = cursor.fetch_add(64); k < out.nodes.size(); k = cursor.fetch_add(64))
-        for (size_t i = k; i < std::min(out.nodes.size(), k + 64); ++i) fill(i);
-    });
+    for_all(threads, out.nodes.size(), [&](size_t i) { fill(i); });
   }
 
   bool leaf(int32_t n) const { return in[n].left < 0; }
@@ -531,7 +540,7 @@ struct Collapser {
       r.e2[a] = t.e2[a];
     }
     r.tri_id = id;
-    r.flags = flags[(size_t)id];
+    r.flags = flags[(size_t)id].load(std::memory_order_relaxed);
     return r;
   }
 
@@ -586,8 +595,9 @@ struct Collapser {
 namespace {
 
 // Leaves whose closed box the closed box b touches.
-int64_t touched_leaves(const PackedScene& scene, const Box& b, std::vector<uint32_t>& stack) {
+int64_t touched_leaves(const PackedScene& scene, const Box& b) {
   int64_t count = 0;
+  static thread_local std::vector<uint32_t> stack;
   stack.assign(1, 0u);
   while (!stack.empty()) {
     const DevNode& d = scene.nodes[stack.back()];
@@ -603,8 +613,7 @@ int64_t touched_leaves(const PackedScene& scene, const Box& b, std::vector<uint3
   return count;
 }
 
-// DevScene::edge_keys of axis a, of a size at which few buckets overflow (a
-// regular mesh has far fewer directions than edges).
+// DevScene::edge_keys of axis a, at most half full.
 void edge_table(const std::vector<DevTri>& tris, int a, std::vector<float>& keys) {
   const int b = (a + 1) % 3, c = (a + 2) % 3;
   auto largest = [&](const DevTri& t) {
@@ -618,31 +627,50 @@ void edge_table(const std::vector<DevTri>& tris, int a, std::vector<float>& keys
   for (const DevTri& t : tris) count += largest(t);
   keys.clear();
   if (count == 0) return;
+  // (A regular mesh has far fewer directions than edges: grown as it fills.)
   std::vector<uint32_t> table;
   uint32_t buckets = 1;
-  while (buckets < count / 2 && buckets < (1u << 27)) buckets *= 2;
-  for (;; buckets *= 2) {
-    size_t full = 0;
+  while (buckets < 1024 && buckets < count) buckets *= 2;
+  for (;; buckets *= 4) {
+    size_t used = 0;
     table.assign(4 * (size_t)buckets, 0u);
     for (const DevTri& t : tris) {
       if (!largest(t)) continue;
       const double r1 = (double)t.e2[b] / t.e2[a], r2 = (double)t.e2[c] / t.e2[a];
       for (uint32_t i = cell(r1 - kEdgeTolerance); i <= cell(r1 + kEdgeTolerance); ++i)
         for (uint32_t j = cell(r2 - kEdgeTolerance); j <= cell(r2 + kEdgeTolerance); ++j) {
-          uint32_t* slot = table.data() + 4 * (size_t)edge_bucket(i, j, buckets);
           const uint32_t tag = edge_tag(i, j);
-          int k = 0;
-          while (k < 4 && slot[k] != 0 && slot[k] != tag && slot[k] != kEdgeAny) ++k;
-          if (k < 4 && slot[k] == 0) slot[k] = tag;
-          if (k < 4) continue;
-          slot[0] = kEdgeAny;
-          ++full;
+          size_t k = 4 * (size_t)edge_bucket(i, j, buckets);
+          while (table[k] != 0 && table[k] != tag) k = k + 1 < table.size() ? k + 1 : 0;
+          used += table[k] == 0;
+          table[k] = tag;
         }
+      if (used > table.size() / 2) break;
     }
-    if (full <= buckets / 1024 || buckets > 4 * count) break;
+    if (used <= table.size() / 2) break;
   }
   keys.resize(table.size());
   memcpy(keys.data(), table.data(), table.size() * sizeof(uint32_t));
+}
+
+// The codes of BvhTri::flags (bits 8-31) with face's at most that of a leaf that
+// ends `gap` beyond it (gap <= 0: it does not).
+uint32_t with_gap(uint32_t codes, int face, float gap, float unit) {
+  if (!(gap > 0.f)) return codes;
+  const int at = 8 + 4 * face;
+  uint32_t c = 0;
+  for (float x = unit; c < 15 && x <= gap; x *= 2) ++c;
+  const uint32_t have = (codes >> at) & 15u;
+  return c < have ? (codes & ~(15u << at)) | (c << at) : codes;
+}
+// Sets f's bits and takes the smaller code of each face.
+void merge_flags(std::atomic<uint32_t>& flags, uint32_t f, uint32_t codes) {
+  for (uint32_t have = flags.load(std::memory_order_relaxed);;) {
+    uint32_t want = (have & 255u) | f;
+    for (int at = 8; at < 32; at += 4)
+      want |= std::min((have >> at) & 15u, (codes >> at) & 15u) << at;
+    if (want == have || flags.compare_exchange_weak(have, want, std::memory_order_relaxed)) return;
+  }
 }
 
 // Bounds that several threads grow.
@@ -736,22 +764,27 @@ bool clip_to_slab(const DevTri& t, const Box& tb, const Plane& p, Box& b) {
 void build_bvh(const float* points, const int32_t* triangles, const PackedScene& scene,
                float scene_eps, int num_threads, PackedBvh& out) {
   const size_t n = scene.tris.size();
-  // A small scene builds in less than it takes to start a thread.
-  const int threads = n <= 8192 ? 1
-                      : num_threads > 0
-                          ? num_threads
-                          : (int)std::max(1u, std::thread::hardware_concurrency());
-  // Per triangle: its bounds, the union of the leaves that list it, how many
-  // do, its flags and its boxes.
-  std::vector<Box> bounds(n), leaves(n);
-  std::vector<int32_t> listed(n, 0);
-  std::vector<uint8_t> flags(n, 0);
+  // The work goes with the leaves' entries; a small scene builds in less than
+  // it takes to start a thread.
+  const size_t cores =
+      num_threads > 0 ? (size_t)num_threads : std::max(1u, std::thread::hardware_concurrency());
+  const int threads =
+      (int)std::max<size_t>(1, std::min(cores, (n + scene.refs.size()) / kWorkPerThread));
+  // Per triangle: its bounds and plane, the union of the leaves that list it,
+  // how many do, its flags and its wide box.
+  std::vector<Box> bounds(n);
   std::vector<Plane> planes(n);
-  std::vector<SharedBox> wide(n);
+  std::vector<SharedBox> wide(n), leaves(n);
+  std::vector<std::atomic<int32_t>> listed(n);
+  std::vector<std::atomic<uint32_t>> flags(n);
   // (scene_eps is 2e-5 of the scene's size.)
   const double scene_size = scene_eps / 2e-5;
-  for (size_t i = 0; i < n; ++i) {
-    leaves[i].reset();
+  for_all(threads, n, [&](size_t i) {
+    Box none;
+    none.reset();
+    leaves[i].set(none);
+    listed[i].store(0, std::memory_order_relaxed);
+    flags[i].store(~255u, std::memory_order_relaxed);
     bounds[i].reset();
     for (int k = 0; k < 3; ++k) {
       const float* v = points + 4 * (size_t)triangles[4 * i + k];
@@ -762,32 +795,10 @@ void build_bvh(const float* points, const int32_t* triangles, const PackedScene&
     }
     planes[i] = plane_of(scene.tris[i], scene_size);
     wide[i].set(bounds[i]);
-  }
-  {
-    std::atomic<size_t> cursor{0};
-    run_threads(threads, [&] {
-      const size_t count = scene.leaves.size(), step = 256;
-      for (size_t i = cursor.fetch_add(step); i < count; i = cursor.fetch_add(step))
-        for (size_t l = i; l < std::min(count, i + step); ++l) {
-          const DevLeaf& L = scene.leaves[l];
-          Box b;
-          for (int a = 0; a < 3; ++a) {
-            b.lo[a] = L.lo[a];
-            b.hi[a] = L.hi[a];
-          }
-          for (int32_t k = 0; k < L.tri_count; ++k) {
-            const size_t id = (size_t)scene.refs[(size_t)L.tri_begin + k];
-            Box part = b;
-            if (planes[id].wide && !wide[id].get().holds(b) &&
-                clip_to_slab(scene.tris[id], bounds[id], planes[id], part))
-              wide[id].add(part);
-          }
-        }
-    });
-  }
-  const float near = kCertainNear * scene_eps;
-  std::vector<int32_t> unique;
-  for (const DevLeaf& L : scene.leaves) {
+  });
+  const float unit = kGapUnit * scene_eps;
+  for_all(threads, scene.leaves.size(), [&](size_t l) {
+    const DevLeaf& L = scene.leaves[l];
     Box b;
     for (int a = 0; a < 3; ++a) {
       b.lo[a] = L.lo[a];
@@ -797,6 +808,7 @@ void build_bvh(const float* points, const int32_t* triangles, const PackedScene&
     int32_t count = L.tri_count;
     bool ascending = true;
     for (int32_t k = 1; k < count; ++k) ascending = ascending && ids[k - 1] < ids[k];
+    std::vector<int32_t> unique;
     if (!ascending) {  // a triangle may be there twice: it counts once
       unique.assign(ids, ids + count);
       std::sort(unique.begin(), unique.end());
@@ -807,39 +819,31 @@ void build_bvh(const float* points, const int32_t* triangles, const PackedScene&
     for (int32_t k = 0; k < count; ++k) {
       const size_t id = (size_t)ids[k];
       leaves[id].add(b);
-      ++listed[id];
+      listed[id].fetch_add(1, std::memory_order_relaxed);
       const Box& t = bounds[id];
-      uint32_t f = ascending ? 0u : kTriUnordered;
+      uint32_t f = ascending ? 0u : kTriUnordered, codes = ~0u;
       for (int a = 0; a < 3; ++a) {
-        const float below = t.lo[a] - b.lo[a], above = b.hi[a] - t.hi[a];
-        if (below > 0.f && below < near) f |= 1u << (2 * a);
-        if (above > 0.f && above < near) f |= 2u << (2 * a);
+        codes = with_gap(codes, 2 * a, t.lo[a] - b.lo[a], unit);
+        codes = with_gap(codes, 2 * a + 1, b.hi[a] - t.hi[a], unit);
         if (b.lo[a] > t.hi[a] || b.hi[a] < t.lo[a]) f |= kTriIrregular;
       }
-      flags[id] |= (uint8_t)f;
+      merge_flags(flags[id], f, codes);
+      Box part = b;
+      if (planes[id].wide && !wide[id].get().holds(b) &&
+          clip_to_slab(scene.tris[id], t, planes[id], part))
+        wide[id].add(part);
     }
-  }
-  {
-    std::atomic<size_t> cursor{0};
-    run_threads(threads, [&] {
-      std::vector<uint32_t> stack;
-      for (size_t i = cursor.fetch_add(1024); i < n; i = cursor.fetch_add(1024))
-        for (size_t k = i; k < std::min(n, i + 1024); ++k)
-          if (listed[k] != touched_leaves(scene, bounds[k], stack))
-            flags[k] |= (uint8_t)kTriIrregular;
-    });
-  }
-  {
-    std::atomic<int> axis{0};
-    run_threads(std::min(threads, 3), [&] {
-      for (int a = axis++; a < 3; a = axis++) edge_table(scene.tris, a, out.edge_keys[a]);
-    });
-  }
+  });
+  for_all(threads, n, [&](size_t i) {
+    if (listed[i].load(std::memory_order_relaxed) != touched_leaves(scene, bounds[i]))
+      flags[i].fetch_or(kTriIrregular, std::memory_order_relaxed);
+  });
+  for_all(threads, 3, [&](size_t a) { edge_table(scene.tris, (int)a, out.edge_keys[a]); });
   std::vector<TriBoxes> boxes(n);
   std::vector<Prim> prims;
   prims.reserve(n);
   for (size_t i = 0; i < n; ++i) {
-    if (!listed[i]) continue;  // no leaf lists it: never tested
+    if (listed[i].load() == 0) continue;  // no leaf lists it: never tested
     TriBoxes& t = boxes[i];
     t.own = bounds[i];
     t.wide = wide[i].get();
@@ -883,8 +887,9 @@ void build_bvh(const float* points, const int32_t* triangles, const PackedScene&
   }
   // Where the certificate's descent starts: the lowest tree node that holds
   // every leaf listing the triangle.
-  for (BvhTri& t : out.tris) {
-    const Box& b = leaves[(size_t)t.tri_id];
+  for_all(threads, out.tris.size(), [&](size_t i) {
+    BvhTri& t = out.tris[i];
+    const Box b = leaves[(size_t)t.tri_id].get();
     uint32_t node = 0;
     while (true) {
       const DevNode& d = scene.nodes[node];
@@ -895,7 +900,7 @@ void build_bvh(const float* points, const int32_t* triangles, const PackedScene&
       else break;
     }
     t.start_node = (int32_t)node;
-  }
+  });
 }
 
 }  // namespace hpt

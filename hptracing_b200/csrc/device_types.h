@@ -85,11 +85,11 @@ static_assert(sizeof(BvhNode) == 160, "160-byte wide node");
 
 // Triangle record in node order: the DevTri values, and for the certificate
 // (bvh_certain in bvh.cuh) the lowest tree node that holds every leaf listing
-// the triangle, and flags. Bit 2a / 2a + 1 of the flags: one of those leaves
-// ends just outside the triangle's lower / upper bound on axis a, by less
-// than kCertainNear. kTriIrregular: the tree does not list the triangle in
-// exactly the leaves its bounds touch. kTriUnordered: in one of them the
-// entries are not in ascending order.
+// the triangle, and flags. kTriIrregular: the tree does not list the triangle
+// in exactly the leaves its bounds touch. kTriUnordered: in one of them the
+// entries are not in ascending order. Bits 8 + 4 f to 11 + 4 f (f = 2a / 2a + 1:
+// the lower / upper bound on axis a): c > 0 when no leaf that lists it ends
+// beyond that bound by less than kGapUnit * scene_eps * 2^(c - 1).
 struct BvhTri {
   float a[3];
   int32_t tri_id;
@@ -101,9 +101,9 @@ struct BvhTri {
 static_assert(sizeof(BvhTri) == 48, "48-byte triangle record");
 constexpr uint32_t kTriIrregular = 64u, kTriUnordered = 128u;
 
-// Leaf faces that count as just outside a triangle's bounds, in units of
-// DevScene::scene_eps (2e-5 of the scene's size).
-constexpr float kCertainNear = 0.8f;
+// The distances in BvhTri::flags, in units of DevScene::scene_eps (2e-5 of the
+// scene's size).
+constexpr float kGapUnit = 0.8f;
 
 // Origins beyond 4 times the scene's size (in units of scene_eps; a coordinate)
 // are walked through the tree: the slabs of the wide boxes are as thick as a
@@ -132,17 +132,16 @@ struct DevTexInfo {
 };
 
 // Hash of edge directions. The other two components over the largest one, r1
-// and r2 in [-1, 1], give a cell of 2^-16 by 2^-16; a bucket of four words holds
-// the tags of the cells that edges are in, within kEdgeTolerance (0: no entry;
-// first one kEdgeAny: more than four).
+// and r2 in [-1, 1], give a cell of 2^-18 by 2^-18; a bucket of four words holds
+// the tags of the cells that edges are in, within kEdgeTolerance (0: none), and
+// where it is full the next one goes on.
 #ifdef __CUDACC__
 #define HPT_SHARED __host__ __device__ __forceinline__
 #else
 #define HPT_SHARED inline
 #endif
-constexpr uint32_t kEdgeAny = 0xFFFFFFFFu;
-constexpr double kEdgeTolerance = 2e-6;
-HPT_SHARED uint32_t edge_cell(float r) { return (uint32_t)((r + 1.f) * 65536.f); }
+constexpr double kEdgeTolerance = 8e-7;
+HPT_SHARED uint32_t edge_cell(float r) { return (uint32_t)((r + 1.f) * 262144.f); }
 HPT_SHARED uint32_t edge_bucket(uint32_t cell1, uint32_t cell2, uint32_t buckets) {
   const uint32_t h = cell1 * 0x9E3779B1u ^ cell2 * 0x85EBCA77u;
   return (h ^ (h >> 15)) & (buckets - 1u);
