@@ -86,8 +86,10 @@ class StageCall {
   // Allocates what was reserved.
   hpt_status begin() {
     HPT_CUDA(cudaSetDevice(h_.scene.device));
-    if (!h_.stage_stream) {
+    if (!h_.stage_stream)
       HPT_CUDA(cudaStreamCreateWithFlags(&h_.stage_stream, cudaStreamNonBlocking));
+    // Each is made if it is missing: one may have failed in an earlier call.
+    if (!h_.stage_pool) {
       cudaMemPoolProps props;
       memset(&props, 0, sizeof props);
       props.allocType = cudaMemAllocationTypePinned;
