@@ -488,6 +488,11 @@ hpt_status upload_scene(const hpt_scene_desc& d, SceneDev& out) {
         ds.finite_shading = 0;
   for (int64_t k = 0; k < 4 * (int64_t)d.num_normals; ++k)
     if ((k & 3) != 3 && !std::isfinite(d.normals[k])) ds.finite_shading = 0;
+  // (A triangle without area has no normal: 0 times NaN.)
+  for (const DevTri& t : pk.tris) {
+    const f3 n = cross(mk(t.e1[0], t.e1[1], t.e1[2]), mk(t.e2[0], t.e2[1], t.e2[2]));
+    if (!(length(n) > 1e-30f)) ds.finite_shading = 0;
+  }
   ds.num_bvh = (int32_t)bvh.nodes.size();
   ds.num_btris = (int32_t)bvh.tris.size();
   ds.nodes = nodes;

@@ -408,15 +408,19 @@ __device__ __forceinline__ int push_open(const EngineParams& P, OpenList* W, int
   return n;
 }
 
-// True when the ray's strength is zero and its hit, whichever it is, adds zero
-// to its path and ends it (a light sampled along the surface it lies in: the
-// ray runs in a split plane, where a certain hit would take a look at the
-// tree). `s`: its scene.
+// True when the ray's strength is zero and its answer, whichever it is, adds
+// zero to its path and ends it (a light sampled along the surface it lies in:
+// the ray runs in a split plane, where a certain hit would take a look at the
+// tree). The answer may be a miss: 0 times an infinite background is not zero.
+// `s`: its scene.
 __device__ __forceinline__ bool no_strength(const EngineParams& P, const DevScene& s, const Ray& r,
                                             int item) {
   const float4 w = P.Q_s[P.ctrl->parity ^ 1][item];
-  return w.x == 0.f && w.y == 0.f && w.z == 0.f && s.finite_shading &&
-         bvh_no_parallel_edge(s, r.d);
+  if (w.x != 0.f || w.y != 0.f || w.z != 0.f || !s.finite_shading) return false;
+  const int slot = __float_as_int(w.w);
+  HPT_DCHECK(&P.ctrl->err, slot >= 0 && slot < P.num_slots, 222, slot, return false);
+  const float* bg = P.jobs[slot].bg;
+  return isfinite(bg[0]) && isfinite(bg[1]) && isfinite(bg[2]) && bvh_no_parallel_edge(s, r.d);
 }
 
 // Writes out one ray of the queue per lane (`have`): a hit goes to the hit
