@@ -187,8 +187,9 @@ HPT_HD uint32_t direction_bytes(const f3& d, float scale127) {
 }
 
 // Starts a walk. Returns false when the ray is to be walked through the tree
-// instead (non-finite rays, directions of extreme length, origins so far away
-// that the roundings outgrow what the boxes and the certificate allow for).
+// instead (non-finite rays; origins so far away that the roundings outgrow what
+// the boxes and the certificate allow for; directions of a length, and scenes
+// of a size, at which products of the test overflow or underflow).
 HPT_HD bool bvh_init(const Ray& r, float scene_eps, BvhRay& b) {
   b.ray = r;
   b.best = kBvhNone;
@@ -211,7 +212,7 @@ HPT_HD bool bvh_init(const Ray& r, float scene_eps, BvhRay& b) {
   b.node_base = 0;
   b.node_bits = (oct << 16) | (1u << 8) | (1u << oct);
   const float omax = fmaxf(fabsf(r.o.x), fmaxf(fabsf(r.o.y), fabsf(r.o.z)));
-  if (!(finite3(r.o) && finite3(r.d) && dmax > 1e-15f && dmax < 1e15f &&
+  if (!(finite3(r.o) && finite3(r.d) && dmax > 1e-9f && dmax < 1e9f && scene_eps < 2e4f &&
         omax <= rn_mul(kMaxOrigin, scene_eps)))
     return false;
   const float len127 = rn_div(127.f, length(r.d));

@@ -723,7 +723,9 @@ Plane plane_of(const DevTri& t, double scene_size) {
     flat = flat || (t.e1[a] == 0.f && t.e2[a] == 0.f);
   }
   l = std::sqrt(l);
-  const double s = l1 > 0 && l2 > 0 ? l / std::sqrt(l1 * l2) : 0;
+  // (Of so small a triangle the test's products underflow: its error is not
+  // relative any more. As one without area.)
+  const double s = l1 * l2 > 1e-52 ? l / std::sqrt(l1 * l2) : 0;
   for (int a = 0; a < 3; ++a) p.n[a] = l > 0 ? p.n[a] / l : 0;
   p.graze = s > kGrazing ? kGrazing / s : 1;
   p.thickness = s > kGrazing ? 14 * kUlp * kMaxDistance * scene_size / s : 0;

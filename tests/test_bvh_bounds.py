@@ -189,3 +189,15 @@ def test_rays_almost_along_a_split_plane(name):
     d = rng.normal(size=(n, 3))
     d[np.arange(n), axis] *= 10.0 ** rng.uniform(-8, -1, n)
     _check(emu.BvhEmu(mesh, nodes, leaf).query(o, _unit(d)))
+
+
+@pytest.mark.parametrize("scale", [1e-14, 1e-12, 1e-8, 1e8, 1e12])
+@pytest.mark.parametrize("length", [1e-14, 1e-8, 1e8, 1e14])
+def test_scenes_and_directions_of_extreme_size(scale, length):
+    """Where products of the test leave the normal numbers, its error is not
+    relative any more."""
+    g = _scene("nine")[0] if scale * length > 1e24 else S.make_scene(3, seed=2, family=2, target_triangles=2000)[0]
+    m = _mesh(g.points[:, :3].astype(np.float64) * scale, g.triangles[:, :3])
+    e = emu.BvhEmu(m, *H.build_kdtree(m.points, m.triangles))
+    for o, d in (_in_plane(m, 20000, 5), S.aabb_random_rays(m, 10000, 3)):
+        _check(e.query(o, d * np.float32(length)))
