@@ -1602,7 +1602,7 @@ hpt_status Engine::ensure_graph(const DevScene* shared_scene, int iterations) {
       (!shared || memcmp(&graph_scene_, shared_scene, sizeof(DevScene)) == 0);
   if (graph_exec_ && same_scene && graph_capacity_ == capacity_ &&
       graph_slots_ == slots_ && graph_iters_ == iterations && graph_tuning_ == isect_variant() &&
-      graph_smem_ == tuning.smem_nodes && graph_refill_ == tuning.refill_chunk &&
+      graph_refill_ == tuning.refill_chunk &&
       graph_steps_ == tuning.trav_steps && graph_max_steps_ == tuning.max_steps &&
       graph_shade_ == tuning.shade_min_blocks)
     return HPT_OK;
@@ -1630,7 +1630,6 @@ hpt_status Engine::ensure_graph(const DevScene* shared_scene, int iterations) {
   graph_slots_ = slots_;
   graph_iters_ = iterations;
   graph_tuning_ = isect_variant();
-  graph_smem_ = tuning.smem_nodes;
   graph_refill_ = tuning.refill_chunk;
   graph_steps_ = tuning.trav_steps;
   graph_max_steps_ = tuning.max_steps;

@@ -13,7 +13,7 @@
 
 namespace hpt {
 
-// Largest shared-memory node prefix a tuning may ask for (64 KB).
+// Largest smem_nodes a tuning may hold (a field without effect).
 constexpr int kMaxSmemNodes = 8192;
 
 struct SceneDev {
@@ -169,7 +169,7 @@ class Engine {
   bool graph_shared_ = false;
   DevScene graph_scene_{};
   int graph_capacity_ = 0, graph_slots_ = 0, graph_iters_ = 0, graph_tuning_ = -1;
-  int graph_smem_ = -1, graph_refill_ = -1, graph_steps_ = -1, graph_max_steps_ = -1;
+  int graph_refill_ = -1, graph_steps_ = -1, graph_max_steps_ = -1;
   int graph_shade_ = -1;
   hpt_status init_status_ = HPT_OK;
   hpt_status init();

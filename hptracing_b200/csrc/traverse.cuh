@@ -173,27 +173,10 @@ struct TravCount {
   uint32_t nodes, leaves, tris, repeats;
 };
 
-// The work counters of a run of traversal units in one register: four
-// 8-bit fields (nodes, leaves, triangle tests, mailbox repeats), added into
-// a TravCount by count_flush before any field can pass 255.
-struct PackedCount {
-  uint32_t v;
-};
 HPT_HD void count_node(TravCount& c) { ++c.nodes; }
 HPT_HD void count_leaf(TravCount& c) { ++c.leaves; }
 HPT_HD void count_test(TravCount& c) { ++c.tris; }
 HPT_HD void count_repeat(TravCount& c) { ++c.repeats; }
-HPT_HD void count_node(PackedCount& c) { c.v += 1u; }
-HPT_HD void count_leaf(PackedCount& c) { c.v += 1u << 8; }
-HPT_HD void count_test(PackedCount& c) { c.v += 1u << 16; }
-HPT_HD void count_repeat(PackedCount& c) { c.v += 1u << 24; }
-HPT_HD void count_flush(PackedCount& p, TravCount& c) {
-  c.nodes += p.v & 255u;
-  c.leaves += (p.v >> 8) & 255u;
-  c.tris += (p.v >> 16) & 255u;
-  c.repeats += p.v >> 24;
-  p.v = 0;
-}
 
 // Starts a query. start_node (>= 0) names a leaf node the origin is
 // expected to lie in (the leaf of the previous hit): if its box contains the
