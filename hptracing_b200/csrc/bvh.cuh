@@ -26,7 +26,7 @@
 // on the split's near side that holds m lists the triangle and ends in (m, X].]
 // The tree walk has to be in one of these leaves that the ray truly crosses
 // (the filter rejects others). It finds its leaf by the rounded point o + t d,
-// so within e = u (4 t |d| + |o + t d|) of a split, on that axis, it may be on
+// so within e = r (4 t |d| + |o + t d|) of a split, r = 2^-24, per axis, it may be on
 // the wrong side, for as long as the ray takes to move away: a ray almost along
 // the split stays there. Of the stretch within `round` of the hit, that is at
 // most 2 e / |d| in t per axis; round is twice what the three need together.

@@ -2,18 +2,18 @@
 //
 // Boxes. A ray has to visit every triangle that the tree walk (traverse.cuh)
 // would accept, and the FP32 Moller-Trumbore test accepts rays that pass
-// beside the triangle. How far beside? With u = 2^-24, T = o - a, n = e1 x e2,
+// beside the triangle. How far beside? With r = 2^-24, T = o - a, n = e1 x e2,
 // S = |e1||e2|, det = -n.d = -c |n||d| (c: sine of the angle between ray and
-// plane), the computed T.(d x e2) and d.(T x e1) are off by at most 7u
-// |T||d||e|, the computed det by 6u |d| S, the reciprocal and the products by
-// 2u more. Let X = a + u e1 + v e2 for the computed u, v: an accepted X is a
+// plane), the computed T.(d x e2) and d.(T x e1) are off by at most 7 r
+// |T||d||e|, the computed det by 6 r |d| S, the reciprocal and the products by
+// 2 r more. Let X = a + u e1 + v e2 for the computed u, v: an accepted X is a
 // point of the triangle, and
-//     (o - X) det = -d (n.T) + E,   |E| <= u |d| S (14 |T| + 8 max|e|).
-// (1) So X is within W = u (14 |T| + 8 max|e|) / (c s) of the ray's line, s =
+//     (o - X) det = -d (n.T) + E,   |E| <= r |d| S (14 |T| + 8 max|e|).
+// (1) So X is within W = r (14 |T| + 8 max|e|) / (c s) of the ray's line, s =
 //     |n| / S, the sine of the angle at vertex a, and by the same steps the
-//     computed t is off by no more than u (15 |T| + 8 max|e|) / (c s |d|). If c
+//     computed t is off by no more than r (15 |T| + 8 max|e|) / (c s |d|). If c
 //     s >= kGrazing, the ray meets a box around the triangle that is grown by
-//     u (36 max-norm |T| + 40 max|e|) / kGrazing (the rest beyond W: where the
+//     r (36 max-norm |T| + 40 max|e|) / kGrazing (the rest beyond W: where the
 //     line's nearest point lies behind the origin). The walk grows boxes by the
 //     first term (kBoxGrowth), the second is part of the box; kCullFactor
 //     covers the error of t. [The first term is what makes origins far away
@@ -21,7 +21,7 @@
 // (2) If c s < kGrazing, the ray runs almost in the plane, and W is no bound.
 //     But |n.(x - X)| <= |n| c |x - X| + |E| / |d| for every point x of the
 //     ray: it stays within a thin slab around the plane, of height h = c |x -
-//     X| + u (14 |T| + 8 max|e|) / s, and the tree walk only tests the triangle
+//     X| + r (14 |T| + 8 max|e|) / s, and the tree walk only tests the triangle
 //     in a leaf that lists it. So the ray meets the part of such a leaf that
 //     lies in the slab. The wide box of a triangle holds these parts; it is
 //     used for rays that are within kGrazing of the plane (a cone per child,
@@ -30,7 +30,7 @@
 //     A triangle with e1 and e2 exactly zero on one axis needs no wide box:
 //     every rounded term of the test then carries d's component on that axis
 //     or the distance along it, and (1) holds without c.
-// A box kept in a node also covers the walk's own rounding (8 u of its largest
+// A box kept in a node also covers the walk's own rounding (8 r of its largest
 // coordinate; the leaf it is in is found by the rounded o + t d).
 // What it costs: 14.6 node visits and 6.6 tests a ray on the 61k-triangle
 // spheres and 19 and 7 on an 842k-triangle terrain, against 11.7 and 6.4, and
@@ -728,7 +728,8 @@ Plane plane_of(const DevTri& t, double scene_size) {
   const double s = l1 * l2 > 1e-52 ? l / std::sqrt(l1 * l2) : 0;
   for (int a = 0; a < 3; ++a) p.n[a] = l > 0 ? p.n[a] / l : 0;
   p.graze = s > kGrazing ? kGrazing / s : 1;
-  p.thickness = s > kGrazing ? 14 * kUlp * kMaxDistance * scene_size / s : 0;
+  // (|T| is at most kMaxDistance sizes, an edge sqrt 3.)
+  p.thickness = s > kGrazing ? 14 * kUlp * (kMaxDistance + 1) * scene_size / s : 0;
   p.wide = p.graze >= 1 || !flat;
   return p;
 }

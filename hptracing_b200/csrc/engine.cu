@@ -766,8 +766,9 @@ __device__ __noinline__ void settle_queued(const EngineParams& P, int i, int par
 // ray; DRAM at 18 % of its rate): hence the one copy of the random direction
 // for two of them (shading.cuh), no atomic that all warps queue for (count_paths,
 // the block's one cursor step and one queue step for BS items - one of each per
-// warp costs 5 % more), and 32 warps per SM against a few spills. Over the 58 M
-// paths of 512x512x64 on 61,476 triangles: 6.94 ms before these three, 6.26 now.
+// warp costs 5 % more), and 32 warps per SM against spills (400 bytes, around the
+// call that settles open hits). Over the 58 M paths of 512x512x64 on 61,476
+// triangles: 6.94 ms before these three, 6.26 with them.
 // MINB: blocks of BS threads per SM the register budget must fit (1 leaves the
 // compiler's natural allocation of ~150); the tuning chooses.
 // kUniform: every job renders P.uscene, whose pointers are constant operands.
@@ -1048,13 +1049,13 @@ void cuda_soft_fail(cudaError_t e, const char* what) {
 hpt_tuning default_tuning() {
   hpt_tuning t;
   memset(&t, 0, sizeof t);
-  // From sweeps on the 512x512, 64 spp spheres frame, the 1920x1080, 4 spp
-  // terrain frame and the 256x256, 16 spp box room: 8 blocks of 128 per SM
-  // (64 registers; 6 / 7 / 8 / 9 blocks: spheres 33.8 / 31.7 / 30.7 / 30.1
-  // ms, terrain 10.0 / 9.6 / 9.5 / 9.6 ms, room 1.17 / 1.15 / 1.17 / 1.20
-  // ms), 16 rounds between refills (8 / 16 / 24: spheres 37.6 / 37.2 / 38.1
-  // ms), a wavefront of 2^24 paths (3.8 GB of queues, allocated only up to
-  // the paths a run has).
+  // From one sweep on the 512x512, 64 spp spheres frame, the 1920x1080, 4 spp
+  // terrain frame and the 256x256, 16 spp box room (device time): 8 blocks of
+  // 128 per SM (64 registers; 6 / 7 / 8 / 9 blocks: spheres 40.1 / 37.8 / 36.8 /
+  // 40.2 ms, terrain 14.3 / 13.7 / 13.9 / 14.7 ms, room 0.88 / 0.86 / 0.87 /
+  // 0.90 ms), 16 rounds between refills (8 / 16 / 24 / 32: spheres 36.9 / 36.8 /
+  // 37.8 / 39.5 ms, terrain 14.0 / 13.9 / 13.7 / 13.9 ms), a wavefront of 2^24
+  // paths (2.7 GB of queues, allocated only up to the paths a run has).
   t.capacity = 1 << 24;
   t.isect_block = 128;
   t.isect_min_blocks = 8;
@@ -1063,8 +1064,9 @@ hpt_tuning default_tuning() {
   t.smem_nodes = 0;
   t.use_graph = 0;
   t.trav_steps = 16;
-  // Shading at 4 blocks of 256 per SM (64 registers): 7.0 instead of 8.4 ms
-  // per spheres frame at the natural 106-register allocation (2 blocks).
+  // Shading at 4 blocks of 256 per SM (64 registers, the settling calls' spills
+  // included): 6.4 ms of a spheres frame, 7.2 at 3 blocks, 14.2 at the natural
+  // allocation.
   t.shade_min_blocks = 4;
   return t;
 }
@@ -1821,7 +1823,12 @@ hpt_status Engine::run(const std::vector<JobSpec>& jobs, hpt_render_stats* stats
   }
   while (!at_once) {
     if (use_graph) {
-      HPT_CUDA(cudaGraphLaunch(graph_exec_, stream));
+      const cudaError_t launch = cudaGraphLaunch(graph_exec_, stream);
+      if (launch != cudaSuccess) {
+        for (auto& b : bufs) free_job(b);
+        HPT_SOFT(cudaStreamSynchronize(stream));
+        return cuda_fail(launch, "graph launch");
+      }
     } else {
       for (int k = 0; k < kBatch; ++k)
         launch_iteration(shared_dev, prof ? &pev[(slot * kBatch + k) * 3] : nullptr, capacity_,
