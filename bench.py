@@ -275,11 +275,11 @@ def reference_scene():
 
 def isect_bytes(stats):
     """Algorithmic bytes of all closest-hit work in one frame: per query 32 B
-    (origin, direction), per hit 16 B written, per hierarchy node visited 80 B,
+    (origin, direction), per hit 16 B written, per hierarchy node visited 160 B,
     per triangle test 48 B."""
     q = stats["intersect_queries"] - stats["primary_rays"]
     hits = max(0, stats["shade_calls"] - stats["paths"])  # hits found by k_trace
-    return 32 * q + 16 * hits + 80 * stats["nodes_visited"] + 48 * stats["triangle_tests"]
+    return 32 * q + 16 * hits + 160 * stats["nodes_visited"] + 48 * stats["triangle_tests"]
 
 
 def cpu_baseline(mesh, nodes, leaf, cam, kind, samples=1):
