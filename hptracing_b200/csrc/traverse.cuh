@@ -478,6 +478,8 @@ HPT_HD bool trav_setup(const Sc& s, TravState& st, TravCold& tc, DevErr* err, Cn
 }
 
 // --- Step-at-a-time traversal ----------------------------------------------
+// No kernel calls it: the host build of the tests compares it, with start hints
+// and the shared node prefix, with trav_leaf, which the kernels' walk_for runs.
 // The same walk as trav_leaf, cut into units of similar cost: one descent
 // step, the set-up of a newly reached leaf, one triangle test, or the exit
 // of a finished leaf through its rope. A warp that calls trav_step in a loop
